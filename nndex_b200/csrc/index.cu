@@ -556,6 +556,12 @@ CudaIndex::TcPlan CudaIndex::plan_tc(uint64_t kcap, bool fp8) const {
     return out;
 }
 
+uint32_t CudaIndex::group_candidates(uint64_t kcap) const {
+    uint64_t want = rerank_width ? std::max<uint64_t>(rerank_width, kcap) : std::max<uint64_t>(32, 2 * kcap);
+    want = std::min<uint64_t>(want, rows);
+    return want <= kMaxGroupCandidates && want >= kcap ? static_cast<uint32_t>(want) : 0u;
+}
+
 int CudaIndex::enqueue_prep_queries(const float* d_raw, uint64_t n, int mode, int path, cudaStream_t s) {
     int st;
     PrepArgs p;
@@ -597,12 +603,9 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
                           cudaStream_t s) {
     int st;
     const TcPlan plan = plan_tc(kcap, fp8);
-    const uint32_t kp = plan.kp, stages = plan.stages;
-    if (!stages || kp < kcap) return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: k'=%u does not fit", kp);
+    if (!plan.stages || plan.kp < kcap)
+        return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: k'=%u does not fit", plan.kp);
     const uint32_t nqb = (n + 127) / 128;
-    uint64_t nranges = 0, range_rows = 0;
-    tc_ranges(nqb, nranges, range_rows);
-    const uint64_t per_query = nranges * kp;
     // Autotuned: when the last batch rarely certified in pass 1, pass 1 only has to produce each
     // query's threshold T, and a sample of the rows (every 8th tile) gives a valid one.
     // The tuner's plan may fix it instead (only bases of ≥ 64 tiles are sampled).
@@ -611,8 +614,38 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     // shared with the index's small-k batches, which may keep it at 1.
     const uint32_t want = forced_stride ? forced_stride : (kcap >= 64 ? 8u : tc_sample_stride);
     const uint32_t stride = (want > 1 && rows >= 256ull * 64) ? want : 1;
+    uint64_t nranges = 0, range_rows = 0;
+    tc_ranges(rows, nqb, nranges, range_rows);
+    // A sampled pass 1 writes group maxima instead of keeping heaps, its ranges split over the sampled
+    // tiles. Groups of 32 columns where a query has at least 64 of them per candidate (two of its best
+    // rows then rarely share one, which would lower T), of as many tiles as still leave 64 (fewer words
+    // to write, read and hold: 512 bytes per candidate at most, what the heaps' slots are admitted
+    // at); groups of 8 columns on smaller samples, and heaps where even those are fewer than four per
+    // candidate.
+    uint32_t gkp = stride > 1 ? group_candidates(kcap) : 0u, group = 0, gm_tiles = 0, span = 1;
+    if (gkp) {
+        const uint64_t sampled = ((rows + 255) / 256 + stride - 1) / stride;
+        uint64_t nr = 0, rr = 0;
+        tc_ranges(sampled * 256, nqb, nr, rr);
+        group = sampled * 8 >= 64ull * gkp ? 32u : (sampled * 32 >= 4ull * gkp ? 8u : 0u);
+        if (group) {
+            nranges = nr;
+            range_rows = rr * stride;
+            const uint64_t per_range = rr / 256;
+            while (group == 32 && span < kMaxGroupSpan && span * 2 <= per_range &&
+                   sampled * 8 >= 64ull * gkp * span * 2)
+                span *= 2;
+            gm_tiles = static_cast<uint32_t>((per_range + span - 1) / span);
+        }
+    }
+    tc_groups = group != 0;
+    const uint32_t kp = tc_groups ? gkp : plan.kp;
+    const uint64_t gm_words = nranges * gm_tiles * (tc_groups ? 256 / group : 0);  // per query, 4 bytes each
+    const uint64_t per_query = tc_groups ? (gm_words + 1) / 2 : nranges * kp;
     if ((st = grow_device(d_thr, cap_thr, n, "tc workspace"))) return st;
     if ((st = grow_device(d_ws, cap_ws, per_query * n, "tc workspace"))) return st;
+    if ((st = grow_device(d_ids, cap_ids, n, "pass-2 buffer"))) return st;
+    if ((st = ensure_fbn())) return st;
     if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_sim, cap_cand_sim, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_cnt, cap_cand_cnt, n, "tc workspace"))) return st;
@@ -621,14 +654,65 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     CUtensorMap tmap_q;
     if ((st = encode_query_tmap(fp8, fp8 ? static_cast<void*>(d_q_fp8) : static_cast<void*>(d_q_bf16), n, &tmap_q)))
         return st;
-    cudaMemsetAsync(d_thr, 0, n * sizeof(unsigned long long), s);
     TcArgs a;
     a.tmap_q = &tmap_q;
     a.tmap_b = fp8 ? &tmap_fp8 : &tmap_bf16;
     a.nranges = static_cast<uint32_t>(nranges);
-    a.stages = stages;
-    a.stream_a = plan.stream_a;
     fill_tc_params(fp8, n, range_rows, a.p);
+    last_tc_stride = stride;
+    stats.pass1_tile_stride = stride;
+    stats.path = fp8 ? 3 : 2;
+    stats.rerank_width = kp;
+    stats.rows_scanned += rows * n;
+    cudaEvent_t ev_a = nullptr;
+    cudaError_t e;
+    if (tc_groups) {
+        const TcPlan plan2 = plan_tc(0, fp8);  // no heaps: pass 2's shared-memory plan
+        a.stages = plan2.stages;
+        a.stream_a = plan2.stream_a;
+        a.p.tile_stride = stride;
+        a.p.gm = reinterpret_cast<uint32_t*>(d_ws);
+        a.p.gm_tiles = gm_tiles;
+        a.p.gm_group = group;
+        a.p.gm_span = span;
+        scan_event_begin(s, ev_a);
+        e = launch_scan_tc(a, fp8, 2, s);
+        scan_event_end(s, ev_a);
+        if (e != cudaSuccess) return cuda_error(e, "tensor-core scan launch");
+        TcThresholdArgs t;
+        t.gm = a.p.gm;
+        t.words = gm_words;
+        t.group = group;
+        t.tiles = gm_tiles;
+        t.span = span;
+        t.stride = stride;
+        t.parts = nranges;
+        t.range_rows = range_rows;
+        t.rows = rows;
+        t.base = d_base;
+        t.ds = static_cast<uint32_t>(ds);
+        t.queries = d_qn;
+        t.nq = n;
+        t.kp = kp;
+        t.k = kcap;
+        t.q_resid = d_q_resid;
+        t.q_scale = fp8 ? d_q_scale : nullptr;
+        t.eps_rows = a.p.eps_rows;
+        t.eps_acc = a.p.eps_acc;
+        t.cand_idx = d_cand_idx;
+        t.cand_sim = d_cand_sim;
+        t.cand_cnt = d_cand_cnt;
+        t.cert = d_cert;
+        t.kth = d_kth;
+        t.ids = d_ids;
+        t.live = d_fbn + 1;
+        if ((e = launch_threshold(t, s)) != cudaSuccess) return cuda_error(e, "threshold launch");
+        stats.kernel_launches += 2;
+        return NNDEX_OK;
+    }
+    cudaMemsetAsync(d_thr, 0, n * sizeof(unsigned long long), s);
+    a.stages = plan.stages;
+    a.stream_a = plan.stream_a;
     a.p.q_resid = d_q_resid;
     a.p.q_scale = fp8 ? d_q_scale : nullptr;
     a.p.kprime = kp;
@@ -636,11 +720,8 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     a.p.thr_global = d_thr;
     a.p.ws_keys = d_ws;
     a.p.tile_stride = stride;
-    last_tc_stride = stride;
-    stats.pass1_tile_stride = stride;
-    cudaEvent_t ev_a = nullptr;
     scan_event_begin(s, ev_a);
-    cudaError_t e = launch_scan_tc(a, fp8, 0, s);
+    e = launch_scan_tc(a, fp8, 0, s);
     scan_event_end(s, ev_a);
     if (e != cudaSuccess) return cuda_error(e, "tensor-core scan launch");
     MergeArgs m;
@@ -672,16 +753,14 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     r.certify = stride == 1;
     if ((e = launch_rerank(r, s)) != cudaSuccess) return cuda_error(e, "rerank launch");
     stats.kernel_launches += 3;
-    stats.path = fp8 ? 3 : 2;
-    stats.rerank_width = kp;
-    stats.rows_scanned += rows * n;
     return NNDEX_OK;
 }
 
-// Row ranges of the tensor-core grid: about four waves of CTAs, each range a multiple of the
-// 256-row tile. Concurrent CTAs share ranges, so a base tile is read from HBM about once.
-void CudaIndex::tc_ranges(uint32_t nqb, uint64_t& nranges, uint64_t& range_rows) const {
-    tc_range_split(rows, nqb, static_cast<uint64_t>(sm_count), nranges, range_rows);
+// Row ranges of the tensor-core grid over `scan_rows` rows: about four waves of CTAs, each range a
+// multiple of the 256-row tile. Concurrent CTAs share ranges, so a base tile is read from HBM about
+// once.
+void CudaIndex::tc_ranges(uint64_t scan_rows, uint32_t nqb, uint64_t& nranges, uint64_t& range_rows) const {
+    tc_range_split(scan_rows, nqb, static_cast<uint64_t>(sm_count), nranges, range_rows);
 }
 
 void CudaIndex::fill_tc_params(bool fp8, uint32_t n, uint64_t range_rows, TcParams& p) const {
@@ -746,15 +825,22 @@ int CudaIndex::enqueue_tc_pass2(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o
         return st;
     uint32_t* d_m = d_fbn + 1;      // uncertified queries
     uint32_t* d_fail = d_fbn + 2;   // of them, collections that overflowed
-    launch_compact_zero_flags(d_cert, n, d_ids, d_m, s);
-    cudaError_t e = launch_gather_queries(d_ids, n, fp8 ? static_cast<const void*>(d_q_fp8)
-                                                         : static_cast<const void*>(d_q_bf16),
-                                          static_cast<uint32_t>(row_bytes), d_q2_lp, d_q_resid, d_q2_resid,
-                                          fp8 ? d_q_scale : nullptr, d_q2_scale, d_kth, d_q2_thr, s, d_m);
-    if (e != cudaSuccess) return cuda_error(e, "gather launch");
+    cudaError_t e = cudaSuccess;
+    if (!tc_groups) {
+        launch_compact_zero_flags(d_cert, n, d_ids, d_m, s);
+        e = launch_gather_queries(d_ids, n, fp8 ? static_cast<const void*>(d_q_fp8)
+                                                : static_cast<const void*>(d_q_bf16),
+                                  static_cast<uint32_t>(row_bytes), d_q2_lp, d_q_resid, d_q2_resid,
+                                  fp8 ? d_q_scale : nullptr, d_q2_scale, d_kth, d_q2_thr, s, d_m);
+        if (e != cudaSuccess) return cuda_error(e, "gather launch");
+        stats.kernel_launches += 2;
+    }
     cudaMemsetAsync(d_cnt2, 0, n * sizeof(uint32_t), s);
+    // after group maxima every query is in pass 2, in the batch's order: its own buffers serve
+    void* q_lp = !tc_groups ? static_cast<void*>(d_q2_lp) : fp8 ? static_cast<void*>(d_q_fp8) : static_cast<void*>(d_q_bf16);
+    const float* q_thr = tc_groups ? d_kth : d_q2_thr;
     CUtensorMap tmap_q2;
-    if ((st = encode_query_tmap(fp8, d_q2_lp, n, &tmap_q2))) return st;
+    if ((st = encode_query_tmap(fp8, q_lp, n, &tmap_q2))) return st;
     TcArgs a;
     a.tmap_q = &tmap_q2;
     a.tmap_b = fp8 ? &tmap_fp8 : &tmap_bf16;
@@ -780,9 +866,9 @@ int CudaIndex::enqueue_tc_pass2(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o
     }
     stats.pass2_query_blocks = a.qb;
     fill_tc_params(fp8, n, 0, a.p);
-    a.p.q_resid = d_q2_resid;
-    a.p.q_scale = fp8 ? d_q2_scale : nullptr;
-    a.p.q_thr = d_q2_thr;
+    a.p.q_resid = tc_groups ? d_q_resid : d_q2_resid;
+    a.p.q_scale = !fp8 ? nullptr : tc_groups ? d_q_scale : d_q2_scale;
+    a.p.q_thr = q_thr;
     a.p.cand_rows = d_rows2;
     a.p.cand_cnt = d_cnt2;
     a.p.cap2 = cap2;
@@ -797,10 +883,10 @@ int CudaIndex::enqueue_tc_pass2(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o
     scan_event_end(s, ev_a);
     if (e != cudaSuccess) return cuda_error(e, "tensor-core scan launch (pass 2)");
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, cap2, kcap,
-                                d_q2_thr, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, d_m);
+                                q_thr, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, d_m);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
     launch_compact_zero_flags(d_ok2, n, d_tcfail, d_fail, s, d_m);
-    stats.kernel_launches += 6;
+    stats.kernel_launches += 4;
     last_tc_n = n;
     return NNDEX_OK;
 }

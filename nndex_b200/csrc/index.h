@@ -117,6 +117,7 @@ struct CudaIndex {
     uint32_t forced_stride = 0;     // the tuned plan's pass-1 tile stride for the current batch (0 = rule)
     uint32_t forced_qb = 0;         // the tuned plan's pass-2 query blocks per CTA (0 = rule)
     uint32_t last_tc_stride = 1;
+    bool tc_groups = false;  // the batch's pass 1 wrote group maxima (every query goes to pass 2)
     float* d_kth = nullptr;  // pass 1: exact k-th score per query
     unsigned long long* d_floor = nullptr;  // TF32 scan: per query, a key its k'-th candidate reaches
     size_t cap_floor = 0;
@@ -298,8 +299,11 @@ struct CudaIndex {
         bool stream_a = false;  // query slabs staged per ring stage instead of resident
     };
     TcPlan plan_tc(uint64_t kcap, bool fp8) const;
+    // k′ of a sampled pass 1 with group maxima: 2k (at least 32) unless set, 0 where the threshold
+    // kernel's lists do not hold it.
+    uint32_t group_candidates(uint64_t kcap) const;
     uint32_t tc_chunks(bool fp8) const;
-    void tc_ranges(uint32_t nqb, uint64_t& nranges, uint64_t& range_rows) const;
+    void tc_ranges(uint64_t scan_rows, uint32_t nqb, uint64_t& nranges, uint64_t& range_rows) const;
     void fill_tc_params(bool fp8, uint32_t n, uint64_t range_rows, TcParams& p) const;
     int encode_query_tmap(bool fp8, void* buf, uint32_t n, CUtensorMap* map) const;
     int enqueue_prep_queries(const float* d_raw, uint64_t n, int mode, int path, cudaStream_t s);

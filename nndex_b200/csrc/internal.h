@@ -147,6 +147,12 @@ struct TcParams {
     const float* q_resid = nullptr;       // ‖q − q̂‖ per query
     float eps_acc = 0.0f;                 // FP32 accumulation error bound
     float eps_rows = 0.0f;                // max ‖x − x̂‖ over the rows
+    // group-maxima pass (mode 2): per query and row range (item mode: per output slot) gm_tiles × 256 /
+    // gm_group words, one per group: the same gm_group (8 or 32) columns of gm_span scanned tiles
+    uint32_t* gm = nullptr;
+    uint32_t gm_tiles = 0;                // spans of tiles per range (item mode: per slot), the most
+    uint32_t gm_group = 0;
+    uint32_t gm_span = 1;                 // a power of two, at most kMaxGroupSpan
     unsigned long long* thr_global = nullptr;  // pass 1: per query, zeroed before the launch
     uint64_t* ws_keys = nullptr;          // pass 1: nq × nranges × kprime
     const float* q_thr = nullptr;         // pass 2: per query T (exact k-th score of pass 1)
@@ -193,7 +199,37 @@ uint32_t tc_stages_for(uint32_t nchunks, uint32_t kprime, bool fp8, bool stream_
 uint32_t tc_pair_stages_for(uint32_t nchunks, bool fp8, size_t smem_limit);
 // Ring stages of a CTA-pair pass 2 (TcArgs::qb = 3) that fit, 0 when none does.
 uint32_t tc_cta_pair_stages_for(uint32_t nchunks, bool fp8, size_t smem_limit);
+// mode 0: pass 1 with heaps; 1: pass 2; 2: a sampled pass 1 that writes group maxima.
 cudaError_t launch_scan_tc(const TcArgs& a, bool fp8, int mode, cudaStream_t stream);
+
+// T (and the candidates it came from) of a group-maxima pass; lists every query for pass 2.
+constexpr uint32_t kMaxGroupSpan = 64;          // 11 low bits of a score name its row
+constexpr uint32_t kMaxGroupCandidates = 512;  // k′ of the threshold kernel's shared-memory lists
+struct TcThresholdArgs {
+    const uint32_t* gm = nullptr;
+    uint64_t words = 0;                   // per query (parts × tiles × 256 / group), without slots
+    uint32_t group = 0, tiles = 0, span = 1, stride = 1;
+    uint64_t parts = 0;                   // row ranges per query
+    uint64_t range_rows = 0;
+    uint64_t rows = 0;
+    const uint32_t* slot_off = nullptr;   // IVF: nq + 1, each query's slots; null: row ranges
+    const uint32_t* slot_row0 = nullptr;  // IVF: first list position of each slot's chunk
+    const float* base = nullptr;          // the rows by candidate (IVF: by list position), stride ds
+    uint32_t ds = 0;
+    const float* queries = nullptr;
+    uint32_t nq = 0, kp = 0, k = 0;
+    const float* q_resid = nullptr;
+    const float* q_scale = nullptr;       // FP8 only
+    float eps_rows = 0.0f, eps_acc = 0.0f;
+    uint64_t* cand_idx = nullptr;         // nq × kp, by approximate score
+    float* cand_sim = nullptr;            // upper bounds of their exact scores
+    uint32_t* cand_cnt = nullptr;
+    uint32_t* cert = nullptr;             // nq: 0
+    float* kth = nullptr;                 // nq: T
+    uint32_t* ids = nullptr;              // nq: 0, 1, 2, …
+    uint32_t* live = nullptr;             // nq
+};
+cudaError_t launch_threshold(const TcThresholdArgs& a, cudaStream_t stream);
 
 // K12: FP32-accurate candidate scan on the tensor cores (three TF32 products per K step), 16
 // queries per CTA; per query and CTA the kp best keys of (s̃ + eps, row) go to ws_keys.

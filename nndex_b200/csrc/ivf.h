@@ -62,6 +62,7 @@ struct IvfScratch {
     uint32_t* d_q_slot_off = nullptr;   size_t cap_q_slot_off = 0; // B + 1
     unsigned long long* d_counters = nullptr; size_t cap_counters = 0;  // work counter, totals, rows probed
     uint64_t* d_ws = nullptr;           size_t cap_ws = 0;         // slots × k keys
+    uint32_t* d_slot_row0 = nullptr;    size_t cap_slot_row0 = 0;  // group maxima: first list position of each slot's chunk
     uint32_t* d_qblock_off = nullptr;   size_t cap_qblock_off = 0; // nlist + 1 (tensor-core scan)
     __nv_bfloat16* d_g16 = nullptr;     size_t cap_g16 = 0;        // gathered query blocks × 128 × kb16
     uint32_t* d_lane_qid = nullptr;     size_t cap_lane_qid = 0;   // gathered blocks × 128

@@ -970,6 +970,7 @@ IvfIndex::~IvfIndex() {
 }
 
 IvfScratch::~IvfScratch() {
+    cudaFree(d_slot_row0);
     cudaFree(d_qblock_off);
     cudaFree(d_g16);
     cudaFree(d_lane_qid);

@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(256)
     ivf_plan_fill_kernel(const uint32_t* __restrict__ probes, uint32_t nq, uint32_t np,
                          const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ list_qoff,
                          uint32_t* __restrict__ list_fill, const uint32_t* __restrict__ q_slot_off,
-                         uint32_t* __restrict__ list_q, uint32_t* __restrict__ list_slot) {
+                         uint32_t* __restrict__ list_q, uint32_t* __restrict__ list_slot,
+                         uint32_t* __restrict__ slot_row0) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (q >= nq) return;
@@ -290,6 +291,9 @@ __global__ void __launch_bounds__(256)
             const uint32_t pos = list_qoff[l] + atomicAdd(&list_fill[l], 1u);
             list_q[pos] = q;
             list_slot[pos] = run + incl - c;
+            // group maxima: the first list position of each of the slots' chunks
+            if (slot_row0)
+                for (uint32_t i = 0; i < c; ++i) slot_row0[run + incl - c + i] = offsets[l] + i * kChunkRows;
         }
         run += __shfl_sync(0xFFFFFFFFu, incl, 31);
     }
@@ -671,7 +675,7 @@ cudaError_t launch_probe_qb(const ProbeLaunch& a, cudaStream_t s) {
 // Probe + plan of n queries: four launches (centroid scores, the selection with its counts, the
 // plan's scans, the pairs).
 cudaError_t launch_probe_plan(uint32_t pqb, const ProbeLaunch& a, uint32_t qb, IvfScratch& w, uint32_t* qblock_off,
-                              cudaStream_t s) {
+                              uint32_t* slot_row0, cudaStream_t s) {
     if ((a.nlist + kProbeCentroids - 1) / kProbeCentroids > 65535u) return cudaErrorInvalidValue;
     cudaError_t e;
     switch (pqb) {
@@ -687,7 +691,7 @@ cudaError_t launch_probe_plan(uint32_t pqb, const ProbeLaunch& a, uint32_t qb, I
     ivf_plan_scan_kernel<<<1, 1024, 0, s>>>(a.nq, a.nlist, a.offsets, qb, w.d_list_cnt, w.d_list_qoff, w.d_item_off,
                                             w.d_q_slot_off, w.d_counters, qblock_off);
     ivf_plan_fill_kernel<<<(a.nq + 7) / 8, 256, 0, s>>>(a.probes, a.nq, a.np, a.offsets, w.d_list_qoff, w.d_list_fill,
-                                                         w.d_q_slot_off, w.d_list_q, w.d_list_slot);
+                                                         w.d_q_slot_off, w.d_list_q, w.d_list_slot, slot_row0);
     count_launch(4);
     return cudaGetLastError();
 }
@@ -773,7 +777,7 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
         const ProbeLaunch pl{qn,          n,          dq,           static_cast<uint32_t>(ix.dp), nlist, np,
                              v.d_cent_t,  v.nlist_pad, v.d_offsets, w.d_pscore, w.d_probes, w.d_list_cnt,
                              w.d_q_slot_off, w.d_counters};
-        cudaError_t e = launch_probe_plan(pqb, pl, qb, w, nullptr, s);
+        cudaError_t e = launch_probe_plan(pqb, pl, qb, w, nullptr, nullptr, s);
         if (e != cudaSuccess) return cuda_error(e, "IVF probe launch");
         a.queries = qn;
         cudaEvent_t ev_a = nullptr;
@@ -823,10 +827,31 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     const uint32_t np = static_cast<uint32_t>(np64);
     const CudaIndex::TcPlan plan = ix.plan_tc(k, false), plan2 = ix.plan_tc(0, false);
     if (plan.kp < k || !plan.stages || !plan2.stages) return ivf_search(ix, ix.d_qn, nq, k, o_idx, o_sim, o_cnt, s);
-    const uint32_t kp = plan.kp;
     const uint32_t pqb = probe_qb(ix.dp, ix.smem_optin);
     if (!pqb) return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: IVF probe shared memory above the limit");
     const uint64_t max_chunks = (v.max_list + kChunkRows - 1) / kChunkRows;
+    // Like the exact path's pass 1: when pass 1 rarely certifies, it only has to give each query its
+    // threshold T, and every 4th tile of its lists gives a valid one (the rule lives in
+    // ivf_finish_tc).
+    // a tuned plan may fix the stride; at k ≥ 64 the rules start sampled (a full pass 1 then carries
+    // the largest heaps and almost never certifies)
+    const uint32_t stride = ix.forced_stride ? ix.forced_stride : (k >= 64 ? ivf_sampled_stride() : w.tc_stride);
+    // A sampled pass 1 writes group maxima: groups of 8 columns (a query's best rows crowd into one or
+    // two lists, so groups of 32 would hold several of them), of as many tiles as keep a slot's words
+    // within its k′ keys; heaps where a query of average lists has fewer than 8 groups per candidate.
+    const uint32_t gkp = stride > 1 ? ix.group_candidates(k) : 0u;
+    uint32_t gm_tiles = 0, span = 1;
+    bool groups = false;
+    if (gkp) {
+        const uint64_t slot_rows = std::min<uint64_t>(v.max_list, kChunkRows);
+        const uint64_t slot_tiles = (slot_rows + 256ull * stride - 1) / (256ull * stride);
+        const uint64_t avg_tiles = (ix.rows / nlist + 256ull * stride - 1) / (256ull * stride);
+        while (span < slot_tiles && slot_tiles * 32 > 2ull * gkp * span) span *= 2;
+        gm_tiles = static_cast<uint32_t>((slot_tiles + span - 1) / span);
+        groups = static_cast<uint64_t>(np) * ((avg_tiles + span - 1) / span) * 32 >= 8ull * gkp;
+    }
+    const uint32_t kp = groups ? gkp : plan.kp;
+    const uint64_t slot_keys = groups ? gm_tiles * 16ull : kp;  // 8-byte words of a slot
     const uint64_t pairs = static_cast<uint64_t>(nq) * np;
     const uint64_t max_blocks = nlist + (pairs + 127) / 128;
     // Σ over lists of (query groups × chunks) ≤ (pairs / 128) · max_chunks + Σ chunks ≤ … + rows / chunk + nlist
@@ -846,7 +871,8 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     if ((st = grow(w.d_list_slot, w.cap_list_slot, pairs, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_q_slot_off, w.cap_q_slot_off, nq + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_counters, w.cap_counters, 10, "IVF plan buffer"))) return st;
-    if ((st = grow(w.d_ws, w.cap_ws, pairs * max_chunks * kp, "IVF slot workspace"))) return st;
+    if ((st = grow(w.d_ws, w.cap_ws, pairs * max_chunks * slot_keys, "IVF slot workspace"))) return st;
+    if (groups && (st = grow(w.d_slot_row0, w.cap_slot_row0, pairs * max_chunks, "IVF slot workspace"))) return st;
     if ((st = grow(w.d_g16, w.cap_g16, max_blocks * 128 * v.kb16, "IVF query blocks"))) return st;
     if ((st = grow(w.d_lane_qid, w.cap_lane_qid, max_blocks * 128, "IVF query blocks"))) return st;
     if ((st = grow(w.d_lane_slot, w.cap_lane_slot, max_blocks * 128, "IVF query blocks"))) return st;
@@ -878,7 +904,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     const ProbeLaunch pl{ix.d_qn,   nq,          static_cast<uint32_t>(ix.ds), static_cast<uint32_t>(ix.dp),
                          nlist,      np,          v.d_cent_t,  v.nlist_pad, v.d_offsets, w.d_pscore, w.d_probes,
                          w.d_list_cnt, w.d_q_slot_off, w.d_counters};
-    cudaError_t e = launch_probe_plan(pqb, pl, 128, w, w.d_qblock_off, s);
+    cudaError_t e = launch_probe_plan(pqb, pl, 128, w, w.d_qblock_off, groups ? w.d_slot_row0 : nullptr, s);
     if (e != cudaSuccess) return cuda_error(e, "IVF probe launch");
     ivf_gather_tc_kernel<<<nlist, 256, 0, s>>>(ix.d_q_bf16, static_cast<uint32_t>(v.kb16), w.d_list_cnt, w.d_list_qoff,
                                                w.d_list_q, w.d_list_slot, w.d_qblock_off, w.d_g16, w.d_lane_qid,
@@ -890,29 +916,18 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     // ---- pass 1 ----
     CUtensorMap tmap_q;
     if ((st = ix.encode_query_tmap(false, w.d_g16, static_cast<uint32_t>(max_blocks * 128), &tmap_q))) return st;
-    cudaMemsetAsync(ix.d_thr, 0, nq * sizeof(unsigned long long), s);
     TcArgs a;
     a.tmap_q = &tmap_q;
     a.tmap_b = &v.tmap_reordered16;
     a.nranges = 1;
-    a.stages = plan.stages;
-    a.stream_a = plan.stream_a;
+    a.stages = groups ? plan2.stages : plan.stages;
+    a.stream_a = groups ? plan2.stream_a : plan.stream_a;
     a.items = static_cast<uint32_t>(max_items);
     ix.fill_tc_params(false, nq, 0, a.p);
     a.p.row_resid = v.d_res16;
     a.p.eps_rows = v.eps16;
     a.p.q_resid = ix.d_q_resid;
-    a.p.kprime = kp;
-    a.p.thr_global = ix.d_thr;
-    a.p.ws_keys = w.d_ws;
-    // Like the exact path's pass 1: when pass 1 rarely certifies, it only has to give each query its
-    // threshold T, and every 4th tile of its lists gives a valid one (the rule lives in
-    // ivf_finish_tc).
-    // a tuned plan may fix the stride; at k ≥ 64 the rules start sampled (a full pass 1 then carries
-    // the largest heaps and almost never certifies)
-    const uint32_t stride = ix.forced_stride ? ix.forced_stride : (k >= 64 ? ivf_sampled_stride() : w.tc_stride);
     a.p.tile_stride = stride;
-    a.p.heap_k = stride > 1 ? std::max(1u, std::min(kp, k)) : kp;  // a sampled pass 1 only yields T
     a.p.it_item_off = w.d_item_off;
     a.p.it_item_list = w.d_item_list;
     a.p.it_list_cnt = w.d_list_cnt;
@@ -924,47 +939,91 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     a.p.it_nlist = nlist;
     a.p.it_chunk_rows = kChunkRows;
     a.p.it_next = w.d_counters + 8;  // the CTAs take items from this counter
-    cudaEvent_t ev_a = nullptr;
-    ix.scan_event_begin(s, ev_a);
-    e = launch_scan_tc(a, false, 0, s);
-    ix.scan_event_end(s, ev_a);
-    if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch");
-    uint32_t p2 = 1;
-    while (p2 < kp) p2 <<= 1;
-    ivf_merge_kernel<<<nq, 512, p2 * sizeof(uint64_t), s>>>(w.d_ws, w.d_q_slot_off, kp, ix.d_cand_idx, ix.d_cand_sim,
-                                                            ix.d_cand_cnt);
-    count_launch();
-    RerankArgs r;
-    r.base = v.d_reordered;  // the slot keys hold list positions
-    r.row_map = v.d_row_map;
-    r.ds = static_cast<uint32_t>(ix.ds);
-    r.queries = ix.d_qn;
-    r.cand_idx = ix.d_cand_idx;
-    r.cand_sim = ix.d_cand_sim;
-    r.cand_cnt = ix.d_cand_cnt;
-    r.nq = nq;
-    r.kp = kp;
-    r.k = k;
-    r.idx_out = o_idx;
-    r.sim_out = o_sim;
-    r.cnt_out = o_cnt;
-    r.cert_out = ix.d_cert;
-    r.kth_out = ix.d_kth;
-    r.certify = stride == 1;
-    if ((e = launch_rerank(r, s)) != cudaSuccess) return cuda_error(e, "rerank launch");
-
-    // ---- pass 2: every probed row whose bound reaches T, for the uncertified queries ----
     uint32_t* d_m = ix.d_fbn + 1;     // uncertified queries
     uint32_t* d_fail = ix.d_fbn + 2;  // of them, collections that overflowed
-    launch_compact_zero_flags(ix.d_cert, nq, ix.d_ids, d_m, s);
-    ivf_pass2_thr_kernel<<<(nq + 255) / 256, 256, 0, s>>>(ix.d_cert, ix.d_kth, nq, ix.d_q2_thr);
-    count_launch();
+    cudaEvent_t ev_a = nullptr;
+    if (groups) {
+        a.p.gm = reinterpret_cast<uint32_t*>(w.d_ws);
+        a.p.gm_tiles = gm_tiles;
+        a.p.gm_group = 8;
+        a.p.gm_span = span;
+        ix.scan_event_begin(s, ev_a);
+        e = launch_scan_tc(a, false, 2, s);
+        ix.scan_event_end(s, ev_a);
+        if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch");
+        TcThresholdArgs t;
+        t.gm = a.p.gm;
+        t.group = 8;
+        t.tiles = gm_tiles;
+        t.span = span;
+        t.stride = stride;
+        t.rows = ix.rows;
+        t.slot_off = w.d_q_slot_off;
+        t.slot_row0 = w.d_slot_row0;
+        t.base = v.d_reordered;
+        t.ds = static_cast<uint32_t>(ix.ds);
+        t.queries = ix.d_qn;
+        t.nq = nq;
+        t.kp = kp;
+        t.k = k;
+        t.q_resid = ix.d_q_resid;
+        t.eps_rows = v.eps16;
+        t.eps_acc = a.p.eps_acc;
+        t.cand_idx = ix.d_cand_idx;
+        t.cand_sim = ix.d_cand_sim;
+        t.cand_cnt = ix.d_cand_cnt;
+        t.cert = ix.d_cert;
+        t.kth = ix.d_kth;
+        t.ids = ix.d_ids;
+        t.live = d_m;
+        if ((e = launch_threshold(t, s)) != cudaSuccess) return cuda_error(e, "threshold launch");
+    } else {
+        cudaMemsetAsync(ix.d_thr, 0, nq * sizeof(unsigned long long), s);
+        a.p.kprime = kp;
+        a.p.heap_k = stride > 1 ? std::max(1u, std::min(kp, k)) : kp;  // a sampled pass 1 only yields T
+        a.p.thr_global = ix.d_thr;
+        a.p.ws_keys = w.d_ws;
+        ix.scan_event_begin(s, ev_a);
+        e = launch_scan_tc(a, false, 0, s);
+        ix.scan_event_end(s, ev_a);
+        if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch");
+        uint32_t p2 = 1;
+        while (p2 < kp) p2 <<= 1;
+        ivf_merge_kernel<<<nq, 512, p2 * sizeof(uint64_t), s>>>(w.d_ws, w.d_q_slot_off, kp, ix.d_cand_idx, ix.d_cand_sim,
+                                                                ix.d_cand_cnt);
+        count_launch();
+        RerankArgs r;
+        r.base = v.d_reordered;  // the slot keys hold list positions
+        r.row_map = v.d_row_map;
+        r.ds = static_cast<uint32_t>(ix.ds);
+        r.queries = ix.d_qn;
+        r.cand_idx = ix.d_cand_idx;
+        r.cand_sim = ix.d_cand_sim;
+        r.cand_cnt = ix.d_cand_cnt;
+        r.nq = nq;
+        r.kp = kp;
+        r.k = k;
+        r.idx_out = o_idx;
+        r.sim_out = o_sim;
+        r.cnt_out = o_cnt;
+        r.cert_out = ix.d_cert;
+        r.kth_out = ix.d_kth;
+        r.certify = stride == 1;
+        if ((e = launch_rerank(r, s)) != cudaSuccess) return cuda_error(e, "rerank launch");
+        launch_compact_zero_flags(ix.d_cert, nq, ix.d_ids, d_m, s);
+        ivf_pass2_thr_kernel<<<(nq + 255) / 256, 256, 0, s>>>(ix.d_cert, ix.d_kth, nq, ix.d_q2_thr);
+        count_launch();
+    }
+    // T by query (a certified one: +inf)
+    const float* q_thr = groups ? ix.d_kth : ix.d_q2_thr;
+
+    // ---- pass 2: every probed row whose bound reaches T, for the uncertified queries ----
     cudaMemsetAsync(ix.d_cnt2, 0, nq * sizeof(uint32_t), s);
     a.stages = plan2.stages;
     a.stream_a = plan2.stream_a;
     a.p.tile_stride = 1;
     a.p.kprime = 0;
-    a.p.q_thr = ix.d_q2_thr;
+    a.p.q_thr = q_thr;
     a.p.cand_rows = ix.d_rows2;
     a.p.cand_cnt = ix.d_cnt2;
     a.p.cap2 = cap2;
@@ -975,7 +1034,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     ix.scan_event_end(s, ev_a);
     if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch (pass 2)");
     e = launch_rerank_collected(v.d_reordered, static_cast<uint32_t>(ix.ds), ix.d_qn, ix.d_ids, nq, ix.d_rows2,
-                                ix.d_cnt2, cap2, k, ix.d_q2_thr, ix.d_rslots, o_idx, o_sim, o_cnt, ix.d_ok2, s, true,
+                                ix.d_cnt2, cap2, k, q_thr, ix.d_rslots, o_idx, o_sim, o_cnt, ix.d_ok2, s, true,
                                 d_m, v.d_row_map);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
     launch_compact_zero_flags(ix.d_ok2, nq, ix.d_tcfail, d_fail, s, d_m);
@@ -983,7 +1042,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     cudaMemcpyAsync(w.h_probed, w.d_counters, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(ix.h_fbn, ix.d_fbn, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     ix.last_tc_n = nq;
-    ix.stats.kernel_launches += 14;
+    ix.stats.kernel_launches += groups ? 11 : 14;
     ix.stats.path = 5;
     ix.stats.nprobe = np;
     ix.stats.rerank_width = kp;

@@ -11,6 +11,9 @@
 //   shared memory, thresholds shared across CTAs through a global per-query key). K4 re-scores the
 //   k′ candidates exactly in FP32; the exact k-th score T is a lower bound of the true k-th score.
 //   If T > the k′-th upper bound, no other row can enter the top-k: the query is done.
+//   When pass 1 is known not to certify it only has to yield T, and a sample of the tiles gives one.
+//   That pass (kMode 2) keeps no per-query state: it writes the largest score of every group of 8 or
+//   32 sampled rows, and threshold_kernel re-scores the rows of each query's k′ largest groups.
 //   Pass 2 (kMode 1), for the other queries only: collect every row with u_r ≥ T (no row with
 //   u_r < T can reach the top-k, since k rows already score ≥ T), and re-score them exactly.
 //   Only a query whose pass-2 set overflows its buffer is re-run on the FP32 scan.
@@ -40,17 +43,18 @@ constexpr int kM = 128;               // queries per CTA (TMEM lanes)
 constexpr int kN = 256;               // base rows per tile (MMA N)
 constexpr uint32_t kAChunk = kM * 128;
 constexpr uint32_t kBChunk = kN * 128;
-// Warps: 0 TMA, 1 MMA, then the epilogue: 4 warps in pass 1 (one thread owns a query's heap), 8 in
-// pass 2 (two warps per TMEM lane quarter, each reading half of the tile's columns: collection has
-// no per-query state beyond the threshold, and the epilogue, not the MMA, bounds the pass).
+// Warps: 0 TMA, 1 MMA, then the epilogue: 4 warps in a pass 1 with heaps (one thread owns a query's
+// heap), 8 in pass 2 and the group-maxima pass (two warps per TMEM lane quarter, each reading half of
+// the tile's columns: neither keeps per-query state that two threads would share).
 template <int kMode>
-constexpr uint32_t epi_warps() { return kMode == 1 ? 8u : 4u; }
+constexpr uint32_t epi_warps() { return kMode == 0 ? 4u : 8u; }
 // Pass 2: rows that pass the cut are staged per epilogue thread and appended to the query's
 // collection kPass2Stage at a time (one atomic per group instead of one per row).
 constexpr uint32_t kPass2Stage = 16;
 template <int kMode>
 constexpr int tc_threads() { return 64 + 32 * static_cast<int>(epi_warps<kMode>()); }
 constexpr uint32_t kTmemCols = 512;   // two 256-column FP32 accumulators
+constexpr uint32_t kNoGroup = 0xFF800000u;  // group maxima: -inf, a group without rows
 
 NNDEX_DEVICE_INLINE uint8_t* align_1024(uint8_t* p) {
     const uint32_t a = smem_u32(p);
@@ -189,6 +193,15 @@ NNDEX_DEVICE_INLINE void epi_survivor(const TcParams& p, EpiState& st, uint64_t*
 // landed, accumulators drained) are the even CTA's, armed for both CTAs' bytes and arrivals; the
 // MMA completions arrive on both CTAs' barriers (slab free, accumulator ready). The tile map's box
 // is 128 rows.
+// kMode 2 (a sampled pass 1): the epilogue keeps, per query and group of rows (the same 8 or 32
+// columns of gm_span consecutive scanned tiles), the group's largest score, its low bits replaced by
+// the row's tile (log2 gm_span bits) and column in its 32-column chunk (5 bits); 0xFF800000: no row. A
+// thread holds 16 running maxima and stores 16 or 64 bytes per gm_span tiles. The heaps it
+// replaces were bound by their inserts, serial per lane and divergent per warp: on 10M x 256 with
+// 4,096 queries at stride 32 the BF16 pass took 1,839 us with them and takes 600 now (its MMAs alone
+// need about 470); on 2M x 512 in FP8 with 1,000 queries at k = 100, stride 8, 1,977 us -> 200 (the
+// heaps also pushed the query slabs out of shared memory); the IVF list scan of 1,024 queries over
+// 2M x 384, 32 of 1,414 lists, stride 4, 339 us -> 142.
 template <bool kFp8, int kST, int kMode, bool kStreamA, bool kItems, int kQB, bool kPair = false>
 __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
     scan_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_b,
@@ -566,8 +579,8 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                     if (pos + i < p.cap2) p.cand_rows[static_cast<size_t>(q) * p.cap2 + pos + i] = my_stage[i];
                 staged = 0;
             };
-            const float qs = (kFp8 && valid_q) ? p.q_scale[q] : 1.0f;
-            const float rq = valid_q ? p.q_resid[q] : 0.0f;
+            const float qs = (kFp8 && kMode != 2 && valid_q) ? p.q_scale[q] : 1.0f;
+            const float rq = (kMode != 2 && valid_q) ? p.q_resid[q] : 0.0f;
             const float b_mul = 1.0f + rq, b_add = rq + p.eps_acc;
             const float slack = fmaf(p.eps_rows, b_mul, b_add);  // the largest u_r − s̃_r over all rows
             EpiState st;
@@ -575,11 +588,24 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
             if (kMode == 0) {
                 st.thr_key = valid_q ? p.thr_global[q] : ~0ull;
                 st.thr_f = !valid_q ? INFINITY : (st.thr_key ? key_score(st.thr_key) : -INFINITY);
+            } else if (kMode == 2) {
+                st.thr_key = 0;
+                st.thr_f = INFINITY;
             } else {
                 st.thr_key = 0;
                 st.thr_f = valid_q ? p.q_thr[q] : INFINITY;
             }
             st.cut = st.thr_f - slack;
+            // group maxima: this thread's words of the (query, range or slot), gm_span tiles at a time
+            uint32_t gacc[16];
+            const uint32_t keep = kMode == 2 ? ~(32u * p.gm_span - 1u) : 0u;
+            const uint32_t gm_words = kMode == 2 ? kN / p.gm_group : 0u;
+            uint32_t* gm = nullptr;
+            if (kMode == 2 && valid_q) {
+                const uint64_t part = kItems ? static_cast<uint64_t>(p.it_lane_slot[q0 + lrow]) + w.chunk
+                                             : static_cast<uint64_t>(q) * nranges + range;
+                gm = p.gm + part * p.gm_tiles * gm_words + c_begin * 32 / p.gm_group;
+            }
             for (uint32_t t = 0; t < w.ntiles; ++t, ++tg) {
                 const uint32_t buf = tg & 1u, ub = tg >> 1;
                 const uint64_t tile_row0 = row_begin + static_cast<uint64_t>(t) * tile_step;
@@ -587,7 +613,7 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                 // so no thread needs the tile's 256 scales unless a score may survive
                 float smin = 0.0f, smax = 0.0f;
                 const float* sc = kFp8 ? p.row_scale + tile_row0 : nullptr;
-                if (kFp8) {
+                if (kFp8 && kMode != 2) {
                     const float2 mm = p.tile_scale[tile_row0 / kN];  // a 128-row tile lies in one 256-row tile
                     smin = mm.x;
                     smax = mm.y;
@@ -616,13 +642,39 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                 // (smallest row scale · query scale) when cut < 0; 2⁻²⁰ of slack covers the roundings
                 // of both sides.
                 float raw_cut = st.cut;
-                if (kFp8) {
+                if (kFp8 && kMode != 2) {
                     const float den = (st.cut >= 0.0f ? smax : smin) * qs;
                     raw_cut = (den > 0.0f) ? st.cut / den : -INFINITY;
                     raw_cut -= fabsf(raw_cut) * 9.5367431640625e-07f;
                     if (!(raw_cut == raw_cut)) raw_cut = -INFINITY;  // an infinite cut filters nothing here
                 }
+                const uint32_t sub = kMode == 2 ? t & (p.gm_span - 1u) : 0u;  // the tile in its groups
                 auto process = [&](const uint32_t(&v)[32], uint32_t c) {
+                    if constexpr (kMode == 2) {
+                        // rows of this chunk inside the CTA's rows (fewer than 32 only at their end)
+                        const uint64_t c_row0 = tile_row0 + c * 32;
+                        const uint32_t live =
+                            c_row0 >= row_end ? 0u : (row_end - c_row0 < 32 ? static_cast<uint32_t>(row_end - c_row0) : 32u);
+#pragma unroll
+                        for (uint32_t g = 0; g < 4; ++g) {
+                            float w8[8];
+#pragma unroll
+                            for (uint32_t j = 0; j < 8; ++j) {
+                                float x = __uint_as_float(v[g * 8 + j]);
+                                // FP8: by row scale only; the query's scale orders nothing
+                                if (kFp8) x *= sc[c * 32 + g * 8 + j];
+                                w8[j] = __uint_as_float((__float_as_uint(x) & keep) | (sub * 32 + g * 8 + j));
+                                if (live < 32 && g * 8 + j >= live) w8[j] = -INFINITY;
+                            }
+#pragma unroll
+                            for (uint32_t h = 4; h > 0; h >>= 1)
+#pragma unroll
+                                for (uint32_t j = 0; j < h; ++j) w8[j] = fmaxf(w8[j], w8[j + h]);
+                            uint32_t& acc = gacc[(c - c_begin) * 4 + g];
+                            acc = __float_as_uint(sub == 0 ? w8[0] : fmaxf(__uint_as_float(acc), w8[0]));
+                        }
+                        return;
+                    }
                     // A padding lane (no query: past nq, or an empty slot of a gathered block) scores
                     // whatever its query row holds, +inf included; it never survives, since its
                     // index would address past the per-query outputs.
@@ -683,6 +735,26 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                         tmem_wait_ld_regs(va);
                     }
                 }
+                if constexpr (kMode == 2) {
+                    static_assert(kChunks == 4, "16 groups of 8 columns per thread and tile");
+                    if (gm && (sub == p.gm_span - 1u || t + 1 == w.ntiles)) {
+                        if (p.gm_group == 8) {
+#pragma unroll
+                            for (uint32_t i = 0; i < 4; ++i)
+                                *reinterpret_cast<uint4*>(gm + i * 4) =
+                                    make_uint4(gacc[i * 4], gacc[i * 4 + 1], gacc[i * 4 + 2], gacc[i * 4 + 3]);
+                        } else {
+                            uint32_t m[4];
+#pragma unroll
+                            for (uint32_t i = 0; i < 4; ++i)
+                                m[i] = __float_as_uint(
+                                    fmaxf(fmaxf(__uint_as_float(gacc[i * 4]), __uint_as_float(gacc[i * 4 + 1])),
+                                          fmaxf(__uint_as_float(gacc[i * 4 + 2]), __uint_as_float(gacc[i * 4 + 3]))));
+                            *reinterpret_cast<uint4*>(gm) = make_uint4(m[0], m[1], m[2], m[3]);
+                        }
+                        gm += gm_words;
+                    }
+                }
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) {
@@ -691,6 +763,12 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                 }
             }
             if (kMode == 1 && staged) flush_stage();
+            if constexpr (kMode == 2) {
+                // tiles that this range or chunk does not have: no rows (the thread's half of the words)
+                for (uint32_t t = (w.ntiles + p.gm_span - 1) / p.gm_span; gm && t < p.gm_tiles; ++t, gm += gm_words)
+                    for (uint32_t i = 0; i < gm_words / 2; i += 4)
+                        *reinterpret_cast<uint4*>(gm + i) = make_uint4(kNoGroup, kNoGroup, kNoGroup, kNoGroup);
+            }
             if (kMode == 0 && valid_q) {
                 uint64_t* dst = kItems ? p.ws_keys + static_cast<size_t>(p.it_lane_slot[q0 + lrow] + w.chunk) * p.kprime
                                        : p.ws_keys + (static_cast<size_t>(q) * nranges + range) * p.kprime;
@@ -828,6 +906,135 @@ __global__ void __launch_bounds__(1024, 1)
         // T: the exact k-th score among the candidates, a lower bound of the true k-th; with fewer
         // than k candidates (a sampled pass 1 over few rows) there is no bound.
         kth_out[q] = kk == k ? key_score(keys[kk - 1]) : -INFINITY;
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// T of a sampled pass 1 from its group maxima (scan_tc_kernel's kMode 2): per query, the rows of the
+// k′ largest groups re-scored exactly in the FP32 scan's order; T is the k-th of those scores, a lower
+// bound of the true k-th (k distinct rows reach it). Fewer than k groups give no bound. Nothing is
+// certified, so every query is listed for pass 2. One block per query:
+//   * each thread keeps the largest of its words, or of each of four shares of them (kR, k′ > 128); the
+//     k′-th largest of these maxima is a cut that at least k′ words reach, and hardly more do (the
+//     words are dealt round-robin);
+//   * the words that reach the cut are listed and sorted, and the first k′ re-scored. A list that
+//     would not fit (mass ties) is truncated: any k rows give a valid T.
+// Bound by its sorts and the gather of the k′ rows. On 10M × 256 with 4,096 queries at k = 10: 107 us,
+// where the merge and rerank of the heaps took 217; 2M × 512 in FP8, 1,000 queries, k = 100: 191 us
+// (four shares; one maximum per thread of 1,024-thread blocks took 284), before 165.
+// ------------------------------------------------------------------------------------------
+namespace {
+constexpr int kThrThreads = 256;
+constexpr uint32_t kThrList = 2048;  // words listed per query
+constexpr uint32_t kThrExact = 1024;  // where the exact keys (≤ 512) start, past the k′ ≤ 512 groups
+
+// Order of a group's word: 0 for a group without rows (or with NaN scores only).
+NNDEX_DEVICE_INLINE uint32_t group_order(uint32_t w) {
+    return (w == kNoGroup || (w & 0x7FFFFFFFu) > 0x7F800000u) ? 0u : float_to_ordered(__uint_as_float(w));
+}
+}  // namespace
+
+template <int kR, bool kItems>
+__global__ void __launch_bounds__(kThrThreads) threshold_kernel(const TcThresholdArgs a) {
+    constexpr int NT = kThrThreads;
+    __shared__ uint64_t keys[kThrList];
+    __shared__ uint32_t count;
+    extern __shared__ __align__(16) float q_s[];  // the query
+    const uint32_t q = blockIdx.x, tid = threadIdx.x;
+    const uint32_t wpt = kN / a.group;            // words per span of tiles
+    const uint32_t slot0 = kItems ? a.slot_off[q] : 0u;
+    const uint64_t nwords = kItems ? static_cast<uint64_t>(a.slot_off[q + 1] - slot0) * a.tiles * wpt : a.words;
+    const uint64_t part0 = kItems ? slot0 : static_cast<uint64_t>(q) * a.parts;  // the query's first range or slot
+    const uint4* words = reinterpret_cast<const uint4*>(a.gm + part0 * a.tiles * wpt);
+    const uint32_t n4 = static_cast<uint32_t>(nwords / 4);
+    for (uint32_t d = tid; d < a.ds; d += NT) q_s[d] = a.queries[static_cast<size_t>(q) * a.ds + d];
+    uint32_t best[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) best[r] = 0;
+    for (uint32_t i0 = tid; i0 < n4; i0 += NT * kR) {
+        uint4 w[kR];
+#pragma unroll
+        for (int r = 0; r < kR; ++r)
+            w[r] = i0 + r * NT < n4 ? words[i0 + r * NT] : make_uint4(kNoGroup, kNoGroup, kNoGroup, kNoGroup);
+#pragma unroll
+        for (int r = 0; r < kR; ++r)
+            best[r] = max(max(best[r], max(group_order(w[r].x), group_order(w[r].y))),
+                          max(group_order(w[r].z), group_order(w[r].w)));
+    }
+#pragma unroll
+    for (int r = 0; r < kR; ++r) keys[tid + r * NT] = best[r];
+    if (tid == 0) count = 0;
+    __syncthreads();
+    block_bitonic_sort_desc(keys, NT * kR);
+    const uint32_t nth = a.kp < static_cast<uint32_t>(NT * kR) ? a.kp : static_cast<uint32_t>(NT * kR);
+    uint32_t cut = static_cast<uint32_t>(keys[nth - 1]);
+    if (cut == 0) cut = 1;  // fewer groups than that: all of them
+    __syncthreads();
+    for (uint32_t i0 = 0; i0 < n4; i0 += NT) {
+        const uint32_t i = i0 + tid;
+        uint4 w = make_uint4(kNoGroup, kNoGroup, kNoGroup, kNoGroup);
+        if (i < n4) w = words[i];
+        const uint32_t o[4] = {group_order(w.x), group_order(w.y), group_order(w.z), group_order(w.w)};
+        if (!__any_sync(0xFFFFFFFFu, max(max(o[0], o[1]), max(o[2], o[3])) >= cut)) continue;
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const bool take = o[u] >= cut;
+            const uint32_t at = warp_append(&count, take);
+            if (take && at < kThrList)
+                keys[at] = (static_cast<uint64_t>(o[u]) << 32) | (0xFFFFFFFFu - (i * 4 + u));
+        }
+    }
+    __syncthreads();
+    uint32_t m = count < kThrList ? count : kThrList;
+    uint32_t p2 = 1;
+    while (p2 < m) p2 <<= 1;
+    for (uint32_t i = m + tid; i < p2; i += NT) keys[i] = 0ull;
+    __syncthreads();
+    block_bitonic_sort_desc(keys, p2);
+    if (m > a.kp) m = a.kp;
+    uint32_t p2k = 1;
+    while (p2k < a.kp) p2k <<= 1;
+    // the bound of a listed row's exact score: its approximate score (up to 32·span − 1 units of the
+    // last place low, under span·2⁻¹⁸ of its magnitude) plus the largest slack
+    const float low = static_cast<float>(a.span) * 7.62939453125e-06f;
+    const float rq = a.q_resid[q], qs = a.q_scale ? a.q_scale[q] : 1.0f;
+    const float slack = fmaf(a.eps_rows, 1.0f + rq, rq + a.eps_acc);
+    const uint32_t ch = tid & 7u, nbox = a.ds / 32;
+    for (uint32_t j0 = 0; j0 < p2k; j0 += NT / 8) {
+        const uint32_t j = j0 + (tid >> 3);
+        bool live = j < m;
+        uint64_t row = 0;
+        float bound = 0.0f;
+        if (live) {
+            const uint32_t o = static_cast<uint32_t>(keys[j] >> 32);
+            const uint32_t wi = 0xFFFFFFFFu - static_cast<uint32_t>(keys[j]);
+            const uint32_t bits = __float_as_uint(ordered_to_float(o));
+            const uint32_t tile = wi / wpt, in_tile = wi % wpt * a.group / 32 * 32 + (bits & 31u);
+            const uint32_t part = tile / a.tiles, t = tile % a.tiles * a.span + (bits >> 5 & (a.span - 1));
+            const uint64_t first = kItems ? a.slot_row0[slot0 + part] : static_cast<uint64_t>(part) * a.range_rows;
+            row = first + static_cast<uint64_t>(t) * a.stride * kN + in_tile;
+            if (row >= a.rows) live = false;  // words of a scan that gave up (its status is reported)
+            const float s = __uint_as_float(bits) * qs;
+            bound = s + fabsf(s) * low + slack;
+        }
+        const float acc = dot_scan_order<8>(a.base + (live ? row : 0) * a.ds, q_s, nbox, ch, live);
+        if (ch == 0 && j < p2k) {
+            keys[kThrExact + j] = live ? make_key(acc, static_cast<uint32_t>(row)) : 0ull;
+            if (j < a.kp) {
+                a.cand_idx[static_cast<size_t>(q) * a.kp + j] = live ? row : 0;
+                a.cand_sim[static_cast<size_t>(q) * a.kp + j] = live ? bound : 0.0f;
+            }
+        }
+    }
+    __syncthreads();
+    block_bitonic_sort_desc(keys + kThrExact, p2k);
+    if (tid == 0) {
+        const uint64_t kth = keys[kThrExact + a.k - 1];
+        a.kth[q] = kth ? key_score(kth) : -INFINITY;
+        a.cand_cnt[q] = m;
+        a.cert[q] = 0;
+        a.ids[q] = q;
+        if (q == 0) *a.live = a.nq;
     }
 }
 
@@ -1047,8 +1254,12 @@ static cudaError_t launch_tc_items(const TcArgs& a, cudaStream_t stream) {
 }
 
 cudaError_t launch_scan_tc(const TcArgs& a, bool fp8, int mode, cudaStream_t stream) {
+    if (mode == 2 && (!a.p.gm || a.p.gm_tiles == 0 || (a.p.gm_group != 8 && a.p.gm_group != 32) || a.qb != 1 ||
+                      a.p.gm_span == 0 || (a.p.gm_span & (a.p.gm_span - 1)) || a.p.gm_span > kMaxGroupSpan))
+        return cudaErrorInvalidValue;
     if (a.items) {
         if (fp8 || a.items > 0x7FFFFFFFu) return cudaErrorInvalidValue;
+        if (mode == 2) return a.stream_a ? launch_tc_items<2, true>(a, stream) : launch_tc_items<2, false>(a, stream);
         if (mode == 0) return a.stream_a ? launch_tc_items<0, true>(a, stream) : launch_tc_items<0, false>(a, stream);
         return a.stream_a ? launch_tc_items<1, true>(a, stream) : launch_tc_items<1, false>(a, stream);
     }
@@ -1073,6 +1284,10 @@ cudaError_t launch_scan_tc(const TcArgs& a, bool fp8, int mode, cudaStream_t str
         }
     }
     if (a.qb != 1) return cudaErrorInvalidValue;
+    if (mode == 2) {
+        if (a.stream_a) return fp8 ? launch_tc_stages<true, 2, true>(a, stream) : launch_tc_stages<false, 2, true>(a, stream);
+        return fp8 ? launch_tc_stages<true, 2, false>(a, stream) : launch_tc_stages<false, 2, false>(a, stream);
+    }
     if (mode == 0) {
         if (a.stream_a) return fp8 ? launch_tc_stages<true, 0, true>(a, stream) : launch_tc_stages<false, 0, true>(a, stream);
         return fp8 ? launch_tc_stages<true, 0, false>(a, stream) : launch_tc_stages<false, 0, false>(a, stream);
@@ -1113,6 +1328,30 @@ cudaError_t launch_gather_queries(const uint32_t* ids, uint32_t m, const void* q
                                                  live);
     count_launch();
     return cudaGetLastError();
+}
+
+template <bool kItems>
+static cudaError_t launch_threshold_impl(const TcThresholdArgs& a, cudaStream_t stream) {
+    const size_t smem = static_cast<size_t>(a.ds) * sizeof(float);
+    // enough maxima that the k′-th largest of them is a tight cut
+    const bool wide = a.kp > 128;
+    auto kern = wide ? threshold_kernel<4, kItems> : threshold_kernel<1, kItems>;
+    if (smem > 24 * 1024) {  // beside the 16 KB of static lists
+        const cudaError_t e =
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<a.nq, kThrThreads, smem, stream>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_threshold(const TcThresholdArgs& a, cudaStream_t stream) {
+    if (a.nq == 0) return cudaSuccess;
+    if (a.k == 0 || a.k > a.kp || a.kp > kMaxGroupCandidates || a.tiles == 0 || (a.group != 8 && a.group != 32) ||
+        a.span == 0 || (a.span & (a.span - 1)) || a.span > kMaxGroupSpan)
+        return cudaErrorInvalidValue;
+    return a.slot_off ? launch_threshold_impl<true>(a, stream) : launch_threshold_impl<false>(a, stream);
 }
 
 uint32_t rerank_chunks(uint32_t cap2) { return (cap2 + kRerankChunk - 1) / kRerankChunk; }
