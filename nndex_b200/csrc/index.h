@@ -117,6 +117,7 @@ struct CudaIndex {
     uint32_t forced_stride = 0;     // the tuned plan's pass-1 tile stride for the current batch (0 = rule)
     uint32_t forced_qb = 0;         // the tuned plan's pass-2 query blocks per CTA (0 = rule)
     uint32_t last_tc_stride = 1;
+    bool tc_patched = false;  // after the batch, results of some queries were written again
     bool tc_groups = false;  // the batch's pass 1 wrote group maxima (every query goes to pass 2)
     float* d_kth = nullptr;  // pass 1: exact k-th score per query
     unsigned long long* d_floor = nullptr;  // TF32 scan: per query, a key its k'-th candidate reaches
@@ -226,7 +227,7 @@ struct CudaIndex {
     // scan, spare}), read back with the statistics.
     uint32_t* d_fbq = nullptr;  // the re-run queries' indices
     size_t cap_fbq = 0;
-    uint32_t* d_fbn = nullptr;  // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, spare}
+    uint32_t* d_fbn = nullptr;  // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, overflows of its retry}
     uint32_t* h_fbn = nullptr;  // pinned copy
     uint32_t* d_tcfail = nullptr;  // TC pass 2: positions (in d_ids) of the queries whose collection overflowed
     size_t cap_tcfail = 0;
@@ -318,6 +319,10 @@ struct CudaIndex {
     // pass-1 stride rule, and the FP32 re-run of any query whose collection overflowed (device
     // outputs patched in place; synchronises the stream again only then).
     int finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
+    // Pass 2 once more for the m queries whose collection overflowed (positions in d_ids: d_tcfail),
+    // against the T of the rows they did collect; the ones that overflow again are left in *failed.
+    int retry_tc_pass2(bool fp8, uint32_t m, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
+                       cudaStream_t s, std::vector<uint32_t>* failed);
     int enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
     // The FP32 scan for the listed queries (rows of d_qn), written into their output slots.
     int rerun_exact_fp32(const std::vector<uint32_t>& qs, uint32_t kcap, uint64_t* o_idx, float* o_sim,

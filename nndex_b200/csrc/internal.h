@@ -303,12 +303,15 @@ cudaError_t launch_gather_queries(const uint32_t* ids, uint32_t m, const void* q
 // Pass 2's exact rerank (two launches: work items of collected rows, then a merge per query).
 // thr: each query's T (indexed like cnt2). vecs: the base by row, or with row_map (IVF) the
 // list-ordered copy by collected position. slot_keys: m × rerank_chunks(cap2) × k keys of scratch.
+// With fail (m positions in ids whose collections overflowed): the k-th exact score of the rows they
+// did collect is a higher T, written to kth (by query), and the queries to fail_ids; no results.
 uint32_t rerank_chunks(uint32_t cap2);
 cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float* queries, const uint32_t* ids,
                                     uint32_t m, const uint32_t* rows2, const uint32_t* cnt2, uint32_t cap2, uint32_t k,
                                     const float* thr, uint64_t* slot_keys, uint64_t* idx_out, float* sim_out,
                                     uint32_t* cnt_out, uint32_t* ok_out, cudaStream_t stream, bool by_query = false,
-                                    const uint32_t* live = nullptr, const uint32_t* row_map = nullptr);
+                                    const uint32_t* live = nullptr, const uint32_t* row_map = nullptr,
+                                    const uint32_t* fail = nullptr, float* kth = nullptr, uint32_t* fail_ids = nullptr);
 cudaError_t launch_max_reduce(const float* v, uint64_t n, unsigned int* out, cudaStream_t stream);
 // FP8: {min, max} row scale of each 256-row tile (tiles = rows_alloc / 256).
 void launch_tile_scale(const float* row_scale, uint64_t rows, uint64_t tiles, float2* out, cudaStream_t s);

@@ -1063,6 +1063,7 @@ int ivf_finish_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     ix.stats.certified = m == 0 ? 1u : 0u;
     ix.stats.second_pass_queries = m;
     ix.stats.fp32_fallback_queries = failed_n;
+    ix.tc_patched = failed_n != 0;
     int st;
     if (m) {
         // rows collected by pass 2 (the counts of the uncertified queries, read after the batch)

@@ -1093,24 +1093,29 @@ NNDEX_DEVICE_INLINE void block_keep_best(uint64_t* keys, uint32_t m, uint32_t kk
 // rows that gave T are among the collected ones, so only those are kept; the item's best k of them
 // go to its slot. `vecs` holds the vectors: the base by row, or (IVF) the list-ordered copy by
 // collected position. Items past a query's collection (or of an overflowed one) return at once.
+// With `fail` (the second threshold of overflowed collections): item i is of uncertified query
+// fail[i], whose first cap2 collected rows are all re-scored.
 __global__ void __launch_bounds__(256)
     rerank_chunk_kernel(const float* __restrict__ vecs, uint32_t ds, const float* __restrict__ queries,
                         const uint32_t* __restrict__ ids, const uint32_t* __restrict__ rows2,
                         const uint32_t* __restrict__ cnt2, uint32_t cap2, uint32_t k, int by_query,
                         const uint32_t* __restrict__ live, const uint32_t* __restrict__ row_map,
-                        const float* __restrict__ thr, uint64_t* __restrict__ slot_keys) {
+                        const float* __restrict__ thr, uint64_t* __restrict__ slot_keys,
+                        const uint32_t* __restrict__ fail) {
     __shared__ uint64_t keys[kRerankChunk];
     __shared__ BlockSelectScratch sel;
     __shared__ uint32_t fill;
     const uint32_t i = blockIdx.x, c = blockIdx.y;
     if (live && i >= *live) return;
-    const uint32_t q = ids[i];
-    const uint32_t qrow = by_query ? q : i;  // collected rows and T indexed by query, or by position in ids
-    const uint32_t total = cnt2[qrow];
+    const uint32_t at0 = fail ? fail[i] : i;
+    const uint32_t q = ids[at0];
+    const uint32_t qrow = by_query ? q : at0;  // collected rows and T indexed by query, or by position in ids
+    uint32_t total = cnt2[qrow];
+    if (fail && total > cap2) total = cap2;
     const uint32_t j_begin = c * kRerankChunk;
     if (total > cap2 || j_begin >= total) return;
     const uint32_t j_end = (total - j_begin) < kRerankChunk ? total : j_begin + kRerankChunk;
-    const float t = thr[qrow];
+    const float t = fail ? -INFINITY : thr[qrow];
     const uint32_t ch = threadIdx.x & 7u, slot = threadIdx.x >> 3, nslots = blockDim.x >> 3;
     const float* qv = queries + static_cast<size_t>(q) * ds;
     const uint32_t nbox = ds / 32;
@@ -1143,14 +1148,17 @@ __global__ void __launch_bounds__(256)
     rerank_merge_kernel(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ cnt2, uint32_t cap2,
                         uint32_t k, int by_query, const uint32_t* __restrict__ live,
                         const uint64_t* __restrict__ slot_keys, uint32_t chunks, uint64_t* __restrict__ idx_out,
-                        float* __restrict__ sim_out, uint32_t* __restrict__ cnt_out, uint32_t* __restrict__ ok_out) {
+                        float* __restrict__ sim_out, uint32_t* __restrict__ cnt_out, uint32_t* __restrict__ ok_out,
+                        const uint32_t* __restrict__ fail, float* __restrict__ kth, uint32_t* __restrict__ fail_ids) {
     extern __shared__ uint64_t keys[];  // chunks·k keys, at least p2(k)
     __shared__ BlockSelectScratch sel;
     const uint32_t i = blockIdx.x;
     if (live && i >= *live) return;
-    const uint32_t q = ids[i];
-    const uint32_t total = cnt2[by_query ? q : i];
-    if (total > cap2) {  // the collected set overflowed: this query goes to the FP32 scan
+    const uint32_t at0 = fail ? fail[i] : i;
+    const uint32_t q = ids[at0];
+    uint32_t total = cnt2[by_query ? q : at0];
+    if (fail && total > cap2) total = cap2;
+    if (total > cap2) {  // the collected set overflowed: finish_tc raises the query's T, or re-runs it
         if (threadIdx.x == 0) ok_out[i] = 0;
         return;
     }
@@ -1169,6 +1177,15 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     const uint32_t kk = m < k ? m : k;
     if (m > kk) block_keep_best(keys, m, kk, sel);
+    if (fail) {  // only the k-th score is wanted: the query's next T, if it is higher
+        if (threadIdx.x == 0) {
+            uint64_t mn = ~0ull;
+            for (uint32_t j = 0; j < kk; ++j) mn = keys[j] < mn ? keys[j] : mn;
+            if (kk == k && key_score(mn) > kth[q]) kth[q] = key_score(mn);
+            fail_ids[i] = q;
+        }
+        return;
+    }
     uint32_t p2 = 1;
     while (p2 < kk) p2 <<= 1;
     for (uint32_t j = kk + threadIdx.x; j < p2; j += blockDim.x) keys[j] = 0ull;
@@ -1360,7 +1377,8 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
                                     uint32_t m, const uint32_t* rows2, const uint32_t* cnt2, uint32_t cap2, uint32_t k,
                                     const float* thr, uint64_t* slot_keys, uint64_t* idx_out, float* sim_out,
                                     uint32_t* cnt_out, uint32_t* ok_out, cudaStream_t stream, bool by_query,
-                                    const uint32_t* live, const uint32_t* row_map) {
+                                    const uint32_t* live, const uint32_t* row_map, const uint32_t* fail, float* kth,
+                                    uint32_t* fail_ids) {
     if (m == 0) return cudaSuccess;
     const uint32_t chunks = rerank_chunks(cap2);
     if (k == 0 || k > kRerankChunk || chunks > 65535u) return cudaErrorInvalidValue;
@@ -1371,7 +1389,7 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
         if (ea != cudaSuccess) return ea;
     }
     rerank_chunk_kernel<<<dim3(m, chunks), 256, qsmem, stream>>>(vecs, ds, queries, ids, rows2, cnt2, cap2, k,
-                                                                by_query ? 1 : 0, live, row_map, thr, slot_keys);
+                                                                by_query ? 1 : 0, live, row_map, thr, slot_keys, fail);
     uint32_t p2 = 1;
     while (p2 < k) p2 <<= 1;
     const size_t smem = std::max<size_t>(static_cast<size_t>(chunks) * k, p2) * sizeof(uint64_t);
@@ -1379,7 +1397,7 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     kern<<<m, 256, smem, stream>>>(ids, cnt2, cap2, k, by_query ? 1 : 0, live, slot_keys, chunks, idx_out, sim_out,
-                                   cnt_out, ok_out);
+                                   cnt_out, ok_out, fail, kth, fail_ids);
     count_launch(2);
     return cudaGetLastError();
 }

@@ -71,3 +71,29 @@ def test_sampled_list_scan_equals_fp32(rows, dims, nq, k, nlist, nprobe, stride)
     assert index.last_search_stats()["path"] == 4
     assert np.array_equal(ti, fi)
     assert np.array_equal(ts, fs)
+
+
+@pytest.mark.parametrize("precision,nq", [("bf16", 70), ("fp8", 150)])
+def test_overflowing_collection_gets_a_second_threshold(precision, nq):
+    # One dense cluster of 30,000 rows the sample never meets (it sits in tiles that stride 32 skips)
+    # next to unrelated rows: T is far too low, every query collects more than 8,192 rows, and the
+    # k-th score of the rows it did collect finishes it without the FP32 scan.
+    rng = np.random.default_rng(nq)
+    dims = 128
+    m = rng.normal(size=(256 * 80, dims)).astype(np.float32)
+    v = rng.normal(size=(1, dims)).astype(np.float32)
+    near = rng.uniform(0.2, 1.2, size=(256 * 62, 1)).astype(np.float32)
+    cluster = v + near * rng.normal(size=(256 * 62, dims)).astype(np.float32)
+    m[256:256 * 32] = cluster[:256 * 31]
+    m[256 * 33:256 * 64] = cluster[256 * 31:]
+    q = (v + np.float32(0.05) * rng.normal(size=(nq, dims))).astype(np.float32)
+    index = NNdex(m, precision=precision)
+    path = {"bf16": 2, "fp8": 3}[precision]
+    force(index, 0, nq, 10, path, 0, path, 32)
+    ti, ts = index.search(q, k=10)
+    st = index.last_search_stats()
+    assert st["path"] == path and st["fp32_fallback_queries"] == 0 and st["kernel_launches"] > 8, st
+    index.set_precision("fp32")
+    fi, fs = index.search(q, k=10)
+    assert np.array_equal(ti, fi)
+    assert np.array_equal(ts, fs)
