@@ -795,8 +795,8 @@ int CudaIndex::encode_query_tmap(bool fp8, void* buf, uint32_t n, CUtensorMap* m
 int CudaIndex::ensure_fbn() {
     if (d_fbn) return NNDEX_OK;
     cudaError_t e;
-    if ((e = cudaMalloc(&d_fbn, 4 * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMallocHost(&h_fbn, 4 * sizeof(uint32_t))) != cudaSuccess)
+    if ((e = cudaMalloc(&d_fbn, kFbnBytes)) != cudaSuccess ||
+        (e = cudaMallocHost(&h_fbn, kFbnBytes)) != cudaSuccess)
         return cuda_error(e, "fallback buffer");
     return NNDEX_OK;
 }
@@ -885,7 +885,7 @@ int CudaIndex::enqueue_tc_pass2(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, cap2, kcap,
                                 q_thr, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, d_m);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
-    launch_compact_zero_flags(d_ok2, n, d_tcfail, d_fail, s, d_m);
+    launch_compact_zero_flags(d_ok2, n, d_tcfail, d_fail, s, d_m, CollectedSum{d_cnt2, nullptr, cap2, d_fbn_rows()});
     stats.kernel_launches += 4;
     last_tc_n = n;
     return NNDEX_OK;
@@ -907,16 +907,7 @@ int CudaIndex::finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_si
     stats.fp32_fallback_queries = 0;
     tc_patched = false;
     int st;
-    if (m) {
-        // rows collected by pass 2 (the counts of its m queries, after the batch)
-        if ((st = grow_host(h_ok2, cap_hok2, n, "pinned buffer"))) return st;
-        cudaMemcpyAsync(h_ok2, d_cnt2, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        const cudaError_t e0 = cudaStreamSynchronize(s);
-        if (e0 != cudaSuccess) return cuda_error(e0, "search");
-        uint64_t total = 0;
-        for (uint32_t i = 0; i < m; ++i) total += std::min<uint32_t>(h_ok2[i], kSecondPassCap);
-        stats.pass2_rows += total;
-    }
+    stats.pass2_rows += h_fbn_rows();
     if (failed_n == 0) return NNDEX_OK;
     std::vector<uint32_t> failed;
     if ((st = retry_tc_pass2(stats.path == 3, failed_n, kcap, o_idx, o_sim, o_cnt, s, &failed))) return st;
@@ -1033,12 +1024,7 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     if ((st = grow_device(d_ws, cap_ws, std::max(per_query, fb_per_query) * n, "scan workspace"))) return st;
     if ((st = grow_device(d_qsub, cap_qsub, static_cast<uint64_t>(n) * ds, "fallback buffer"))) return st;
     if ((st = grow_device(d_fbq, cap_fbq, n, "fallback buffer"))) return st;
-    if (!d_fbn) {
-        cudaError_t e0;
-        if ((e0 = cudaMalloc(&d_fbn, 4 * sizeof(uint32_t))) != cudaSuccess ||
-            (e0 = cudaMallocHost(&h_fbn, 4 * sizeof(uint32_t))) != cudaSuccess)
-            return cuda_error(e0, "fallback buffer");
-    }
+    if ((st = ensure_fbn())) return st;
     if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_sim, cap_cand_sim, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_cnt, cap_cand_cnt, n, "tc workspace"))) return st;
@@ -1238,7 +1224,7 @@ int CudaIndex::enqueue_host_batch(uint64_t n, uint64_t kcap, int mode, int path)
                                    d_cnt, stream)))
             return st;
         // pass 2's counts come back with the results (finish_tc reads them once the batch is done)
-        cudaMemcpyAsync(h_fbn, d_fbn, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
+        cudaMemcpyAsync(h_fbn, d_fbn, kFbnBytes, cudaMemcpyDeviceToHost, stream);
     }
     if (error_report)
         serr_record(static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt, stream);
@@ -1416,9 +1402,7 @@ int CudaIndex::run_device_chunk(const float* dq, uint64_t n, uint64_t kcap, int 
     if (path == 5) {
         *synced = true;
         if ((st = ivf_search_tc(*this, n32, k32, oi, os, oc, s))) return st;
-        h_flags[1] = 0;
-        cudaMemcpyAsync(&h_flags[0], d_err, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(&h_flags[1], d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);  // err, status
         const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_error(e, "IVF search");
         if ((st = check_device_words())) return st;
@@ -1433,10 +1417,8 @@ int CudaIndex::run_device_chunk(const float* dq, uint64_t n, uint64_t kcap, int 
     }
     if ((st = enqueue_tc(path == 3, n32, k32, oi, os, oc, s))) return st;
     if ((st = enqueue_tc_pass2(path == 3, n32, k32, oi, os, oc, s))) return st;
-    cudaMemcpyAsync(h_fbn, d_fbn, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    h_flags[1] = 0;
-    cudaMemcpyAsync(&h_flags[0], d_err, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&h_flags[1], d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(h_fbn, d_fbn, kFbnBytes, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);  // err, status
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(e, "search");
     if ((st = check_device_words())) return st;
@@ -1456,7 +1438,7 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
     if (error_report && (st = serr_begin(nq, kcap, s))) return st;
     cudaMemsetAsync(d_err, 0xFF, sizeof(unsigned long long), s);
     cudaMemsetAsync(d_status, 0, sizeof(uint32_t), s);
-    bool synced = false;
+    bool synced = false, done = false;  // done: the last piece waited and its status words were clean
     for (uint64_t q0 = 0; q0 < nq; q0 += kMaxBatchChunk) {
         const uint64_t n = std::min<uint64_t>(kMaxBatchChunk, nq - q0);
         uint64_t* oi = d_idx_out + q0 * kcap;
@@ -1516,19 +1498,24 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
         }
         forced_stride = plan.stride;
         forced_qb = plan.qb;
-        st = run_device_chunk(dq, n, kcap, plan.path, oi, os, oc, s, &synced);
+        done = false;
+        st = run_device_chunk(dq, n, kcap, plan.path, oi, os, oc, s, &done);
         forced_stride = 0;
         forced_qb = 0;
         if (st) return st;
+        synced |= done;
         if (error_report) {
+            done = false;
             serr_off = q0;
             serr_record(static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), oi, os, oc, s);
         }
     }
+    if (done) {  // nothing was enqueued since
+        mark_done(s);
+        return NNDEX_OK;
+    }
     if (synchronize || synced) {
-        h_flags[1] = 0;
-        cudaMemcpyAsync(&h_flags[0], d_err, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(&h_flags[1], d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);  // err, status
         mark_done(s);
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_error(e, "search");

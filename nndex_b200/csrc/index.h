@@ -227,11 +227,15 @@ struct CudaIndex {
     // scan, spare}), read back with the statistics.
     uint32_t* d_fbq = nullptr;  // the re-run queries' indices
     size_t cap_fbq = 0;
-    uint32_t* d_fbn = nullptr;  // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, overflows of its retry}
+    // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, spare, rows pass 2 collected (64 bits)}
+    static constexpr size_t kFbnBytes = 6 * sizeof(uint32_t);
+    uint32_t* d_fbn = nullptr;
     uint32_t* h_fbn = nullptr;  // pinned copy
     uint32_t* d_tcfail = nullptr;  // TC pass 2: positions (in d_ids) of the queries whose collection overflowed
     size_t cap_tcfail = 0;
     int ensure_fbn();
+    unsigned long long* d_fbn_rows() const { return reinterpret_cast<unsigned long long*>(d_fbn + 4); }
+    uint64_t h_fbn_rows() const { return *reinterpret_cast<const unsigned long long*>(h_fbn + 4); }
     cudaStream_t fbn_stream = nullptr;
     bool fbn_pending = false;
     int fetch_fallback_stats();

@@ -263,8 +263,14 @@ cudaError_t launch_tf32_row_norms(const float* base, uint64_t rows, uint32_t ds,
 
 // Device-side certificate fallback: compaction of the zero flags (one block), a gather of their rows
 // (zeros past the count), and a scatter of re-run results back to their queries' slots.
+struct CollectedSum {
+    const uint32_t* cnt = nullptr;  // collected rows per query
+    const uint32_t* by = nullptr;   // optional: cnt is indexed by[i] rather than i
+    uint32_t cap = 0;
+    unsigned long long* sum = nullptr;
+};
 void launch_compact_zero_flags(const uint32_t* flags, uint32_t n, uint32_t* ids, uint32_t* count, cudaStream_t s,
-                               const uint32_t* live = nullptr);
+                               const uint32_t* live = nullptr, const CollectedSum& rows = CollectedSum{});
 void launch_gather_rows(const float* src, uint32_t ds, const uint32_t* ids, const uint32_t* count, uint32_t n,
                         float* dst, cudaStream_t s);
 void launch_scatter_results(const uint64_t* fb_idx, const float* fb_sim, const uint32_t* fb_cnt, const uint32_t* ids,

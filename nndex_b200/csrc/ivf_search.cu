@@ -1037,10 +1037,11 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
                                 ix.d_cnt2, cap2, k, q_thr, ix.d_rslots, o_idx, o_sim, o_cnt, ix.d_ok2, s, true,
                                 d_m, v.d_row_map);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
-    launch_compact_zero_flags(ix.d_ok2, nq, ix.d_tcfail, d_fail, s, d_m);
+    launch_compact_zero_flags(ix.d_ok2, nq, ix.d_tcfail, d_fail, s, d_m,
+                              CollectedSum{ix.d_cnt2, ix.d_ids, cap2, ix.d_fbn_rows()});
     // the plan's totals and the pass counts come back with the results
     cudaMemcpyAsync(w.h_probed, w.d_counters, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ix.h_fbn, ix.d_fbn, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(ix.h_fbn, ix.d_fbn, CudaIndex::kFbnBytes, cudaMemcpyDeviceToHost, s);
     ix.last_tc_n = nq;
     ix.stats.kernel_launches += groups ? 11 : 14;
     ix.stats.path = 5;
@@ -1065,19 +1066,7 @@ int ivf_finish_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     ix.stats.fp32_fallback_queries = failed_n;
     ix.tc_patched = failed_n != 0;
     int st;
-    if (m) {
-        // rows collected by pass 2 (the counts of the uncertified queries, read after the batch)
-        if ((st = grow_pinned(ix.h_ok2, ix.cap_hok2, nq, "pinned buffer"))) return st;
-        if ((st = grow_pinned(ix.h_ids, ix.cap_hids, nq, "pinned buffer"))) return st;
-        cudaMemcpyAsync(ix.h_ok2, ix.d_cnt2, nq * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(ix.h_ids, ix.d_cert, nq * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        const cudaError_t e0 = cudaStreamSynchronize(s);
-        if (e0 != cudaSuccess) return cuda_error(e0, "IVF search");
-        uint64_t total = 0;
-        for (uint32_t i = 0; i < nq; ++i)
-            if (!ix.h_ids[i]) total += std::min<uint32_t>(ix.h_ok2[i], kSecondPassCap);
-        ix.stats.pass2_rows += total;
-    }
+    ix.stats.pass2_rows += ix.h_fbn_rows();
     // the rule learns from batches that ran its own stride (a full pass 1 that certified few)
     if (!ix.forced_stride && w.tc_stride == 1 && ix.stats.pass1_tile_stride == 1 && m * 2 > nq) {
         w.tc_stride = ivf_sampled_stride();
