@@ -652,19 +652,20 @@ def run_mixed(args, dev, L, world):
     os_ = torch.empty((nq, k), dtype=torch.float32, device=dev)
     stats = _lib.SearchStats()
     out = {}
+    # The FP32 arm is the plain FP32 scan (the index's own choice for FP32 batches of this size is the
+    # TF32 scan with FP32 rerank): a plan in the tuner's cache, with --mixed-stride / --mixed-qb also the
+    # given stride and blocks for both low precisions.
+    n = C.c_uint64(0)
+    L.nndex_cuda_autotune_export(h, None, 0, C.byref(n))
+    buf = C.create_string_buffer(n.value)
+    L.nndex_cuda_autotune_export(h, buf, n.value, C.byref(n))
+    nqb, kb = 1 << (nq - 1).bit_length(), 1 << (k - 1).bit_length()
+    text = buf.value.decode() + f"shape ivf=0 nq={nqb} k={kb} precision=1 nprobe=0 plan path=1 stride=0 qb=0 ms=0\n"
     if args.mixed_stride or args.mixed_qb:
-        # the tuner's cache with the given stride / blocks for both tensor-core precisions at this shape
-        n = C.c_uint64(0)
-        L.nndex_cuda_autotune_export(h, None, 0, C.byref(n))
-        buf = C.create_string_buffer(n.value)
-        L.nndex_cuda_autotune_export(h, buf, n.value, C.byref(n))
-        nqb, kb = 1 << (nq - 1).bit_length(), 1 << (k - 1).bit_length()
-        text = buf.value.decode() + "".join(
-            f"shape ivf=0 nq={nqb} k={kb} precision={p} nprobe=0 plan path={p} stride={args.mixed_stride} "
-            f"qb={args.mixed_qb} ms=0\n"
-            for p in (2, 3))
-        if L.nndex_cuda_autotune_import(h, text.encode()) != 0:
-            raise RuntimeError(_lib.last_error())
+        text += "".join(f"shape ivf=0 nq={nqb} k={kb} precision={p} nprobe=0 plan path={p} "
+                        f"stride={args.mixed_stride} qb={args.mixed_qb} ms=0\n" for p in (2, 3))
+    if L.nndex_cuda_autotune_import(h, text.encode()) != 0:
+        raise RuntimeError(_lib.last_error())
     sample = min(args.mixed_oracle_queries, nq)
     ref_i, ref_s = fp64_topk(base, q[:sample], k)
     for name, prec in (("fp32", NNDEX_PRECISION_FP32), ("bf16", NNDEX_PRECISION_BF16), ("fp8", NNDEX_PRECISION_FP8)):

@@ -55,7 +55,7 @@ extern "C" {
 
 /* ---- precision of the exact scan ------------------------------------------------------ */
 #define NNDEX_PRECISION_AUTO 0u /* autotuner: FP32 at small batches, low precision + rerank */
-#define NNDEX_PRECISION_FP32 1u /* plain FP32 scan (CUDA cores)                               */
+#define NNDEX_PRECISION_FP32 1u /* FP32 results from the FP32 rows alone (no BF16/FP8 copy)   */
 #define NNDEX_PRECISION_BF16 2u /* BF16 tensor-core scan + exact FP32 rerank                  */
 #define NNDEX_PRECISION_FP8  3u /* FP8-E4M3 tensor-core scan + exact FP32 rerank              */
 
@@ -104,7 +104,8 @@ typedef struct nndex_cuda_search_stats {
     uint32_t path;             /* 1 = FP32 scan, 2 = BF16 scan+rerank, 3 = FP8 scan+rerank,
                                   4 = IVF probe + rerank, 5 = IVF list scan on the tensor
                                   cores + rerank, 6 = TF32 candidate scan + rerank
-                                  (9-16 queries of a batch)                                    */
+                                  (9-16 queries of a batch), 7 = two-pass TF32 scan + rerank
+                                  (17 queries and more of an FP32 batch)                       */
     uint32_t kernel_launches;  /* kernels this library launched for the call                */
     uint32_t rerank_width;     /* k' of a low-precision scan's first pass (0 otherwise)     */
     uint32_t certified;        /* 1 = every query certified after the first pass            */
@@ -113,7 +114,8 @@ typedef struct nndex_cuda_search_stats {
     uint64_t rows_scanned;     /* base rows scored (sum over queries for IVF)               */
     double   device_ms;        /* CUDA-event time of the device part of the call            */
     uint32_t fp32_fallback_queries; /* queries re-run on the FP32 scan (pass-2 overflow, or
-                                       an uncertified query of path 6)                       */
+                                       an uncertified query of path 6, a collection
+                                       overflow of path 7)                                   */
     uint32_t pass1_tile_stride;     /* first pass scanned every n-th 256-row tile (1 = all) */
     uint64_t ivf_rows_streamed;     /* IVF: rows read by the list scan (a list once per query group) */
     uint64_t ivf_rows_union;        /* IVF: rows in the union of the probed lists               */
@@ -265,9 +267,9 @@ NNDEX_API int nndex_cuda_search_batch_device(nndex_cuda_index* index, const floa
 NNDEX_API int nndex_cuda_set_precision(nndex_cuda_index* index, uint32_t precision, uint32_t rerank_width);
 
 /*
- * Candidates of the last exact low-precision search on this index (paths 2, 3 and 6; diagnostics
+ * Candidates of the last exact low-precision search on this index (paths 2, 3, 6 and 7; diagnostics
  * and error reports):
- * for each of `query_rows` queries, the k' rows ranked by approximate (BF16/FP8) score, with those
+ * for each of `query_rows` queries, the k' rows ranked by approximate (BF16/FP8/TF32) score, with those
  * approximate scores, the bound eps the exactness certificate used for this index's copy (max row
  * residual) and, per query, whether its certificate held (0 = re-run on the FP32 scan). Host
  * buffers of query_rows × k' entries (certified_out: query_rows); *kprime receives k'.
@@ -361,7 +363,7 @@ NNDEX_API int nndex_cuda_set_graphs(nndex_cuda_index* index, int enable);
  * The autotuner (replaces src/profiles.rs:65-185, which maps a shape to a CPU strategy by fixed
  * thresholds). mode 1 (the default): the first batch of each shape — exact or IVF, queries and k
  * rounded up to powers of two, nprobe and precision — runs every plan that returns the same
- * results (the FP32 scan or the TF32 candidate scan for small batches; BF16 or FP8 tensor-core
+ * results (the FP32 scan or a TF32 scan for FP32 batches; BF16 or FP8 tensor-core
  * scans with pass-1 tile strides 1, 8 and 32 for large ones; the FP32 or the tensor-core IVF list
  * scan, the latter with pass-1 strides 1, 2, 4 and 16), times each, and keeps the fastest for later
  * batches of that shape. mode 0: the fixed

@@ -66,7 +66,7 @@ bool parse_entry(const char* line, uint64_t* key, CudaIndex::TuneEntry* e) {
                         "shape ivf=%u nq=%llu k=%llu precision=%u nprobe=%u plan path=%d stride=%u qb=%u ms=%lf",
                         &ivf, &nq, &k, &prec, &nprobe, &path, &stride, &qb, &ms);
     if (n != 9 || ivf > 1 || !is_pow2(nq) || nq > kMaxBatchChunk || !is_pow2(k) || k > (1ull << 20) || prec > 3 ||
-        path < 1 || path > 6 || stride > 64 || qb > 3 || !(ms >= 0.0))
+        path < 1 || path > 7 || stride > 64 || qb > 3 || !(ms >= 0.0))
         return false;
     if (ivf ? (path != 4 && path != 5) : (path == 4 || path == 5)) return false;
     if (path == 4 && stride) return false;
@@ -187,9 +187,13 @@ std::vector<CudaIndex::TunePlan> CudaIndex::tune_candidates(uint64_t nq, uint64_
         return c;
     }
     const bool tf32 = plan_tf32(nq, kcap).kp != 0;
+    // From 17 queries the two-pass TF32 scan replaces the FP32 scan where its rule takes it (timing
+    // the FP32 scan beside it would cost more than it could ever save: 17 times as much on 10M × 256
+    // with 4,096 queries).
+    const int fp32_path = plan_tf32_batch(nq, kcap).kp ? 7 : 1;
     switch (precision) {
         case NNDEX_PRECISION_FP32:
-            c.push_back({1, 0});
+            c.push_back({fp32_path, 0});
             if (tf32) c.push_back({6, 0});
             break;
         case NNDEX_PRECISION_BF16:
@@ -201,7 +205,7 @@ std::vector<CudaIndex::TunePlan> CudaIndex::tune_candidates(uint64_t nq, uint64_
         }
         default:  // AUTO: the FP32 scans for small batches, the tensor cores beside them from 64
             if (nq <= 256) {
-                c.push_back({1, 0});
+                c.push_back({fp32_path, 0});
                 if (tf32) c.push_back({6, 0});
             }
             if (nq >= 64) {

@@ -421,7 +421,7 @@ int CudaIndex::choose_path(uint64_t nq, uint64_t kcap) const {
     // Small batches (plan_tf32's range): the TF32 candidate scan, which reads the same FP32 base and
     // returns the same bits as the FP32 scan at the HBM rate, where the FP32 scan is bound by its
     // FMA issue.
-    const int fp32_path = plan_tf32(nq, kcap).kp ? 6 : 1;
+    const int fp32_path = plan_tf32(nq, kcap).kp ? 6 : plan_tf32_batch(nq, kcap).kp ? 7 : 1;
     switch (precision) {
         case NNDEX_PRECISION_FP32: return fp32_path;
         case NNDEX_PRECISION_BF16: return (has16 && tc_ok(false)) ? 2 : 1;
@@ -466,6 +466,41 @@ CudaIndex::Tf32Plan CudaIndex::plan_tf32(uint64_t nq, uint64_t kcap) const {
     p.kp_cta = kp_cta;
     p.cap = cap;
     p.stages = stages;
+    return p;
+}
+
+// Batches of 17 queries and more of an FP32 index: the FP32 scan is bound by its FMAs there, the
+// tensor cores read the same base at the HBM rate.
+CudaIndex::Tf32BatchPlan CudaIndex::plan_tf32_batch(uint64_t nq, uint64_t kcap) const {
+    Tf32BatchPlan p;
+    static const bool off = [] {
+        const char* v = getenv("NNDEX_TF32_SCAN");  // 0: FP32 batches always take the FP32 scan
+        return v && v[0] == '0';
+    }();
+    if (off || !d_tfnorm || nq < 17 || kcap == 0 || kcap > kMaxGroupCandidates / 2) return p;
+    if (rows * ds * nq < kTf32BatchMinWork) return p;
+    const uint64_t kp = std::min<uint64_t>(rows, std::max<uint64_t>(32, 2 * kcap));
+    // Pass 1 on every stride-th tile: few enough that the groups of 8 rows are at least 16 per
+    // candidate, and that pass 2 collects about stride × k ≤ 2,048 rows per query.
+    const uint64_t tiles = (rows + 255) / 256;
+    uint32_t stride = 32;
+    while (stride > 1 && ((tiles + stride - 1) / stride * 32 < 16 * kp || stride * kcap > 2048 ||
+                          (stride > 8 && tiles < 16384)))
+        stride /= 2;
+    if (tiles * 32 < 4 * kp) return p;
+    const uint32_t nchunks = static_cast<uint32_t>(ds / 32);
+    // the query block resident beside at least three ring stages, else its slabs with every stage
+    uint32_t stages = tc_stages_for(nchunks, 0, false, false, smem_optin);
+    const bool stream_a = stages < 3;
+    if (stream_a) stages = tc_stages_for(nchunks, 0, false, true, smem_optin);
+    if (!stages) return p;
+    plan_groups(static_cast<uint32_t>((nq + 127) / 128), static_cast<uint32_t>(kp), stride, p.group, p.span, p.gm_tiles,
+                p.nranges, p.range_rows);
+    if (!p.group) return p;
+    p.stride = stride;
+    p.stages = stages;
+    p.stream_a = stream_a;
+    p.kp = static_cast<uint32_t>(kp);
     return p;
 }
 
@@ -616,28 +651,10 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     const uint32_t stride = (want > 1 && rows >= 256ull * 64) ? want : 1;
     uint64_t nranges = 0, range_rows = 0;
     tc_ranges(rows, nqb, nranges, range_rows);
-    // A sampled pass 1 writes group maxima instead of keeping heaps, its ranges split over the sampled
-    // tiles. Groups of 32 columns where a query has at least 64 of them per candidate (two of its best
-    // rows then rarely share one, which would lower T), of as many tiles as still leave 64 (fewer words
-    // to write, read and hold: 512 bytes per candidate at most, what the heaps' slots are admitted
-    // at); groups of 8 columns on smaller samples, and heaps where even those are fewer than four per
-    // candidate.
-    uint32_t gkp = stride > 1 ? group_candidates(kcap) : 0u, group = 0, gm_tiles = 0, span = 1;
-    if (gkp) {
-        const uint64_t sampled = ((rows + 255) / 256 + stride - 1) / stride;
-        uint64_t nr = 0, rr = 0;
-        tc_ranges(sampled * 256, nqb, nr, rr);
-        group = sampled * 8 >= 64ull * gkp ? 32u : (sampled * 32 >= 4ull * gkp ? 8u : 0u);
-        if (group) {
-            nranges = nr;
-            range_rows = rr * stride;
-            const uint64_t per_range = rr / 256;
-            while (group == 32 && span < kMaxGroupSpan && span * 2 <= per_range &&
-                   sampled * 8 >= 64ull * gkp * span * 2)
-                span *= 2;
-            gm_tiles = static_cast<uint32_t>((per_range + span - 1) / span);
-        }
-    }
+    // A sampled pass 1 writes group maxima instead of keeping heaps, where plan_groups finds enough.
+    const uint32_t gkp = stride > 1 ? group_candidates(kcap) : 0u;
+    uint32_t group = 0, gm_tiles = 0, span = 1;
+    if (gkp) plan_groups(nqb, gkp, stride, group, span, gm_tiles, nranges, range_rows);
     tc_groups = group != 0;
     const uint32_t kp = tc_groups ? gkp : plan.kp;
     const uint64_t gm_words = nranges * gm_tiles * (tc_groups ? 256 / group : 0);  // per query, 4 bytes each
@@ -676,7 +693,7 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
         a.p.gm_group = group;
         a.p.gm_span = span;
         scan_event_begin(s, ev_a);
-        e = launch_scan_tc(a, fp8, 2, s);
+        e = launch_scan_tc(a, fp8 ? kTcFp8 : kTcBf16, 2, s);
         scan_event_end(s, ev_a);
         if (e != cudaSuccess) return cuda_error(e, "tensor-core scan launch");
         TcThresholdArgs t;
@@ -721,7 +738,7 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     a.p.ws_keys = d_ws;
     a.p.tile_stride = stride;
     scan_event_begin(s, ev_a);
-    e = launch_scan_tc(a, fp8, 0, s);
+    e = launch_scan_tc(a, fp8 ? kTcFp8 : kTcBf16, 0, s);
     scan_event_end(s, ev_a);
     if (e != cudaSuccess) return cuda_error(e, "tensor-core scan launch");
     MergeArgs m;
@@ -756,11 +773,33 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     return NNDEX_OK;
 }
 
+// The groups of a sampled pass 1 (every stride-th tile) for kp candidates per query, and its ranges,
+// split over the sampled tiles. Groups of 32 columns where a query has at least 64 of them per
+// candidate (two of its best rows then rarely share one, which would lower T), of as many tiles as
+// still leave 64 (fewer words to write, read and hold: 512 bytes per candidate at most, what the
+// heaps' slots are admitted at); groups of 8 columns on smaller samples, and none (group 0, the ranges
+// as they were) where even those are fewer than four per candidate.
+void CudaIndex::plan_groups(uint32_t nqb, uint32_t kp, uint32_t stride, uint32_t& group, uint32_t& span,
+                            uint32_t& gm_tiles, uint64_t& nranges, uint64_t& range_rows) const {
+    const uint64_t sampled = ((rows + 255) / 256 + stride - 1) / stride;
+    group = sampled * 8 >= 64ull * kp ? 32u : (sampled * 32 >= 4ull * kp ? 8u : 0u);
+    span = 1;
+    if (!group) return;
+    uint64_t nr = 0, rr = 0;
+    tc_ranges(sampled * 256, nqb, nr, rr, 256);
+    const uint64_t per_range = rr / 256;
+    while (group == 32 && span < kMaxGroupSpan && span * 2 <= per_range && sampled * 8 >= 64ull * kp * span * 2) span *= 2;
+    nranges = nr;
+    range_rows = rr * stride;
+    gm_tiles = static_cast<uint32_t>((per_range + span - 1) / span);
+}
+
 // Row ranges of the tensor-core grid over `scan_rows` rows: about four waves of CTAs, each range a
 // multiple of the 256-row tile. Concurrent CTAs share ranges, so a base tile is read from HBM about
 // once.
-void CudaIndex::tc_ranges(uint64_t scan_rows, uint32_t nqb, uint64_t& nranges, uint64_t& range_rows) const {
-    tc_range_split(scan_rows, nqb, static_cast<uint64_t>(sm_count), nranges, range_rows);
+void CudaIndex::tc_ranges(uint64_t scan_rows, uint32_t nqb, uint64_t& nranges, uint64_t& range_rows,
+                          uint64_t min_rows) const {
+    tc_range_split(scan_rows, nqb, static_cast<uint64_t>(sm_count), nranges, range_rows, min_rows);
 }
 
 void CudaIndex::fill_tc_params(bool fp8, uint32_t n, uint64_t range_rows, TcParams& p) const {
@@ -879,7 +918,7 @@ int CudaIndex::enqueue_tc_pass2(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o
     a.live_items = 8u * static_cast<uint32_t>(sm_count) + static_cast<uint32_t>(n_alloc / 128) + 1u;
     cudaEvent_t ev_a = nullptr;
     scan_event_begin(s, ev_a);
-    e = launch_scan_tc(a, fp8, 1, s);
+    e = launch_scan_tc(a, fp8 ? kTcFp8 : kTcBf16, 1, s);
     scan_event_end(s, ev_a);
     if (e != cudaSuccess) return cuda_error(e, "tensor-core scan launch (pass 2)");
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, cap2, kcap,
@@ -947,7 +986,7 @@ int CudaIndex::retry_tc_pass2(bool fp8, uint32_t m, uint32_t kcap, uint64_t* o_i
     a.stages = plan2.stages;
     a.stream_a = plan2.stream_a;
     uint64_t nranges = 0, range_rows = 0;
-    tc_ranges(rows, (m + 127) / 128, nranges, range_rows);
+    tc_ranges(rows, (m + 127) / 128, nranges, range_rows, 256);
     a.nranges = static_cast<uint32_t>(nranges);
     fill_tc_params(fp8, m, range_rows, a.p);
     a.p.q_resid = d_q2_resid;
@@ -958,7 +997,7 @@ int CudaIndex::retry_tc_pass2(bool fp8, uint32_t m, uint32_t kcap, uint64_t* o_i
     a.p.cap2 = cap2;
     cudaEvent_t ev_a = nullptr;
     scan_event_begin(s, ev_a);
-    e = launch_scan_tc(a, fp8, 1, s);
+    e = launch_scan_tc(a, fp8 ? kTcFp8 : kTcBf16, 1, s);
     scan_event_end(s, ev_a);
     if (e != cudaSuccess) return cuda_error(e, "tensor-core scan launch (overflow)");
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_fbq, m, d_rows2, d_cnt2, cap2, kcap, d_q2_thr,
@@ -1022,7 +1061,6 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
         return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: no FP32 scan plan for k=%u", kcap);
     const uint64_t fb_per_query = static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap;
     if ((st = grow_device(d_ws, cap_ws, std::max(per_query, fb_per_query) * n, "scan workspace"))) return st;
-    if ((st = grow_device(d_qsub, cap_qsub, static_cast<uint64_t>(n) * ds, "fallback buffer"))) return st;
     if ((st = grow_device(d_fbq, cap_fbq, n, "fallback buffer"))) return st;
     if ((st = ensure_fbn())) return st;
     if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
@@ -1089,15 +1127,28 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     r.fb_count = d_fbn;
     cudaMemsetAsync(d_fbn, 0, sizeof(uint32_t), s);
     if ((e = launch_rerank(r, s)) != cudaSuccess) return cuda_error(e, "rerank launch");
-    // Uncertified queries re-run on the FP32 scan, on the device: the rerank listed them, then a
-    // gather, the scan and its merge (all return at once when every query certified), the merge
-    // writing each result into the query's own output row.
-    launch_gather_rows(d_qn, static_cast<uint32_t>(ds), d_fbq, d_fbn, n, d_qsub, s);
+    // Uncertified queries re-run on the FP32 scan, on the device: the rerank listed them.
+    if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
+    last_tc_n = n;
+    fbn_stream = s;
+    fbn_pending = true;
+    stats.kernel_launches += 5;
+    stats.path = 6;
+    stats.rerank_width = kp;
+    stats.rows_scanned += rows * n;
+    return NNDEX_OK;
+}
+
+// The scan reads the listed queries' rows, the merge writes each result into the query's own output
+// row; both return at once when none is listed.
+int CudaIndex::enqueue_fp32_fallback(const ScanPlan& plan, uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim,
+                                     uint32_t* o_cnt, cudaStream_t s) {
+    const uint64_t per_query = static_cast<uint64_t>(plan.ctas_per_group) * kcap;
     ScanArgs fa;
     fa.tmap = &tmap_f32;
     fa.tmap_tile = &tmap_f32_176;
     fa.tmap_112 = &tmap_f32_112;
-    fa.queries = d_qsub;
+    fa.queries = d_qn;
     fa.nq = n;
     fa.dq = static_cast<uint32_t>(ds);
     fa.rows = rows;
@@ -1105,11 +1156,13 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     fa.ws_keys = d_ws;
     fa.status = d_status;
     fa.live = d_fbn;
-    if ((e = launch_scan_fp32(fa, fb_plan, s)) != cudaSuccess) return cuda_error(e, "fallback scan launch");
+    fa.ids = d_fbq;
+    cudaError_t e;
+    if ((e = launch_scan_fp32(fa, plan, s)) != cudaSuccess) return cuda_error(e, "fallback scan launch");
     MergeArgs fm;
     fm.ws_keys = d_ws;
     fm.nq = n;
-    fm.per_query = fb_per_query;
+    fm.per_query = per_query;
     fm.k = kcap;
     fm.out_stride = kcap;
     fm.idx_out = o_idx;
@@ -1117,14 +1170,137 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     fm.count_out = o_cnt;
     fm.live = d_fbn;
     fm.out_rows = d_fbq;
-    if ((st = merge_workspace(fb_per_query, n, kcap, fm, s))) return st;
+    int st;
+    if ((st = merge_workspace(per_query, n, kcap, fm, s))) return st;
     if ((e = launch_merge_topk(fm, s)) != cudaSuccess) return cuda_error(e, "fallback merge launch");
+    return NNDEX_OK;
+}
+
+int CudaIndex::grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t kcap, uint64_t fb_keys) {
+    int st;
+    const uint64_t words = plan.nranges * plan.gm_tiles * (256 / plan.group);
+    if ((st = grow_device(d_ws, cap_ws, std::max((words + 1) / 2, fb_keys) * n, "scan workspace"))) return st;
+    if ((st = grow_device(d_q_resid, cap_q_resid, n, "query buffer"))) return st;
+    if ((st = grow_device(d_ids, cap_ids, n, "pass-2 buffer"))) return st;
+    if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * plan.kp, "tc workspace"))) return st;
+    if ((st = grow_device(d_cand_sim, cap_cand_sim, static_cast<uint64_t>(n) * plan.kp, "tc workspace"))) return st;
+    if ((st = grow_device(d_cand_cnt, cap_cand_cnt, n, "tc workspace"))) return st;
+    if ((st = grow_device(d_cert, cap_cert, n, "tc workspace"))) return st;
+    if ((st = grow_device(d_kth, cap_kth, n, "tc workspace"))) return st;
+    if ((st = grow_device(d_rows2, cap_rows2, static_cast<uint64_t>(n) * kSecondPassCap, "pass-2 buffer"))) return st;
+    if ((st = grow_device(d_cnt2, cap_cnt2, n, "pass-2 buffer"))) return st;
+    if ((st = grow_device(d_ok2, cap_ok2, n, "pass-2 buffer"))) return st;
+    if ((st = grow_device(d_rslots, cap_rslots, static_cast<uint64_t>(n) * rerank_chunks(kSecondPassCap) * kcap,
+                          "pass-2 buffer")))
+        return st;
+    if ((st = grow_device(d_fbq, cap_fbq, n, "fallback buffer"))) return st;
+    return ensure_fbn();
+}
+
+// Two-pass TF32 scan (FP32 indexes, 17 queries and more): K3's sampled pass 1 and collecting pass 2 on
+// the FP32 base itself, read as TF32 by the tensor cores, with K12's bound at the rows' largest norms
+// as every query's slack. The exact rerank sums in the FP32 scan's order, so rows and scores are the
+// FP32 scan's bit for bit; a query whose collection overflows is re-run on it, on the device.
+int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
+                                  cudaStream_t s) {
+    int st;
+    const Tf32BatchPlan plan = plan_tf32_batch(n, kcap);
+    ScanPlan fb_plan;
+    // (a tuned plan is shared by the shapes of a power of two, some of which the rule may not take)
+    if (!plan.kp || !plan_scan_fp32(n, static_cast<uint32_t>(ds), kcap, rows, sm_count, smem_optin, fb_plan))
+        return enqueue_exact_fp32(d_qn, n, kcap, kcap, o_idx, o_sim, o_cnt, s);
+    // The fallback usually has few queries: up to a CTA per SM for each group of 16, within 256 MB of keys.
+    const uint64_t fb_per = std::min<uint64_t>(static_cast<uint64_t>(sm_count), (32ull << 20) / (static_cast<uint64_t>(n) * kcap));
+    fb_plan.ctas_per_group = static_cast<uint32_t>(std::max<uint64_t>(fb_plan.ctas_per_group, fb_per));
+    if ((st = grow_tf32_batch(plan, n, kcap, static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap))) {
+        // without memory for the collections: the FP32 scan, whose workspace is far smaller
+        if (st != NNDEX_ERR_OUT_OF_MEMORY) return st;
+        cudaGetLastError();
+        clear_error();
+        return enqueue_exact_fp32(d_qn, n, kcap, kcap, o_idx, o_sim, o_cnt, s);
+    }
+    CUtensorMap tmap_q;  // the queries straight from the prepared buffer: rows past n read as zeros
+    if (!encode_tmap_2d(&tmap_q, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d_qn, ds, n, ds * sizeof(float), 32, 128,
+                        CU_TENSOR_MAP_SWIZZLE_128B))
+        return set_error(NNDEX_ERR_CUDA, "cuda execution error: cuTensorMapEncodeTiled failed (queries, driver "
+                                         "result %d)", last_encode_result());
+    cudaError_t e = launch_tf32_slack(d_qn, n, static_cast<uint32_t>(ds), d_tfnorm + rows, tf32_c_norm(), d_q_resid,
+                                      d_cnt2, kSecondPassCap + 1, d_fbn, s);
+    if (e != cudaSuccess) return cuda_error(e, "TF32 slack launch");
+    TcArgs a;
+    a.tmap_q = &tmap_q;
+    a.tmap_b = &tmap_f32_256;
+    a.stages = plan.stages;
+    a.stream_a = plan.stream_a;
+    a.nranges = static_cast<uint32_t>(plan.nranges);
+    a.p.nq = n;
+    a.p.nchunks = static_cast<uint32_t>(ds / 32);
+    a.p.rows = rows;
+    a.p.range_rows = plan.range_rows;
+    a.p.status = d_status;
+    a.p.q_resid = d_q_resid;
+    a.p.tile_stride = plan.stride;
+    a.p.gm = reinterpret_cast<uint32_t*>(d_ws);
+    a.p.gm_tiles = plan.gm_tiles;
+    a.p.gm_group = plan.group;
+    a.p.gm_span = plan.span;
+    cudaEvent_t ev_a = nullptr;
+    scan_event_begin(s, ev_a);
+    e = launch_scan_tc(a, kTcTf32, 2, s);
+    scan_event_end(s, ev_a);
+    if (e != cudaSuccess) return cuda_error(e, "TF32 scan launch");
+    TcThresholdArgs t;
+    t.gm = a.p.gm;
+    t.words = plan.nranges * plan.gm_tiles * (256 / plan.group);
+    t.group = plan.group;
+    t.tiles = plan.gm_tiles;
+    t.span = plan.span;
+    t.stride = plan.stride;
+    t.parts = plan.nranges;
+    t.range_rows = plan.range_rows;
+    t.rows = rows;
+    t.base = d_base;
+    t.ds = static_cast<uint32_t>(ds);
+    t.queries = d_qn;
+    t.nq = n;
+    t.kp = plan.kp;
+    t.k = kcap;
+    t.q_resid = d_q_resid;
+    t.whole_slack = true;
+    t.cand_idx = d_cand_idx;
+    t.cand_sim = d_cand_sim;
+    t.cand_cnt = d_cand_cnt;
+    t.cert = d_cert;
+    t.kth = d_kth;
+    t.ids = d_ids;
+    t.live = d_fbn + 1;
+    if ((e = launch_threshold(t, s)) != cudaSuccess) return cuda_error(e, "threshold launch");
+    uint64_t nranges = 0, range_rows = 0;
+    tc_ranges(rows, (n + 127) / 128, nranges, range_rows, 256);
+    a.nranges = static_cast<uint32_t>(nranges);
+    a.p.range_rows = range_rows;
+    a.p.tile_stride = 1;
+    a.p.q_thr = d_kth;
+    a.p.cand_rows = d_rows2;
+    a.p.cand_cnt = d_cnt2;
+    a.p.cap2 = kSecondPassCap;
+    scan_event_begin(s, ev_a);
+    e = launch_scan_tc(a, kTcTf32, 1, s);
+    scan_event_end(s, ev_a);
+    if (e != cudaSuccess) return cuda_error(e, "TF32 scan launch (pass 2)");
+    e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, kSecondPassCap, kcap,
+                                d_kth, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, nullptr, nullptr, nullptr, nullptr,
+                                nullptr, d_fbq, d_fbn);
+    if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
+    if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
     last_tc_n = n;
     fbn_stream = s;
     fbn_pending = true;
-    stats.kernel_launches += 6;
-    stats.path = 6;
-    stats.rerank_width = kp;
+    stats.kernel_launches += 8;
+    stats.path = 7;
+    stats.rerank_width = plan.kp;
+    stats.pass1_tile_stride = plan.stride;
+    stats.second_pass_queries += n;
     stats.rows_scanned += rows * n;
     return NNDEX_OK;
 }
@@ -1216,6 +1392,9 @@ int CudaIndex::enqueue_host_batch(uint64_t n, uint64_t kcap, int mode, int path)
     } else if (path == 6) {
         if ((st = enqueue_tf32(static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt, stream)))
             return st;
+    } else if (path == 7) {
+        if ((st = enqueue_tf32_batch(static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt, stream)))
+            return st;
     } else {
         if ((st = enqueue_tc(path == 3, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt,
                              stream)))
@@ -1238,10 +1417,10 @@ int CudaIndex::enqueue_host_batch(uint64_t n, uint64_t kcap, int mode, int path)
 // the capture); otherwise directly. No path needs a host decision in the middle of its batch: the
 // FP32 scan (1), the tensor-core scans (2, 3, 5: pass 2 and its compaction run on the device; the
 // rare FP32 re-run of an overflowed collection follows the batch), the IVF list scan (4) and the
-// TF32 candidate scan (6, its certificate's fallback on the device).
+// TF32 scans (6 and 7, their fallback on the device).
 int CudaIndex::run_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
     const bool graphable = use_graphs && !scan_timing && !error_report && !sync_check_enabled() &&
-                           path >= 1 && path <= 6 &&
+                           path >= 1 && path <= 7 &&
                            !(graph_failed_paths & (1u << path));
     if (!graphable) return enqueue_host_batch(n, kcap, mode, path);
     const uint64_t epoch = alloc_epoch();
@@ -1269,7 +1448,7 @@ int CudaIndex::run_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
         stats.ivf_rows_union = acc.ivf_rows_union;
         count_launch(static_cast<uint32_t>(graphs[i].launches));
         stats.graph = 2;
-        if (path == 6) {  // the replayed fallback's count is read back with the statistics
+        if (path == 6 || path == 7) {  // the replayed fallback's count is read back with the statistics
             fbn_stream = stream;
             fbn_pending = true;
         }
@@ -1409,12 +1588,10 @@ int CudaIndex::run_device_chunk(const float* dq, uint64_t n, uint64_t kcap, int 
         return ivf_finish_tc(*this, n32, k32, oi, os, oc, s);
     }
     if (path == 1) return enqueue_exact_fp32(d_qn, n32, k32, k32, oi, os, oc, s);
-    // the certificates' fallbacks need the host: these paths synchronise
+    if (path == 6) return enqueue_tf32(n32, k32, oi, os, oc, s);  // its fallback runs on the device
+    if (path == 7) return enqueue_tf32_batch(n32, k32, oi, os, oc, s);
+    // the overflowed collections' re-runs need the host: these paths synchronise
     *synced = true;
-    if (path == 6) {
-        *synced = false;  // the certificate's fallback runs on the device
-        return enqueue_tf32(n32, k32, oi, os, oc, s);
-    }
     if ((st = enqueue_tc(path == 3, n32, k32, oi, os, oc, s))) return st;
     if ((st = enqueue_tc_pass2(path == 3, n32, k32, oi, os, oc, s))) return st;
     cudaMemcpyAsync(h_fbn, d_fbn, kFbnBytes, cudaMemcpyDeviceToHost, s);
@@ -1740,7 +1917,9 @@ int index_finish(CudaIndex* ix) {
         !encode_tmap_2d(&ix->tmap_f32_176, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ix->d_base, ix->ds, ix->rows_alloc,
                         ix->ds * sizeof(float), 32, 176, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tmap_2d(&ix->tmap_f32_112, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ix->d_base, ix->ds, ix->rows_alloc,
-                        ix->ds * sizeof(float), 32, 112, CU_TENSOR_MAP_SWIZZLE_128B))
+                        ix->ds * sizeof(float), 32, 112, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_tmap_2d(&ix->tmap_f32_256, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ix->d_base, ix->ds, ix->rows_alloc,
+                        ix->ds * sizeof(float), 32, 256, CU_TENSOR_MAP_SWIZZLE_128B))
         return fail(set_error(NNDEX_ERR_CUDA, "cuda execution error: cuTensorMapEncodeTiled failed"));
     if (ix->d_base_bf16 &&
         (!encode_tmap_2d(&ix->tmap_bf16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ix->d_base_bf16, ix->kb16,
@@ -1762,9 +1941,11 @@ int index_finish(CudaIndex* ix) {
     }
     // Row norms of K12's bound (8 bytes per row, one pass over the base). Without them (no memory)
     // small batches take the FP32 scan.
-    if (cudaMalloc(&ix->d_tfnorm, ix->rows * sizeof(float2)) == cudaSuccess) {
+    if (cudaMalloc(&ix->d_tfnorm, (ix->rows + 1) * sizeof(float2)) == cudaSuccess) {
+        cudaMemsetAsync(ix->d_tfnorm + ix->rows, 0, sizeof(float2), ix->stream);
         if ((e = launch_tf32_row_norms(ix->d_base, ix->rows, static_cast<uint32_t>(ix->ds), ix->d_tfnorm,
-                                       static_cast<uint32_t>(ix->sm_count), ix->stream)) != cudaSuccess)
+                                       ix->d_tfnorm + ix->rows, static_cast<uint32_t>(ix->sm_count), ix->stream)) !=
+            cudaSuccess)
             return fail(cuda_error(e, "row norms launch"));
     } else {
         ix->d_tfnorm = nullptr;
@@ -1859,6 +2040,7 @@ int make_view(const CudaIndex& src, CudaIndex** out) {
     v->tmap_f32 = src.tmap_f32;
     v->tmap_f32_176 = src.tmap_f32_176;
     v->tmap_f32_112 = src.tmap_f32_112;
+    v->tmap_f32_256 = src.tmap_f32_256;
     v->precision = src.precision;
     v->kb16 = src.kb16;
     v->kf8 = src.kf8;
@@ -2098,7 +2280,7 @@ int nndex_cuda_last_candidates(nndex_cuda_index* index, uint64_t query_rows, uin
     const uint32_t kp = ix->stats.rerank_width;
     if (kprime) *kprime = kp;
     if (eps_rows)
-        *eps_rows = ix->stats.path == 3 ? ix->eps_fp8 : ix->stats.path == 6 ? ix->tf32_eps() : ix->eps_bf16;
+        *eps_rows = ix->stats.path == 3 ? ix->eps_fp8 : ix->stats.path >= 6 ? ix->tf32_eps() : ix->eps_bf16;
     if (kp == 0 || !ix->d_cand_idx) return set_error(NNDEX_ERR_INVALID_ARGUMENT, "cuda execution error: no low-precision search yet");
     if (ix->stats.path == 5)
         return set_error(NNDEX_ERR_UNSUPPORTED,

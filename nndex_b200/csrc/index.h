@@ -18,6 +18,14 @@ constexpr uint64_t kMaxBatchChunk = 16384;
 // Rows a pass-2 query may collect before it is re-run on the FP32 scan.
 constexpr uint32_t kSecondPassCap = 8192;
 
+// FP32 batches take the two-pass TF32 scan from this much work (rows × stored dims × queries). Its nine
+// launches cost about 45 us whatever the batch, the FP32 scan's FMAs about 20 us per 1e8 beyond its own
+// 50. Batches in a row through device buffers, FP32 scan against two-pass scan: 50k × 128 with 17
+// queries (1.1e8) 61 / 70 us, 32 (2.0e8) 66 / 71, 64 (4.1e8) 94 / 72, 256 (1.6e9) 216 / 78;
+// 5k × 768, 32 queries (1.2e8) 67 / 80; 300k × 100, 37 queries 232 / 111; 1M × 768, 256 queries
+// 11,410 / 962.
+constexpr uint64_t kTf32BatchMinWork = 250000000ull;
+
 // Incremented whenever a scratch or staging buffer of any index is (re)allocated: a captured
 // CUDA graph is valid only while the epoch it was captured in lasts.
 uint64_t alloc_epoch();
@@ -68,6 +76,7 @@ struct CudaIndex {
     CUtensorMap tmap_f32{};
     CUtensorMap tmap_f32_176{};  // box {32 floats, 176 rows}: the 11-warp wide FP32 scan's tiles
     CUtensorMap tmap_f32_112{};  // box {32 floats, 112 rows}: the 7-warp wide FP32 scan's tiles
+    CUtensorMap tmap_f32_256{};  // box {32 floats, 256 rows}: the two-pass TF32 scan's tiles
 
     // Low-precision scoring copies (NNDEX_FLAG_BF16 / NNDEX_FLAG_FP8), K3.
     uint32_t precision = NNDEX_PRECISION_AUTO;
@@ -89,7 +98,8 @@ struct CudaIndex {
     size_t cap_q_fp8 = 0;
     float* d_q_scale = nullptr;
     size_t cap_q_scale = 0;
-    float2* d_tfnorm = nullptr;  // K12: per row {‖x‖, ‖x − tf32_head(x)‖}, rounded up (shared by views)
+    float2* d_tfnorm = nullptr;  // TF32 scans: per row {‖x‖, ‖x − tf32_head(x)‖}, rounded up; the last
+                                 // entry (index rows) holds the largest of each (shared by views)
     float* d_q_resid = nullptr;
     size_t cap_q_resid = 0;
     unsigned long long* d_thr = nullptr;
@@ -261,7 +271,8 @@ struct CudaIndex {
     int run_device_chunk(const float* dq, uint64_t n, uint64_t kcap, int path, uint64_t* oi, float* os,
                          uint32_t* oc, cudaStream_t s, bool* synced);
     // Path choice for a batch: 1 = FP32 scan, 2 = BF16 tensor-core scan, 3 = FP8 tensor-core scan,
-    // 6 = TF32 tensor-core candidate scan + exact FP32 rerank (small batches of an FP32 index).
+    // 6 = TF32 tensor-core candidate scan + exact FP32 rerank (small batches of an FP32 index),
+    // 7 = two-pass TF32 tensor-core scan + exact FP32 rerank (its larger batches).
     int choose_path(uint64_t nq, uint64_t kcap) const;
     // K12's plan for k results: candidates per query and CTA (0: no plan), buffer, ring depth.
     struct Tf32Plan {
@@ -270,6 +281,16 @@ struct CudaIndex {
         uint32_t cap = 0, stages = 0;
     };
     Tf32Plan plan_tf32(uint64_t nq, uint64_t kcap) const;
+    // The two-pass TF32 scan's plan for larger FP32 batches (kp 0: none): sampled pass 1 with group
+    // maxima, then a collecting pass.
+    struct Tf32BatchPlan {
+        uint32_t kp = 0;  // candidates per query whose exact scores give T
+        uint32_t stride = 1, group = 0, span = 1, gm_tiles = 0;
+        uint64_t nranges = 0, range_rows = 0;  // pass 1
+        uint32_t stages = 0;
+        bool stream_a = false;
+    };
+    Tf32BatchPlan plan_tf32_batch(uint64_t nq, uint64_t kcap) const;
     float tf32_c_norm() const;  // C of K12's bound: ε = ‖q‖(‖d_x‖ + C‖x‖) + ‖d_q‖(‖x‖ + ‖d_x‖)
     float tf32_eps() const;     // the largest ε for unit rows and queries
     int ivf_path(uint64_t nq, uint64_t kcap) const;
@@ -308,7 +329,10 @@ struct CudaIndex {
     // kernel's lists do not hold it.
     uint32_t group_candidates(uint64_t kcap) const;
     uint32_t tc_chunks(bool fp8) const;
-    void tc_ranges(uint64_t scan_rows, uint32_t nqb, uint64_t& nranges, uint64_t& range_rows) const;
+    void plan_groups(uint32_t nqb, uint32_t kp, uint32_t stride, uint32_t& group, uint32_t& span, uint32_t& gm_tiles,
+                     uint64_t& nranges, uint64_t& range_rows) const;
+    void tc_ranges(uint64_t scan_rows, uint32_t nqb, uint64_t& nranges, uint64_t& range_rows,
+                   uint64_t min_rows = 2048) const;
     void fill_tc_params(bool fp8, uint32_t n, uint64_t range_rows, TcParams& p) const;
     int encode_query_tmap(bool fp8, void* buf, uint32_t n, CUtensorMap* map) const;
     int enqueue_prep_queries(const float* d_raw, uint64_t n, int mode, int path, cudaStream_t s);
@@ -328,6 +352,12 @@ struct CudaIndex {
     int retry_tc_pass2(bool fp8, uint32_t m, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
                        cudaStream_t s, std::vector<uint32_t>* failed);
     int enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
+    int enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
+    int grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t kcap, uint64_t fb_keys);
+    // The FP32 scan of the d_fbn[0] queries listed in d_fbq, into their own output rows (enqueued
+    // for up to n of them; its launches return at once when there are none).
+    int enqueue_fp32_fallback(const ScanPlan& plan, uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim,
+                              uint32_t* o_cnt, cudaStream_t s);
     // The FP32 scan for the listed queries (rows of d_qn), written into their output slots.
     int rerun_exact_fp32(const std::vector<uint32_t>& qs, uint32_t kcap, uint64_t* o_idx, float* o_sim,
                          uint32_t* o_cnt, cudaStream_t s);

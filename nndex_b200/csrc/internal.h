@@ -67,7 +67,10 @@ struct ScanArgs {
     const uint32_t* row_map = nullptr;  // optional: stored position → original row index
     uint64_t* ws_keys = nullptr;        // nq × ctas_per_group × k
     uint32_t* status = nullptr;
-    const uint32_t* live = nullptr;     // optional: a device count; 0 makes the whole launch return
+    // optional: a device count of the queries to run (a certificate's fallback; 0: the launch returns
+    // at once), and their rows in `queries`
+    const uint32_t* live = nullptr;
+    const uint32_t* ids = nullptr;
 };
 
 // Picks queries-per-CTA, grid and candidate capacity for (nq, dq, k) within the shared-memory
@@ -102,16 +105,18 @@ cudaError_t launch_merge_topk(const MergeArgs& a, cudaStream_t stream);
 // 256-row tiles, so the launch takes ceil(groups × ranges / sms) rounds of one range's tiles: the
 // split minimises that product over 1 to 8 rounds. (Four ranges per SM with 32 query blocks made
 // 608 CTAs on 148 SMs: 4.1 rounds, the fifth with 16 CTAs and 132 SMs idle.) A range holds at
-// least 2,048 rows. The host derives pass 1's grid with it, pass 2's CTAs from the live query count.
+// least min_rows rows: 2,048 where a CTA has its own set-up per range (heaps and their merge), one tile
+// where it has none (group maxima, collections), so that small bases still fill the SMs. The host
+// derives pass 1's grid with it, pass 2's CTAs from the live query count.
 __host__ __device__ inline void tc_range_split(uint64_t rows, uint64_t groups, uint64_t sms, uint64_t& nranges,
-                                               uint64_t& range_rows) {
+                                               uint64_t& range_rows, uint64_t min_rows = 2048) {
     const uint64_t tiles = (rows + 255) / 256;
     if (tiles == 0 || groups == 0 || sms == 0) {
         nranges = 1;
         range_rows = 256;
         return;
     }
-    uint64_t nr_max = (rows + 2047) / 2048;
+    uint64_t nr_max = (rows + min_rows - 1) / min_rows;
     if (nr_max < 1) nr_max = 1;
     uint64_t best_tpr = tiles, best_cost = ~0ull;
     for (uint64_t m = 1; m <= 8; ++m) {
@@ -129,6 +134,9 @@ __host__ __device__ inline void tc_range_split(uint64_t rows, uint64_t groups, u
     nranges = (rows + range_rows - 1) / range_rows;
 }
 
+// Operands of the tensor-core scan: the BF16 or the FP8 copy, or the FP32 base itself as TF32.
+enum TcType : int { kTcBf16 = 0, kTcFp8 = 1, kTcTf32 = 2 };
+
 struct TcParams {
     uint32_t nq = 0;
     uint32_t nchunks = 0;                 // K bytes / 128
@@ -144,7 +152,7 @@ struct TcParams {
     const float2* tile_scale = nullptr;   // FP8 only: per 256-row tile, {min, max} of its rows' scales
     const float* q_scale = nullptr;       // FP8 only
     const float* row_resid = nullptr;     // ‖x − x̂‖ per row
-    const float* q_resid = nullptr;       // ‖q − q̂‖ per query
+    const float* q_resid = nullptr;       // ‖q − q̂‖ per query (TF32: its largest bound slack)
     float eps_acc = 0.0f;                 // FP32 accumulation error bound
     float eps_rows = 0.0f;                // max ‖x − x̂‖ over the rows
     // group-maxima pass (mode 2): per query and row range (item mode: per output slot) gm_tiles × 256 /
@@ -200,7 +208,7 @@ uint32_t tc_pair_stages_for(uint32_t nchunks, bool fp8, size_t smem_limit);
 // Ring stages of a CTA-pair pass 2 (TcArgs::qb = 3) that fit, 0 when none does.
 uint32_t tc_cta_pair_stages_for(uint32_t nchunks, bool fp8, size_t smem_limit);
 // mode 0: pass 1 with heaps; 1: pass 2; 2: a sampled pass 1 that writes group maxima.
-cudaError_t launch_scan_tc(const TcArgs& a, bool fp8, int mode, cudaStream_t stream);
+cudaError_t launch_scan_tc(const TcArgs& a, int type, int mode, cudaStream_t stream);
 
 // T (and the candidates it came from) of a group-maxima pass; lists every query for pass 2.
 constexpr uint32_t kMaxGroupSpan = 64;          // 11 low bits of a score name its row
@@ -221,6 +229,7 @@ struct TcThresholdArgs {
     const float* q_resid = nullptr;
     const float* q_scale = nullptr;       // FP8 only
     float eps_rows = 0.0f, eps_acc = 0.0f;
+    bool whole_slack = false;             // TF32: q_resid is the whole slack
     uint64_t* cand_idx = nullptr;         // nq × kp, by approximate score
     float* cand_sim = nullptr;            // upper bounds of their exact scores
     uint32_t* cand_cnt = nullptr;
@@ -257,12 +266,18 @@ uint32_t tf32_stages_for(uint32_t cap, size_t smem_limit);
 // queries (nq rows; the rows past nq read as zeros), box {32 floats, 16 rows}, 128-byte swizzle.
 cudaError_t launch_scan_tf32(const CUtensorMap& tmap_x, const CUtensorMap& tmap_q, const Tf32ScanArgs& a,
                              uint32_t stages, uint32_t ctas, cudaStream_t stream);
-// Per row of the base (stride ds): {‖x‖, ‖x − tf32_head(x)‖}, FP64 sums rounded up.
-cudaError_t launch_tf32_row_norms(const float* base, uint64_t rows, uint32_t ds, float2* out, uint32_t sm_count,
-                                  cudaStream_t stream);
+// Per row of the base (stride ds): {‖x‖, ‖x − tf32_head(x)‖}, FP64 sums rounded up; and the largest of
+// each over the rows, raised into *max (zeroed before; non-negative floats order as their bits).
+cudaError_t launch_tf32_row_norms(const float* base, uint64_t rows, uint32_t ds, float2* out, float2* max,
+                                  uint32_t sm_count, cudaStream_t stream);
+// Per query (stride ds): the largest bound slack over all rows, ‖q‖(‖d_x‖ + C‖x‖) + ‖d_q‖(‖x‖ + ‖d_x‖) at
+// the rows' maxima, and collected[q] = 0. A query whose products could overflow FP32 gets an infinite
+// slack and over_cap in collected[q] (its collection then counts as overflowed). *over_count = 0.
+cudaError_t launch_tf32_slack(const float* queries, uint32_t nq, uint32_t ds, const float2* row_max, float c_norm,
+                              float* slack, uint32_t* collected, uint32_t over_cap, uint32_t* over_count,
+                              cudaStream_t stream);
 
-// Device-side certificate fallback: compaction of the zero flags (one block), a gather of their rows
-// (zeros past the count), and a scatter of re-run results back to their queries' slots.
+// Device-side certificate fallback: compaction of the zero flags (one block).
 struct CollectedSum {
     const uint32_t* cnt = nullptr;  // collected rows per query
     const uint32_t* by = nullptr;   // optional: cnt is indexed by[i] rather than i
@@ -271,11 +286,6 @@ struct CollectedSum {
 };
 void launch_compact_zero_flags(const uint32_t* flags, uint32_t n, uint32_t* ids, uint32_t* count, cudaStream_t s,
                                const uint32_t* live = nullptr, const CollectedSum& rows = CollectedSum{});
-void launch_gather_rows(const float* src, uint32_t ds, const uint32_t* ids, const uint32_t* count, uint32_t n,
-                        float* dst, cudaStream_t s);
-void launch_scatter_results(const uint64_t* fb_idx, const float* fb_sim, const uint32_t* fb_cnt, const uint32_t* ids,
-                            const uint32_t* count, uint32_t n, uint32_t k, uint64_t* idx, float* sim, uint32_t* cnt,
-                            cudaStream_t s);
 
 struct RerankArgs {
     const float* base = nullptr;  // FP32 base, stride ds (with row_map: the list-ordered copy)
@@ -311,13 +321,15 @@ cudaError_t launch_gather_queries(const uint32_t* ids, uint32_t m, const void* q
 // list-ordered copy by collected position. slot_keys: m × rerank_chunks(cap2) × k keys of scratch.
 // With fail (m positions in ids whose collections overflowed): the k-th exact score of the rows they
 // did collect is a higher T, written to kth (by query), and the queries to fail_ids; no results.
+// With over_ids: queries whose collection overflowed are appended there, counted in over_count.
 uint32_t rerank_chunks(uint32_t cap2);
 cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float* queries, const uint32_t* ids,
                                     uint32_t m, const uint32_t* rows2, const uint32_t* cnt2, uint32_t cap2, uint32_t k,
                                     const float* thr, uint64_t* slot_keys, uint64_t* idx_out, float* sim_out,
                                     uint32_t* cnt_out, uint32_t* ok_out, cudaStream_t stream, bool by_query = false,
                                     const uint32_t* live = nullptr, const uint32_t* row_map = nullptr,
-                                    const uint32_t* fail = nullptr, float* kth = nullptr, uint32_t* fail_ids = nullptr);
+                                    const uint32_t* fail = nullptr, float* kth = nullptr, uint32_t* fail_ids = nullptr,
+                                    uint32_t* over_ids = nullptr, uint32_t* over_count = nullptr);
 cudaError_t launch_max_reduce(const float* v, uint64_t n, unsigned int* out, cudaStream_t stream);
 // FP8: {min, max} row scale of each 256-row tile (tiles = rows_alloc / 256).
 void launch_tile_scale(const float* row_scale, uint64_t rows, uint64_t tiles, float2* out, cudaStream_t s);

@@ -45,8 +45,12 @@ __global__ void __launch_bounds__(ScanShape<QB, NCW>::kThreads, 1)
     scan_fp32_kernel(const __grid_constant__ CUtensorMap tmap, const float* __restrict__ queries, uint32_t nq,
                      uint32_t dq, uint64_t rows, uint32_t k, uint32_t cap,
                      const uint32_t* __restrict__ row_map, uint64_t* __restrict__ ws_keys,
-                     uint32_t* __restrict__ status, const uint32_t* __restrict__ live) {
-    if (live && *live == 0) return;  // a fallback launch with nothing to re-run
+                     uint32_t* __restrict__ status, const uint32_t* __restrict__ live,
+                     const uint32_t* __restrict__ ids) {
+    if (live) {  // a fallback launch: only the queries to re-run
+        if (*live < nq) nq = *live;
+        if (blockIdx.y * QB >= nq) return;
+    }
     using S = ScanShape<QB, NCW>;
     using Consumer = ScanConsumer<QB, NCW, ST>;
     constexpr int TR = S::kTileRows;
@@ -92,7 +96,7 @@ __global__ void __launch_bounds__(ScanShape<QB, NCW>::kThreads, 1)
     }
     for (uint32_t i = tid; i < static_cast<uint32_t>(QB) * dq; i += blockDim.x) {
         const uint32_t b = i / dq, d = i - b * dq;
-        q_s[i] = b < nqg ? queries[static_cast<size_t>(q0 + b) * dq + d] : 0.0f;
+        q_s[i] = b < nqg ? queries[static_cast<size_t>(ids ? ids[q0 + b] : q0 + b) * dq + d] : 0.0f;
     }
     if (tid < static_cast<uint32_t>(QB)) {
         cnt[tid] = 0;
@@ -166,8 +170,12 @@ __global__ void __launch_bounds__((W + 1) * 32, 1)
     scan_fp32_wide_kernel(const __grid_constant__ CUtensorMap tmap, const float* __restrict__ queries, uint32_t nq,
                           uint32_t dq, uint64_t rows, uint32_t k, uint32_t cap,
                           const uint32_t* __restrict__ row_map, uint64_t* __restrict__ ws_keys,
-                          uint32_t* __restrict__ status, const uint32_t* __restrict__ live) {
-    if (live && *live == 0) return;  // a fallback launch with nothing to re-run
+                          uint32_t* __restrict__ status, const uint32_t* __restrict__ live,
+                     const uint32_t* __restrict__ ids) {
+    if (live) {  // a fallback launch: only the queries to re-run
+        if (*live < nq) nq = *live;
+        if (blockIdx.y * QB >= nq) return;
+    }
     using Consumer = ScanConsumerWide<QB, W, ST>;
     constexpr int TR = Consumer::kTileRows;
     constexpr uint32_t kStageBytes = Consumer::kStageBytes;
@@ -213,7 +221,8 @@ __global__ void __launch_bounds__((W + 1) * 32, 1)
     // queries slab-major (ScanConsumerWide::q_slab_index)
     for (uint32_t i = tid; i < static_cast<uint32_t>(QB) * dq; i += blockDim.x) {
         const uint32_t b = i / dq, d = i - b * dq;
-        q_s[Consumer::q_slab_index(b, d)] = b < nqg ? queries[static_cast<size_t>(q0 + b) * dq + d] : 0.0f;
+        q_s[Consumer::q_slab_index(b, d)] =
+            b < nqg ? queries[static_cast<size_t>(ids ? ids[q0 + b] : q0 + b) * dq + d] : 0.0f;
     }
     if (tid < static_cast<uint32_t>(QB)) {
         cnt[tid] = 0;
@@ -498,7 +507,7 @@ cudaError_t launch_qb_st(const ScanArgs& a, const ScanPlan& p, cudaStream_t stre
     if (e != cudaSuccess) return e;
     dim3 grid(p.ctas_per_group, p.groups);
     kern<<<grid, ScanShape<QB, kNcw>::kThreads, p.smem_bytes, stream>>>(*a.tmap, a.queries, a.nq, a.dq, a.rows, a.k, p.cap,
-                                                              a.row_map, a.ws_keys, a.status, a.live);
+                                                              a.row_map, a.ws_keys, a.status, a.live, a.ids);
     count_launch();
     return cudaGetLastError();
 }
@@ -530,7 +539,7 @@ cudaError_t launch_wide_st(const ScanArgs& a, const ScanPlan& p, cudaStream_t st
     if (!tm) return cudaErrorInvalidValue;
     dim3 grid(p.ctas_per_group, p.groups);
     kern<<<grid, (W + 1) * 32, p.smem_bytes, stream>>>(*tm, a.queries, a.nq, a.dq, a.rows, a.k, p.cap, a.row_map,
-                                                       a.ws_keys, a.status, a.live);
+                                                       a.ws_keys, a.status, a.live, a.ids);
     count_launch();
     return cudaGetLastError();
 }

@@ -202,16 +202,20 @@ NNDEX_DEVICE_INLINE void epi_survivor(const TcParams& p, EpiState& st, uint64_t*
 // need about 470); on 2M x 512 in FP8 with 1,000 queries at k = 100, stride 8, 1,977 us -> 200 (the
 // heaps also pushed the query slabs out of shared memory); the IVF list scan of 1,024 queries over
 // 2M x 384, 32 of 1,414 lists, stride 4, 339 us -> 142.
-template <bool kFp8, int kST, int kMode, bool kStreamA, bool kItems, int kQB, bool kPair = false>
+// kT = kTcTf32 (modes 1 and 2): the FP32 base and queries themselves, read by kind::tf32 MMAs (sign,
+// exponent, top 10 mantissa bits); p.q_resid then holds each query's whole bound slack.
+template <int kT, int kST, int kMode, bool kStreamA, bool kItems, int kQB, bool kPair = false>
 __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
     scan_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_b,
                    const TcParams p) {
+    constexpr bool kFp8 = kT == kTcFp8, kTf32 = kT == kTcTf32;
+    static_assert(!kTf32 || (kMode != 0 && !kItems && kQB == 1 && !kPair), "TF32: exact scans without heaps");
     static_assert(kQB == 1 || (kQB == 2 && kMode == 1 && !kStreamA && !kItems), "two query blocks: pass 2 only");
     static_assert(!kPair || (kQB == 1 && kMode == 1 && !kStreamA && !kItems), "CTA pairs: pass 2 only");
     constexpr uint32_t kNT = kQB == 2 ? kN / 2 : kN;  // base rows per tile (MMA N)
     constexpr uint32_t kLoadRows = kPair ? kN / 2 : kNT;  // base rows per tile this CTA loads
     constexpr uint32_t kQC = kM * kQB;                // queries per CTA
-    constexpr uint32_t kElems = kFp8 ? 128 : 64;      // K elements per 128-byte slab
+    constexpr uint32_t kElems = kFp8 ? 128 : kTf32 ? 32 : 64;  // K elements per 128-byte slab
     constexpr uint32_t kStage = kStreamA ? kAChunk + kBChunk : kLoadRows * 128;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align_1024(smem_raw);
@@ -458,7 +462,8 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
     } else if (warp == 1) {
         // ---------------- MMA issuer (pairs: the even CTA's, for both) ----------------
         if (lane == 0 && leader) {
-            constexpr uint32_t idesc = tc::instr_desc<kFp8, kPair ? 2 * kM : kM, kNT>();
+            constexpr uint32_t idesc =
+                kTf32 ? tc::instr_desc_tf32<kM, kNT>() : tc::instr_desc<kFp8, kPair ? 2 * kM : kM, kNT>();
             const uint32_t a_addr0 = smem_u32(a_smem), b_addr0 = smem_u32(b_smem);
             uint32_t it = 0, tg = 0;  // slabs and tiles over all of the CTA's work
             for (uint32_t j = 0;; ++j) {
@@ -515,6 +520,10 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                                         tc::mma_pair<kFp8>(d, tc::smem_desc_sw128(a_addr + kk * 32),
                                                            tc::smem_desc_sw128(b_addr + kk * 32), idesc,
                                                            (c | kk) != 0u ? 1u : 0u);
+                                    else if constexpr (kTf32)
+                                        tc::mma_tf32(d, tc::smem_desc_sw128(a_addr + kk * 32),
+                                                     tc::smem_desc_sw128(b_addr + kk * 32), idesc,
+                                                     (c | kk) != 0u ? 1u : 0u);
                                     else
                                         tc::mma<kFp8>(d + b * kNT, tc::smem_desc_sw128(a_addr + kk * 32),
                                                       tc::smem_desc_sw128(b_addr + kk * 32), idesc,
@@ -582,7 +591,7 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
             const float qs = (kFp8 && kMode != 2 && valid_q) ? p.q_scale[q] : 1.0f;
             const float rq = (kMode != 2 && valid_q) ? p.q_resid[q] : 0.0f;
             const float b_mul = 1.0f + rq, b_add = rq + p.eps_acc;
-            const float slack = fmaf(p.eps_rows, b_mul, b_add);  // the largest u_r − s̃_r over all rows
+            const float slack = kTf32 ? rq : fmaf(p.eps_rows, b_mul, b_add);  // the largest u_r − s̃_r over all rows
             EpiState st;
             st.n = 0;
             if (kMode == 0) {
@@ -998,7 +1007,7 @@ __global__ void __launch_bounds__(kThrThreads) threshold_kernel(const TcThreshol
     // last place low, under span·2⁻¹⁸ of its magnitude) plus the largest slack
     const float low = static_cast<float>(a.span) * 7.62939453125e-06f;
     const float rq = a.q_resid[q], qs = a.q_scale ? a.q_scale[q] : 1.0f;
-    const float slack = fmaf(a.eps_rows, 1.0f + rq, rq + a.eps_acc);
+    const float slack = a.whole_slack ? rq : fmaf(a.eps_rows, 1.0f + rq, rq + a.eps_acc);
     const uint32_t ch = tid & 7u, nbox = a.ds / 32;
     for (uint32_t j0 = 0; j0 < p2k; j0 += NT / 8) {
         const uint32_t j = j0 + (tid >> 3);
@@ -1149,7 +1158,8 @@ __global__ void __launch_bounds__(256)
                         uint32_t k, int by_query, const uint32_t* __restrict__ live,
                         const uint64_t* __restrict__ slot_keys, uint32_t chunks, uint64_t* __restrict__ idx_out,
                         float* __restrict__ sim_out, uint32_t* __restrict__ cnt_out, uint32_t* __restrict__ ok_out,
-                        const uint32_t* __restrict__ fail, float* __restrict__ kth, uint32_t* __restrict__ fail_ids) {
+                        const uint32_t* __restrict__ fail, float* __restrict__ kth, uint32_t* __restrict__ fail_ids,
+                        uint32_t* __restrict__ over_ids, uint32_t* __restrict__ over_count) {
     extern __shared__ uint64_t keys[];  // chunks·k keys, at least p2(k)
     __shared__ BlockSelectScratch sel;
     const uint32_t i = blockIdx.x;
@@ -1159,7 +1169,10 @@ __global__ void __launch_bounds__(256)
     uint32_t total = cnt2[by_query ? q : at0];
     if (fail && total > cap2) total = cap2;
     if (total > cap2) {  // the collected set overflowed: finish_tc raises the query's T, or re-runs it
-        if (threadIdx.x == 0) ok_out[i] = 0;
+        if (threadIdx.x == 0) {
+            ok_out[i] = 0;
+            if (over_ids) over_ids[atomicAdd(over_count, 1u)] = q;
+        }
         return;
     }
     const uint32_t items = (total + kRerankChunk - 1) / kRerankChunk;
@@ -1204,12 +1217,12 @@ __global__ void __launch_bounds__(256)
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
-template <bool kFp8, int kST, int kMode, bool kStreamA, bool kItems = false, int kQB = 1, bool kPair = false>
+template <int kT, int kST, int kMode, bool kStreamA, bool kItems = false, int kQB = 1, bool kPair = false>
 static cudaError_t launch_tc_impl(const TcArgs& a, cudaStream_t stream) {
-    auto kern = scan_tc_kernel<kFp8, kST, kMode, kStreamA, kItems, kQB, kPair>;
+    auto kern = scan_tc_kernel<kT, kST, kMode, kStreamA, kItems, kQB, kPair>;
     const uint32_t kp = kMode == 0 ? a.p.kprime : 0;
     if (kMode == 0 && (a.p.heap_k == 0 || a.p.heap_k > kp)) return cudaErrorInvalidValue;
-    const size_t smem = tc_smem_bytes(a.p.nchunks, kp, kST, kFp8, kStreamA, kPair ? 3 : kQB);
+    const size_t smem = tc_smem_bytes(a.p.nchunks, kp, kST, kT == kTcFp8, kStreamA, kPair ? 3 : kQB);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     dim3 grid = kItems ? dim3(a.items, 1)
@@ -1223,9 +1236,9 @@ static cudaError_t launch_tc_impl(const TcArgs& a, cudaStream_t stream) {
     TcParams p = a.p;
     p.kprime = kp;
     if (sync_check_enabled())
-        set_launch_note("scan_tc fp8 %d stages %d mode %d stream_a %d items %d query blocks %d: grid (%u, %u), nq %u, "
+        set_launch_note("scan_tc type %d stages %d mode %d stream_a %d items %d query blocks %d: grid (%u, %u), nq %u, "
                         "k' %u, tile stride %u, range rows %llu, rows %llu, smem %zu",
-                        kFp8, kST, kMode, kStreamA, kItems, kQB, grid.x, grid.y, p.nq, kp, p.tile_stride,
+                        kT, kST, kMode, kStreamA, kItems, kQB, grid.x, grid.y, p.nq, kp, p.tile_stride,
                         (unsigned long long)p.range_rows, (unsigned long long)p.rows, smem);
     if (kPair) {
         cudaLaunchConfig_t cfg = {};
@@ -1249,12 +1262,12 @@ static cudaError_t launch_tc_impl(const TcArgs& a, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <bool kFp8, int kMode, bool kStreamA>
+template <int kT, int kMode, bool kStreamA>
 static cudaError_t launch_tc_stages(const TcArgs& a, cudaStream_t stream) {
     switch (a.stages) {
-        case 4: return launch_tc_impl<kFp8, 4, kMode, kStreamA>(a, stream);
-        case 3: return launch_tc_impl<kFp8, 3, kMode, kStreamA>(a, stream);
-        case 2: return launch_tc_impl<kFp8, 2, kMode, kStreamA>(a, stream);
+        case 4: return launch_tc_impl<kT, 4, kMode, kStreamA>(a, stream);
+        case 3: return launch_tc_impl<kT, 3, kMode, kStreamA>(a, stream);
+        case 2: return launch_tc_impl<kT, 2, kMode, kStreamA>(a, stream);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -1263,17 +1276,26 @@ static cudaError_t launch_tc_stages(const TcArgs& a, cudaStream_t stream) {
 template <int kMode, bool kStreamA>
 static cudaError_t launch_tc_items(const TcArgs& a, cudaStream_t stream) {
     switch (a.stages) {
-        case 4: return launch_tc_impl<false, 4, kMode, kStreamA, true>(a, stream);
-        case 3: return launch_tc_impl<false, 3, kMode, kStreamA, true>(a, stream);
-        case 2: return launch_tc_impl<false, 2, kMode, kStreamA, true>(a, stream);
+        case 4: return launch_tc_impl<kTcBf16, 4, kMode, kStreamA, true>(a, stream);
+        case 3: return launch_tc_impl<kTcBf16, 3, kMode, kStreamA, true>(a, stream);
+        case 2: return launch_tc_impl<kTcBf16, 2, kMode, kStreamA, true>(a, stream);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t launch_scan_tc(const TcArgs& a, bool fp8, int mode, cudaStream_t stream) {
+cudaError_t launch_scan_tc(const TcArgs& a, int type, int mode, cudaStream_t stream) {
+    const bool fp8 = type == kTcFp8;
     if (mode == 2 && (!a.p.gm || a.p.gm_tiles == 0 || (a.p.gm_group != 8 && a.p.gm_group != 32) || a.qb != 1 ||
                       a.p.gm_span == 0 || (a.p.gm_span & (a.p.gm_span - 1)) || a.p.gm_span > kMaxGroupSpan))
         return cudaErrorInvalidValue;
+    if (type == kTcTf32) {
+        if (a.items || a.qb != 1) return cudaErrorInvalidValue;
+        if (mode == 1)
+            return a.stream_a ? launch_tc_stages<kTcTf32, 1, true>(a, stream) : launch_tc_stages<kTcTf32, 1, false>(a, stream);
+        if (mode == 2)
+            return a.stream_a ? launch_tc_stages<kTcTf32, 2, true>(a, stream) : launch_tc_stages<kTcTf32, 2, false>(a, stream);
+        return cudaErrorInvalidValue;
+    }
     if (a.items) {
         if (fp8 || a.items > 0x7FFFFFFFu) return cudaErrorInvalidValue;
         if (mode == 2) return a.stream_a ? launch_tc_items<2, true>(a, stream) : launch_tc_items<2, false>(a, stream);
@@ -1283,34 +1305,34 @@ cudaError_t launch_scan_tc(const TcArgs& a, bool fp8, int mode, cudaStream_t str
     if (mode == 1 && a.qb == 2) {
         if (a.stream_a || a.p.range_rows % kN) return cudaErrorInvalidValue;
         switch (a.stages) {
-            case 5: return fp8 ? launch_tc_impl<true, 5, 1, false, false, 2>(a, stream)
-                               : launch_tc_impl<false, 5, 1, false, false, 2>(a, stream);
-            case 4: return fp8 ? launch_tc_impl<true, 4, 1, false, false, 2>(a, stream)
-                               : launch_tc_impl<false, 4, 1, false, false, 2>(a, stream);
+            case 5: return fp8 ? launch_tc_impl<kTcFp8, 5, 1, false, false, 2>(a, stream)
+                               : launch_tc_impl<kTcBf16, 5, 1, false, false, 2>(a, stream);
+            case 4: return fp8 ? launch_tc_impl<kTcFp8, 4, 1, false, false, 2>(a, stream)
+                               : launch_tc_impl<kTcBf16, 4, 1, false, false, 2>(a, stream);
             default: return cudaErrorInvalidValue;
         }
     }
     if (mode == 1 && a.qb == 3) {
         if (a.stream_a || a.p.range_rows % kN) return cudaErrorInvalidValue;
         switch (a.stages) {
-            case 8: return fp8 ? launch_tc_impl<true, 8, 1, false, false, 1, true>(a, stream)
-                               : launch_tc_impl<false, 8, 1, false, false, 1, true>(a, stream);
-            case 6: return fp8 ? launch_tc_impl<true, 6, 1, false, false, 1, true>(a, stream)
-                               : launch_tc_impl<false, 6, 1, false, false, 1, true>(a, stream);
+            case 8: return fp8 ? launch_tc_impl<kTcFp8, 8, 1, false, false, 1, true>(a, stream)
+                               : launch_tc_impl<kTcBf16, 8, 1, false, false, 1, true>(a, stream);
+            case 6: return fp8 ? launch_tc_impl<kTcFp8, 6, 1, false, false, 1, true>(a, stream)
+                               : launch_tc_impl<kTcBf16, 6, 1, false, false, 1, true>(a, stream);
             default: return cudaErrorInvalidValue;
         }
     }
     if (a.qb != 1) return cudaErrorInvalidValue;
     if (mode == 2) {
-        if (a.stream_a) return fp8 ? launch_tc_stages<true, 2, true>(a, stream) : launch_tc_stages<false, 2, true>(a, stream);
-        return fp8 ? launch_tc_stages<true, 2, false>(a, stream) : launch_tc_stages<false, 2, false>(a, stream);
+        if (a.stream_a) return fp8 ? launch_tc_stages<kTcFp8, 2, true>(a, stream) : launch_tc_stages<kTcBf16, 2, true>(a, stream);
+        return fp8 ? launch_tc_stages<kTcFp8, 2, false>(a, stream) : launch_tc_stages<kTcBf16, 2, false>(a, stream);
     }
     if (mode == 0) {
-        if (a.stream_a) return fp8 ? launch_tc_stages<true, 0, true>(a, stream) : launch_tc_stages<false, 0, true>(a, stream);
-        return fp8 ? launch_tc_stages<true, 0, false>(a, stream) : launch_tc_stages<false, 0, false>(a, stream);
+        if (a.stream_a) return fp8 ? launch_tc_stages<kTcFp8, 0, true>(a, stream) : launch_tc_stages<kTcBf16, 0, true>(a, stream);
+        return fp8 ? launch_tc_stages<kTcFp8, 0, false>(a, stream) : launch_tc_stages<kTcBf16, 0, false>(a, stream);
     }
-    if (a.stream_a) return fp8 ? launch_tc_stages<true, 1, true>(a, stream) : launch_tc_stages<false, 1, true>(a, stream);
-    return fp8 ? launch_tc_stages<true, 1, false>(a, stream) : launch_tc_stages<false, 1, false>(a, stream);
+    if (a.stream_a) return fp8 ? launch_tc_stages<kTcFp8, 1, true>(a, stream) : launch_tc_stages<kTcBf16, 1, true>(a, stream);
+    return fp8 ? launch_tc_stages<kTcFp8, 1, false>(a, stream) : launch_tc_stages<kTcBf16, 1, false>(a, stream);
 }
 
 cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t stream) {
@@ -1378,7 +1400,7 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
                                     const float* thr, uint64_t* slot_keys, uint64_t* idx_out, float* sim_out,
                                     uint32_t* cnt_out, uint32_t* ok_out, cudaStream_t stream, bool by_query,
                                     const uint32_t* live, const uint32_t* row_map, const uint32_t* fail, float* kth,
-                                    uint32_t* fail_ids) {
+                                    uint32_t* fail_ids, uint32_t* over_ids, uint32_t* over_count) {
     if (m == 0) return cudaSuccess;
     const uint32_t chunks = rerank_chunks(cap2);
     if (k == 0 || k > kRerankChunk || chunks > 65535u) return cudaErrorInvalidValue;
@@ -1397,15 +1419,14 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     kern<<<m, 256, smem, stream>>>(ids, cnt2, cap2, k, by_query ? 1 : 0, live, slot_keys, chunks, idx_out, sim_out,
-                                   cnt_out, ok_out, fail, kth, fail_ids);
+                                   cnt_out, ok_out, fail, kth, fail_ids, over_ids, over_count);
     count_launch(2);
     return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------------
-// Device-side fallback of a certificate: the queries whose certificate failed are compacted,
-// gathered, re-run on the FP32 scan (whose launch returns at once when there are none) and their
-// results scattered back, all on the stream, with no host round trip.
+// Device-side fallback of a certificate: the queries whose certificate failed are compacted for the
+// pass that follows (whose launch returns at once when there are none), with no host round trip.
 // ------------------------------------------------------------------------------------------
 
 // One block of 1024 threads: ids[0..m) = the indices i < n with flags[i] == 0, in order; count[0] = m.
@@ -1460,52 +1481,9 @@ __global__ void __launch_bounds__(1024) compact_zero_flags_kernel(const uint32_t
     }
 }
 
-// Row i of dst (stride ds floats) = row ids[i] of src for i < count[0], zeros for the rest of n.
-__global__ void gather_rows_kernel(const float* __restrict__ src, uint32_t ds, const uint32_t* __restrict__ ids,
-                                   const uint32_t* __restrict__ count, float* __restrict__ dst) {
-    const uint32_t i = blockIdx.x;
-    float4* d = reinterpret_cast<float4*>(dst + static_cast<size_t>(i) * ds);
-    if (i >= count[0]) {
-        for (uint32_t t = threadIdx.x; t < ds / 4; t += blockDim.x) d[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
-    }
-    const float4* a = reinterpret_cast<const float4*>(src + static_cast<size_t>(ids[i]) * ds);
-    for (uint32_t t = threadIdx.x; t < ds / 4; t += blockDim.x) d[t] = a[t];
-}
-
-// The results of re-run query i (< count[0]) into the slots of query ids[i].
-__global__ void scatter_results_kernel(const uint64_t* __restrict__ fb_idx, const float* __restrict__ fb_sim,
-                                       const uint32_t* __restrict__ fb_cnt, const uint32_t* __restrict__ ids,
-                                       const uint32_t* __restrict__ count, uint32_t k, uint64_t* __restrict__ idx,
-                                       float* __restrict__ sim, uint32_t* __restrict__ cnt) {
-    const uint32_t i = blockIdx.x;
-    if (i >= count[0]) return;
-    const uint32_t q = ids[i];
-    for (uint32_t j = threadIdx.x; j < k; j += blockDim.x) {
-        idx[static_cast<size_t>(q) * k + j] = fb_idx[static_cast<size_t>(i) * k + j];
-        sim[static_cast<size_t>(q) * k + j] = fb_sim[static_cast<size_t>(i) * k + j];
-    }
-    if (threadIdx.x == 0 && cnt) cnt[q] = fb_cnt[i];
-}
-
 void launch_compact_zero_flags(const uint32_t* flags, uint32_t n, uint32_t* ids, uint32_t* count, cudaStream_t s,
                                const uint32_t* live, const CollectedSum& rows) {
     compact_zero_flags_kernel<<<1, 1024, 0, s>>>(flags, n, ids, count, live, rows);
-    count_launch();
-}
-
-void launch_gather_rows(const float* src, uint32_t ds, const uint32_t* ids, const uint32_t* count, uint32_t n,
-                        float* dst, cudaStream_t s) {
-    if (n == 0) return;
-    gather_rows_kernel<<<n, 128, 0, s>>>(src, ds, ids, count, dst);
-    count_launch();
-}
-
-void launch_scatter_results(const uint64_t* fb_idx, const float* fb_sim, const uint32_t* fb_cnt, const uint32_t* ids,
-                            const uint32_t* count, uint32_t n, uint32_t k, uint64_t* idx, float* sim, uint32_t* cnt,
-                            cudaStream_t s) {
-    if (n == 0) return;
-    scatter_results_kernel<<<n, 128, 0, s>>>(fb_idx, fb_sim, fb_cnt, ids, count, k, idx, sim, cnt);
     count_launch();
 }
 

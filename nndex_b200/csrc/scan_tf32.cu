@@ -302,23 +302,62 @@ __global__ void __launch_bounds__(kTfThreads, 1)
     }
 }
 
-// Per row of the base: {‖x‖, ‖x − tf32_head(x)‖}, rounded up (one warp per row).
+// Per row of the base: {‖x‖, ‖x − tf32_head(x)‖}, rounded up (one warp per row), and their maxima (a
+// NaN norm, of an overflowing sum, compares above every finite one as bits).
 __global__ void tf32_row_norms_kernel(const float* __restrict__ base, uint64_t rows, uint32_t ds,
-                                      float2* __restrict__ out) {
+                                      float2* __restrict__ out, float2* __restrict__ max) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t w0 = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nw = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+    uint32_t mx = 0, my = 0;
     for (uint64_t r = w0; r < rows; r += nw) {
         const float2 n = warp_tf32_norms(base + r * ds, ds, lane);
         if (lane == 0) out[r] = n;
+        mx = ::max(mx, __float_as_uint(n.x));
+        my = ::max(my, __float_as_uint(n.y));
+    }
+    if (lane == 0 && w0 < rows) {
+        atomicMax(reinterpret_cast<unsigned int*>(&max->x), mx);
+        atomicMax(reinterpret_cast<unsigned int*>(&max->y), my);
     }
 }
 
-cudaError_t launch_tf32_row_norms(const float* base, uint64_t rows, uint32_t ds, float2* out, uint32_t sm_count,
-                                  cudaStream_t stream) {
+// One warp per query: its norms, then the bound of |s̃ − the FP32 scan's score| over all rows.
+__global__ void tf32_slack_kernel(const float* __restrict__ queries, uint32_t nq, uint32_t ds,
+                                  const float2* __restrict__ row_max, float c_norm, float* __restrict__ slack,
+                                  uint32_t* __restrict__ collected, uint32_t over_cap,
+                                  uint32_t* __restrict__ over_count) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (q >= nq) return;
+    const float2 n = warp_tf32_norms(queries + static_cast<size_t>(q) * ds, ds, lane);
+    if (lane != 0) return;
+    const float2 x = *row_max;
+    // the last term: products and operands below FP32's normal range, which either side may flush
+    const float e = (n.x * fmaf(c_norm, x.x, x.y) + n.y * (x.x + x.y)) * 1.01f +
+              (n.x + x.x + 1.0f) * static_cast<float>(ds) * 7.5231638e-37f;
+    // every partial sum of a score stays below ‖q‖‖x‖: far from overflow, or no bound is trusted
+    const bool trusted = n.x * x.x <= 1e37f && e <= 1e37f;
+    slack[q] = trusted ? e : INFINITY;
+    collected[q] = trusted ? 0u : over_cap;
+    if (q == 0) *over_count = 0;
+}
+
+cudaError_t launch_tf32_slack(const float* queries, uint32_t nq, uint32_t ds, const float2* row_max, float c_norm,
+                              float* slack, uint32_t* collected, uint32_t over_cap, uint32_t* over_count,
+                              cudaStream_t stream) {
+    if (nq == 0) return cudaSuccess;
+    tf32_slack_kernel<<<(nq + 3) / 4, 128, 0, stream>>>(queries, nq, ds, row_max, c_norm, slack, collected, over_cap,
+                                                        over_count);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tf32_row_norms(const float* base, uint64_t rows, uint32_t ds, float2* out, float2* max,
+                                  uint32_t sm_count, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
     const uint64_t blocks = std::min<uint64_t>((rows + 7) / 8, static_cast<uint64_t>(sm_count) * 8);
-    tf32_row_norms_kernel<<<static_cast<uint32_t>(blocks), 256, 0, stream>>>(base, rows, ds, out);
+    tf32_row_norms_kernel<<<static_cast<uint32_t>(blocks), 256, 0, stream>>>(base, rows, ds, out, max);
     count_launch();
     return cudaGetLastError();
 }

@@ -21,6 +21,14 @@ def force(index, ivf, nq, k, precision, nprobe, path, stride):
                           f"plan path={path} stride={stride} qb=0 ms=1.0\n")
 
 
+def fp32_scan(index, q, k):
+    """The FP32 scan's results: it serves batches of up to eight queries."""
+    index.set_precision("fp32")
+    parts = [index.search(np.vstack([q[lo:lo + 7], q[:1]]), k=k) for lo in range(0, len(q), 7)]
+    assert index.last_search_stats()["path"] == 1
+    return np.vstack([p[0][:-1] for p in parts]), np.vstack([p[1][:-1] for p in parts])
+
+
 @pytest.mark.parametrize("precision,rows,dims,nq,k,stride", [
     ("bf16", 16_384, 64, 1, 1, 8),         # the smallest sampled base, one query, one slab
     ("bf16", 16_641, 100, 129, 10, 8),     # one row in the last tile, one query in the last block
@@ -43,8 +51,7 @@ def test_sampled_pass_equals_fp32(precision, rows, dims, nq, k, stride):
     ti, ts = index.search(np.vstack([q, q[:1]]) if nq == 1 else q, k=k)
     st = index.last_search_stats()
     assert st["path"] == {"bf16": 2, "fp8": 3}[precision]
-    index.set_precision("fp32")
-    fi, fs = index.search(np.vstack([q, q[:1]]) if nq == 1 else q, k=k)
+    fi, fs = fp32_scan(index, np.vstack([q, q[:1]]) if nq == 1 else q, k)
     assert np.array_equal(ti, fi)
     assert np.array_equal(ts, fs)
     if nq > 1:
@@ -93,7 +100,6 @@ def test_overflowing_collection_gets_a_second_threshold(precision, nq):
     ti, ts = index.search(q, k=10)
     st = index.last_search_stats()
     assert st["path"] == path and st["fp32_fallback_queries"] == 0 and st["kernel_launches"] > 8, st
-    index.set_precision("fp32")
-    fi, fs = index.search(q, k=10)
+    fi, fs = fp32_scan(index, q, 10)
     assert np.array_equal(ti, fi)
     assert np.array_equal(ts, fs)
