@@ -40,6 +40,11 @@ NNDEX_DEVICE_INLINE uint64_t make_key(float score, uint32_t row) {
 NNDEX_DEVICE_INLINE float key_score(uint64_t key) { return ordered_to_float(static_cast<uint32_t>(key >> 32)); }
 NNDEX_DEVICE_INLINE uint32_t key_row(uint64_t key) { return 0xFFFFFFFFu - static_cast<uint32_t>(key & 0xFFFFFFFFu); }
 
+// ---- TF32 --------------------------------------------------------------------------------
+
+// The sign, exponent and top 10 mantissa bits of v: the least a kind::tf32 MMA reads of it.
+NNDEX_DEVICE_INLINE float tf32_head(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFFE000u); }
+
 // ---- shared-memory addresses -----------------------------------------------------------
 
 NNDEX_DEVICE_INLINE uint32_t smem_u32(const void* p) {

@@ -47,7 +47,7 @@ int nndex_cuda_check_bounded_wait(nndex_cuda_index* index, uint64_t budget_cycle
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "wait check launch");
-    ix->h_flags[0] = ~0ull;  // no validation error involved
+    ix->h_flags[0] = 0;  // no validation error involved
     ix->h_flags[1] = 0;
     cudaMemcpyAsync(&ix->h_flags[1], ix->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ix->stream);
     cudaMemsetAsync(ix->d_status, 0, sizeof(uint32_t), ix->stream);

@@ -357,7 +357,7 @@ int CudaIndex::enqueue_exact_fp32(const float* d_queries, uint32_t nq, uint32_t 
     a.rows = rows;
     a.k = k;
     a.ws_keys = d_ws;
-    a.status = d_status;
+    a.status = w_status;
     cudaEvent_t ev_a = nullptr;
     scan_event_begin(s, ev_a);
     cudaError_t e = launch_scan_fp32(a, plan, s);
@@ -392,7 +392,7 @@ int CudaIndex::enqueue_query_prep(uint64_t nq, int mode, cudaStream_t s) {
     p.out = d_qn;
     p.out_stride = static_cast<uint32_t>(ds);
     p.mode = mode;
-    p.err = d_err;
+    p.err = w_err;
     p.sm_count = sm_count;
     launch_prep_rows(p, s);
     stats.kernel_launches += 1;
@@ -403,7 +403,7 @@ int CudaIndex::check_device_words() {
     // h_flags[0] = err word, h_flags[1] = status word (copied with the results).
     const uint64_t err = h_flags[0];
     const uint32_t status = static_cast<uint32_t>(h_flags[1]);
-    if (err != ~0ull) return err_code(static_cast<int>(err & 0xFF));
+    if (err != 0) return err_code(static_cast<int>(~err & 0xFF));
     if (status == kStatusTimeout)
         return set_error(NNDEX_ERR_TIMEOUT, "cuda execution error: a bounded device wait timed out");
     if (status != 0) return set_error(NNDEX_ERR_CUDA, "cuda execution error: device status %u", status);
@@ -606,8 +606,30 @@ int CudaIndex::enqueue_prep_queries(const float* d_raw, uint64_t n, int mode, in
     p.out = d_qn;
     p.out_stride = static_cast<uint32_t>(ds);
     p.mode = mode;
-    p.err = d_err;
+    p.err = w_err;
     p.sm_count = sm_count;
+    // What the path's later kernels expect zeroed, and the two-pass TF32 scan's slack.
+    if (path == 4 || path == 5) {
+        if ((st = ivf_plan_words(*this, &p.zero[0], &p.zero_words[0]))) return st;
+    } else if (path == 6) {
+        if ((st = grow_device(d_floor, cap_floor, n, "tc workspace"))) return st;
+        if ((st = ensure_fbn())) return st;
+        p.zero[0] = reinterpret_cast<uint32_t*>(d_floor);
+        p.zero_words[0] = 2 * n;
+        p.zero[1] = d_fbn;
+        p.zero_words[1] = 1;
+    } else if (path == 7) {
+        if ((st = grow_device(d_q_resid, cap_q_resid, n, "query buffer"))) return st;
+        if ((st = grow_device(d_cnt2, cap_cnt2, n, "pass-2 buffer"))) return st;
+        if ((st = ensure_fbn())) return st;
+        p.tf_slack = d_q_resid;
+        p.tf_row_max = d_tfnorm + rows;
+        p.tf_c_norm = tf32_c_norm();
+        p.tf_collected = d_cnt2;
+        p.tf_over = kSecondPassCap + 1;
+        p.zero[1] = d_fbn;
+        p.zero_words[1] = 1;
+    }
     if (path == 2 || path == 3 || path == 5) {
         const uint64_t nq_alloc = (n + 127) / 128 * 128;
         if ((st = grow_device(d_q_resid, cap_q_resid, n, "query buffer"))) return st;
@@ -814,7 +836,7 @@ void CudaIndex::fill_tc_params(bool fp8, uint32_t n, uint64_t range_rows, TcPara
     p.eps_rows = fp8 ? eps_fp8 : eps_bf16;
     // FP32 accumulation of kb exact products (|Σ| ≤ 1 + ε): kb·2^-23, with a 4× margin.
     p.eps_acc = 4.0f * static_cast<float>(kb) * 1.1920929e-07f;
-    p.status = d_status;
+    p.status = w_status;
 }
 
 int CudaIndex::encode_query_tmap(bool fp8, void* buf, uint32_t n, CUtensorMap* map) const {
@@ -924,10 +946,23 @@ int CudaIndex::enqueue_tc_pass2(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, cap2, kcap,
                                 q_thr, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, d_m);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
-    launch_compact_zero_flags(d_ok2, n, d_tcfail, d_fail, s, d_m, CollectedSum{d_cnt2, nullptr, cap2, d_fbn_rows()});
+    launch_compact_zero_flags(d_ok2, n, d_tcfail, d_fail, s, d_m, batch_report());
     stats.kernel_launches += 4;
     last_tc_n = n;
     return NNDEX_OK;
+}
+
+// What the host reads after a tensor-core batch, written by its last kernel.
+BatchReport CudaIndex::batch_report() const {
+    BatchReport r;
+    r.cnt = d_cnt2;
+    r.cap = kSecondPassCap;
+    r.host_counts = h_fbn;
+    if (w_err == d_err) {
+        r.flags = d_err;
+        r.host_flags = reinterpret_cast<unsigned long long*>(h_flags);
+    }
+    return r;
 }
 
 int CudaIndex::finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
@@ -1008,7 +1043,7 @@ int CudaIndex::retry_tc_pass2(bool fp8, uint32_t m, uint32_t kcap, uint64_t* o_i
     if ((st = grow_host(h_ok2, cap_hok2, m, "pinned buffer"))) return st;
     cudaMemcpyAsync(h_ids, d_fbq, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(h_ok2, d_ok2, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&h_flags[1], d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    if (w_err == d_err) cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(e, "search");
     if ((st = check_device_words())) return st;
@@ -1068,7 +1103,6 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     if ((st = grow_device(d_cand_cnt, cap_cand_cnt, n, "tc workspace"))) return st;
     if ((st = grow_device(d_cert, cap_cert, n, "tc workspace"))) return st;
     if ((st = grow_device(d_kth, cap_kth, n, "tc workspace"))) return st;
-    if ((st = grow_device(d_floor, cap_floor, n, "tc workspace"))) return st;
     // The queries straight from the prepared buffer: rows past n read as zeros.
     CUtensorMap tmap_q;
     if (!encode_tmap_2d(&tmap_q, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d_qn, ds, n, ds * sizeof(float), 32, 16,
@@ -1088,8 +1122,7 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     a.evict_first = n <= 16;
     a.ws_keys = d_ws;
     a.floor_keys = d_floor;
-    a.status = d_status;
-    cudaMemsetAsync(d_floor, 0, n * sizeof(unsigned long long), s);
+    a.status = w_status;
     cudaEvent_t ev_a = nullptr;
     scan_event_begin(s, ev_a);
     cudaError_t e = launch_scan_tf32(tmap_f32, tmap_q, a, plan.stages, ctas, s);
@@ -1125,7 +1158,6 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     r.floor_keys = d_floor;  // rows the CTAs' lists left out score below it
     r.fb_ids = d_fbq;
     r.fb_count = d_fbn;
-    cudaMemsetAsync(d_fbn, 0, sizeof(uint32_t), s);
     if ((e = launch_rerank(r, s)) != cudaSuccess) return cuda_error(e, "rerank launch");
     // Uncertified queries re-run on the FP32 scan, on the device: the rerank listed them.
     if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
@@ -1154,7 +1186,7 @@ int CudaIndex::enqueue_fp32_fallback(const ScanPlan& plan, uint32_t n, uint32_t 
     fa.rows = rows;
     fa.k = kcap;
     fa.ws_keys = d_ws;
-    fa.status = d_status;
+    fa.status = w_status;
     fa.live = d_fbn;
     fa.ids = d_fbq;
     cudaError_t e;
@@ -1180,7 +1212,6 @@ int CudaIndex::grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t k
     int st;
     const uint64_t words = plan.nranges * plan.gm_tiles * (256 / plan.group);
     if ((st = grow_device(d_ws, cap_ws, std::max((words + 1) / 2, fb_keys) * n, "scan workspace"))) return st;
-    if ((st = grow_device(d_q_resid, cap_q_resid, n, "query buffer"))) return st;
     if ((st = grow_device(d_ids, cap_ids, n, "pass-2 buffer"))) return st;
     if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * plan.kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_sim, cap_cand_sim, static_cast<uint64_t>(n) * plan.kp, "tc workspace"))) return st;
@@ -1188,13 +1219,11 @@ int CudaIndex::grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t k
     if ((st = grow_device(d_cert, cap_cert, n, "tc workspace"))) return st;
     if ((st = grow_device(d_kth, cap_kth, n, "tc workspace"))) return st;
     if ((st = grow_device(d_rows2, cap_rows2, static_cast<uint64_t>(n) * kSecondPassCap, "pass-2 buffer"))) return st;
-    if ((st = grow_device(d_cnt2, cap_cnt2, n, "pass-2 buffer"))) return st;
     if ((st = grow_device(d_ok2, cap_ok2, n, "pass-2 buffer"))) return st;
     if ((st = grow_device(d_rslots, cap_rslots, static_cast<uint64_t>(n) * rerank_chunks(kSecondPassCap) * kcap,
                           "pass-2 buffer")))
         return st;
-    if ((st = grow_device(d_fbq, cap_fbq, n, "fallback buffer"))) return st;
-    return ensure_fbn();
+    return grow_device(d_fbq, cap_fbq, n, "fallback buffer");
 }
 
 // Two-pass TF32 scan (FP32 indexes, 17 queries and more): K3's sampled pass 1 and collecting pass 2 on
@@ -1224,9 +1253,7 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
                         CU_TENSOR_MAP_SWIZZLE_128B))
         return set_error(NNDEX_ERR_CUDA, "cuda execution error: cuTensorMapEncodeTiled failed (queries, driver "
                                          "result %d)", last_encode_result());
-    cudaError_t e = launch_tf32_slack(d_qn, n, static_cast<uint32_t>(ds), d_tfnorm + rows, tf32_c_norm(), d_q_resid,
-                                      d_cnt2, kSecondPassCap + 1, d_fbn, s);
-    if (e != cudaSuccess) return cuda_error(e, "TF32 slack launch");
+    cudaError_t e = cudaSuccess;
     TcArgs a;
     a.tmap_q = &tmap_q;
     a.tmap_b = &tmap_f32_256;
@@ -1237,7 +1264,7 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
     a.p.nchunks = static_cast<uint32_t>(ds / 32);
     a.p.rows = rows;
     a.p.range_rows = plan.range_rows;
-    a.p.status = d_status;
+    a.p.status = w_status;
     a.p.q_resid = d_q_resid;
     a.p.tile_stride = plan.stride;
     a.p.gm = reinterpret_cast<uint32_t*>(d_ws);
@@ -1296,7 +1323,7 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
     last_tc_n = n;
     fbn_stream = s;
     fbn_pending = true;
-    stats.kernel_launches += 8;
+    stats.kernel_launches += 7;
     stats.path = 7;
     stats.rerank_width = plan.kp;
     stats.pass1_tile_stride = plan.stride;
@@ -1373,10 +1400,9 @@ int CudaIndex::tune_host(uint64_t n, uint64_t kcap, int mode, TunePlan* plan) {
 // resets, upload, prep, the path's scan and merge, and the downloads into the pinned buffers.
 int CudaIndex::enqueue_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
     int st;
-    cudaMemsetAsync(d_err, 0xFF, sizeof(unsigned long long), stream);
-    cudaMemsetAsync(d_status, 0, sizeof(uint32_t), stream);
-    cudaMemcpyAsync(d_qraw, h_q, n * dims * sizeof(float), cudaMemcpyHostToDevice, stream);
-    if ((st = enqueue_prep_queries(d_qraw, n, mode, path, stream))) return st;
+    h_flags[0] = h_flags[1] = 0;  // (a replay's are reset by run_host_batch)
+    if (!mapped_io) cudaMemcpyAsync(d_qraw, h_q, n * dims * sizeof(float), cudaMemcpyHostToDevice, stream);
+    if ((st = enqueue_prep_queries(mapped_io ? h_q : d_qraw, n, mode, path, stream))) return st;
     if (path == 4) {
         if ((st = ivf_search(*this, d_qn, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt,
                              stream)))
@@ -1402,13 +1428,10 @@ int CudaIndex::enqueue_host_batch(uint64_t n, uint64_t kcap, int mode, int path)
         if ((st = enqueue_tc_pass2(path == 3, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim,
                                    d_cnt, stream)))
             return st;
-        // pass 2's counts come back with the results (finish_tc reads them once the batch is done)
-        cudaMemcpyAsync(h_fbn, d_fbn, kFbnBytes, cudaMemcpyDeviceToHost, stream);
     }
     if (error_report)
         serr_record(static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt, stream);
-    cudaMemcpyAsync(h_res, d_res, res_bytes, cudaMemcpyDeviceToHost, stream);  // idx, sim, cnt
-    cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream);  // err, status
+    if (!mapped_io) cudaMemcpyAsync(h_res, d_res, res_bytes, cudaMemcpyDeviceToHost, stream);  // idx, sim, cnt
     return NNDEX_OK;
 }
 
@@ -1435,6 +1458,7 @@ int CudaIndex::run_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
             graphs.erase(graphs.begin() + static_cast<long>(i));
             break;
         }
+        h_flags[0] = h_flags[1] = 0;
         const cudaError_t e = cudaGraphLaunch(graphs[i].exec, stream);
         if (e != cudaSuccess) return cuda_error(e, "graph launch");
         // the capture's statistics: counters added to this call's, the rest as captured
@@ -1504,6 +1528,7 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
     cudaSetDevice(device);
     stats = nndex_cuda_search_stats{};
     order_after_previous(stream);
+    use_host_words();
     const uint64_t kcap = std::min<uint64_t>(k, rows);
     if (kcap > kMaxFusedK)
         return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: k=%llu above the fused top-k limit %u",
@@ -1517,6 +1542,15 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
         int st;
         if ((st = ensure_query_capacity(n))) return st;
         if ((st = ensure_result_capacity(n, kcap))) return st;
+        // Each copy of a small batch costs the GPU more (4 to 12 us with the gaps around it) than the
+        // kernels' own reads and writes of pinned memory over PCIe: up to 64 KB each way, rows that
+        // query prep reads once (prep.cu). One query against 50k × 128: 82 -> 57 us a call.
+        mapped_io = !error_report && dims <= 1024 && n * dims * sizeof(float) <= kMappedIoBytes && res_bytes <= kMappedIoBytes;
+        if (mapped_io) {
+            d_idx = h_idx;
+            d_sim = h_sim;
+            d_cnt = h_cnt;
+        }
         std::memcpy(h_q, queries + q0 * dims, n * dims * sizeof(float));
         bool measure = false;
         TunePlan plan = plan_for(n, kcap, &measure);
@@ -1548,7 +1582,7 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
                            : finish_tc(static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt,
                                        stream);
             if (st) return st;
-            if (tc_patched) {
+            if (tc_patched && !mapped_io) {
                 cudaMemcpyAsync(h_res, d_res, res_bytes, cudaMemcpyDeviceToHost, stream);
                 if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_error(e, "search");
             }
@@ -1563,10 +1597,8 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
         if (counts_out)
             for (uint64_t i = 0; i < n; ++i) counts_out[q0 + i] = h_cnt[i];
     }
-    mark_done(stream);
-    float ms = 0.0f;
-    if (nq) cudaEventElapsedTime(&ms, ev0, ev1);
-    stats.device_ms = ms;
+    done_stream = nullptr;  // every batch was waited for: nothing for a later call to be ordered after
+    ms_pending = nq != 0;   // the device time between ev0 and ev1, read with the statistics
     return NNDEX_OK;
 }
 
@@ -1581,7 +1613,6 @@ int CudaIndex::run_device_chunk(const float* dq, uint64_t n, uint64_t kcap, int 
     if (path == 5) {
         *synced = true;
         if ((st = ivf_search_tc(*this, n32, k32, oi, os, oc, s))) return st;
-        cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);  // err, status
         const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_error(e, "IVF search");
         if ((st = check_device_words())) return st;
@@ -1594,8 +1625,6 @@ int CudaIndex::run_device_chunk(const float* dq, uint64_t n, uint64_t kcap, int 
     *synced = true;
     if ((st = enqueue_tc(path == 3, n32, k32, oi, os, oc, s))) return st;
     if ((st = enqueue_tc_pass2(path == 3, n32, k32, oi, os, oc, s))) return st;
-    cudaMemcpyAsync(h_fbn, d_fbn, kFbnBytes, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);  // err, status
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(e, "search");
     if ((st = check_device_words())) return st;
@@ -1613,8 +1642,8 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
     int st;
     if ((st = ensure_query_capacity(std::min<uint64_t>(nq, kMaxBatchChunk)))) return st;
     if (error_report && (st = serr_begin(nq, kcap, s))) return st;
-    cudaMemsetAsync(d_err, 0xFF, sizeof(unsigned long long), s);
-    cudaMemsetAsync(d_status, 0, sizeof(uint32_t), s);
+    use_device_words();
+    cudaMemsetAsync(d_err, 0, 2 * sizeof(unsigned long long), s);
     bool synced = false, done = false;  // done: the last piece waited and its status words were clean
     for (uint64_t q0 = 0; q0 < nq; q0 += kMaxBatchChunk) {
         const uint64_t n = std::min<uint64_t>(kMaxBatchChunk, nq - q0);
@@ -1752,6 +1781,7 @@ int CudaIndex::serr_fetch_stats() {
 // The index's scratch buffers are shared by every call: work enqueued on one stream must not
 // overlap work of an earlier call on another stream.
 void CudaIndex::order_after_previous(cudaStream_t s) {
+    ms_pending = false;
     if (done_ev && done_stream && done_stream != s) cudaStreamWaitEvent(s, done_ev, 0);
 }
 void CudaIndex::mark_done(cudaStream_t s) {
@@ -1763,10 +1793,8 @@ void CudaIndex::mark_done(cudaStream_t s) {
 int CudaIndex::stream_status() {
     std::lock_guard<std::mutex> lock(mu);
     cudaSetDevice(device);
-    h_flags[1] = 0;
     cudaStreamSynchronize(stream);
-    cudaMemcpy(&h_flags[0], d_err, sizeof(uint64_t), cudaMemcpyDeviceToHost);
-    cudaMemcpy(&h_flags[1], d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+    cudaMemcpy(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost);
     return check_device_words();
 }
 
@@ -1840,8 +1868,16 @@ int index_begin(uint64_t rows, uint64_t dims, uint32_t flags, const nndex_cuda_o
     const size_t base_bytes = ix->rows_alloc * ix->ds * sizeof(float);
     if ((e = cudaMalloc(&ix->d_base, base_bytes)) != cudaSuccess) return fail(cuda_error(e, "base allocation"));
     cudaMemsetAsync(ix->d_base + rows * ix->ds, 0, (ix->rows_alloc - rows) * ix->ds * sizeof(float), ix->stream);
-    cudaMemsetAsync(ix->d_err, 0xFF, sizeof(unsigned long long), ix->stream);
-    cudaMemsetAsync(ix->d_status, 0, sizeof(uint32_t), ix->stream);
+    cudaMemsetAsync(ix->d_err, 0, 2 * sizeof(unsigned long long), ix->stream);
+    ix->use_device_words();
+    // Row norms of the TF32 scans' bounds (8 bytes per row, written by K1; the last entry their maxima).
+    // Without them (no memory) FP32 batches take the FP32 scan.
+    if (cudaMalloc(&ix->d_tfnorm, (rows + 1) * sizeof(float2)) == cudaSuccess) {
+        cudaMemsetAsync(ix->d_tfnorm + rows, 0, sizeof(float2), ix->stream);
+    } else {
+        ix->d_tfnorm = nullptr;
+        cudaGetLastError();
+    }
     // Low-precision scoring copies (K1 writes them in the same pass) and their residual norms.
     if (flags & NNDEX_FLAG_BF16) {
         ix->kb16 = (dims + 63) / 64 * 64;
@@ -1874,6 +1910,10 @@ void index_prep_rows(CudaIndex* ix, const float* d_src, uint64_t row0, uint64_t 
     p.mode = ix->normalized ? 2 : 0;
     p.err = ix->d_err;
     p.sm_count = ix->sm_count;
+    if (ix->d_tfnorm) {
+        p.tf_norms = ix->d_tfnorm + row0;
+        p.tf_max = ix->d_tfnorm + ix->rows;
+    }
     if (ix->d_base_bf16) {
         p.out_bf16 = ix->d_base_bf16 + row0 * ix->kb16;
         p.bf16_stride = static_cast<uint32_t>(ix->kb16);
@@ -1896,7 +1936,7 @@ int index_finish(CudaIndex* ix) {
     cudaError_t e;
     cudaMemcpyAsync(&ix->h_flags[0], ix->d_err, sizeof(uint64_t), cudaMemcpyDeviceToHost, ix->stream);
     if ((e = cudaStreamSynchronize(ix->stream)) != cudaSuccess) return fail(cuda_error(e, "upload"));
-    if (ix->h_flags[0] != ~0ull) return fail(err_code(static_cast<int>(ix->h_flags[0] & 0xFF)));
+    if (ix->h_flags[0] != 0) return fail(err_code(static_cast<int>(~ix->h_flags[0] & 0xFF)));
     if (ix->d_res16 || ix->d_res8) {
         // ε of the certificate: the largest residual norm ‖x − x̂‖ over the rows.
         unsigned int* d_max = nullptr;
@@ -1938,18 +1978,6 @@ int index_finish(CudaIndex* ix) {
         if ((e = cudaMalloc(&ix->d_tile_scale, ix->rows_alloc / 256 * sizeof(float2))) != cudaSuccess)
             return fail(cuda_error(e, "FP8 tile scales"));
         launch_tile_scale(ix->d_row_scale, ix->rows, ix->rows_alloc / 256, ix->d_tile_scale, ix->stream);
-    }
-    // Row norms of K12's bound (8 bytes per row, one pass over the base). Without them (no memory)
-    // small batches take the FP32 scan.
-    if (cudaMalloc(&ix->d_tfnorm, (ix->rows + 1) * sizeof(float2)) == cudaSuccess) {
-        cudaMemsetAsync(ix->d_tfnorm + ix->rows, 0, sizeof(float2), ix->stream);
-        if ((e = launch_tf32_row_norms(ix->d_base, ix->rows, static_cast<uint32_t>(ix->ds), ix->d_tfnorm,
-                                       ix->d_tfnorm + ix->rows, static_cast<uint32_t>(ix->sm_count), ix->stream)) !=
-            cudaSuccess)
-            return fail(cuda_error(e, "row norms launch"));
-    } else {
-        ix->d_tfnorm = nullptr;
-        cudaGetLastError();
     }
     if (ix->approx) {
         // src/approx.rs:46-100, built once at construction instead of on the first approx search.
@@ -2074,8 +2102,8 @@ int make_view(const CudaIndex& src, CudaIndex** out) {
         return cuda_error(e, "index view");
     }
     v->d_status = reinterpret_cast<uint32_t*>(v->d_err + 1);
-    cudaMemsetAsync(v->d_err, 0xFF, sizeof(unsigned long long), v->stream);
-    cudaMemsetAsync(v->d_status, 0, sizeof(uint32_t), v->stream);
+    cudaMemsetAsync(v->d_err, 0, 2 * sizeof(unsigned long long), v->stream);
+    v->use_device_words();
     cudaStreamSynchronize(v->stream);
     *out = v;
     return NNDEX_OK;
@@ -2311,6 +2339,13 @@ int nndex_cuda_last_search_stats(const nndex_cuda_index* index, nndex_cuda_searc
     if (!index || !out) return set_error(NNDEX_ERR_INVALID_ARGUMENT, "cuda execution error: null argument");
     CudaIndex* ix = index->impl;
     std::lock_guard<std::mutex> lock(ix->mu);
+    if (ix->ms_pending) {
+        cudaSetDevice(ix->device);
+        float ms = 0.0f;
+        if (cudaEventElapsedTime(&ms, ix->ev0, ix->ev1) != cudaSuccess) cudaGetLastError();
+        ix->stats.device_ms = ms;
+        ix->ms_pending = false;
+    }
     if (ix->serr_pending || ix->fbn_pending) {
         cudaSetDevice(ix->device);
         int st = ix->serr_fetch_stats();

@@ -18,6 +18,9 @@ constexpr uint64_t kMaxBatchChunk = 16384;
 // Rows a pass-2 query may collect before it is re-run on the FP32 scan.
 constexpr uint32_t kSecondPassCap = 8192;
 
+// Host-buffer batches up to this size, queries and results each, run without copies.
+constexpr size_t kMappedIoBytes = 64 << 10;
+
 // FP32 batches take the two-pass TF32 scan from this much work (rows × stored dims × queries). Its nine
 // launches cost about 45 us whatever the batch, the FP32 scan's FMAs about 20 us per 1e8 beyond its own
 // 50. Batches in a row through device buffers, FP32 scan against two-pass scan: 50k × 128 with 17
@@ -70,6 +73,7 @@ struct CudaIndex {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t done_ev = nullptr;        // completion of the last call's device work
     cudaStream_t done_stream = nullptr;   // the stream it ran on
+    bool ms_pending = false;              // stats.device_ms is still to be read from ev0 and ev1
     std::mutex mu;
 
     float* d_base = nullptr;  // rows_alloc × ds FP32, normalised, zero padded
@@ -180,10 +184,25 @@ struct CudaIndex {
     float* h_sim = nullptr;
     uint32_t* h_cnt = nullptr;
     size_t res_bytes = 0;        // bytes of the current batch's results
-    // Status words, adjacent in one 16-byte allocation (d_status = the word after d_err), read back
-    // with one copy into h_flags.
+    // Status words, adjacent in one 16-byte allocation (d_status = the word after d_err), zero when
+    // clean: of construction and of device-buffer searches, read back with one copy into h_flags.
     unsigned long long* d_err = nullptr;
     uint32_t* d_status = nullptr;
+    // The current call's: d_err / d_status, or for a host-buffer search h_flags itself (the kernels
+    // only ever write them on an error, and a host-buffer search waits before it reads them).
+    unsigned long long* w_err = nullptr;
+    uint32_t* w_status = nullptr;
+    void use_device_words() {
+        w_err = d_err;
+        w_status = d_status;
+    }
+    void use_host_words() {
+        w_err = reinterpret_cast<unsigned long long*>(h_flags);
+        w_status = reinterpret_cast<uint32_t*>(h_flags + 1);
+    }
+    // Small host-buffer batches: the kernels read the queries from the pinned buffer and write the
+    // results into the pinned buffer (d_idx, d_sim, d_cnt are its views), so that no copy runs.
+    bool mapped_io = false;
     float* h_q = nullptr;
     size_t cap_hq = 0;
     uint64_t* h_flags = nullptr;
@@ -244,7 +263,6 @@ struct CudaIndex {
     uint32_t* d_tcfail = nullptr;  // TC pass 2: positions (in d_ids) of the queries whose collection overflowed
     size_t cap_tcfail = 0;
     int ensure_fbn();
-    unsigned long long* d_fbn_rows() const { return reinterpret_cast<unsigned long long*>(d_fbn + 4); }
     uint64_t h_fbn_rows() const { return *reinterpret_cast<const unsigned long long*>(h_fbn + 4); }
     cudaStream_t fbn_stream = nullptr;
     bool fbn_pending = false;
@@ -346,6 +364,7 @@ struct CudaIndex {
     // Once the stream has completed a tensor-core batch (h_fbn read back with it): statistics, the
     // pass-1 stride rule, and the FP32 re-run of any query whose collection overflowed (device
     // outputs patched in place; synchronises the stream again only then).
+    BatchReport batch_report() const;
     int finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
     // Pass 2 once more for the m queries whose collection overflowed (positions in d_ids: d_tcfail),
     // against the T of the rows they did collect; the ones that overflow again are left in *failed.

@@ -32,7 +32,7 @@ struct PrepArgs {
     float* out = nullptr;        // rows × out_stride
     uint32_t out_stride = 0;
     int mode = 0;                // 0 normalize_rows, 1 normalize_vector, 2 finite check + pad
-    unsigned long long* err = nullptr;  // (row << 8) | code, reduced with atomicMin
+    unsigned long long* err = nullptr;  // ~((row << 8) | code), reduced with atomicMax (0: no error)
     __nv_bfloat16* out_bf16 = nullptr;
     uint32_t bf16_stride = 0;
     uint8_t* out_fp8 = nullptr;
@@ -40,6 +40,20 @@ struct PrepArgs {
     float* fp8_scale = nullptr;
     float* resid_bf16 = nullptr;
     float* resid_fp8 = nullptr;
+    // TF32 scans. Rows of the base: {‖x‖, ‖x − tf32_head(x)‖} each, rounded up, and the largest of each
+    // raised into *tf_max (zeroed before; non-negative floats order as their bits).
+    float2* tf_norms = nullptr;
+    float2* tf_max = nullptr;
+    // Queries of the two-pass scan: the largest bound slack over all rows,
+    // ‖q‖(‖d_x‖ + C‖x‖) + ‖d_q‖(‖x‖ + ‖d_x‖) at the rows' maxima tf_row_max, and 0 collected rows. A query
+    // whose products could overflow FP32 gets an infinite slack and tf_over collected rows.
+    float* tf_slack = nullptr;
+    const float2* tf_row_max = nullptr;
+    float tf_c_norm = 0.0f;
+    uint32_t* tf_collected = nullptr;
+    uint32_t tf_over = 0;
+    uint32_t* zero[2] = {nullptr, nullptr};  // words to zero for the kernels behind this one
+    uint64_t zero_words[2] = {0, 0};
     int sm_count = 148;
 };
 void launch_prep_rows(const PrepArgs& a, cudaStream_t stream);
@@ -266,26 +280,24 @@ uint32_t tf32_stages_for(uint32_t cap, size_t smem_limit);
 // queries (nq rows; the rows past nq read as zeros), box {32 floats, 16 rows}, 128-byte swizzle.
 cudaError_t launch_scan_tf32(const CUtensorMap& tmap_x, const CUtensorMap& tmap_q, const Tf32ScanArgs& a,
                              uint32_t stages, uint32_t ctas, cudaStream_t stream);
-// Per row of the base (stride ds): {‖x‖, ‖x − tf32_head(x)‖}, FP64 sums rounded up; and the largest of
-// each over the rows, raised into *max (zeroed before; non-negative floats order as their bits).
-cudaError_t launch_tf32_row_norms(const float* base, uint64_t rows, uint32_t ds, float2* out, float2* max,
-                                  uint32_t sm_count, cudaStream_t stream);
-// Per query (stride ds): the largest bound slack over all rows, ‖q‖(‖d_x‖ + C‖x‖) + ‖d_q‖(‖x‖ + ‖d_x‖) at
-// the rows' maxima, and collected[q] = 0. A query whose products could overflow FP32 gets an infinite
-// slack and over_cap in collected[q] (its collection then counts as overflowed). *over_count = 0.
-cudaError_t launch_tf32_slack(const float* queries, uint32_t nq, uint32_t ds, const float2* row_max, float c_norm,
-                              float* slack, uint32_t* collected, uint32_t over_cap, uint32_t* over_count,
-                              cudaStream_t stream);
 
 // Device-side certificate fallback: compaction of the zero flags (one block).
-struct CollectedSum {
-    const uint32_t* cnt = nullptr;  // collected rows per query
-    const uint32_t* by = nullptr;   // optional: cnt is indexed by[i] rather than i
+// What the last compaction of a tensor-core batch adds for the host: Σ min(cnt[j], cap) over the flags i
+// that count, j = by[i] (by given) or i (pass 2's collected rows); its counts ({·, live, zero flags, ·,
+// Σ} as 32-bit words, Σ in two), the IVF plan's counters and the batch's status words, each written to
+// pinned memory by the kernel.
+struct BatchReport {
+    const uint32_t* cnt = nullptr;
+    const uint32_t* by = nullptr;
     uint32_t cap = 0;
-    unsigned long long* sum = nullptr;
+    uint32_t* host_counts = nullptr;
+    const unsigned long long* counters = nullptr;  // 8 of them
+    unsigned long long* host_counters = nullptr;
+    const unsigned long long* flags = nullptr;     // 2: the error word, the status word
+    unsigned long long* host_flags = nullptr;
 };
 void launch_compact_zero_flags(const uint32_t* flags, uint32_t n, uint32_t* ids, uint32_t* count, cudaStream_t s,
-                               const uint32_t* live = nullptr, const CollectedSum& rows = CollectedSum{});
+                               const uint32_t* live = nullptr, const BatchReport& report = BatchReport{});
 
 struct RerankArgs {
     const float* base = nullptr;  // FP32 base, stride ds (with row_map: the list-ordered copy)

@@ -52,15 +52,20 @@ struct IvfScratch {
     uint32_t tc_stride = 1;             // tensor-core scan: pass 1 on every n-th tile (autotuned)
     uint32_t* d_probes = nullptr;       size_t cap_probes = 0;
     float* d_pscore = nullptr;          size_t cap_pscore = 0;     // B·nlist: centroid scores of the probe
-    uint32_t* d_list_cnt = nullptr;     size_t cap_list_cnt = 0;   // nlist: queries probing each list
-    uint32_t* d_list_fill = nullptr;    size_t cap_list_fill = 0;
+    // The words a search starts from zero, in one buffer: 16 counters (work counters, totals, rows
+    // probed), then per list the queries probing it and its fill. Query prep zeroes them for the
+    // search behind it (zeroed); the views below point into it.
+    uint32_t* d_plan0 = nullptr;        size_t cap_plan0 = 0;
+    bool zeroed = false;
+    uint32_t* d_list_cnt = nullptr;     // nlist
+    uint32_t* d_list_fill = nullptr;    // nlist
+    unsigned long long* d_counters = nullptr;  // 16
     uint32_t* d_list_qoff = nullptr;    size_t cap_list_qoff = 0;  // nlist + 1
     uint32_t* d_item_off = nullptr;     size_t cap_item_off = 0;   // nlist + 1
     uint32_t* d_item_list = nullptr;    size_t cap_item_list = 0;  // tensor-core scan: list of each work item
     uint32_t* d_list_q = nullptr;       size_t cap_list_q = 0;     // B·nprobe: query of each (list, query) pair
     uint32_t* d_list_slot = nullptr;    size_t cap_list_slot = 0;  // B·nprobe: its first output slot
     uint32_t* d_q_slot_off = nullptr;   size_t cap_q_slot_off = 0; // B + 1
-    unsigned long long* d_counters = nullptr; size_t cap_counters = 0;  // work counter, totals, rows probed
     uint64_t* d_ws = nullptr;           size_t cap_ws = 0;         // slots × k keys
     uint32_t* d_slot_row0 = nullptr;    size_t cap_slot_row0 = 0;  // group maxima: first list position of each slot's chunk
     uint32_t* d_qblock_off = nullptr;   size_t cap_qblock_off = 0; // nlist + 1 (tensor-core scan)
@@ -84,6 +89,8 @@ int ivf_restore(CudaIndex& ix, uint64_t nlist, const float* centroids, const uin
 // Position-sensitive 64-bit fingerprint of the stored (normalised, padded) rows.
 int base_checksum(CudaIndex& ix, uint64_t* out);
 
+// The words an IVF search starts from zero, for query prep to zero (the next search then does not).
+int ivf_plan_words(CudaIndex& ix, uint32_t** words, uint64_t* n);
 // Enqueues the IVF search of `nq` normalised queries (stride ds) with capped k into the device
 // outputs (rows of `k` slots), on the FP32 list scan. Returns an NNDEX status.
 int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uint64_t* o_idx, float* o_sim,

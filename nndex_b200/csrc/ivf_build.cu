@@ -977,15 +977,13 @@ IvfScratch::~IvfScratch() {
     cudaFree(d_lane_slot);
     cudaFree(d_probes);
     cudaFree(d_pscore);
-    cudaFree(d_list_cnt);
-    cudaFree(d_list_fill);
+    cudaFree(d_plan0);
     cudaFree(d_list_qoff);
     cudaFree(d_item_off);
     cudaFree(d_item_list);
     cudaFree(d_list_q);
     cudaFree(d_list_slot);
     cudaFree(d_q_slot_off);
-    cudaFree(d_counters);
     cudaFree(d_ws);
     cudaFreeHost(h_probed);
 }

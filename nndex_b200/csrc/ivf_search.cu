@@ -481,10 +481,13 @@ __global__ void __launch_bounds__(IvfScanShape<QB>::kThreads, 1)
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(512)
     ivf_merge_kernel(const uint64_t* __restrict__ ws, const uint32_t* __restrict__ q_slot_off, uint32_t k,
-                     uint64_t* __restrict__ idx_out, float* __restrict__ sim_out, uint32_t* __restrict__ count_out) {
+                     uint64_t* __restrict__ idx_out, float* __restrict__ sim_out, uint32_t* __restrict__ count_out,
+                     const unsigned long long* __restrict__ counters, unsigned long long* __restrict__ host_probed) {
     __shared__ BlockSelectScratch s;
     extern __shared__ uint64_t sorted[];
     const uint32_t q = blockIdx.x;
+    // the plan's row totals for the statistics, into pinned memory
+    if (host_probed && q == 0 && threadIdx.x < 3) host_probed[threadIdx.x] = counters[3 + threadIdx.x];
     const uint64_t* keys = ws + static_cast<uint64_t>(q_slot_off[q]) * k;
     const uint64_t n = static_cast<uint64_t>(q_slot_off[q + 1] - q_slot_off[q]) * k;
     if (threadIdx.x == 0) s.count = 0;
@@ -605,6 +608,22 @@ int grow(T*& p, size_t& cap, size_t n, const char* what) {
     return NNDEX_OK;
 }
 
+constexpr uint32_t kPlanCounters = 16;
+
+int plan_buffer(IvfScratch& w, uint32_t nlist) {
+    const int st = grow(w.d_plan0, w.cap_plan0, 2 * kPlanCounters + 2 * static_cast<size_t>(nlist), "IVF plan buffer");
+    if (st) return st;
+    w.d_counters = reinterpret_cast<unsigned long long*>(w.d_plan0);
+    w.d_list_cnt = w.d_plan0 + 2 * kPlanCounters;
+    w.d_list_fill = w.d_list_cnt + nlist;
+    return NNDEX_OK;
+}
+
+void zero_plan(IvfScratch& w, uint32_t nlist, cudaStream_t s) {
+    if (!w.zeroed) cudaMemsetAsync(w.d_plan0, 0, (2 * kPlanCounters + 2 * static_cast<size_t>(nlist)) * sizeof(uint32_t), s);
+    w.zeroed = false;
+}
+
 // Tile rows of the list scan at qb queries per item (IvfScanShape).
 uint32_t ivf_scan_tile_rows(uint32_t qb) { return qb >= 16 ? 8 * 16 : 16 * 16; }
 
@@ -714,6 +733,17 @@ int grow_pinned(T*& p, size_t& cap, size_t n, const char* what) {
 
 }  // namespace
 
+int ivf_plan_words(CudaIndex& ix, uint32_t** words, uint64_t* n) {
+    IvfScratch& w = ix.ivf_scratch;
+    const uint32_t nlist = static_cast<uint32_t>(ix.ivf->nlist);
+    const int st = plan_buffer(w, nlist);
+    if (st) return st;
+    *words = w.d_plan0;
+    *n = 2 * kPlanCounters + 2 * static_cast<uint64_t>(nlist);
+    w.zeroed = true;
+    return NNDEX_OK;
+}
+
 int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uint64_t* o_idx, float* o_sim,
                uint32_t* o_cnt, cudaStream_t s) {
     const IvfIndex& v = *ix.ivf;
@@ -742,14 +772,12 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
     uint32_t sub = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(nq, ws_budget / per_query)));
     if ((st = grow(w.d_probes, w.cap_probes, static_cast<size_t>(sub) * np, "IVF probe buffer"))) return st;
     if ((st = grow(w.d_pscore, w.cap_pscore, static_cast<size_t>(sub) * nlist, "IVF probe buffer"))) return st;
-    if ((st = grow(w.d_list_cnt, w.cap_list_cnt, nlist, "IVF plan buffer"))) return st;
-    if ((st = grow(w.d_list_fill, w.cap_list_fill, nlist, "IVF plan buffer"))) return st;
+    if ((st = plan_buffer(w, nlist))) return st;
     if ((st = grow(w.d_list_qoff, w.cap_list_qoff, nlist + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_item_off, w.cap_item_off, nlist + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_list_q, w.cap_list_q, static_cast<size_t>(sub) * np, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_list_slot, w.cap_list_slot, static_cast<size_t>(sub) * np, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_q_slot_off, w.cap_q_slot_off, sub + 1, "IVF plan buffer"))) return st;
-    if ((st = grow(w.d_counters, w.cap_counters, 8, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_ws, w.cap_ws, static_cast<size_t>(sub) * np * max_chunks * k, "IVF slot workspace"))) return st;
     IvfScanArgs a;
     a.dq = dq;
@@ -765,15 +793,17 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
     a.list_slot = w.d_list_slot;
     a.counters = w.d_counters;
     a.ws = w.d_ws;
-    a.status = ix.d_status;
+    a.status = ix.w_status;
     uint32_t p2 = 1;
     while (p2 < k) p2 <<= 1;
-    cudaMemsetAsync(w.d_counters, 0, 8 * sizeof(unsigned long long), s);
+    if (!w.h_probed) bump_alloc_epoch();
+    if (!w.h_probed && cudaMallocHost(&w.h_probed, 8 * sizeof(unsigned long long)) != cudaSuccess)
+        return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
+    zero_plan(w, nlist, s);
     for (uint32_t q0 = 0; q0 < nq; q0 += sub) {
         const uint32_t n = std::min(sub, nq - q0);
         const float* qn = queries + static_cast<uint64_t>(q0) * ix.ds;
-        cudaMemsetAsync(w.d_list_cnt, 0, nlist * sizeof(uint32_t), s);
-        cudaMemsetAsync(w.d_list_fill, 0, nlist * sizeof(uint32_t), s);
+        if (q0) cudaMemsetAsync(w.d_list_cnt, 0, 2 * nlist * sizeof(uint32_t), s);  // and the fills behind it
         const ProbeLaunch pl{qn,          n,          dq,           static_cast<uint32_t>(ix.dp), nlist, np,
                              v.d_cent_t,  v.nlist_pad, v.d_offsets, w.d_pscore, w.d_probes, w.d_list_cnt,
                              w.d_q_slot_off, w.d_counters};
@@ -791,15 +821,11 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
         if (e != cudaSuccess) return cuda_error(e, "IVF scan launch");
         ivf_merge_kernel<<<n, 512, p2 * sizeof(uint64_t), s>>>(w.d_ws, w.d_q_slot_off, k, o_idx + static_cast<uint64_t>(q0) * k,
                                                                o_sim + static_cast<uint64_t>(q0) * k,
-                                                               o_cnt ? o_cnt + q0 : nullptr);
+                                                               o_cnt ? o_cnt + q0 : nullptr, w.d_counters, w.h_probed);
         count_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "IVF merge launch");
         ix.stats.kernel_launches += 6;
     }
-    if (!w.h_probed) bump_alloc_epoch();
-    if (!w.h_probed && cudaMallocHost(&w.h_probed, 8 * sizeof(unsigned long long)) != cudaSuccess)
-        return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
-    cudaMemcpyAsync(w.h_probed, w.d_counters + 3, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
     ix.stats.path = 4;
     ix.stats.nprobe = np;
     return NNDEX_OK;
@@ -862,15 +888,13 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     int st;
     if ((st = grow(w.d_probes, w.cap_probes, pairs, "IVF probe buffer"))) return st;
     if ((st = grow(w.d_pscore, w.cap_pscore, static_cast<size_t>(nq) * nlist, "IVF probe buffer"))) return st;
-    if ((st = grow(w.d_list_cnt, w.cap_list_cnt, nlist, "IVF plan buffer"))) return st;
-    if ((st = grow(w.d_list_fill, w.cap_list_fill, nlist, "IVF plan buffer"))) return st;
+    if ((st = plan_buffer(w, nlist))) return st;
     if ((st = grow(w.d_list_qoff, w.cap_list_qoff, nlist + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_item_off, w.cap_item_off, nlist + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_qblock_off, w.cap_qblock_off, nlist + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_list_q, w.cap_list_q, pairs, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_list_slot, w.cap_list_slot, pairs, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_q_slot_off, w.cap_q_slot_off, nq + 1, "IVF plan buffer"))) return st;
-    if ((st = grow(w.d_counters, w.cap_counters, 10, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_ws, w.cap_ws, pairs * max_chunks * slot_keys, "IVF slot workspace"))) return st;
     if (groups && (st = grow(w.d_slot_row0, w.cap_slot_row0, pairs * max_chunks, "IVF slot workspace"))) return st;
     if ((st = grow(w.d_g16, w.cap_g16, max_blocks * 128 * v.kb16, "IVF query blocks"))) return st;
@@ -897,10 +921,8 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
         return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
 
     // ---- probe + plan (groups of 128 queries) + gathered query blocks ----
-    // [8] and [9]: the work-item counters of the two tensor-core passes
-    cudaMemsetAsync(w.d_counters, 0, 10 * sizeof(unsigned long long), s);
-    cudaMemsetAsync(w.d_list_cnt, 0, nlist * sizeof(uint32_t), s);
-    cudaMemsetAsync(w.d_list_fill, 0, nlist * sizeof(uint32_t), s);
+    // counters [8] and [9]: the work-item counters of the two tensor-core passes
+    zero_plan(w, nlist, s);
     const ProbeLaunch pl{ix.d_qn,   nq,          static_cast<uint32_t>(ix.ds), static_cast<uint32_t>(ix.dp),
                          nlist,      np,          v.d_cent_t,  v.nlist_pad, v.d_offsets, w.d_pscore, w.d_probes,
                          w.d_list_cnt, w.d_q_slot_off, w.d_counters};
@@ -990,7 +1012,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
         uint32_t p2 = 1;
         while (p2 < kp) p2 <<= 1;
         ivf_merge_kernel<<<nq, 512, p2 * sizeof(uint64_t), s>>>(w.d_ws, w.d_q_slot_off, kp, ix.d_cand_idx, ix.d_cand_sim,
-                                                                ix.d_cand_cnt);
+                                                                ix.d_cand_cnt, nullptr, nullptr);
         count_launch();
         RerankArgs r;
         r.base = v.d_reordered;  // the slot keys hold list positions
@@ -1037,11 +1059,12 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
                                 ix.d_cnt2, cap2, k, q_thr, ix.d_rslots, o_idx, o_sim, o_cnt, ix.d_ok2, s, true,
                                 d_m, v.d_row_map);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
-    launch_compact_zero_flags(ix.d_ok2, nq, ix.d_tcfail, d_fail, s, d_m,
-                              CollectedSum{ix.d_cnt2, ix.d_ids, cap2, ix.d_fbn_rows()});
     // the plan's totals and the pass counts come back with the results
-    cudaMemcpyAsync(w.h_probed, w.d_counters, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ix.h_fbn, ix.d_fbn, CudaIndex::kFbnBytes, cudaMemcpyDeviceToHost, s);
+    BatchReport report = ix.batch_report();
+    report.by = ix.d_ids;
+    report.counters = w.d_counters;
+    report.host_counters = w.h_probed;
+    launch_compact_zero_flags(ix.d_ok2, nq, ix.d_tcfail, d_fail, s, d_m, report);
     ix.last_tc_n = nq;
     ix.stats.kernel_launches += groups ? 11 : 14;
     ix.stats.path = 5;

@@ -112,8 +112,7 @@ int search_device_noalloc(CudaIndex* ix, const float* d_queries, uint64_t nq, ui
         return code;
     };
     // The array keeps the previous call's contents: reset the words that must start clean.
-    cudaMemsetAsync(d_err, 0xFF, sizeof(unsigned long long), s);
-    cudaMemsetAsync(d_status, 0, sizeof(uint32_t), s);
+    cudaMemsetAsync(d_err, 0, 2 * sizeof(unsigned long long), s);
     for (uint64_t q0 = 0; q0 < nq; q0 += kMaxBatchChunk) {
         const uint64_t n = std::min<uint64_t>(kMaxBatchChunk, nq - q0);
         ScanPlan pl;

@@ -1430,24 +1430,24 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
 // ------------------------------------------------------------------------------------------
 
 // One block of 1024 threads: ids[0..m) = the indices i < n with flags[i] == 0, in order; count[0] = m.
-// With `live`, only the first live[0] flags count. With `sum`: also Σ min(cnt[j], cap) over the flags i
-// that count, j = by[i] (by given) or i — pass 2's collected rows, for the statistics.
+// With `live`, only the first live[0] flags count. With a report, what the host reads after the batch
+// (BatchReport), written to pinned memory here rather than by copies behind the kernel.
 __global__ void __launch_bounds__(1024) compact_zero_flags_kernel(const uint32_t* __restrict__ flags, uint32_t n,
                                                                   uint32_t* __restrict__ ids,
                                                                   uint32_t* __restrict__ count,
                                                                   const uint32_t* __restrict__ live,
-                                                                  const CollectedSum rows) {
+                                                                  const BatchReport rep) {
     __shared__ uint32_t warp_sum[32];
     __shared__ uint32_t base;
     __shared__ uint32_t warp_rows[32];
     if (live && *live < n) n = *live;
     if (threadIdx.x == 0) base = 0;
     __syncthreads();
-    if (rows.sum) {
+    if (rep.cnt) {
         uint32_t mine = 0;  // 16,384 flags of ≤ 8,192 rows: below 2³²
         for (uint32_t i = threadIdx.x; i < n; i += 1024) {
-            const uint32_t c = rows.cnt[rows.by ? rows.by[i] : i];
-            mine += c < rows.cap ? c : rows.cap;
+            const uint32_t c = rep.cnt[rep.by ? rep.by[i] : i];
+            mine += c < rep.cap ? c : rep.cap;
         }
         mine = __reduce_add_sync(0xFFFFFFFFu, mine);
         if ((threadIdx.x & 31u) == 0) warp_rows[threadIdx.x >> 5] = mine;
@@ -1473,17 +1473,21 @@ __global__ void __launch_bounds__(1024) compact_zero_flags_kernel(const uint32_t
     }
     if (threadIdx.x == 0) {
         count[0] = base;
-        if (rows.sum) {
+        if (rep.host_counts) {
             unsigned long long total = 0;
             for (uint32_t w = 0; w < 32; ++w) total += warp_rows[w];
-            *rows.sum = total;
+            rep.host_counts[1] = n;
+            rep.host_counts[2] = base;
+            *reinterpret_cast<unsigned long long*>(rep.host_counts + 4) = total;
         }
     }
+    if (rep.host_counters && threadIdx.x < 8) rep.host_counters[threadIdx.x] = rep.counters[threadIdx.x];
+    if (rep.host_flags && threadIdx.x < 2) rep.host_flags[threadIdx.x] = rep.flags[threadIdx.x];
 }
 
 void launch_compact_zero_flags(const uint32_t* flags, uint32_t n, uint32_t* ids, uint32_t* count, cudaStream_t s,
-                               const uint32_t* live, const CollectedSum& rows) {
-    compact_zero_flags_kernel<<<1, 1024, 0, s>>>(flags, n, ids, count, live, rows);
+                               const uint32_t* live, const BatchReport& report) {
+    compact_zero_flags_kernel<<<1, 1024, 0, s>>>(flags, n, ids, count, live, report);
     count_launch();
 }
 

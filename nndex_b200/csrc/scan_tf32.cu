@@ -14,7 +14,7 @@
 // (Cauchy–Schwarz on q·(x − x̂) + (q − q̂)·x̂). C·‖q‖‖x‖ bounds the rest: the tensor core's FP32
 // accumulation of ds products (4·ds·2⁻²³ of Σ|q̂_i x̂_i| ≤ ‖q‖‖x‖, the margin the BF16 scan takes),
 // the FP32 scan's own rounding ((ds/8 + 3)·2⁻²⁴) and the rounding of u itself (2⁻²²). The norms are
-// FP64 sums rounded up: ‖x‖ and ‖d_x‖ per row once per index (row_norms), ‖q‖ and ‖d_q‖ per query
+// FP64 sums rounded up: ‖x‖ and ‖d_x‖ per row once per index (row_norms, written by prep.cu with the rows), ‖q‖ and ‖d_q‖ per query
 // by the epilogue warps before the first tile.
 //
 // Each CTA keeps, per query, the k′ rows with the largest u. The merge keeps each query's k′ best,
@@ -57,8 +57,6 @@ constexpr int kTfThreads = 192;
 constexpr int kTfAcc = 8;                             // accumulators in flight
 constexpr uint32_t kTfTmemCols = 128;                 // kTfAcc × 16 columns
 constexpr uint32_t kTfIdesc = tc::instr_desc_tf32<kTfM, kTfN>();
-
-NNDEX_DEVICE_INLINE float tf32_head(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFFE000u); }
 
 NNDEX_DEVICE_INLINE uint8_t* align_1024(uint8_t* p) {
     const uint32_t a = smem_u32(p);
@@ -300,66 +298,6 @@ __global__ void __launch_bounds__(kTfThreads, 1)
         tc::fence_after_sync();
         tc::tmem_dealloc(tmem_base, kTfTmemCols);
     }
-}
-
-// Per row of the base: {‖x‖, ‖x − tf32_head(x)‖}, rounded up (one warp per row), and their maxima (a
-// NaN norm, of an overflowing sum, compares above every finite one as bits).
-__global__ void tf32_row_norms_kernel(const float* __restrict__ base, uint64_t rows, uint32_t ds,
-                                      float2* __restrict__ out, float2* __restrict__ max) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t w0 = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-    uint32_t mx = 0, my = 0;
-    for (uint64_t r = w0; r < rows; r += nw) {
-        const float2 n = warp_tf32_norms(base + r * ds, ds, lane);
-        if (lane == 0) out[r] = n;
-        mx = ::max(mx, __float_as_uint(n.x));
-        my = ::max(my, __float_as_uint(n.y));
-    }
-    if (lane == 0 && w0 < rows) {
-        atomicMax(reinterpret_cast<unsigned int*>(&max->x), mx);
-        atomicMax(reinterpret_cast<unsigned int*>(&max->y), my);
-    }
-}
-
-// One warp per query: its norms, then the bound of |s̃ − the FP32 scan's score| over all rows.
-__global__ void tf32_slack_kernel(const float* __restrict__ queries, uint32_t nq, uint32_t ds,
-                                  const float2* __restrict__ row_max, float c_norm, float* __restrict__ slack,
-                                  uint32_t* __restrict__ collected, uint32_t over_cap,
-                                  uint32_t* __restrict__ over_count) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (q >= nq) return;
-    const float2 n = warp_tf32_norms(queries + static_cast<size_t>(q) * ds, ds, lane);
-    if (lane != 0) return;
-    const float2 x = *row_max;
-    // the last term: products and operands below FP32's normal range, which either side may flush
-    const float e = (n.x * fmaf(c_norm, x.x, x.y) + n.y * (x.x + x.y)) * 1.01f +
-              (n.x + x.x + 1.0f) * static_cast<float>(ds) * 7.5231638e-37f;
-    // every partial sum of a score stays below ‖q‖‖x‖: far from overflow, or no bound is trusted
-    const bool trusted = n.x * x.x <= 1e37f && e <= 1e37f;
-    slack[q] = trusted ? e : INFINITY;
-    collected[q] = trusted ? 0u : over_cap;
-    if (q == 0) *over_count = 0;
-}
-
-cudaError_t launch_tf32_slack(const float* queries, uint32_t nq, uint32_t ds, const float2* row_max, float c_norm,
-                              float* slack, uint32_t* collected, uint32_t over_cap, uint32_t* over_count,
-                              cudaStream_t stream) {
-    if (nq == 0) return cudaSuccess;
-    tf32_slack_kernel<<<(nq + 3) / 4, 128, 0, stream>>>(queries, nq, ds, row_max, c_norm, slack, collected, over_cap,
-                                                        over_count);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_tf32_row_norms(const float* base, uint64_t rows, uint32_t ds, float2* out, float2* max,
-                                  uint32_t sm_count, cudaStream_t stream) {
-    if (rows == 0) return cudaSuccess;
-    const uint64_t blocks = std::min<uint64_t>((rows + 7) / 8, static_cast<uint64_t>(sm_count) * 8);
-    tf32_row_norms_kernel<<<static_cast<uint32_t>(blocks), 256, 0, stream>>>(base, rows, ds, out, max);
-    count_launch();
-    return cudaGetLastError();
 }
 
 // Deepest ring (8 down to 2 stages) whose footprint fits `smem_limit`; 0 if none.
