@@ -109,6 +109,7 @@ struct MergeArgs {
     const uint32_t* live = nullptr;     // optional: a device count; queries at or past it are skipped
     const uint32_t* out_rows = nullptr;  // optional: query q's results go to output row out_rows[q]
 };
+constexpr uint32_t kMergeBestK = 256;  // up to this k a query's keys are merged by one block
 uint32_t merge_parts(uint64_t per_query, uint32_t k, uint32_t nq);
 cudaError_t launch_merge_topk(const MergeArgs& a, cudaStream_t stream);
 

@@ -479,6 +479,58 @@ __global__ void __launch_bounds__(IvfScanShape<QB>::kThreads, 1)
 // ------------------------------------------------------------------------------------------
 // 4. Merge: per query, the k best keys of its slots, sorted; unused result slots (0, 0.0f).
 // ------------------------------------------------------------------------------------------
+// k ≤ kMergeBestK (block_merge_best).
+__global__ void __launch_bounds__(256)
+    ivf_merge_best_kernel(const uint64_t* __restrict__ ws, const uint32_t* __restrict__ q_slot_off, uint32_t k,
+                          uint64_t* __restrict__ idx_out, float* __restrict__ sim_out, uint32_t* __restrict__ count_out,
+                          const unsigned long long* __restrict__ counters,
+                          unsigned long long* __restrict__ host_probed) {
+    __shared__ MergeScratch<256> s;
+    const uint32_t q = blockIdx.x;
+    // the plan's row totals for the statistics, into pinned memory
+    if (host_probed && q == 0 && threadIdx.x < 3) host_probed[threadIdx.x] = counters[3 + threadIdx.x];
+    const uint64_t* keys = ws + static_cast<uint64_t>(q_slot_off[q]) * k;
+    const uint32_t n = (q_slot_off[q + 1] - q_slot_off[q]) * k;
+    uint64_t* oi = idx_out + static_cast<uint64_t>(q) * k;
+    float* os = sim_out + static_cast<uint64_t>(q) * k;
+    const uint32_t kk = block_merge_best<256>(
+        keys, n, k, s,
+        [&](uint32_t j, uint64_t key) {
+            oi[j] = key_row(key);
+            os[j] = key_score(key);
+        },
+        [&]() {
+            // more keys above the cut than the list holds: the exact k-th by radix selection
+            __shared__ BlockSelectScratch sel;
+            const uint64_t kth = block_radix_kth(keys, n, k, sel);
+            if (threadIdx.x == 0) s.count = 0;
+            __syncthreads();
+            for (uint32_t i0 = 0; i0 < n; i0 += blockDim.x) {
+                const uint32_t i = i0 + threadIdx.x;
+                const uint64_t key = i < n ? keys[i] : 0ull;
+                const bool take = key != 0ull && key >= kth;
+                const uint32_t at = warp_append(&s.count, take);
+                if (take && at < k) s.list[at] = key;
+            }
+            __syncthreads();
+            const uint32_t c = s.count < k ? s.count : k;
+            uint32_t p2 = 1;
+            while (p2 < c) p2 <<= 1;
+            for (uint32_t i = c + threadIdx.x; i < p2; i += blockDim.x) s.list[i] = 0ull;
+            block_bitonic_sort_desc(s.list, p2);
+            for (uint32_t j = threadIdx.x; j < c; j += blockDim.x) {
+                oi[j] = key_row(s.list[j]);
+                os[j] = key_score(s.list[j]);
+            }
+            return c;
+        });
+    for (uint32_t j = kk + threadIdx.x; j < k; j += blockDim.x) {
+        oi[j] = 0;
+        os[j] = 0.0f;
+    }
+    if (threadIdx.x == 0 && count_out) count_out[q] = kk;
+}
+
 __global__ void __launch_bounds__(512)
     ivf_merge_kernel(const uint64_t* __restrict__ ws, const uint32_t* __restrict__ q_slot_off, uint32_t k,
                      uint64_t* __restrict__ idx_out, float* __restrict__ sim_out, uint32_t* __restrict__ count_out,
@@ -649,6 +701,19 @@ cudaError_t launch_scan(const CUtensorMap& tmap, const IvfScanArgs& a, uint32_t 
     return cudaGetLastError();
 }
 
+void launch_ivf_merge(const IvfScratch& w, uint32_t nq, uint32_t k, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
+                      const unsigned long long* counters, unsigned long long* host_probed, cudaStream_t s) {
+    if (k <= kMergeBestK) {
+        ivf_merge_best_kernel<<<nq, 256, 0, s>>>(w.d_ws, w.d_q_slot_off, k, o_idx, o_sim, o_cnt, counters, host_probed);
+    } else {
+        uint32_t p2 = 1;
+        while (p2 < k) p2 <<= 1;
+        ivf_merge_kernel<<<nq, 512, p2 * sizeof(uint64_t), s>>>(w.d_ws, w.d_q_slot_off, k, o_idx, o_sim, o_cnt, counters,
+                                                               host_probed);
+    }
+    count_launch();
+}
+
 // The sampled pass-1 stride of the tensor-core list scan's rules.
 uint32_t ivf_sampled_stride() {
     static const uint32_t sampled = [] {
@@ -794,8 +859,6 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
     a.counters = w.d_counters;
     a.ws = w.d_ws;
     a.status = ix.w_status;
-    uint32_t p2 = 1;
-    while (p2 < k) p2 <<= 1;
     if (!w.h_probed) bump_alloc_epoch();
     if (!w.h_probed && cudaMallocHost(&w.h_probed, 8 * sizeof(unsigned long long)) != cudaSuccess)
         return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
@@ -819,10 +882,8 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
         }
         ix.scan_event_end(s, ev_a);
         if (e != cudaSuccess) return cuda_error(e, "IVF scan launch");
-        ivf_merge_kernel<<<n, 512, p2 * sizeof(uint64_t), s>>>(w.d_ws, w.d_q_slot_off, k, o_idx + static_cast<uint64_t>(q0) * k,
-                                                               o_sim + static_cast<uint64_t>(q0) * k,
-                                                               o_cnt ? o_cnt + q0 : nullptr, w.d_counters, w.h_probed);
-        count_launch();
+        launch_ivf_merge(w, n, k, o_idx + static_cast<uint64_t>(q0) * k, o_sim + static_cast<uint64_t>(q0) * k,
+                         o_cnt ? o_cnt + q0 : nullptr, w.d_counters, w.h_probed, s);
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "IVF merge launch");
         ix.stats.kernel_launches += 6;
     }
@@ -1009,11 +1070,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
         e = launch_scan_tc(a, false, 0, s);
         ix.scan_event_end(s, ev_a);
         if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch");
-        uint32_t p2 = 1;
-        while (p2 < kp) p2 <<= 1;
-        ivf_merge_kernel<<<nq, 512, p2 * sizeof(uint64_t), s>>>(w.d_ws, w.d_q_slot_off, kp, ix.d_cand_idx, ix.d_cand_sim,
-                                                                ix.d_cand_cnt, nullptr, nullptr);
-        count_launch();
+        launch_ivf_merge(w, nq, kp, ix.d_cand_idx, ix.d_cand_sim, ix.d_cand_cnt, nullptr, nullptr, s);
         RerankArgs r;
         r.base = v.d_reordered;  // the slot keys hold list positions
         r.row_map = v.d_row_map;

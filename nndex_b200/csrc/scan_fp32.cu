@@ -357,6 +357,43 @@ NNDEX_DEVICE_INLINE void merge_final(const uint64_t* keys, uint64_t n, uint32_t 
 
 }  // namespace
 
+// k ≤ kMergeBestK: one block per query (block_merge_best). Bound by latency: two rounds of loads, one
+// warp's selection, the ranks. One query's 148 lists of 10: 6.5 us, where the split kernel below spent
+// 12.5; 148 lists of 100: 13.6 (20); 16 queries with 148 lists of 64, 256 kept: 19 (29). Blocks of
+// 1,024 threads were no faster on the long lists.
+template <int NT>
+__global__ void __launch_bounds__(NT) merge_best_kernel(const uint64_t* __restrict__ ws_keys, uint64_t per_query,
+                                                        uint32_t k, uint32_t out_stride, uint64_t* __restrict__ idx_out,
+                                                        float* __restrict__ sim_out, uint32_t* __restrict__ count_out,
+                                                        const uint32_t* __restrict__ live,
+                                                        const uint32_t* __restrict__ out_rows) {
+    if (live && blockIdx.x >= *live) return;  // a fallback merge: only the queries re-run
+    __shared__ MergeScratch<NT> s;
+    const uint32_t q = blockIdx.x, oq = out_rows ? out_rows[q] : q;
+    const uint64_t* keys = ws_keys + static_cast<size_t>(q) * per_query;
+    uint64_t* oi = idx_out + static_cast<size_t>(oq) * out_stride;
+    float* os = sim_out + static_cast<size_t>(oq) * out_stride;
+    bool done = false;
+    const uint32_t kk = block_merge_best<NT>(
+        keys, static_cast<uint32_t>(per_query), k, s,
+        [&](uint32_t j, uint64_t key) {
+            oi[j] = key_row(key);
+            os[j] = key_score(key);
+        },
+        [&]() {
+            __shared__ BlockSelectScratch sel;
+            merge_final(keys, per_query, k, oq, out_stride, idx_out, sim_out, count_out, sel, s.list);
+            done = true;
+            return k;
+        });
+    if (done) return;
+    for (uint32_t j = kk + threadIdx.x; j < out_stride; j += NT) {
+        oi[j] = 0;
+        os[j] = 0.0f;
+    }
+    if (threadIdx.x == 0 && count_out) count_out[oq] = kk;
+}
+
 // grid (parts, nq); dynamic shared memory: p2(k) keys for the sort, plus parts·k keys when
 // parts > 1 (the survivors, staged for the final merge).
 __global__ void __launch_bounds__(512) merge_topk_kernel(const uint64_t* __restrict__ ws_keys, uint64_t per_query,
@@ -690,6 +727,7 @@ cudaError_t launch_scan_fp32(const ScanArgs& a, const ScanPlan& p, cudaStream_t 
 }
 
 uint32_t merge_parts(uint64_t per_query, uint32_t k, uint32_t nq) {
+    if (k <= kMergeBestK) return 1;  // merge_best_kernel
     const uint64_t lists = k ? per_query / k : 0;
     uint64_t parts = lists < 16 ? lists : 16;
     while (parts > 1 && parts * k > 4096) --parts;  // survivors staged in shared memory
@@ -702,6 +740,17 @@ uint32_t merge_parts(uint64_t per_query, uint32_t k, uint32_t nq) {
 }
 
 cudaError_t launch_merge_topk(const MergeArgs& a, cudaStream_t stream) {
+    if (a.k <= kMergeBestK && a.per_query < (1ull << 31)) {
+        // few keys: small blocks, of which many fit an SM
+        if (a.k <= 64 && a.per_query <= 1024)
+            merge_best_kernel<128><<<a.nq, 128, 0, stream>>>(a.ws_keys, a.per_query, a.k, a.out_stride, a.idx_out,
+                                                             a.sim_out, a.count_out, a.live, a.out_rows);
+        else
+            merge_best_kernel<512><<<a.nq, 512, 0, stream>>>(a.ws_keys, a.per_query, a.k, a.out_stride, a.idx_out,
+                                                             a.sim_out, a.count_out, a.live, a.out_rows);
+        count_launch();
+        return cudaGetLastError();
+    }
     uint32_t p2 = 1;
     while (p2 < a.k) p2 <<= 1;
     const uint32_t parts = (a.part_keys && a.part_done) ? merge_parts(a.per_query, a.k, a.nq) : 1u;

@@ -217,4 +217,85 @@ NNDEX_DEVICE_INLINE void block_bitonic_sort_desc(uint64_t* a, uint32_t n) {
     __syncthreads();
 }
 
+// ---- the k best of a query's candidate keys, by one block ------------------------------------
+//
+// Each thread keeps the largest of the keys it reads (dealt round-robin); the k-th largest of these
+// maxima (one warp's radix select) is a cut that at least k keys reach and hardly more do, so one
+// more read lists about k keys, and their ranks among themselves place them. Exact whatever the
+// keys: only a list that does not hold every key above the cut sends the block to `overflow`.
+template <int NT>
+struct MergeScratch {
+    static constexpr uint32_t kList = 1024;
+    uint64_t list[kList];
+    uint32_t hist[256];
+    unsigned long long cut;
+    uint32_t count;
+};
+
+// put(j, key) for each of the min(k, non-empty keys) best of keys[0, n) (distinct; 0 = empty slot) at its
+// rank j; returns their number. k ≤ NT. overflow() returns the count after doing the same another way.
+template <int NT, class Put, class Overflow>
+NNDEX_DEVICE_INLINE uint32_t block_merge_best(const uint64_t* __restrict__ keys, uint32_t n, uint32_t k,
+                                              MergeScratch<NT>& s, Put&& put, Overflow&& overflow) {
+    static_assert(NT <= static_cast<int>(MergeScratch<NT>::kList), "the maxima share the list");
+    constexpr int U = 8;  // loads in flight; the keys stay in registers where one round reads them all
+    const uint32_t tid = threadIdx.x;
+    uint64_t best = 0, x[U];
+    for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? keys[i0 + u * NT + tid] : 0ull;
+#pragma unroll
+        for (int u = 0; u < U; ++u) best = x[u] > best ? x[u] : best;
+    }
+    // small k: the maxima of 2, 4, … threads together, still four times as many as k
+    uint32_t o = 1;
+    for (; o < 32 && NT / (2 * o) >= 4 * k && NT / (2 * o) >= 32; o <<= 1) {
+        const uint64_t other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other > best ? other : best;
+    }
+    if ((tid & (o - 1)) == 0) s.list[tid / o] = best;
+    if (tid == 0) s.count = 0;
+    __syncthreads();
+    if (tid < 32) {
+        const uint64_t kth = warp_radix_kth(s.list, NT / o, k, s.hist);
+        if (tid == 0) s.cut = kth ? kth : 1ull;  // fewer keys than that: all of them
+    }
+    __syncthreads();
+    const uint64_t cut = s.cut;
+    for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
+        if (n > U * NT) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? keys[i0 + u * NT + tid] : 0ull;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool take = x[u] >= cut;
+            const uint32_t at = warp_append(&s.count, take);
+            if (take && at < MergeScratch<NT>::kList) s.list[at] = x[u];
+        }
+    }
+    __syncthreads();
+    const uint32_t c = s.count;
+    if (c > MergeScratch<NT>::kList) {
+        __syncthreads();
+        return overflow();
+    }
+    const uint32_t kk = c < k ? c : k;
+    if (c <= 192) {
+        for (uint32_t t = tid; t < c; t += NT) {
+            const uint64_t mine = s.list[t];
+            uint32_t rank = 0;
+            for (uint32_t j = 0; j < c; ++j) rank += s.list[j] > mine ? 1u : 0u;
+            if (rank < kk) put(rank, mine);
+        }
+        return kk;
+    }
+    uint32_t p2 = 256;
+    while (p2 < c) p2 <<= 1;
+    for (uint32_t t = c + tid; t < p2; t += NT) s.list[t] = 0ull;
+    block_bitonic_sort_desc(s.list, p2);
+    for (uint32_t j = tid; j < kk; j += NT) put(j, s.list[j]);
+    return kk;
+}
+
 }  // namespace nndex
