@@ -489,10 +489,8 @@ CudaIndex::Tf32BatchPlan CudaIndex::plan_tf32_batch(uint64_t nq, uint64_t kcap) 
         stride /= 2;
     if (tiles * 32 < 4 * kp) return p;
     const uint32_t nchunks = static_cast<uint32_t>(ds / 32);
-    // the query block resident beside at least three ring stages, else its slabs with every stage
-    uint32_t stages = tc_stages_for(nchunks, 0, false, false, smem_optin);
-    const bool stream_a = stages < 3;
-    if (stream_a) stages = tc_stages_for(nchunks, 0, false, true, smem_optin);
+    bool stream_a = false;
+    const uint32_t stages = tc_tf32_stages_for(nchunks, smem_optin, &stream_a);
     if (!stages) return p;
     plan_groups(static_cast<uint32_t>((nq + 127) / 128), static_cast<uint32_t>(kp), stride, p.group, p.span, p.gm_tiles,
                 p.nranges, p.range_rows);

@@ -392,6 +392,10 @@ struct CudaIndex {
     void mark_done(cudaStream_t s);
 };
 
+// Tensor map of a row-major matrix (inner × outer elements), 2-D boxes.
+bool encode_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
+                    uint64_t inner, uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner,
+                    uint32_t box_outer, CUtensorMapSwizzle swizzle);
 int make_view(const CudaIndex& src, CudaIndex** out);
 int index_begin(uint64_t rows, uint64_t dims, uint32_t flags, const nndex_cuda_opts* opts, CudaIndex** out);
 void index_prep_rows(CudaIndex* ix, const float* d_src, uint64_t row0, uint64_t n);

@@ -178,6 +178,8 @@ struct TcParams {
     uint32_t gm_span = 1;                 // a power of two, at most kMaxGroupSpan
     unsigned long long* thr_global = nullptr;  // pass 1: per query, zeroed before the launch
     uint64_t* ws_keys = nullptr;          // pass 1: nq × nranges × kprime
+    float* scores = nullptr;              // mode 3: nq × score_stride (a multiple of 256, ≥ rows)
+    uint64_t score_stride = 0;
     const float* q_thr = nullptr;         // pass 2: per query T (exact k-th score of pass 1)
     uint32_t* cand_rows = nullptr;        // pass 2: nq × cap2
     uint32_t* cand_cnt = nullptr;         // pass 2: nq, zeroed before the launch
@@ -217,12 +219,15 @@ struct TcArgs {
 size_t tc_smem_bytes(uint32_t nchunks, uint32_t kprime, uint32_t stages, bool fp8, bool stream_a, uint32_t qb = 1);
 // Deepest base ring (4, 3 or 2 stages) that fits k′ heaps in `smem_limit`; 0 if none fits.
 uint32_t tc_stages_for(uint32_t nchunks, uint32_t kprime, bool fp8, bool stream_a, size_t smem_limit);
+// TF32 scans (32 values per slab): the query block resident beside at least three ring stages, else its
+// slabs with every stage.
+uint32_t tc_tf32_stages_for(uint32_t nchunks, size_t smem_limit, bool* stream_a);
 // Pass 2 with two resident query blocks per CTA: the deepest ring (5 or 4 stages of 128-row slabs)
 // that fits beside both blocks' query slabs; 0 if none (large D).
 uint32_t tc_pair_stages_for(uint32_t nchunks, bool fp8, size_t smem_limit);
 // Ring stages of a CTA-pair pass 2 (TcArgs::qb = 3) that fit, 0 when none does.
 uint32_t tc_cta_pair_stages_for(uint32_t nchunks, bool fp8, size_t smem_limit);
-// mode 0: pass 1 with heaps; 1: pass 2; 2: a sampled pass 1 that writes group maxima.
+// mode 0: pass 1 with heaps; 1: pass 2; 2: a sampled pass 1 that writes group maxima; 3: every score.
 cudaError_t launch_scan_tc(const TcArgs& a, int type, int mode, cudaStream_t stream);
 
 // T (and the candidates it came from) of a group-maxima pass; lists every query for pass 2.

@@ -27,6 +27,8 @@ struct IvfIndex {
     uint64_t nlist_pad = 0;      // nlist rounded up to 256 (assignment GEMM tiles, dims-major stride)
     float* d_centroids = nullptr;  // nlist × ds FP32, final centroids (zero padded)
     float* d_cent_t = nullptr;     // ds × nlist_pad FP32, the same centroids dims-major (probe)
+    CUtensorMap tmap_cent{};       // the centroids, box {32 floats, 256 rows} (probe scores)
+    float2* d_cent_max = nullptr;  // the largest ‖c‖ and ‖c − tf32_head(c)‖, rounded up
     float* d_reordered = nullptr;  // rows_alloc × ds FP32, cluster-contiguous copy of the base
     uint32_t* d_row_map = nullptr; // rows: reordered position → original row
     uint32_t* d_offsets = nullptr; // nlist + 1
@@ -51,7 +53,7 @@ struct IvfScratch {
     uint32_t nprobe = 0;                // 0 = choose_nprobe per search
     uint32_t tc_stride = 1;             // tensor-core scan: pass 1 on every n-th tile (autotuned)
     uint32_t* d_probes = nullptr;       size_t cap_probes = 0;
-    float* d_pscore = nullptr;          size_t cap_pscore = 0;     // B·nlist: centroid scores of the probe
+    float* d_pscore = nullptr;          size_t cap_pscore = 0;     // B·nlist_pad: centroid scores of the probe
     // The words a search starts from zero, in one buffer: 16 counters (work counters, totals, rows
     // probed), then per list the queries probing it and its fill. Query prep zeroes them for the
     // search behind it (zeroed); the views below point into it.

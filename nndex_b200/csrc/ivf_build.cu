@@ -45,10 +45,6 @@
 
 namespace nndex {
 
-bool encode_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
-                    uint64_t inner, uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner,
-                    uint32_t box_outer, CUtensorMapSwizzle swizzle);
-
 namespace {
 
 NNDEX_DEVICE_INLINE uint8_t* align_1024(uint8_t* p) {
@@ -955,6 +951,28 @@ __global__ void centroid_normalize_kernel(const double* __restrict__ sums, uint3
         out[d] = d < dp ? __double2float_rn(__dmul_rn(sc[d], inv_norm)) : 0.0f;
 }
 
+// The largest ‖c‖ and ‖c − tf32_head(c)‖ over the final centroids, rounded up, raised into *max (zeroed
+// before): the probe's TF32 bound. One warp per centroid.
+__global__ void centroid_tf32_max_kernel(const float* __restrict__ cent, uint32_t ds, uint32_t nlist,
+                                         float2* __restrict__ max) {
+    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (c >= nlist) return;
+    double n2 = 0.0, r2 = 0.0;
+    for (uint32_t d = lane; d < ds; d += 32) {
+        const float v = cent[static_cast<uint64_t>(c) * ds + d];
+        const float e = v - tf32_head(v);
+        n2 = fma(static_cast<double>(v), static_cast<double>(v), n2);
+        r2 = fma(static_cast<double>(e), static_cast<double>(e), r2);
+    }
+    n2 = warp_sum_d(n2);
+    r2 = warp_sum_d(r2);
+    if (lane == 0) {
+        atomicMax(reinterpret_cast<unsigned int*>(&max->x), __float_as_uint(sqrt_up(n2)));
+        atomicMax(reinterpret_cast<unsigned int*>(&max->y), __float_as_uint(sqrt_up(r2)));
+    }
+}
+
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
@@ -964,6 +982,7 @@ IvfIndex::~IvfIndex() {
     cudaFree(d_res16);
     cudaFree(d_centroids);
     cudaFree(d_cent_t);
+    cudaFree(d_cent_max);
     cudaFree(d_reordered);
     cudaFree(d_row_map);
     cudaFree(d_offsets);
@@ -1059,6 +1078,11 @@ static cudaError_t ivf_enqueue_layout(CudaIndex& ix, IvfIndex& v, unsigned int* 
     const cudaStream_t s = ix.stream;
     const uint64_t kb16 = (ix.dims + 63) / 64 * 64;
     cudaError_t e;
+    if ((e = cudaMalloc(&v.d_cent_max, sizeof(float2))) != cudaSuccess) return e;
+    cudaMemsetAsync(v.d_cent_max, 0, sizeof(float2), s);
+    centroid_tf32_max_kernel<<<static_cast<unsigned>((v.nlist * 32 + 255) / 256), 256, 0, s>>>(
+        v.d_centroids, static_cast<uint32_t>(ds), static_cast<uint32_t>(v.nlist), v.d_cent_max);
+    count_launch();
     if ((e = cudaMalloc(&v.d_reordered, ix.rows_alloc * ds * sizeof(float))) != cudaSuccess) return e;
     cudaMemsetAsync(v.d_reordered + rows * ds, 0, (ix.rows_alloc - rows) * ds * sizeof(float), s);
     const uint32_t gb = static_cast<uint32_t>(std::min<uint64_t>((rows * 32 + 255) / 256, ix.sm_count * 16ull));
@@ -1084,7 +1108,9 @@ static int ivf_complete_layout(CudaIndex& ix, IvfIndex& v, unsigned int eps_bits
     if (!encode_tmap_2d(&v.tmap_reordered, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, v.d_reordered, ix.ds, ix.rows_alloc,
                         ix.ds * sizeof(float), 32, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tmap_2d(&v.tmap_reordered16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, v.d_reordered16, v.kb16,
-                        ix.rows_alloc, v.kb16 * 2, 64, 256, CU_TENSOR_MAP_SWIZZLE_128B))
+                        ix.rows_alloc, v.kb16 * 2, 64, 256, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_tmap_2d(&v.tmap_cent, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, v.d_centroids, ix.ds, v.nlist,
+                        ix.ds * sizeof(float), 32, 256, CU_TENSOR_MAP_SWIZZLE_128B))
         return set_error(NNDEX_ERR_CUDA, "cuda execution error: cuTensorMapEncodeTiled failed (IVF rows)");
     std::memcpy(&v.eps16, &eps_bits, sizeof(float));
     if (ix.kb16 == 0) ix.kb16 = v.kb16;  // BF16 query copies for the tensor-core list scan

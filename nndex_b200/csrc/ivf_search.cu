@@ -2,9 +2,9 @@
 //
 // Replaces candidate_clusters(_batch) (src/approx.rs:159-300) and search_approx /
 // search_batch_approx (src/cpu.rs:425-502). A batch runs as six launches and no host round trip:
-//   1. probe (two launches): per query, dot_small against every centroid (FP64 in index order, f32
-//      result — the reference's value; up to 8 queries share each read of a centroid) and the nprobe
-//      best clusters (score desc, lower index on ties).
+//   1. probe (two launches): per query, the nprobe best clusters by dot_small (FP64 in index order, f32
+//      result — the reference's value; score desc, lower index on ties): TF32 scores of every centroid
+//      from the tensor cores with a rigorous bound, and exact scores only of the clusters it leaves open.
 //   2. plan (a one-block scan, then one warp per query): the (list, query) pairs grouped by list,
 //      each list cut into chunks of at most kChunkRows rows, and work items (list chunk × group of up
 //      to QB queries probing it), with every (query, list chunk) owning one output slot of k keys.
@@ -16,6 +16,7 @@
 // Lists probed by many queries are read once per group of QB queries: the list scan is bounded by
 // the union of probed rows, not by the sum over queries.
 #include <algorithm>
+#include <cfloat>
 
 #include "common.cuh"
 #include "index.h"
@@ -133,6 +134,34 @@ NNDEX_DEVICE_INLINE uint64_t warp_radix_kth(const float* scores, uint32_t n, uin
     return prefix;
 }
 
+// The reference's f32 dot (FP64 accumulation in index order, src/approx.rs:539-552) of a query in shared
+// memory, as doubles, and a centroid row, n values (a multiple of 8), by 8 consecutive lanes (j of 8, all
+// of the warp calling); every lane returns it. The lanes add in another order: both sums are within
+// n·2⁻⁵³·Σ|xy| ≤ err / 2 of the exact value, so where every value within err rounds to one f32, that is the
+// reference's. Where it does not (about once in 10⁷) they add in index order.
+NNDEX_DEVICE_INLINE float dot_f64_row8(const double* q_s, const float* __restrict__ row, uint32_t n, double err,
+                                       uint32_t j, bool live) {
+    double s = 0.0;
+    if (live) {
+#pragma unroll 4
+        for (uint32_t d = 4 * j; d < n; d += 32) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(row + d));
+            s = fma(q_s[d], static_cast<double>(v.x), s);
+            s = fma(q_s[d + 1], static_cast<double>(v.y), s);
+            s = fma(q_s[d + 2], static_cast<double>(v.z), s);
+            s = fma(q_s[d + 3], static_cast<double>(v.w), s);
+        }
+    }
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
+    s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
+    if (live && __double2float_rn(s - err) != __double2float_rn(s + err)) {
+        s = 0.0;
+        for (uint32_t d = 0; d < n; ++d) s = fma(q_s[d], static_cast<double>(row[d]), s);
+    }
+    return __double2float_rn(s);
+}
+
 constexpr uint32_t kProbeCentroids = 256;  // centroids per scoring block
 constexpr uint32_t kProbeThreads = 128;    // two centroids per thread
 
@@ -221,6 +250,154 @@ __global__ void __launch_bounds__(256)
     if (lane == 0) {
         q_slot_off[q] = slots;
         atomicAdd(&counters[3], rows);  // zeroed once per search: Σ over sub-batches
+    }
+}
+
+// The probe of up to kProbePick lists, also in two launches:
+//    (a) Scores: the tensor cores score every centroid as TF32 (scan_tc_kernel's kMode 3).
+//    (b) Pick: one block per query. With ε a bound of |TF32 score − the reference's f32 score| over all
+//        centroids and L the np-th largest TF32 score, a list above L + 2ε is probed and one below L − 2ε
+//        is not, whatever their exact scores; only the few between them are scored as the reference
+//        does (FP64 in index order), and the best of those fill the remaining places. The same lists as
+//        from exact scores, in another order, which nothing depends on. Writes the lists and the plan's
+//        counts like the selection above.
+//    Bound by latency (its barriers, then the rows between the bounds from L2). 1,024 queries against 1,414
+//    centroids of 384 dims: scores 17 us + pick 36, where the FP64 scores of every pair and the warp
+//    selection took 94 + 25; one query against 512 of 128: 4.5 + 8.2, before 15 + 7.4. (Exact scores
+//    as one thread's chain of FP64 adds per list: pick 54 and 10 us.)
+constexpr uint32_t kProbePick = 512;
+constexpr uint32_t kProbeBand = 256;  // lists between the certain ones scored from shared memory
+
+template <int NT>
+__global__ void __launch_bounds__(NT, NT <= 128 ? 8 : 1)
+    ivf_probe_pick_kernel(float* __restrict__ scores, uint64_t stride, uint32_t nlist, uint32_t np,
+                          const float* __restrict__ queries, uint32_t ds, uint32_t dp,
+                          const float* __restrict__ centroids, const float2* __restrict__ cent_max, float c_norm,
+                          const uint32_t* __restrict__ offsets, uint32_t* __restrict__ probes,
+                          uint32_t* __restrict__ list_cnt, uint32_t* __restrict__ q_slot_off,
+                          unsigned long long* __restrict__ counters) {
+    __shared__ MergeScratch<NT> s;
+    __shared__ uint64_t band_key[kProbeBand];
+    __shared__ uint32_t picked[kProbePick], band[kProbeBand];
+    __shared__ double norm_part[2][NT / 32];
+    __shared__ uint32_t n_in, n_band, n_slots;
+    __shared__ unsigned long long n_rows;
+    __shared__ float sh_l, sh_e2;
+    __shared__ double sh_err;
+    extern __shared__ __align__(16) double q_d[];
+    const uint32_t q = blockIdx.x, tid = threadIdx.x;
+    const float* qv = queries + static_cast<uint64_t>(q) * ds;
+    float* sq = scores + static_cast<uint64_t>(q) * stride;
+    double s1 = 0.0, s2 = 0.0;
+    for (uint32_t d = tid; d < ds; d += NT) {
+        const float x = qv[d], e = x - tf32_head(x);
+        q_d[d] = static_cast<double>(x);
+        s1 = fma(static_cast<double>(x), static_cast<double>(x), s1);
+        s2 = fma(static_cast<double>(e), static_cast<double>(e), s2);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s1 += __shfl_xor_sync(0xFFFFFFFFu, s1, o);
+        s2 += __shfl_xor_sync(0xFFFFFFFFu, s2, o);
+    }
+    if ((tid & 31u) == 0) {
+        norm_part[0][tid >> 5] = s1;
+        norm_part[1][tid >> 5] = s2;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        n_in = n_band = n_slots = 0;
+        n_rows = 0;
+        s1 = s2 = 0.0;
+        for (uint32_t w = 0; w < NT / 32; ++w) {
+            s1 += norm_part[0][w];
+            s2 += norm_part[1][w];
+        }
+        // (1e-12: the sums' own rounding)
+        const float nq = __double2float_ru(__dsqrt_ru(s1 * (1.0 + 1e-12)));
+        const float rq = __double2float_ru(__dsqrt_ru(s2 * (1.0 + 1e-12)));
+        const float2 c = *cent_max;
+        // K12's ε at the centroids' maxima; the last term covers values below FP32's normal range
+        const float e = (nq * fmaf(c_norm, c.x, c.y) + rq * (c.x + c.y)) * 1.01f +
+                        (nq + c.x + 1.0f) * static_cast<float>(ds) * 7.5231638e-37f;
+        sh_e2 = (nq * c.x <= 1e37f && e <= 1e37f) ? 2.0f * e : INFINITY;
+        sh_l = -INFINITY;
+        sh_err = static_cast<double>(nq) * static_cast<double>(c.x) * static_cast<double>(dp) * 4.5e-16;  // 2·2⁻⁵³·2
+    }
+    __syncthreads();
+    bool all_exact = !(sh_e2 <= FLT_MAX);  // no bound: every list by its exact score
+    if (np < nlist && !all_exact) {
+        block_merge_best<NT>(
+            [&](uint32_t i) { return make_key(sq[i], i); }, nlist, np, s,
+            [&](uint32_t j, uint64_t key) {
+                if (j == np - 1) sh_l = key_score(key);
+            },
+            [&]() {
+                all_exact = true;  // (mass ties)
+                return 0u;
+            });
+        __syncthreads();
+    }
+    const float hi = sh_l + sh_e2, lo = sh_l - sh_e2;
+    for (uint32_t i0 = 0; i0 < nlist; i0 += NT) {
+        const uint32_t i = i0 + tid;
+        const float x = i < nlist ? sq[i] : 0.0f;
+        const bool in = i < nlist && (np >= nlist || (!all_exact && x > hi));
+        const bool maybe = i < nlist && !in && (all_exact || x >= lo);
+        const uint32_t a = warp_append(&n_in, in), b = warp_append(&n_band, maybe);
+        if (in && a < kProbePick) picked[a] = i;
+        if (maybe && b < kProbeBand) band[b] = i;
+    }
+    __syncthreads();
+    const uint32_t nb = n_band, nin = n_in, r = np < nlist ? np - nin : 0u;  // places left
+    if (nb <= kProbeBand) {
+        for (uint32_t t0 = 0; t0 < nb; t0 += NT / 8) {
+            const uint32_t t = t0 + tid / 8;
+            const uint32_t c = t < nb ? band[t] : 0u;
+            const float x = dot_f64_row8(q_d, centroids + static_cast<uint64_t>(c) * ds, dp, sh_err, tid & 7u, t < nb);
+            if (t < nb && (tid & 7u) == 0) band_key[t] = make_key(fold_zero(x), c);
+        }
+        __syncthreads();
+        for (uint32_t t = tid; t < nb; t += NT) {
+            uint32_t rank = 0;
+            for (uint32_t j = 0; j < nb; ++j) rank += band_key[j] > band_key[t] ? 1u : 0u;
+            if (rank < r) picked[nin + rank] = band[t];
+        }
+    } else {
+        // too many to hold: their exact scores replace the approximate ones, the others' are set apart
+        for (uint32_t i0 = 0; i0 < nlist; i0 += NT / 8) {
+            const uint32_t i = i0 + tid / 8;
+            const bool maybe = i < nlist && (all_exact || (sq[i] <= hi && sq[i] >= lo));
+            const float x = dot_f64_row8(q_d, centroids + static_cast<uint64_t>(maybe ? i : 0) * ds, dp, sh_err, tid & 7u, maybe);
+            if (i < nlist && (tid & 7u) == 0) sq[i] = maybe ? fold_zero(x) : -FLT_MAX;
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < nlist; i += NT) {
+            if (sq[i] == -FLT_MAX) continue;
+            const uint64_t key = make_key(sq[i], i);
+            uint32_t rank = 0;
+            for (uint32_t j = 0; j < nlist; ++j) rank += (sq[j] != -FLT_MAX && make_key(sq[j], j) > key) ? 1u : 0u;
+            if (rank < r) picked[nin + rank] = i;
+        }
+    }
+    __syncthreads();
+    const uint32_t n = np < nlist ? np : nlist;
+    uint32_t slots = 0;
+    unsigned long long rows = 0;
+    for (uint32_t t = tid; t < n; t += NT) {
+        const uint32_t c = picked[t];
+        probes[static_cast<uint64_t>(q) * np + t] = c;
+        atomicAdd(&list_cnt[c], 1u);
+        const uint32_t len = offsets[c + 1] - offsets[c];
+        slots += (len + kChunkRows - 1) / kChunkRows;
+        rows += len;
+    }
+    if (slots) atomicAdd(&n_slots, slots);
+    if (rows) atomicAdd(&n_rows, rows);
+    __syncthreads();
+    if (tid == 0) {
+        q_slot_off[q] = n_slots;
+        atomicAdd(&counters[3], n_rows);  // zeroed once per search: Σ over sub-batches
     }
 }
 
@@ -494,7 +671,7 @@ __global__ void __launch_bounds__(256)
     uint64_t* oi = idx_out + static_cast<uint64_t>(q) * k;
     float* os = sim_out + static_cast<uint64_t>(q) * k;
     const uint32_t kk = block_merge_best<256>(
-        keys, n, k, s,
+        [&](uint32_t i) { return keys[i]; }, n, k, s,
         [&](uint32_t j, uint64_t key) {
             oi[j] = key_row(key);
             os[j] = key_score(key);
@@ -733,12 +910,13 @@ uint32_t probe_qb(uint64_t dp, size_t smem_optin) {
 }
 
 struct ProbeLaunch {
+    const CudaIndex* ix;
     const float* queries;
     uint32_t nq, ds, dp, nlist, np;
     const float* cent_t;
     uint64_t ct_stride;
     const uint32_t* offsets;
-    float* scores;  // nq × nlist
+    float* scores;  // nq × nlist, or nq × nlist_pad (ct_stride) from the tensor cores
     uint32_t* probes;
     uint32_t* list_cnt;
     uint32_t* q_slot_off;
@@ -760,23 +938,60 @@ cudaError_t launch_probe_qb(const ProbeLaunch& a, cudaStream_t s) {
 // plan's scans, the pairs).
 cudaError_t launch_probe_plan(uint32_t pqb, const ProbeLaunch& a, uint32_t qb, IvfScratch& w, uint32_t* qblock_off,
                               uint32_t* slot_row0, cudaStream_t s) {
-    if ((a.nlist + kProbeCentroids - 1) / kProbeCentroids > 65535u) return cudaErrorInvalidValue;
     cudaError_t e;
-    switch (pqb) {
-        case 8: e = launch_probe_qb<8>(a, s); break;
-        case 4: e = launch_probe_qb<4>(a, s); break;
-        case 2: e = launch_probe_qb<2>(a, s); break;
-        case 1: e = launch_probe_qb<1>(a, s); break;
-        default: return cudaErrorInvalidValue;
+    bool stream_a = false;
+    const uint32_t stages = a.np <= kProbePick ? tc_tf32_stages_for(a.ds / 32, a.ix->smem_optin, &stream_a) : 0;
+    if (stages && a.ds * sizeof(double) <= 64 * 1024) {
+        const CudaIndex& ix = *a.ix;
+        CUtensorMap tmap_q;
+        if (!encode_tmap_2d(&tmap_q, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(a.queries), a.ds, a.nq,
+                            a.ds * sizeof(float), 32, 128, CU_TENSOR_MAP_SWIZZLE_128B))
+            return cudaErrorInvalidValue;
+        TcArgs t;
+        t.tmap_q = &tmap_q;
+        t.tmap_b = &ix.ivf->tmap_cent;
+        t.stages = stages;
+        t.stream_a = stream_a;
+        uint64_t nranges = 0, range_rows = 0;
+        tc_range_split(a.nlist, (a.nq + 127) / 128, static_cast<uint64_t>(ix.sm_count), nranges, range_rows, 256);
+        t.nranges = static_cast<uint32_t>(nranges);
+        t.p.nq = a.nq;
+        t.p.nchunks = a.ds / 32;
+        t.p.rows = a.nlist;
+        t.p.range_rows = range_rows;
+        t.p.scores = a.scores;
+        t.p.score_stride = a.ct_stride;
+        t.p.status = ix.w_status;
+        if ((e = launch_scan_tc(t, kTcTf32, 3, s)) != cudaSuccess) return e;
+        const size_t smem = a.ds * sizeof(double);
+        // a few lists: small blocks, of which many fit an SM
+        auto pick = a.np <= 64 ? ivf_probe_pick_kernel<128> : ivf_probe_pick_kernel<512>;
+        if (smem > 24 * 1024 &&
+            (e = cudaFuncSetAttribute(pick, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))) != cudaSuccess)
+            return e;
+        pick<<<a.nq, a.np <= 64 ? 128 : 512, smem, s>>>(a.scores, a.ct_stride, a.nlist, a.np, a.queries, a.ds, a.dp,
+                                                        ix.ivf->d_centroids, ix.ivf->d_cent_max, ix.tf32_c_norm(),
+                                                        a.offsets, a.probes, a.list_cnt, a.q_slot_off, a.counters);
+        count_launch();
+    } else {
+        if ((a.nlist + kProbeCentroids - 1) / kProbeCentroids > 65535u) return cudaErrorInvalidValue;
+        switch (pqb) {
+            case 8: e = launch_probe_qb<8>(a, s); break;
+            case 4: e = launch_probe_qb<4>(a, s); break;
+            case 2: e = launch_probe_qb<2>(a, s); break;
+            case 1: e = launch_probe_qb<1>(a, s); break;
+            default: return cudaErrorInvalidValue;
+        }
+        if (e != cudaSuccess) return e;
+        ivf_probe_select_kernel<<<(a.nq + 7) / 8, 256, 0, s>>>(a.scores, a.nq, a.nlist, a.np, a.offsets, a.probes,
+                                                               a.list_cnt, a.q_slot_off, a.counters);
+        count_launch(2);
     }
-    if (e != cudaSuccess) return e;
-    ivf_probe_select_kernel<<<(a.nq + 7) / 8, 256, 0, s>>>(a.scores, a.nq, a.nlist, a.np, a.offsets, a.probes,
-                                                           a.list_cnt, a.q_slot_off, a.counters);
     ivf_plan_scan_kernel<<<1, 1024, 0, s>>>(a.nq, a.nlist, a.offsets, qb, w.d_list_cnt, w.d_list_qoff, w.d_item_off,
                                             w.d_q_slot_off, w.d_counters, qblock_off);
     ivf_plan_fill_kernel<<<(a.nq + 7) / 8, 256, 0, s>>>(a.probes, a.nq, a.np, a.offsets, w.d_list_qoff, w.d_list_fill,
                                                          w.d_q_slot_off, w.d_list_q, w.d_list_slot, slot_row0);
-    count_launch(4);
+    count_launch(2);
     return cudaGetLastError();
 }
 
@@ -836,7 +1051,7 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
     uint64_t per_query = std::max<uint64_t>(1, static_cast<uint64_t>(np) * max_chunks * k * 8);
     uint32_t sub = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(nq, ws_budget / per_query)));
     if ((st = grow(w.d_probes, w.cap_probes, static_cast<size_t>(sub) * np, "IVF probe buffer"))) return st;
-    if ((st = grow(w.d_pscore, w.cap_pscore, static_cast<size_t>(sub) * nlist, "IVF probe buffer"))) return st;
+    if ((st = grow(w.d_pscore, w.cap_pscore, static_cast<size_t>(sub) * v.nlist_pad, "IVF probe buffer"))) return st;
     if ((st = plan_buffer(w, nlist))) return st;
     if ((st = grow(w.d_list_qoff, w.cap_list_qoff, nlist + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_item_off, w.cap_item_off, nlist + 1, "IVF plan buffer"))) return st;
@@ -867,7 +1082,7 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
         const uint32_t n = std::min(sub, nq - q0);
         const float* qn = queries + static_cast<uint64_t>(q0) * ix.ds;
         if (q0) cudaMemsetAsync(w.d_list_cnt, 0, 2 * nlist * sizeof(uint32_t), s);  // and the fills behind it
-        const ProbeLaunch pl{qn,          n,          dq,           static_cast<uint32_t>(ix.dp), nlist, np,
+        const ProbeLaunch pl{&ix, qn,          n,          dq,           static_cast<uint32_t>(ix.dp), nlist, np,
                              v.d_cent_t,  v.nlist_pad, v.d_offsets, w.d_pscore, w.d_probes, w.d_list_cnt,
                              w.d_q_slot_off, w.d_counters};
         cudaError_t e = launch_probe_plan(pqb, pl, qb, w, nullptr, nullptr, s);
@@ -948,7 +1163,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     const uint32_t cap2 = kSecondPassCap;
     int st;
     if ((st = grow(w.d_probes, w.cap_probes, pairs, "IVF probe buffer"))) return st;
-    if ((st = grow(w.d_pscore, w.cap_pscore, static_cast<size_t>(nq) * nlist, "IVF probe buffer"))) return st;
+    if ((st = grow(w.d_pscore, w.cap_pscore, static_cast<size_t>(nq) * v.nlist_pad, "IVF probe buffer"))) return st;
     if ((st = plan_buffer(w, nlist))) return st;
     if ((st = grow(w.d_list_qoff, w.cap_list_qoff, nlist + 1, "IVF plan buffer"))) return st;
     if ((st = grow(w.d_item_off, w.cap_item_off, nlist + 1, "IVF plan buffer"))) return st;
@@ -984,7 +1199,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     // ---- probe + plan (groups of 128 queries) + gathered query blocks ----
     // counters [8] and [9]: the work-item counters of the two tensor-core passes
     zero_plan(w, nlist, s);
-    const ProbeLaunch pl{ix.d_qn,   nq,          static_cast<uint32_t>(ix.ds), static_cast<uint32_t>(ix.dp),
+    const ProbeLaunch pl{&ix, ix.d_qn,   nq,          static_cast<uint32_t>(ix.ds), static_cast<uint32_t>(ix.dp),
                          nlist,      np,          v.d_cent_t,  v.nlist_pad, v.d_offsets, w.d_pscore, w.d_probes,
                          w.d_list_cnt, w.d_q_slot_off, w.d_counters};
     cudaError_t e = launch_probe_plan(pqb, pl, 128, w, w.d_qblock_off, groups ? w.d_slot_row0 : nullptr, s);

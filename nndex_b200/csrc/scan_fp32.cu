@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(NT) merge_best_kernel(const uint64_t* __restri
     float* os = sim_out + static_cast<size_t>(oq) * out_stride;
     bool done = false;
     const uint32_t kk = block_merge_best<NT>(
-        keys, static_cast<uint32_t>(per_query), k, s,
+        [&](uint32_t i) { return keys[i]; }, static_cast<uint32_t>(per_query), k, s,
         [&](uint32_t j, uint64_t key) {
             oi[j] = key_row(key);
             os[j] = key_score(key);

@@ -101,6 +101,12 @@ uint32_t tc_stages_for(uint32_t nchunks, uint32_t kprime, bool fp8, bool stream_
     return 0;
 }
 
+uint32_t tc_tf32_stages_for(uint32_t nchunks, size_t smem_limit, bool* stream_a) {
+    const uint32_t stages = tc_stages_for(nchunks, 0, false, false, smem_limit);
+    *stream_a = stages < 3;
+    return *stream_a ? tc_stages_for(nchunks, 0, false, true, smem_limit) : stages;
+}
+
 uint32_t tc_pair_stages_for(uint32_t nchunks, bool fp8, size_t smem_limit) {
     for (uint32_t st = 5; st >= 4; --st)
         if (tc_smem_bytes(nchunks, 0, st, fp8, false, 2) <= smem_limit) return st;
@@ -202,7 +208,8 @@ NNDEX_DEVICE_INLINE void epi_survivor(const TcParams& p, EpiState& st, uint64_t*
 // need about 470); on 2M x 512 in FP8 with 1,000 queries at k = 100, stride 8, 1,977 us -> 200 (the
 // heaps also pushed the query slabs out of shared memory); the IVF list scan of 1,024 queries over
 // 2M x 384, 32 of 1,414 lists, stride 4, 339 us -> 142.
-// kT = kTcTf32 (modes 1 and 2): the FP32 base and queries themselves, read by kind::tf32 MMAs (sign,
+// kMode 3 (TF32): every score is written out, p.scores row by query (the IVF probe's centroid scores).
+// kT = kTcTf32 (modes 1 to 3): the FP32 base and queries themselves, read by kind::tf32 MMAs (sign,
 // exponent, top 10 mantissa bits); p.q_resid then holds each query's whole bound slack.
 template <int kT, int kST, int kMode, bool kStreamA, bool kItems, int kQB, bool kPair = false>
 __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
@@ -588,8 +595,8 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                     if (pos + i < p.cap2) p.cand_rows[static_cast<size_t>(q) * p.cap2 + pos + i] = my_stage[i];
                 staged = 0;
             };
-            const float qs = (kFp8 && kMode != 2 && valid_q) ? p.q_scale[q] : 1.0f;
-            const float rq = (kMode != 2 && valid_q) ? p.q_resid[q] : 0.0f;
+            const float qs = (kFp8 && kMode < 2 && valid_q) ? p.q_scale[q] : 1.0f;
+            const float rq = (kMode < 2 && valid_q) ? p.q_resid[q] : 0.0f;
             const float b_mul = 1.0f + rq, b_add = rq + p.eps_acc;
             const float slack = kTf32 ? rq : fmaf(p.eps_rows, b_mul, b_add);  // the largest u_r − s̃_r over all rows
             EpiState st;
@@ -597,7 +604,7 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
             if (kMode == 0) {
                 st.thr_key = valid_q ? p.thr_global[q] : ~0ull;
                 st.thr_f = !valid_q ? INFINITY : (st.thr_key ? key_score(st.thr_key) : -INFINITY);
-            } else if (kMode == 2) {
+            } else if (kMode >= 2) {
                 st.thr_key = 0;
                 st.thr_f = INFINITY;
             } else {
@@ -659,6 +666,16 @@ __global__ void __launch_bounds__(tc_threads<kMode>(), 1)
                 }
                 const uint32_t sub = kMode == 2 ? t & (p.gm_span - 1u) : 0u;  // the tile in its groups
                 auto process = [&](const uint32_t(&v)[32], uint32_t c) {
+                    if constexpr (kMode == 3) {
+                        if (!valid_q) return;
+                        float4* o = reinterpret_cast<float4*>(p.scores + static_cast<size_t>(q) * p.score_stride +
+                                                              tile_row0 + c * 32);
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j)
+                            o[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                               __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                        return;
+                    }
                     if constexpr (kMode == 2) {
                         // rows of this chunk inside the CTA's rows (fewer than 32 only at their end)
                         const uint64_t c_row0 = tile_row0 + c * 32;
@@ -1294,6 +1311,8 @@ cudaError_t launch_scan_tc(const TcArgs& a, int type, int mode, cudaStream_t str
             return a.stream_a ? launch_tc_stages<kTcTf32, 1, true>(a, stream) : launch_tc_stages<kTcTf32, 1, false>(a, stream);
         if (mode == 2)
             return a.stream_a ? launch_tc_stages<kTcTf32, 2, true>(a, stream) : launch_tc_stages<kTcTf32, 2, false>(a, stream);
+        if (mode == 3 && a.p.scores && a.p.score_stride % 256 == 0 && a.p.score_stride >= a.p.rows)
+            return a.stream_a ? launch_tc_stages<kTcTf32, 3, true>(a, stream) : launch_tc_stages<kTcTf32, 3, false>(a, stream);
         return cudaErrorInvalidValue;
     }
     if (a.items) {

@@ -232,18 +232,19 @@ struct MergeScratch {
     uint32_t count;
 };
 
-// put(j, key) for each of the min(k, non-empty keys) best of keys[0, n) (distinct; 0 = empty slot) at its
-// rank j; returns their number. k ≤ NT. overflow() returns the count after doing the same another way.
-template <int NT, class Put, class Overflow>
-NNDEX_DEVICE_INLINE uint32_t block_merge_best(const uint64_t* __restrict__ keys, uint32_t n, uint32_t k,
-                                              MergeScratch<NT>& s, Put&& put, Overflow&& overflow) {
+// put(j, key) for each of the min(k, non-empty keys) best of the keys get(0 … n) (distinct; 0 = empty
+// slot) at its rank j; returns their number. k ≤ NT. overflow() returns the count after doing the same
+// another way.
+template <int NT, class Get, class Put, class Overflow>
+NNDEX_DEVICE_INLINE uint32_t block_merge_best(Get&& get, uint32_t n, uint32_t k, MergeScratch<NT>& s, Put&& put,
+                                              Overflow&& overflow) {
     static_assert(NT <= static_cast<int>(MergeScratch<NT>::kList), "the maxima share the list");
     constexpr int U = 8;  // loads in flight; the keys stay in registers where one round reads them all
     const uint32_t tid = threadIdx.x;
     uint64_t best = 0, x[U];
     for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? keys[i0 + u * NT + tid] : 0ull;
+        for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? get(i0 + u * NT + tid) : 0ull;
 #pragma unroll
         for (int u = 0; u < U; ++u) best = x[u] > best ? x[u] : best;
     }
@@ -265,7 +266,7 @@ NNDEX_DEVICE_INLINE uint32_t block_merge_best(const uint64_t* __restrict__ keys,
     for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
         if (n > U * NT) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? keys[i0 + u * NT + tid] : 0ull;
+            for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? get(i0 + u * NT + tid) : 0ull;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
