@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 8 : 1)
                           const float* __restrict__ centroids, const float2* __restrict__ cent_max, float c_norm,
                           const uint32_t* __restrict__ offsets, uint32_t* __restrict__ probes,
                           uint32_t* __restrict__ list_cnt, uint32_t* __restrict__ q_slot_off,
-                          unsigned long long* __restrict__ counters) {
+                          unsigned long long* __restrict__ counters, int no_plan) {
     __shared__ MergeScratch<NT> s;
     __shared__ uint64_t band_key[kProbeBand];
     __shared__ uint32_t picked[kProbePick], band[kProbeBand];
@@ -383,21 +383,23 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 8 : 1)
     __syncthreads();
     const uint32_t n = np < nlist ? np : nlist;
     uint32_t slots = 0;
-    unsigned long long rows = 0;
+    unsigned long long rows = 0, first = 0;  // rows of the query's lists, of those no other query had taken
     for (uint32_t t = tid; t < n; t += NT) {
         const uint32_t c = picked[t];
         probes[static_cast<uint64_t>(q) * np + t] = c;
-        atomicAdd(&list_cnt[c], 1u);
         const uint32_t len = offsets[c + 1] - offsets[c];
+        if (atomicAdd(&list_cnt[c], 1u) == 0u) first += len;
         slots += (len + kChunkRows - 1) / kChunkRows;
         rows += len;
     }
     if (slots) atomicAdd(&n_slots, slots);
     if (rows) atomicAdd(&n_rows, rows);
+    if (no_plan && first) atomicAdd(&counters[5], first);  // otherwise the plan's
     __syncthreads();
     if (tid == 0) {
         q_slot_off[q] = n_slots;
         atomicAdd(&counters[3], n_rows);  // zeroed once per search: Σ over sub-batches
+        if (no_plan) atomicAdd(&counters[4], n_rows);
     }
 }
 
@@ -654,20 +656,123 @@ __global__ void __launch_bounds__(IvfScanShape<QB>::kThreads, 1)
 }
 
 // ------------------------------------------------------------------------------------------
+// Small batches: no plan. CTA (c, j, q) scans chunk c of query q's j-th probed list for that query alone
+// (a list serves about one query on average, so there is little to share), with the FP32 scan's
+// consumer, FMA order and addition tree, and fills the slot of the same number; a list without that
+// chunk leaves its slot empty. The chunks spread a query's lists over the SMs: one query's 16 lists of
+// 780 rows × 128 ran 22 us as 16 items of the persistent scan, behind 9 us of plan; 8.7 us here.
+// ------------------------------------------------------------------------------------------
+constexpr int kPairW = 8;  // consumer warps: 128-row tiles, three CTAs per SM at 128 dims
+
+__global__ void __launch_bounds__((kPairW + 1) * 32)
+    ivf_scan_pair_kernel(const __grid_constant__ CUtensorMap tmap, const IvfScanArgs a,
+                         const uint32_t* __restrict__ probes, uint32_t np, uint32_t chunk_rows) {
+    using Consumer = ScanConsumerWide<1, kPairW, kStages>;
+    constexpr int TR = Consumer::kTileRows;
+    constexpr uint32_t kStage = Consumer::kStageBytes;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t q = blockIdx.z, j = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t k = a.k, cap = a.cap, dq = a.dq, nbox = dq / 32;
+    uint64_t* slot = a.ws + ((static_cast<uint64_t>(q) * np + j) * gridDim.x + blockIdx.x) * k;
+    const uint32_t l = probes[static_cast<uint64_t>(q) * np + j];
+    const uint32_t le = a.offsets[l + 1];
+    const uint64_t row_begin = static_cast<uint64_t>(a.offsets[l]) + static_cast<uint64_t>(blockIdx.x) * chunk_rows;
+    if (row_begin >= le) {
+        for (uint32_t i = tid; i < k; i += blockDim.x) slot[i] = 0ull;
+        return;
+    }
+    const uint64_t row_end = row_begin + chunk_rows < le ? row_begin + chunk_rows : le;
+    const uint32_t ntiles = static_cast<uint32_t>((row_end - row_begin + TR - 1) / TR);
+    uint8_t* stage_base = align_1024(smem_raw);
+    float* q_s = reinterpret_cast<float*>(stage_base + static_cast<size_t>(kStages) * kStage);
+    uint64_t* cand = reinterpret_cast<uint64_t*>(q_s + dq);
+    uint32_t* hist = reinterpret_cast<uint32_t*>(cand + cap);
+    uint64_t* thr = reinterpret_cast<uint64_t*>(hist + kPairW * 256);
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(thr + 1);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(cnt + 2);
+    uint64_t* empty_bar = full_bar + kStages;
+    volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(empty_bar + kStages);
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], kPairW * 32);
+        }
+        *abort_flag = 0;
+        fence_mbar_init();
+        cnt[0] = 0;
+        thr[0] = 0ull;
+    }
+    // (one query: its slab-major order is the row's own)
+    for (uint32_t i = tid; i < dq; i += blockDim.x) q_s[i] = a.queries[static_cast<uint64_t>(q) * dq + i];
+    __syncthreads();
+    if (warp == kPairW) {
+        // ---------------- producer ----------------
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool stop = false;
+            for (uint32_t t = 0; t < ntiles && !stop; ++t) {
+                const int32_t y = static_cast<int32_t>(row_begin + static_cast<uint64_t>(t) * TR);
+                for (uint32_t bx = 0; bx < nbox; ++bx) {
+                    const uint32_t s = it % kStages, u = it / kStages;
+                    if (*abort_flag) {
+                        stop = true;
+                        break;
+                    }
+                    if (u > 0 && !mbar_wait_bounded(&empty_bar[s], (u - 1) & 1u, kWaitBudgetCycles)) {
+                        *abort_flag = 1;
+                        record_status(a.status, kStatusTimeout);
+                        stop = true;
+                        break;
+                    }
+                    mbar_arrive_expect_tx(&full_bar[s], kStage);
+                    tma_load_2d(stage_base + static_cast<size_t>(s) * kStage, &tmap, &full_bar[s],
+                                static_cast<int32_t>(bx * 32), y);
+                    ++it;
+                }
+            }
+            // Drain: every issued copy has landed before the CTA may exit.
+            const uint32_t used = it < static_cast<uint32_t>(kStages) ? it : kStages;
+            for (uint32_t s = 0; s < used; ++s) {
+                const uint32_t uses = (it - s + kStages - 1) / kStages;
+                if (!mbar_wait_bounded(&full_bar[s], (uses - 1) & 1u, kWaitBudgetCycles))
+                    record_status(a.status, kStatusTimeout);
+            }
+        }
+        return;
+    }
+    // ---------------- consumers ----------------
+    const Consumer con(warp, lane, stage_base, q_s);
+    auto row_key = [&](uint64_t r) { return a.row_map[r]; };
+    float acc[4][1];
+    RingPos<kStages> pos;
+    for (uint32_t t = 0; t < ntiles; ++t) {
+        con.accumulate(acc, nbox, pos, full_bar, empty_bar, abort_flag, a.status);
+        con.insert(acc, row_begin + static_cast<uint64_t>(t) * TR, row_end, 1, row_key, thr, cnt, cand, cap, a.status);
+        scan_flush_g<1, kPairW, TR>(t + 1 == ntiles, 1, k, cap, warp, lane, cnt, thr, cand, hist);
+    }
+    if (warp == 0) {
+        const uint32_t n = cnt[0] < k ? cnt[0] : k;
+        for (uint32_t i = lane; i < k; i += 32) slot[i] = i < n ? cand[i] : 0ull;
+    }
+}
+
+// ------------------------------------------------------------------------------------------
 // 4. Merge: per query, the k best keys of its slots, sorted; unused result slots (0, 0.0f).
 // ------------------------------------------------------------------------------------------
 // k ≤ kMergeBestK (block_merge_best).
 __global__ void __launch_bounds__(256)
-    ivf_merge_best_kernel(const uint64_t* __restrict__ ws, const uint32_t* __restrict__ q_slot_off, uint32_t k,
-                          uint64_t* __restrict__ idx_out, float* __restrict__ sim_out, uint32_t* __restrict__ count_out,
+    ivf_merge_best_kernel(const uint64_t* __restrict__ ws, const uint32_t* __restrict__ q_slot_off, uint32_t slots,
+                          uint32_t k, uint64_t* __restrict__ idx_out, float* __restrict__ sim_out, uint32_t* __restrict__ count_out,
                           const unsigned long long* __restrict__ counters,
                           unsigned long long* __restrict__ host_probed) {
     __shared__ MergeScratch<256> s;
     const uint32_t q = blockIdx.x;
     // the plan's row totals for the statistics, into pinned memory
     if (host_probed && q == 0 && threadIdx.x < 3) host_probed[threadIdx.x] = counters[3 + threadIdx.x];
-    const uint64_t* keys = ws + static_cast<uint64_t>(q_slot_off[q]) * k;
-    const uint32_t n = (q_slot_off[q + 1] - q_slot_off[q]) * k;
+    // a plan's slots, or `slots` of every query
+    const uint64_t slot0 = q_slot_off ? q_slot_off[q] : static_cast<uint64_t>(q) * slots;
+    const uint64_t* keys = ws + slot0 * k;
+    const uint32_t n = (q_slot_off ? q_slot_off[q + 1] - q_slot_off[q] : slots) * k;
     uint64_t* oi = idx_out + static_cast<uint64_t>(q) * k;
     float* os = sim_out + static_cast<uint64_t>(q) * k;
     const uint32_t kk = block_merge_best<256>(
@@ -868,6 +973,16 @@ size_t ivf_scan_smem(uint32_t qb, uint32_t dq, uint32_t cap) {
     return b;
 }
 
+// (query, list) pairs of a batch scanned without a plan. Batches in a row, without / with a plan: 400k ×
+// 128, 16 of 512 lists, 1 query 41 / 70 us, 32 queries 80 / 107; 2M × 384, 32 of 1,414 lists, 8
+// queries 151 / 205, 16 (512 pairs) 246 / 274, 32 431 / 377; 8 lists, 64 queries 355 / 327.
+constexpr uint64_t kPairLimit = 512;
+
+size_t ivf_pair_smem(uint32_t dq, uint32_t cap) {
+    return 1024 + static_cast<size_t>(kStages) * kPairW * 16 * 128 + static_cast<size_t>(dq) * 4 +
+           static_cast<size_t>(cap) * 8 + kPairW * 256 * 4 + 8 + 8 + kStages * 16 + 16;
+}
+
 template <int QB>
 cudaError_t launch_scan(const CUtensorMap& tmap, const IvfScanArgs& a, uint32_t grid, size_t smem, cudaStream_t s) {
     auto kern = ivf_scan_kernel<QB>;
@@ -881,7 +996,8 @@ cudaError_t launch_scan(const CUtensorMap& tmap, const IvfScanArgs& a, uint32_t 
 void launch_ivf_merge(const IvfScratch& w, uint32_t nq, uint32_t k, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
                       const unsigned long long* counters, unsigned long long* host_probed, cudaStream_t s) {
     if (k <= kMergeBestK) {
-        ivf_merge_best_kernel<<<nq, 256, 0, s>>>(w.d_ws, w.d_q_slot_off, k, o_idx, o_sim, o_cnt, counters, host_probed);
+        ivf_merge_best_kernel<<<nq, 256, 0, s>>>(w.d_ws, w.d_q_slot_off, 0, k, o_idx, o_sim, o_cnt, counters,
+                                                 host_probed);
     } else {
         uint32_t p2 = 1;
         while (p2 < k) p2 <<= 1;
@@ -934,14 +1050,21 @@ cudaError_t launch_probe_qb(const ProbeLaunch& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// Probe + plan of n queries: four launches (centroid scores, the selection with its counts, the
-// plan's scans, the pairs).
-cudaError_t launch_probe_plan(uint32_t pqb, const ProbeLaunch& a, uint32_t qb, IvfScratch& w, uint32_t* qblock_off,
-                              uint32_t* slot_row0, cudaStream_t s) {
+// Whether the probe can pick its lists from TF32 scores (ivf_probe_pick_kernel).
+bool probe_picks(const CudaIndex& ix, uint32_t np, uint32_t* stages, bool* stream_a) {
+    *stages = np <= kProbePick && ix.ds * sizeof(double) <= 64 * 1024
+                  ? tc_tf32_stages_for(static_cast<uint32_t>(ix.ds / 32), ix.smem_optin, stream_a)
+                  : 0u;
+    return *stages != 0;
+}
+
+// The probe of n queries: two launches (centroid scores, the selection with its counts; no_plan: the
+// totals a plan would count too).
+cudaError_t launch_probe(uint32_t pqb, const ProbeLaunch& a, bool no_plan, cudaStream_t s) {
     cudaError_t e;
     bool stream_a = false;
-    const uint32_t stages = a.np <= kProbePick ? tc_tf32_stages_for(a.ds / 32, a.ix->smem_optin, &stream_a) : 0;
-    if (stages && a.ds * sizeof(double) <= 64 * 1024) {
+    uint32_t stages = 0;
+    if (probe_picks(*a.ix, a.np, &stages, &stream_a)) {
         const CudaIndex& ix = *a.ix;
         CUtensorMap tmap_q;
         if (!encode_tmap_2d(&tmap_q, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(a.queries), a.ds, a.nq,
@@ -971,7 +1094,8 @@ cudaError_t launch_probe_plan(uint32_t pqb, const ProbeLaunch& a, uint32_t qb, I
             return e;
         pick<<<a.nq, a.np <= 64 ? 128 : 512, smem, s>>>(a.scores, a.ct_stride, a.nlist, a.np, a.queries, a.ds, a.dp,
                                                         ix.ivf->d_centroids, ix.ivf->d_cent_max, ix.tf32_c_norm(),
-                                                        a.offsets, a.probes, a.list_cnt, a.q_slot_off, a.counters);
+                                                        a.offsets, a.probes, a.list_cnt, a.q_slot_off, a.counters,
+                                                        no_plan ? 1 : 0);
         count_launch();
     } else {
         if ((a.nlist + kProbeCentroids - 1) / kProbeCentroids > 65535u) return cudaErrorInvalidValue;
@@ -987,6 +1111,14 @@ cudaError_t launch_probe_plan(uint32_t pqb, const ProbeLaunch& a, uint32_t qb, I
                                                                a.list_cnt, a.q_slot_off, a.counters);
         count_launch(2);
     }
+    return cudaGetLastError();
+}
+
+// Probe + plan of n queries: four launches (the probe, the plan's scans, the pairs).
+cudaError_t launch_probe_plan(uint32_t pqb, const ProbeLaunch& a, uint32_t qb, IvfScratch& w, uint32_t* qblock_off,
+                              uint32_t* slot_row0, cudaStream_t s) {
+    const cudaError_t e = launch_probe(pqb, a, false, s);
+    if (e != cudaSuccess) return e;
     ivf_plan_scan_kernel<<<1, 1024, 0, s>>>(a.nq, a.nlist, a.offsets, qb, w.d_list_cnt, w.d_list_qoff, w.d_item_off,
                                             w.d_q_slot_off, w.d_counters, qblock_off);
     ivf_plan_fill_kernel<<<(a.nq + 7) / 8, 256, 0, s>>>(a.probes, a.nq, a.np, a.offsets, w.d_list_qoff, w.d_list_fill,
@@ -1044,8 +1176,61 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
         return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: IVF scan needs %zu bytes of shared memory", smem);
     const uint32_t pqb = probe_qb(ix.dp, ix.smem_optin);
     if (!pqb) return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: IVF probe shared memory above the limit");
-    const uint64_t max_chunks = (v.max_list + kChunkRows - 1) / kChunkRows;
     int st;
+    // Small batches whose lists serve at most one query on average: (query, list, chunk) CTAs, no plan.
+    // Chunks of as many 256 rows as give every SM about two (of the longest list at most 32).
+    const uint64_t pairs = static_cast<uint64_t>(nq) * np;
+    if (pairs <= nlist && pairs <= kPairLimit && k <= kMergeBestK) {
+        const uint64_t rows_est = pairs * (ix.rows / nlist + 1);
+        uint64_t chunk = std::max<uint64_t>(rows_est / (2 * static_cast<uint64_t>(ix.sm_count)), (v.max_list + 31) / 32);
+        chunk = std::max<uint64_t>(256, (chunk + 255) / 256 * 256);
+        const uint32_t chunks = static_cast<uint32_t>(std::max<uint64_t>(1, (v.max_list + chunk - 1) / chunk));
+        const uint32_t pcap = ((k + 2 * kPairW * 16) + 31) / 32 * 32;
+        const size_t psmem = ivf_pair_smem(dq, pcap);
+        uint32_t stages = 0;
+        bool stream_a = false;
+        if (psmem <= ix.smem_optin && probe_picks(ix, np, &stages, &stream_a)) {
+            if ((st = grow(w.d_probes, w.cap_probes, pairs, "IVF probe buffer"))) return st;
+            if ((st = grow(w.d_pscore, w.cap_pscore, static_cast<size_t>(nq) * v.nlist_pad, "IVF probe buffer"))) return st;
+            if ((st = plan_buffer(w, nlist))) return st;
+            if ((st = grow(w.d_q_slot_off, w.cap_q_slot_off, nq + 1, "IVF plan buffer"))) return st;
+            if ((st = grow(w.d_ws, w.cap_ws, pairs * chunks * k, "IVF slot workspace"))) return st;
+            if (!w.h_probed) bump_alloc_epoch();
+            if (!w.h_probed && cudaMallocHost(&w.h_probed, 8 * sizeof(unsigned long long)) != cudaSuccess)
+                return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
+            zero_plan(w, nlist, s);
+            const ProbeLaunch pl{&ix, queries, nq, dq, static_cast<uint32_t>(ix.dp), nlist, np, v.d_cent_t, v.nlist_pad,
+                                 v.d_offsets, w.d_pscore, w.d_probes, w.d_list_cnt, w.d_q_slot_off, w.d_counters};
+            cudaError_t e = launch_probe(pqb, pl, true, s);
+            if (e != cudaSuccess) return cuda_error(e, "IVF probe launch");
+            IvfScanArgs a;
+            a.dq = dq;
+            a.k = k;
+            a.cap = pcap;
+            a.queries = queries;
+            a.offsets = v.d_offsets;
+            a.row_map = v.d_row_map;
+            a.ws = w.d_ws;
+            a.status = ix.w_status;
+            if ((e = cudaFuncSetAttribute(ivf_scan_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(psmem))) != cudaSuccess)
+                return cuda_error(e, "IVF scan launch");
+            cudaEvent_t ev_a = nullptr;
+            ix.scan_event_begin(s, ev_a);
+            ivf_scan_pair_kernel<<<dim3(chunks, np, nq), (kPairW + 1) * 32, psmem, s>>>(v.tmap_reordered, a, w.d_probes, np,
+                                                                                       static_cast<uint32_t>(chunk));
+            ix.scan_event_end(s, ev_a);
+            ivf_merge_best_kernel<<<nq, 256, 0, s>>>(w.d_ws, nullptr, np * chunks, k, o_idx, o_sim, o_cnt, w.d_counters,
+                                                     w.h_probed);
+            count_launch(2);
+            if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "IVF scan launch");
+            ix.stats.kernel_launches += 4;
+            ix.stats.path = 4;
+            ix.stats.nprobe = np;
+            return NNDEX_OK;
+        }
+    }
+    const uint64_t max_chunks = (v.max_list + kChunkRows - 1) / kChunkRows;
     // Sub-batches so the slot workspace (Σ slots × k keys) stays bounded.
     const uint64_t ws_budget = 256ull << 20;
     uint64_t per_query = std::max<uint64_t>(1, static_cast<uint64_t>(np) * max_chunks * k * 8);

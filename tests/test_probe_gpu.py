@@ -65,3 +65,32 @@ def test_probed_lists(nlist, nprobe, dims, nq, kind):
             assert set(idx[i].tolist()) == set(want[i].tolist()), i
         else:
             assert set(idx[i].tolist()) <= set(want[i].tolist()), i
+
+
+@pytest.mark.parametrize("rows,dims,nlist,nprobe,k,sizes", [
+    (20_000, 40, 64, 8, 10, (1, 3)),         # lists of a few hundred rows, one chunk
+    (120_000, 128, 300, 20, 100, (1, 9)),
+    (60_000, 96, 40, 3, 256, (1, 13)),       # lists of several chunks, the longest merge
+    (5_000, 1_100, 100, 60, 1, (1,)),
+])
+def test_small_batches_equal_large_ones(rows, dims, nlist, nprobe, k, sizes):
+    # a few queries are scanned per (query, list, chunk) without a plan, a large batch by the plan's
+    # items: the same rows and scores
+    rng = np.random.default_rng(rows + dims)
+    c = rng.standard_normal((37, dims), dtype=np.float32)
+    w = np.arange(1, 38) ** -1.2
+    pick = rng.choice(37, size=rows + 300, p=w / w.sum())  # uneven lists
+    x = c[pick] + np.float32(0.4) * rng.standard_normal((rows + 300, dims), dtype=np.float32)
+    index = NNdex(x[:rows], approx=True, nlist=nlist, kmeans_iters=3, seed=1, precision="fp32")
+    index.set_nprobe(nprobe)
+    q = x[rows:]
+    bi, bs = index.search(q, k=k)
+    streamed = index.last_search_stats()["ivf_rows_streamed"]
+    for n in sizes:
+        for lo in (0, 111):
+            i, s = index.search(np.vstack([q[lo:lo + n], q[:1]]) if n == 1 else q[lo:lo + n], k=k)
+            st = index.last_search_stats()
+            assert st["path"] == 4 and 0 < st["ivf_rows_union"] <= st["ivf_rows_streamed"] <= st["rows_scanned"]
+            np.testing.assert_array_equal(i[:n], bi[lo:lo + n])
+            np.testing.assert_array_equal(s[:n].view(np.uint32), bs[lo:lo + n].view(np.uint32))
+    assert streamed > 0
