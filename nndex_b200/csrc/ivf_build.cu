@@ -8,11 +8,12 @@
 // value: products of two f32 are exact in FP64, and the sum is accumulated in index order.
 //
 // Where the time goes and how it is spent on B200:
-//   * seeding: nlist − 1 sequential passes over the rows. Each pass screens every row with an FP16
-//     dot (half the bytes of FP32) and a rigorous error bound; only rows whose distance could drop
-//     below their running minimum are re-scored exactly (FP64 sequential dot). The running sum of
-//     the minima and the threshold search are exact: every distance is a multiple of 2^-24, so FP64
-//     sums below 2^29 carry no rounding and any summation order gives the reference's value.
+//   * seeding: nlist − 1 sequential passes over the rows. Each pass screens every row with an INT8
+//     dot (a quarter of FP32's bytes; the copy of 200,000 × 256 stays in L2) and a rigorous error
+//     bound; only rows whose distance could drop below their running minimum (2% of them) are scored
+//     exactly, eight lanes each. The running sum of the minima and the threshold search are exact:
+//     every distance is a multiple of 2^-24, so FP64 sums below 2^29 carry no rounding and any
+//     summation order gives the reference's value.
 //   * assignment: a tcgen05 FP16 GEMM rows × centroids (M = 128 rows in TMEM lanes, N = 256
 //     centroids), run twice. Pass A keeps each row's best approximate score s1. Pass B repeats the
 //     GEMM and lists every centroid whose approximate score reaches s1 − 2e (e = the row's error
@@ -73,6 +74,36 @@ NNDEX_DEVICE_INLINE float dot_f64_seq(const float* __restrict__ x, const float* 
     return __double2float_rn(s);
 }
 
+// The same value by 8 consecutive lanes (j of 8, all of the warp calling; every lane returns it): y in
+// shared memory, n a multiple of 4. The lanes add in another order: both sums are within n·2⁻⁵³·Σ|xy| ≤
+// err / 2 of the exact value, so where every value within err rounds to one f32, that is the
+// reference's; where it does not (about once in 10⁷), or err is not finite, they add in index order.
+NNDEX_DEVICE_INLINE float dot_f64_lanes8(const float* __restrict__ x, const float* y, uint32_t n, double err,
+                                         uint32_t j, bool live) {
+    double s = 0.0;
+    if (live) {
+#pragma unroll 8
+        for (uint32_t d = 4 * j; d < n; d += 32) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(x + d));
+            const float4 b = *reinterpret_cast<const float4*>(y + d);
+            s = fma(static_cast<double>(a.x), static_cast<double>(b.x), s);
+            s = fma(static_cast<double>(a.y), static_cast<double>(b.y), s);
+            s = fma(static_cast<double>(a.z), static_cast<double>(b.z), s);
+            s = fma(static_cast<double>(a.w), static_cast<double>(b.w), s);
+        }
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    if (live && !(__double2float_rn(s - err) == __double2float_rn(s + err))) return dot_f64_seq(x, y, n);
+    return __double2float_rn(s);
+}
+
+// err of dot_f64_lanes8 from upper bounds of the operands' norms.
+NNDEX_DEVICE_INLINE double dot_f64_err(float nx, float ny, uint32_t n) {
+    return static_cast<double>(nx) * static_cast<double>(ny) * static_cast<double>(n) * 4.5e-16;  // 2·2·2⁻⁵³
+}
+
 // Same with the second operand dims-major (column c of a [n × stride] matrix).
 NNDEX_DEVICE_INLINE float dot_f64_seq_col(const float* __restrict__ x, const float* __restrict__ ct, uint64_t stride,
                                           uint32_t c, uint32_t n) {
@@ -105,8 +136,8 @@ NNDEX_DEVICE_INLINE float sqrt_up(double v) {
 }  // namespace
 
 // ------------------------------------------------------------------------------------------
-// Row preparation: FP16 copy and per row upper bounds of ‖x‖ and of the residual ‖x − x̂‖. One
-// warp per row.
+// Row preparation: the FP16 copy (K slabs of 64, zero past the row) and upper bounds of ‖x‖ and of the
+// residual ‖x − x̂‖. One warp per row, four values a lane.
 // ------------------------------------------------------------------------------------------
 __global__ void ivf_row_prep_kernel(const float* __restrict__ src, uint32_t ds, uint64_t rows,
                                     __half* __restrict__ out16, uint32_t kb, float* __restrict__ norm_up,
@@ -115,21 +146,73 @@ __global__ void ivf_row_prep_kernel(const float* __restrict__ src, uint32_t ds, 
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
     for (uint64_t r = warp; r < rows; r += nwarps) {
-        const float* x = src + r * ds;
         double n2 = 0.0, r2 = 0.0;
-        for (uint32_t d = lane; d < kb; d += 32) {
-            const float v = d < ds ? x[d] : 0.0f;
-            float e;
-            const __half b = to_f16(v, e);
-            n2 = fma(static_cast<double>(v), static_cast<double>(v), n2);
-            r2 = fma(static_cast<double>(e), static_cast<double>(e), r2);
-            out16[r * kb + d] = b;
+        for (uint32_t d = 4 * lane; d < kb; d += 128) {
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (d < ds) v = *reinterpret_cast<const float4*>(src + r * ds + d);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+            union {
+                __half h[4];
+                uint2 u;
+            } o;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float e;
+                o.h[i] = to_f16(x[i], e);
+                n2 = fma(static_cast<double>(x[i]), static_cast<double>(x[i]), n2);
+                r2 = fma(static_cast<double>(e), static_cast<double>(e), r2);
+            }
+            *reinterpret_cast<uint2*>(out16 + r * kb + d) = o.u;
         }
         n2 = warp_sum_d(n2);
         r2 = warp_sum_d(r2);
         if (lane == 0) {
             norm_up[r] = sqrt_up(n2);
             res_up[r] = sqrt_up(r2);
+        }
+    }
+}
+
+// The same with an INT8 copy, x̂ = scale · q with scale = max|x| / 127: what the seeding screens. The
+// residual is that of the scale and the q that are stored, so its bound holds for whatever they round
+// to; a value that is not finite makes it infinite or NaN, and its row is always scored exactly.
+__global__ void ivf_row_prep8_kernel(const float* __restrict__ src, uint32_t ds, uint64_t rows,
+                                     signed char* __restrict__ out8, float* __restrict__ norm_up,
+                                     float2* __restrict__ res_scale) {
+    const uint64_t warp = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+    for (uint64_t r = warp; r < rows; r += nwarps) {
+        const float* x = src + r * ds;
+        float m = 0.0f;
+        for (uint32_t d = 4 * lane; d < ds; d += 128) {
+            const float4 v = *reinterpret_cast<const float4*>(x + d);
+            m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float scale = m / 127.0f, inv = m > 0.0f ? 127.0f / m : 0.0f;
+        double n2 = 0.0, r2 = 0.0;
+        for (uint32_t d = 4 * lane; d < ds; d += 128) {
+            const float4 v4 = *reinterpret_cast<const float4*>(x + d);
+            const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+            char4 o;
+            signed char* ob = reinterpret_cast<signed char*>(&o);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int q = __float2int_rn(fminf(fmaxf(v[i] * inv, -127.0f), 127.0f));
+                const double e = static_cast<double>(v[i]) - static_cast<double>(scale) * static_cast<double>(q);
+                ob[i] = static_cast<signed char>(q);
+                n2 = fma(static_cast<double>(v[i]), static_cast<double>(v[i]), n2);
+                r2 = fma(e, e, r2);
+            }
+            *reinterpret_cast<char4*>(out8 + r * ds + d) = o;
+        }
+        n2 = warp_sum_d(n2);
+        r2 = warp_sum_d(r2);
+        if (lane == 0) {
+            norm_up[r] = sqrt_up(n2);
+            res_scale[r] = make_float2(sqrt_up(r2), scale);
         }
     }
 }
@@ -198,11 +281,27 @@ __global__ void __launch_bounds__(64, 1)
         }
         const uint8_t* st = ring + s * kColStageBytes;
         const uint32_t nr = (rows - static_cast<uint64_t>(t) * 128) < 128 ? static_cast<uint32_t>(rows - t * 128ull) : 128u;
-        for (uint32_t r = 0; r < nr; ++r) {
-            const float v =
-                *reinterpret_cast<const volatile float*>(st + r * 128 + ((chunk ^ (r & 7u)) * 16) + within);
-            sum = __dadd_rn(sum, static_cast<double>(v));
+        // The chain of FP64 adds in row order is the bound (14 cycles each): the next 16 values load while
+        // 16 are added. 200,000 rows: 2.7 ms with each value loaded when it is added, 1.45 so.
+        auto value = [&](uint32_t row) {
+            return *reinterpret_cast<const volatile float*>(st + row * 128 + ((chunk ^ (row & 7u)) * 16) + within);
+        };
+        uint32_t r = 0;
+        if (nr == 128) {
+            float v[2][16];
+#pragma unroll
+            for (uint32_t u = 0; u < 16; ++u) v[0][u] = value(u);
+#pragma unroll
+            for (uint32_t b = 0; b < 8; ++b) {
+                if (b + 1 < 8)
+#pragma unroll
+                    for (uint32_t u = 0; u < 16; ++u) v[(b + 1) & 1][u] = value((b + 1) * 16 + u);
+#pragma unroll
+                for (uint32_t u = 0; u < 16; ++u) sum = __dadd_rn(sum, static_cast<double>(v[b & 1][u]));
+            }
+            r = 128;
         }
+        for (; r < nr; ++r) sum = __dadd_rn(sum, static_cast<double>(value(r)));
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
     }
@@ -231,6 +330,11 @@ __global__ void medoid_kernel(const float* __restrict__ base, uint32_t ds, uint3
 // k-means++ seeding step c (src/approx.rs:370-402): min_d[r] = min(min_d[r], max(1 − dot(r, c−1),
 // 0)); total = Σ min_d; the LCG draws a threshold; the chosen row is the first whose running sum
 // reaches it. One launch per centroid; the last block to finish does the draw and the search.
+// What a step of 200,000 × 256 took: 60 µs with an FP16 screen and each row's exact dot by one lane, in
+// its place in the loop (the step waited for the warps with most of them); 32 with eight lanes a dot; 21
+// with the INT8 screen and the dots after the loop; 18.4 with the next step's blocks in place before this
+// one's end and no more registers than the rows' loads need (5 blocks an SM). 51 MB at L2's rate would be
+// about 6: the rest is the chain from the drawn row to its values, the dots, the block count and the draw.
 // ------------------------------------------------------------------------------------------
 struct KppState {
     unsigned long long rng;
@@ -241,111 +345,219 @@ struct KppState {
 
 namespace {
 constexpr uint32_t kKppThreads = 256;
-constexpr uint32_t kKppScanChunk = 2048;
+constexpr uint32_t kKppSegment = 1024;  // rows a block screens before it scores those that need it
+
+// A block's search in n values that are not negative, added up in order: every thread has a run of
+// them, the first kHeld of it in registers.
+template <class V>
+struct RunSearch {
+    static constexpr uint32_t kHeld = 4;
+    V v;
+    uint32_t b, e;
+    double held[kHeld], start, sum;  // start: what stands before the run
+
+    // The sum of all; wsum holds a double per warp.
+    NNDEX_DEVICE_INLINE double scan(uint32_t n, double* wsum) {
+        const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+        const uint32_t per = (n + kKppThreads - 1) / kKppThreads;
+        b = tid * per < n ? tid * per : n;
+        e = b + per < n ? b + per : n;
+#pragma unroll
+        for (uint32_t u = 0; u < kHeld; ++u) held[u] = b + u < e ? v(b + u) : 0.0;
+        sum = 0.0;
+#pragma unroll
+        for (uint32_t u = 0; u < kHeld; ++u) sum += held[u];
+        for (uint32_t i = b + kHeld; i < e; ++i) sum += v(i);
+        double incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= static_cast<uint32_t>(o)) incl += x;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        start = incl - sum;
+        double total = 0.0;
+#pragma unroll
+        for (uint32_t w = 0; w < kKppThreads / 32; ++w) {
+            if (w < warp) start += wsum[w];
+            total += wsum[w];
+        }
+        return total;
+    }
+
+    // The first i of scan's n with before + v(0) + … + v(i) ≥ thr (n if none has); before then is the sum
+    // in front of it.
+    NNDEX_DEVICE_INLINE uint32_t first_reaching(uint32_t n, double thr, double& before, uint32_t* sh_at,
+                                                double* sh_before) {
+        if (threadIdx.x == 0) {
+            *sh_at = before >= thr ? 0 : n;
+            *sh_before = before;
+        }
+        __syncthreads();
+        double at = before + start;
+        if (at < thr && at + sum >= thr) {  // one run crosses it
+            for (uint32_t i = b; i < e; ++i) {
+                double x = 0.0;
+                if (i - b < kHeld) {
+#pragma unroll
+                    for (uint32_t u = 0; u < kHeld; ++u)
+                        if (u == i - b) x = held[u];
+                } else {
+                    x = v(i);
+                }
+                if (at + x >= thr) {
+                    *sh_at = i;
+                    *sh_before = at;
+                    break;
+                }
+                at += x;
+            }
+        }
+        __syncthreads();
+        before = *sh_before;
+        return *sh_at;
+    }
+};
 }  // namespace
 
+// The seeding's first centroid, and its state.
+__global__ void kpp_init_kernel(const unsigned long long* __restrict__ best, unsigned long long rng,
+                                KppState* __restrict__ st, uint32_t* __restrict__ chosen) {
+    st->rng = rng;
+    st->done = 0;
+    st->pad = 0;
+    st->exact_rows = 0;
+    chosen[0] = key_row(*best);
+}
+
+// kL lanes screen a row: each has up to kPre 16-byte chunks of it in flight.
+template <int kL, int kPre>
 __global__ void __launch_bounds__(kKppThreads)
-    kpp_step_kernel(const float* __restrict__ base, const __half* __restrict__ b16, uint32_t ds, uint32_t kb,
-                    uint32_t dp, uint64_t rows, uint64_t rows_per_block, const float* __restrict__ norm_up,
-                    const float* __restrict__ res_up, float gamma, float* __restrict__ min_d,
-                    double* __restrict__ partial, KppState* __restrict__ st, uint32_t* __restrict__ chosen,
-                    uint32_t c) {
+    kpp_step_kernel(const float* __restrict__ base, const signed char* __restrict__ b8, uint32_t ds, uint32_t dp,
+                    uint64_t rows, uint64_t rows_per_block, const float* __restrict__ norm_up,
+                    const float2* __restrict__ res_scale, float* __restrict__ min_d, double* __restrict__ partial,
+                    KppState* __restrict__ st, uint32_t* __restrict__ chosen, uint32_t c) {
     extern __shared__ uint8_t smem_raw[];
-    float* cf = reinterpret_cast<float*>(smem_raw);                        // ds
-    __half* cb = reinterpret_cast<__half*>(cf + ds);                      // kb
-    float* scan_buf = reinterpret_cast<float*>(cb + kb);                   // kKppScanChunk (last block)
+    float* cf = reinterpret_cast<float*>(smem_raw);                       // ds
+    int4* cq = reinterpret_cast<int4*>(cf + ds);                          // ds bytes
+    __shared__ uint2 queue[kKppSegment];                                  // rows to score, their minimum so far
+    __shared__ uint32_t queued;
     __shared__ double wsum[kKppThreads / 32];
     __shared__ unsigned int is_last;
-    __shared__ double sh_total, sh_thr, sh_before;
-    __shared__ unsigned long long sh_blk;
-    __shared__ unsigned int sh_found;
-    __shared__ unsigned long long sh_exact;
+    __shared__ double sh_before;
+    __shared__ uint32_t sh_at;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t prev = chosen[c - 1];
-    for (uint32_t d = tid; d < ds; d += blockDim.x) cf[d] = base[static_cast<uint64_t>(prev) * ds + d];
-    for (uint32_t d = tid; d < kb; d += blockDim.x) cb[d] = b16[static_cast<uint64_t>(prev) * kb + d];
-    if (tid == 0) sh_exact = 0;
+    // The next step's blocks may take the places that this one's leave; each waits here for the whole step
+    // before it, whose choice it needs.
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t prev = __ldcg(&chosen[c - 1]);
+    const float nc = norm_up[prev];
+    const float2 cs = res_scale[prev];
+    const uint32_t nch = ds / 16;  // 16-byte chunks of an INT8 row
+    for (uint32_t d = tid; d < ds / 4; d += blockDim.x)
+        reinterpret_cast<float4*>(cf)[d] = reinterpret_cast<const float4*>(base + static_cast<uint64_t>(prev) * ds)[d];
+    for (uint32_t d = tid; d < nch; d += blockDim.x)
+        cq[d] = reinterpret_cast<const int4*>(b8 + static_cast<uint64_t>(prev) * ds)[d];
+    if (tid == 0) queued = 0;
     __syncthreads();
-    const float nc = norm_up[prev], rc = res_up[prev];
     const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * rows_per_block;
     const uint64_t r1 = (r0 + rows_per_block) < rows ? (r0 + rows_per_block) : rows;
-    const uint32_t g = lane >> 3, j = lane & 7u;  // 4 rows per warp, 8 lanes per row
-    const uint32_t nch = kb / 8;                    // 16-byte chunks of a BF16 row
+    constexpr uint32_t kW = 32 / kL;  // rows of a warp at a time
+    const uint32_t g = lane / kL, j = lane % kL;
     double acc = 0.0;
     uint32_t exact_here = 0;
-    const uint4* cr = reinterpret_cast<const uint4*>(cb);
-    for (uint64_t rb = r0 + warp * 4; rb < r1; rb += (kKppThreads / 32) * 4) {
-        const uint64_t r = rb + g;
-        const bool live = r < r1;
-        // Every load of the row first (its FP16 chunks; lane 0 of the group: min_d and the row's
-        // bounds), so a row costs one memory round trip.
-        float m = 0.0f, nr = 0.0f, rr = 0.0f;
-        if (live && j == 0) {
-            m = min_d[r];
-            nr = norm_up[r];
-            rr = res_up[r];
-        }
-        constexpr int kPre = 8;  // chunks per lane in flight (rows up to 512 FP16 values)
-        const uint4* xr = reinterpret_cast<const uint4*>(b16 + (live ? r : r0) * kb);
-        uint4 xa[kPre];
-#pragma unroll
-        for (int u = 0; u < kPre; ++u) {
-            const uint32_t ch = j + 8u * u;
-            xa[u] = (live && ch < nch) ? xr[ch] : make_uint4(0u, 0u, 0u, 0u);
-        }
-        float sd = 0.0f;
-        auto dot_chunk = [&](const uint4& a, const uint4& b) {
-            const __half2* a2 = reinterpret_cast<const __half2*>(&a);
-            const __half2* b2 = reinterpret_cast<const __half2*>(&b);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 fa = __half22float2(a2[i]), fb = __half22float2(b2[i]);
-                sd = fmaf(fa.x, fb.x, sd);
-                sd = fmaf(fa.y, fb.y, sd);
+    for (uint64_t s0 = r0; s0 < r1; s0 += kKppSegment) {
+        const uint64_t s1 = s0 + kKppSegment < r1 ? s0 + kKppSegment : r1;
+        for (uint64_t rb = s0 + warp * kW; rb < s1; rb += (kKppThreads / 32) * kW) {
+            const uint64_t r = rb + g;
+            const bool live = r < s1;
+            // Every load of the row first (its chunks; the group's first lane: min_d and the row's
+            // bounds), so a row costs one memory round trip.
+            float m = 0.0f, nr = 0.0f;
+            float2 rs = make_float2(0.0f, 0.0f);
+            if (live && j == 0) {
+                m = __ldcg(&min_d[r]);
+                nr = norm_up[r];
+                rs = res_scale[r];
             }
-        };
+            const int4* xr = reinterpret_cast<const int4*>(b8 + (live ? r : s0) * ds);
+            int4 xa[kPre];
 #pragma unroll
-        for (int u = 0; u < kPre; ++u) {
-            const uint32_t ch = j + 8u * u;
-            if (ch < nch) dot_chunk(xa[u], cr[ch]);
-        }
-        if (live)
-            for (uint32_t ch = j + 8u * kPre; ch < nch; ch += 8) dot_chunk(xr[ch], cr[ch]);
-        sd += __shfl_xor_sync(0xffffffffu, sd, 1);
-        sd += __shfl_xor_sync(0xffffffffu, sd, 2);
-        sd += __shfl_xor_sync(0xffffffffu, sd, 4);
-        if (live && j == 0) {
-            bool need = m > 0.0f;
-            if (need && m < FLT_MAX) {
-                // |x·c − x̂·ĉ| ≤ ‖δx‖‖c‖ + ‖x̂‖‖δc‖; + FP32 accumulation of the screen; + the f32
-                // rounding of the exact dot and of 1 − dot.
-                const float xh = nr + rr, chn = nc + rc;
-                const float e = (rr * nc + xh * rc + gamma * xh * chn + 2.4e-7f * fmaxf(1.0f, nr * nc)) * 1.001f;
-                const double lb = 1.0 - (static_cast<double>(sd) + static_cast<double>(e));
-                need = !(static_cast<double>(m) <= lb);  // a NaN bound (overflowed copy) scores exactly
+            for (int u = 0; u < kPre; ++u) {
+                const uint32_t ch = j + kL * u;
+                xa[u] = (live && ch < nch) ? __ldg(xr + ch) : make_int4(0, 0, 0, 0);
             }
-            if (need) {
-                const float dot = dot_f64_seq(base + r * ds, cf, dp);
+            int si = 0;  // |si| ≤ 127² · ds: exact below 133,000 dimensions
+            auto dot_chunk = [&](const int4& a, const int4& b) {
+                si = __dp4a(a.x, b.x, si);
+                si = __dp4a(a.y, b.y, si);
+                si = __dp4a(a.z, b.z, si);
+                si = __dp4a(a.w, b.w, si);
+            };
+#pragma unroll
+            for (int u = 0; u < kPre; ++u) {
+                const uint32_t ch = j + kL * u;
+                if (ch < nch) dot_chunk(xa[u], cq[ch]);
+            }
+            if (live)
+                for (uint32_t ch = j + kL * kPre; ch < nch; ch += kL) dot_chunk(xr[ch], cq[ch]);
+#pragma unroll
+            for (int o = 1; o < kL; o <<= 1) si += __shfl_xor_sync(0xffffffffu, si, o);
+            if (live && j == 0) {
+                bool need = m > 0.0f;
+                if (need && m < FLT_MAX) {
+                    // |x·c − x̂·ĉ| ≤ ‖δx‖‖c‖ + ‖x̂‖‖δc‖; + the roundings of the screen's product; + the
+                    // f32 rounding of the exact dot and of 1 − dot.
+                    const float sd = rs.y * cs.y * static_cast<float>(si);
+                    const float xh = nr + rs.x, chn = nc + cs.x;
+                    const float e =
+                        (rs.x * nc + xh * cs.x + 3.0e-7f * xh * chn + 2.4e-7f * fmaxf(1.0f, nr * nc)) * 1.001f;
+                    const double lb = 1.0 - (static_cast<double>(sd) + static_cast<double>(e));
+                    need = !(static_cast<double>(m) <= lb);  // a NaN bound scores exactly
+                }
+                if (need)
+                    queue[atomicAdd(&queued, 1u)] = make_uint2(static_cast<uint32_t>(r - s0), __float_as_uint(m));
+                else
+                    acc += static_cast<double>(m);
+            }
+        }
+        // The segment's rows that need it, eight lanes each: all at once, where in the loop above each
+        // would have held up its warp.
+        __syncthreads();
+        const uint32_t nq = queued;
+        const uint32_t j8 = lane & 7u;
+        for (uint32_t i0 = warp * 4; i0 < nq; i0 += kKppThreads / 8) {
+            const uint32_t i = i0 + (lane >> 3);
+            const bool on = i < nq;
+            const uint2 q = on ? queue[i] : make_uint2(0u, 0u);
+            const uint64_t r = s0 + q.x;
+            const float dot = dot_f64_lanes8(base + r * ds, cf, dp, dot_f64_err(norm_up[r], nc, dp), j8, on);
+            if (on && j8 == 0) {
+                float m = __uint_as_float(q.y);
                 const float dist = fmaxf(1.0f - dot, 0.0f);  // (1.0 - dot).max(0.0) in f32
                 if (dist < m) {
                     m = dist;
                     min_d[r] = m;
                 }
-                ++exact_here;
+                acc += static_cast<double>(m);
             }
-            acc += static_cast<double>(m);
         }
+        if (tid == 0) exact_here += nq;
+        __syncthreads();
+        if (tid == 0) queued = 0;
+        __syncthreads();
     }
     __threadfence();  // this thread's min_d writes, before the block's ticket below
     acc = warp_sum_d(acc);
     if (lane == 0) wsum[warp] = acc;
-    if (exact_here) atomicAdd(&sh_exact, static_cast<unsigned long long>(exact_here));
     __syncthreads();
     if (tid == 0) {
         double b = 0.0;
         for (uint32_t w = 0; w < kKppThreads / 32; ++w) b += wsum[w];
         partial[blockIdx.x] = b;  // exact: a sum of multiples of 2^-24 below 2^29
-        atomicAdd(&st->exact_rows, sh_exact);
+        if (exact_here) atomicAdd(&st->exact_rows, static_cast<unsigned long long>(exact_here));
         __threadfence();
         is_last = (atomicAdd(&st->done, 1u) == gridDim.x - 1) ? 1u : 0u;
     }
@@ -354,14 +566,9 @@ __global__ void __launch_bounds__(kKppThreads)
     __threadfence();
     // ---- last block: total, threshold, chosen row ----
     const uint32_t nb = gridDim.x;
-    if (warp == 0) {
-        double t = 0.0;
-        for (uint32_t b = lane; b < nb; b += 32) t += __ldcg(&partial[b]);
-        t = warp_sum_d(t);
-        if (lane == 0) sh_total = t;
-    }
-    __syncthreads();
-    const double total = sh_total;
+    auto block_sum = [&](uint32_t i) { return __ldcg(&partial[i]); };
+    RunSearch<decltype(block_sum)> in_blocks{block_sum};
+    const double total = in_blocks.scan(nb, wsum);
     if (total <= 0.0) {
         if (tid == 0) {
             chosen[c] = prev;  // duplicate of the previous centroid; the LCG does not advance
@@ -369,73 +576,25 @@ __global__ void __launch_bounds__(kKppThreads)
         }
         return;
     }
-    if (warp == 0) {
-        const unsigned long long rng = st->rng * 6364136223846793005ull + 1ull;
-        const double thr = __dmul_rn(__ddiv_rn(__ull2double_rn(rng), __ull2double_rn(~0ull)), total);
-        // First block whose running sum reaches thr (sums are exact, so this is the row-order scan).
-        double before = 0.0;
-        unsigned long long blk = nb;  // none
-        for (uint32_t b0 = 0; b0 < nb && blk == nb; b0 += 32) {
-            const double v = (b0 + lane < nb) ? __ldcg(&partial[b0 + lane]) : 0.0;
-            double incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double n = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= static_cast<uint32_t>(o)) incl += n;
-            }
-            const unsigned hit = __ballot_sync(0xffffffffu, (b0 + lane < nb) && (before + incl >= thr));
-            if (hit) {
-                const int l = __ffs(hit) - 1;
-                blk = b0 + l;
-                before += __shfl_sync(0xffffffffu, incl - v, l);
-            } else {
-                before += __shfl_sync(0xffffffffu, incl, 31);
-            }
-        }
-        if (lane == 0) {
-            st->rng = rng;
-            sh_thr = thr;
-            sh_before = before;
-            sh_blk = blk;
-            sh_found = 0;
-        }
-    }
-    __syncthreads();
+    const unsigned long long rng = st->rng * 6364136223846793005ull + 1ull;
+    const double thr = __dmul_rn(__ddiv_rn(__ull2double_rn(rng), __ull2double_rn(~0ull)), total);
+    // First block, then first row of it, whose running sum reaches thr (sums are exact, so any
+    // grouping gives the row-order scan).
+    double before = 0.0;
+    const uint32_t blk = in_blocks.first_reaching(nb, thr, before, &sh_at, &sh_before);
     uint64_t chosen_row = rows - 1;
-    if (sh_blk < nb) {
-        const uint64_t b0 = sh_blk * rows_per_block;
+    if (blk < nb) {
+        const uint64_t b0 = static_cast<uint64_t>(blk) * rows_per_block;
         const uint64_t b1 = (b0 + rows_per_block) < rows ? (b0 + rows_per_block) : rows;
-        double before = sh_before;
-        for (uint64_t s0 = b0; s0 < b1; s0 += kKppScanChunk) {
-            const uint32_t n = static_cast<uint32_t>((b1 - s0) < kKppScanChunk ? (b1 - s0) : kKppScanChunk);
-            for (uint32_t i = tid; i < n; i += blockDim.x) scan_buf[i] = __ldcg(&min_d[s0 + i]);
-            __syncthreads();
-            if (warp == 0) {
-                for (uint32_t i0 = 0; i0 < n; i0 += 32) {
-                    const double v = (i0 + lane < n) ? static_cast<double>(scan_buf[i0 + lane]) : 0.0;
-                    double incl = v;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const double nn = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= static_cast<uint32_t>(o)) incl += nn;
-                    }
-                    const unsigned hit = __ballot_sync(0xffffffffu, (i0 + lane < n) && (before + incl >= sh_thr));
-                    if (hit) {
-                        if (lane == 0) {
-                            sh_found = 1;
-                            sh_blk = s0 + i0 + (__ffs(hit) - 1);  // reuse: the chosen row
-                        }
-                        break;
-                    }
-                    before += __shfl_sync(0xffffffffu, incl, 31);
-                }
-            }
-            __syncthreads();
-            if (sh_found) break;
-        }
-        if (sh_found) chosen_row = sh_blk;
+        const uint32_t n = static_cast<uint32_t>(b1 - b0);
+        auto row_min = [&](uint32_t i) { return static_cast<double>(__ldcg(&min_d[b0 + i])); };
+        RunSearch<decltype(row_min)> in_rows{row_min};
+        in_rows.scan(n, wsum);
+        const uint32_t at = in_rows.first_reaching(n, thr, before, &sh_at, &sh_before);
+        if (at < b1 - b0) chosen_row = b0 + at;
     }
     if (tid == 0) {
+        st->rng = rng;
         chosen[c] = static_cast<uint32_t>(chosen_row);
         st->done = 0;
     }
@@ -565,6 +724,9 @@ struct AssignParams {
 // every centroid whose approximate score reaches s1 − 2e is a candidate (any other scores strictly
 // lower than the best, exactly). One candidate: assigned. Up to kCandCap: queued for the exact
 // decision among them. More (or a non-finite bound): queued for the all-centroid exact pass.
+// The epilogue's instructions bound both passes: pass A takes a tree of maxima over 32 scores (68 → 43 µs
+// at 200,000 × 447 × 256), pass B one bit a score and then the few that are set (169 → 53 µs; a branch for
+// each score, which nearly every warp takes for some row, was the 169).
 template <int kMode>
 __global__ void __launch_bounds__(kAsThreads, 1)
     kmeans_assign_tc_kernel(const __grid_constant__ CUtensorMap tmap_rows, const __grid_constant__ CUtensorMap tmap_cent,
@@ -702,14 +864,34 @@ __global__ void __launch_bounds__(kAsThreads, 1)
                 uint32_t va[32], vb[32];
                 auto process = [&](const uint32_t(&v)[32], uint32_t c) {
                     const uint32_t id0 = ct * kAsN + c * 32;
+                    if (id0 >= p.nlist) return;
+                    const uint32_t valid = p.nlist - id0 < 32 ? (1u << (p.nlist - id0)) - 1u : 0xffffffffu;
+                    if (kMode == 0) {
+                        if (valid == 0xffffffffu) {
+                            float m[16];
 #pragma unroll
-                    for (uint32_t jj = 0; jj < 32; ++jj) {
-                        const float sv = __uint_as_float(v[jj]);
-                        if (kMode == 0) {
-                            if (sv > s1 && id0 + jj < p.nlist) s1 = sv;
-                        } else if (sv >= thr && id0 + jj < p.nlist) {
-                            if (ncand == 0) first = id0 + jj;
-                            if (ncand < kCandCap) my_list[ncand] = id0 + jj;
+                            for (uint32_t jj = 0; jj < 16; ++jj)
+                                m[jj] = fmaxf(__uint_as_float(v[jj]), __uint_as_float(v[jj + 16]));
+#pragma unroll
+                            for (uint32_t h = 8; h > 0; h >>= 1)
+#pragma unroll
+                                for (uint32_t jj = 0; jj < h; ++jj) m[jj] = fmaxf(m[jj], m[jj + h]);
+                            s1 = fmaxf(s1, m[0]);  // skips NaN, like the comparison below
+                        } else {
+#pragma unroll
+                            for (uint32_t jj = 0; jj < 32; ++jj)
+                                if (((valid >> jj) & 1u) && __uint_as_float(v[jj]) > s1) s1 = __uint_as_float(v[jj]);
+                        }
+                    } else {
+                        // one bit per score first: nearly every warp has a row with a candidate here
+                        uint32_t pass = 0;
+#pragma unroll
+                        for (uint32_t jj = 0; jj < 32; ++jj)
+                            if (__uint_as_float(v[jj]) >= thr) pass |= 1u << jj;
+                        for (pass &= valid; pass; pass &= pass - 1u) {
+                            const uint32_t id = id0 + __ffs(pass) - 1;
+                            if (ncand == 0) first = id;
+                            if (ncand < kCandCap) my_list[ncand] = id;
                             ++ncand;
                         }
                     }
@@ -820,56 +1002,78 @@ __global__ void __launch_bounds__(256)
 // Stable counting sort of rows by cluster: per-block histograms (cluster-major), one exclusive
 // scan, and a scatter that keeps row order inside each cluster (warp match + running cursors).
 // ------------------------------------------------------------------------------------------
-namespace {
-constexpr uint32_t kSortRows = 2048;  // rows per histogram / scatter block
-}
-
 __global__ void cluster_hist_kernel(const uint32_t* __restrict__ assign, uint64_t rows, uint32_t nlist,
-                                    uint32_t nblk, uint32_t* __restrict__ hist) {
+                                    uint32_t nblk, uint32_t sort_rows, uint32_t* __restrict__ hist) {
     extern __shared__ uint32_t h[];
     for (uint32_t c = threadIdx.x; c < nlist; c += blockDim.x) h[c] = 0;
     __syncthreads();
-    const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * kSortRows;
-    const uint64_t r1 = (r0 + kSortRows) < rows ? (r0 + kSortRows) : rows;
+    const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * sort_rows;
+    const uint64_t r1 = (r0 + sort_rows) < rows ? (r0 + sort_rows) : rows;
     for (uint64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) atomicAdd(&h[assign[r]], 1u);
     __syncthreads();
     for (uint32_t c = threadIdx.x; c < nlist; c += blockDim.x)
         hist[static_cast<uint64_t>(c) * nblk + blockIdx.x] = h[c];
 }
 
-// Exclusive scan of n u32 in place (one block; n up to a few million). out[n] = total.
-__global__ void __launch_bounds__(1024) exclusive_scan_kernel(uint32_t* __restrict__ v, uint64_t n) {
-    __shared__ uint32_t part[1024];
-    const uint32_t t = threadIdx.x;
-    const uint64_t per = (n + 1023) / 1024;
-    const uint64_t b = t * per, e = (b + per) < n ? (b + per) : n;
-    uint32_t s = 0;
-    for (uint64_t i = b; i < e; ++i) s += v[i];
-    part[t] = s;
-    __syncthreads();
-    for (uint32_t o = 1; o < 1024; o <<= 1) {
-        const uint32_t x = t >= o ? part[t - o] : 0u;
-        __syncthreads();
-        part[t] += x;
-        __syncthreads();
+// Per cluster: its blocks' counts → what stands before each block's, and the cluster's size. One warp
+// per cluster.
+__global__ void cluster_prefix_kernel(uint32_t* __restrict__ hist, uint32_t nlist, uint32_t nblk,
+                                      uint32_t* __restrict__ size) {
+    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (c >= nlist) return;
+    uint32_t* h = hist + static_cast<uint64_t>(c) * nblk;
+    uint32_t run = 0;
+    for (uint32_t b0 = 0; b0 < nblk; b0 += 32) {
+        const uint32_t x = b0 + lane < nblk ? h[b0 + lane] : 0u;
+        uint32_t incl = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= static_cast<uint32_t>(o)) incl += y;
+        }
+        if (b0 + lane < nblk) h[b0 + lane] = run + incl - x;
+        run += __shfl_sync(0xffffffffu, incl, 31);
     }
-    uint32_t run = part[t] - s;
-    for (uint64_t i = b; i < e; ++i) {
-        const uint32_t x = v[i];
-        v[i] = run;
-        run += x;
+    if (lane == 0) size[c] = run;
+}
+
+// List offsets: the exclusive scan of the clusters' sizes, and the number of rows after the last. One block.
+__global__ void __launch_bounds__(1024) list_offsets_kernel(const uint32_t* __restrict__ size, uint32_t nlist,
+                                                            uint32_t* __restrict__ offsets) {
+    __shared__ uint32_t wsum[32];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    uint32_t run = 0;
+    for (uint32_t c0 = 0; c0 < nlist; c0 += 1024) {
+        const uint32_t x = c0 + t < nlist ? size[c0 + t] : 0u;
+        uint32_t incl = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= static_cast<uint32_t>(o)) incl += y;
+        }
+        __syncthreads();
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        uint32_t before = run, total = 0;
+        for (uint32_t w = 0; w < 32; ++w) {
+            before += w < warp ? wsum[w] : 0u;
+            total += wsum[w];
+        }
+        if (c0 + t < nlist) offsets[c0 + t] = before + incl - x;
+        run += total;
     }
-    if (t == 1023) v[n] = part[1023];
+    if (t == 0) offsets[nlist] = run;
 }
 
 __global__ void cluster_scatter_kernel(const uint32_t* __restrict__ assign, uint64_t rows, uint32_t nlist,
-                                       uint32_t nblk, const uint32_t* __restrict__ off, uint32_t* __restrict__ perm) {
+                                       uint32_t nblk, uint32_t sort_rows, const uint32_t* __restrict__ hist,
+                                       const uint32_t* __restrict__ offsets, uint32_t* __restrict__ perm) {
     extern __shared__ uint32_t cursor[];
     const uint32_t lane = threadIdx.x;  // one warp per block
-    for (uint32_t c = lane; c < nlist; c += 32) cursor[c] = off[static_cast<uint64_t>(c) * nblk + blockIdx.x];
+    for (uint32_t c = lane; c < nlist; c += 32) cursor[c] = offsets[c] + hist[static_cast<uint64_t>(c) * nblk + blockIdx.x];
     __syncwarp();
-    const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * kSortRows;
-    const uint64_t r1 = (r0 + kSortRows) < rows ? (r0 + kSortRows) : rows;
+    const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * sort_rows;
+    const uint64_t r1 = (r0 + sort_rows) < rows ? (r0 + sort_rows) : rows;
     const uint32_t lt = (1u << lane) - 1u;
     for (uint64_t rb = r0; rb < r1; rb += 32) {
         const uint64_t r = rb + lane;
@@ -888,14 +1092,6 @@ __global__ void cluster_scatter_kernel(const uint32_t* __restrict__ assign, uint
     }
 }
 
-// list offsets: offsets[c] = off[c·nblk] (the first block's position of cluster c); offsets[nlist] = rows.
-__global__ void list_offsets_kernel(const uint32_t* __restrict__ off, uint32_t nlist, uint32_t nblk, uint64_t rows,
-                                    uint32_t* __restrict__ offsets) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < nlist) offsets[c] = off[static_cast<uint64_t>(c) * nblk];
-    if (c == nlist) offsets[c] = static_cast<uint32_t>(rows);
-}
-
 // ------------------------------------------------------------------------------------------
 // Centroid update (src/approx.rs:495-531). Sums: grid (nlist, ds/32), one warp, lane = dimension,
 // the cluster's rows in row order; the loads run ahead of the (sequential) FP64 additions.
@@ -908,7 +1104,7 @@ __global__ void __launch_bounds__(32)
     const uint32_t b = offsets[c], e = offsets[c + 1];
     double s = 0.0;
     uint32_t i = b;
-    constexpr uint32_t U = 16;
+    constexpr uint32_t U = 32;
     for (; i + U <= e; i += U) {
         uint32_t r[U];
         float v[U];
@@ -1145,11 +1341,14 @@ int ivf_build(CudaIndex& ix) {
     cudaMemsetAsync(v.d_cent_t, 0, ds * v.nlist_pad * sizeof(float), s);
 
     // ---- scratch ----
-    __half* b16 = nullptr;  // FP16 rows of the build (screens and the assignment GEMM)
+    // FP16 rows of the assignment GEMM; the seeding before it has its INT8 rows (ds ≤ kb bytes each) there.
+    __half* b16 = nullptr;
     if ((e = tmp.alloc(b16, ix.rows_alloc * kb)) != cudaSuccess) return oom("IVF FP16 rows");
-    cudaMemsetAsync(b16, 0, ix.rows_alloc * kb * sizeof(__half), s);
+    if (ix.rows_alloc > rows)
+        cudaMemsetAsync(b16 + rows * kb, 0, (ix.rows_alloc - rows) * kb * sizeof(__half), s);
     float *norm_up, *res_up, *min_d, *mean_f32;
-    uint32_t *chosen, *assign, *amb, *amb_cnt, *hist, *perm;
+    float2* res_scale;
+    uint32_t *chosen, *assign, *amb, *amb_cnt, *hist, *list_size, *perm;
     unsigned int* cmax;
     unsigned long long* best;
     double *partial, *sums;
@@ -1158,11 +1357,16 @@ int ivf_build(CudaIndex& ix) {
     uint2* cand;
     uint32_t *cand_cnt, *cand_list;
     float* smax;
-    const uint32_t nblk_sort = static_cast<uint32_t>((rows + kSortRows - 1) / kSortRows);
+    // Rows of a sort block: a warp scatters them 32 at a time, one after another, so few, until the blocks'
+    // histograms (nlist counts each) would outweigh the rows. 200,000 rows, 447 lists: 2,048 → 512 rows
+    // took the scatter from 29 to 11 µs.
+    const uint64_t sort_rows = nlist <= 1024 ? 512 : 2048;
+    const uint32_t nblk_sort = static_cast<uint32_t>((rows + sort_rows - 1) / sort_rows);
     if ((e = tmp.alloc(norm_up, rows)) || (e = tmp.alloc(res_up, rows)) || (e = tmp.alloc(min_d, rows)) ||
+        (e = tmp.alloc(res_scale, rows)) || (e = tmp.alloc(list_size, nlist)) ||
         (e = tmp.alloc(mean_f32, ds)) || (e = tmp.alloc(chosen, nlist)) || (e = tmp.alloc(assign, rows)) ||
         (e = tmp.alloc(amb, rows)) || (e = tmp.alloc(amb_cnt, 1)) ||
-        (e = tmp.alloc(hist, nlist * nblk_sort + 1)) || (e = tmp.alloc(cmax, 2)) || (e = tmp.alloc(best, 1)) ||
+        (e = tmp.alloc(hist, nlist * nblk_sort)) || (e = tmp.alloc(cmax, 2)) || (e = tmp.alloc(best, 1)) ||
         (e = tmp.alloc(sums, nlist * ds)) || (e = tmp.alloc(kst, 1)) || (e = tmp.alloc(c16, v.nlist_pad * kb)) ||
         (e = tmp.alloc(cand, rows)) || (e = tmp.alloc(cand_cnt, 1)) || (e = tmp.alloc(smax, rows)) ||
         (e = tmp.alloc(cand_list, rows * kCandCap)))
@@ -1173,13 +1377,10 @@ int ivf_build(CudaIndex& ix) {
     Timer t_all, t_seed, t_km, t_lay;
     cudaEventRecord(t_all.a, s);
     cudaEventRecord(t_seed.a, s);
-    // Row bounds (and the BF16 copy when the index keeps none).
-    {
-        const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((rows + 7) / 8, ix.sm_count * 16ull));
-        ivf_row_prep_kernel<<<blocks, 256, 0, s>>>(ix.d_base, static_cast<uint32_t>(ds), rows, b16,
-                                                   static_cast<uint32_t>(kb), norm_up, res_up);
-        count_launch();
-    }
+    const uint32_t prep_blocks = static_cast<uint32_t>(std::min<uint64_t>((rows + 7) / 8, ix.sm_count * 16ull));
+    signed char* b8 = reinterpret_cast<signed char*>(b16);
+    ivf_row_prep8_kernel<<<prep_blocks, 256, 0, s>>>(ix.d_base, static_cast<uint32_t>(ds), rows, b8, norm_up, res_scale);
+    count_launch();
     // Medoid.
     {
         const size_t smem = 1024 + kColStages * kColStageBytes + 2 * kColStages * 8 + 16;
@@ -1194,20 +1395,14 @@ int ivf_build(CudaIndex& ix) {
                                                                static_cast<uint32_t>(dp), rows, mean_f32, best);
         count_launch();
     }
-    unsigned long long h_best = 0;
-    cudaMemcpyAsync(&h_best, best, sizeof(h_best), cudaMemcpyDeviceToHost, s);
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(e, "IVF medoid");
-    const uint32_t medoid = 0xFFFFFFFFu - static_cast<uint32_t>(h_best & 0xFFFFFFFFu);
-    cudaMemcpyAsync(chosen, &medoid, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
 
     // k-means++ seeding.
-    const float gamma = static_cast<float>(kb) * 1.2e-7f;  // K · 2^-23: FP32 accumulation of K products
     {
-        KppState h{};
-        h.rng = ix.opts.has_seed ? ix.opts.seed : rows * 2654435761ull + dp;
-        cudaMemcpyAsync(kst, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-        const size_t smem = ds * sizeof(float) + kb * sizeof(__half) + kKppScanChunk * sizeof(float);
-        auto kern = kpp_step_kernel;
+        kpp_init_kernel<<<1, 1, 0, s>>>(best, ix.opts.has_seed ? ix.opts.seed : rows * 2654435761ull + dp, kst, chosen);
+        count_launch();
+        const size_t smem = ds * sizeof(float) + ds;
+        // Four lanes a row while they have all of it in flight (8 chunks of 16 values each), else eight.
+        auto kern = ds <= 256 ? kpp_step_kernel<4, 4> : ds <= 512 ? kpp_step_kernel<8, 4> : kpp_step_kernel<8, 8>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         // One resident wave: every block streams its row range once, none waits for a second wave.
         int per_sm = 0;
@@ -1221,10 +1416,22 @@ int ivf_build(CudaIndex& ix) {
         fill_f32_kernel<<<static_cast<unsigned>(std::min<uint64_t>((rows + 255) / 256, 65535)), 256, 0, s>>>(
             min_d, rows, FLT_MAX);
         count_launch();
+        cudaLaunchAttribute overlap{};
+        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        overlap.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(nb);
+        cfg.blockDim = dim3(kKppThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cfg.attrs = &overlap;
+        cfg.numAttrs = 1;
         for (uint64_t c = 1; c < nlist; ++c) {
-            kern<<<nb, kKppThreads, smem, s>>>(ix.d_base, b16, static_cast<uint32_t>(ds), static_cast<uint32_t>(kb),
-                                               static_cast<uint32_t>(dp), rows, rpb, norm_up, res_up, gamma, min_d,
-                                               partial, kst, chosen, static_cast<uint32_t>(c));
+            if ((e = cudaLaunchKernelEx(&cfg, kern, static_cast<const float*>(ix.d_base), static_cast<const signed char*>(b8),
+                                        static_cast<uint32_t>(ds), static_cast<uint32_t>(dp), rows, rpb,
+                                        static_cast<const float*>(norm_up), static_cast<const float2*>(res_scale), min_d,
+                                        partial, kst, chosen, static_cast<uint32_t>(c))) != cudaSuccess)
+                return cuda_error(e, "IVF seeding launch");
         }
         count_launch(static_cast<uint32_t>(nlist - 1));
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "IVF seeding launch");
@@ -1236,6 +1443,10 @@ int ivf_build(CudaIndex& ix) {
 
     // Spherical k-means.
     cudaEventRecord(t_km.a, s);
+    ivf_row_prep_kernel<<<prep_blocks, 256, 0, s>>>(ix.d_base, static_cast<uint32_t>(ds), rows, b16,
+                                                    static_cast<uint32_t>(kb), norm_up, res_up);
+    count_launch();
+    const float gamma = static_cast<float>(kb) * 1.2e-7f;  // K · 2^-23: FP32 accumulation of K products
     CUtensorMap tmap_rows{}, tmap_cent{};
     if (!encode_tmap_2d(&tmap_rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, b16, kb, ix.rows_alloc, kb * 2, 64, 128,
                         CU_TENSOR_MAP_SWIZZLE_128B) ||
@@ -1294,12 +1505,12 @@ int ivf_build(CudaIndex& ix) {
         cudaMemcpyAsync(d_amb_hist + 2 * it + 1, cand_cnt, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
         // Lists of this assignment (stable by row).
         cluster_hist_kernel<<<nblk_sort, 256, nlist * sizeof(uint32_t), s>>>(assign, rows, static_cast<uint32_t>(nlist),
-                                                                             nblk_sort, hist);
-        exclusive_scan_kernel<<<1, 1024, 0, s>>>(hist, nlist * nblk_sort);
-        cluster_scatter_kernel<<<nblk_sort, 32, nlist * sizeof(uint32_t), s>>>(assign, rows, static_cast<uint32_t>(nlist),
-                                                                               nblk_sort, hist, perm);
-        list_offsets_kernel<<<static_cast<unsigned>((nlist + 1 + 255) / 256), 256, 0, s>>>(
-            hist, static_cast<uint32_t>(nlist), nblk_sort, rows, v.d_offsets);
+                                                                             nblk_sort, static_cast<uint32_t>(sort_rows),
+                                                                             hist);
+        cluster_prefix_kernel<<<cp_blocks, 256, 0, s>>>(hist, static_cast<uint32_t>(nlist), nblk_sort, list_size);
+        list_offsets_kernel<<<1, 1024, 0, s>>>(list_size, static_cast<uint32_t>(nlist), v.d_offsets);
+        cluster_scatter_kernel<<<nblk_sort, 32, nlist * sizeof(uint32_t), s>>>(
+            assign, rows, static_cast<uint32_t>(nlist), nblk_sort, static_cast<uint32_t>(sort_rows), hist, v.d_offsets, perm);
         // New centroids.
         centroid_sum_kernel<<<dim3(static_cast<unsigned>(nlist), static_cast<unsigned>(ds / 32)), 32, 0, s>>>(
             ix.d_base, static_cast<uint32_t>(ds), perm, v.d_offsets, sums);
