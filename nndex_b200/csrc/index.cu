@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -231,6 +232,39 @@ void CudaIndex::drop_graphs() {
     graphs.clear();
 }
 
+// The host's words (kHostWordBytes, pinned). A page of the heap, registered, takes a third of the time that
+// a pinned allocation does (0.3 ms; the driver maps 2 MB for the first one of a process: 0.9 to 2.7).
+cudaError_t CudaIndex::alloc_words() {
+    words_page = std::aligned_alloc(kHostWordBytes, kHostWordBytes);
+    void* seen = nullptr;
+    if (words_page && cudaHostRegister(words_page, kHostWordBytes, cudaHostRegisterMapped) == cudaSuccess) {
+        if (cudaHostGetDevicePointer(&seen, words_page, 0) != cudaSuccess || seen != words_page)
+            cudaHostUnregister(words_page);  // the kernels are given the host's address
+        else
+            h_flags = static_cast<uint64_t*>(words_page);
+    }
+    if (!h_flags) {
+        cudaGetLastError();
+        std::free(words_page);
+        words_page = nullptr;
+        const cudaError_t e = cudaMallocHost(&h_flags, kHostWordBytes);
+        if (e != cudaSuccess) return e;
+    }
+    uint8_t* const at = reinterpret_cast<uint8_t*>(h_flags);
+    h_fbn = reinterpret_cast<uint32_t*>(at + kFbnAt);
+    ivf_scratch.h_probed = reinterpret_cast<unsigned long long*>(at + kProbedAt);
+    return cudaSuccess;
+}
+
+void CudaIndex::free_words() {
+    if (words_page) {
+        cudaHostUnregister(words_page);
+        std::free(words_page);
+    } else {
+        cudaFreeHost(h_flags);
+    }
+}
+
 CudaIndex::~CudaIndex() {
     cudaSetDevice(device);
     cudaStreamSynchronize(stream);
@@ -239,34 +273,24 @@ CudaIndex::~CudaIndex() {
         cudaEventDestroy(p.first);
         cudaEventDestroy(p.second);
     }
-    if (owns_base) cudaFree(d_base);
+    cudaFree(d_mem);  // an owner's rows and copies, and the device words; a view's words
     cudaFree(d_qraw);
     cudaFree(d_qn);
     cudaFree(d_ws);
     cudaFree(d_res);
-    cudaFree(d_err);  // d_status lives in the same allocation
     cudaFree(d_part_keys);
     cudaFree(d_part_done);
     cudaFreeHost(h_q);
     cudaFreeHost(h_res);
-    cudaFreeHost(h_flags);
-    if (owns_base) cudaFree(d_base_bf16);
-    if (owns_base) cudaFree(d_base_fp8);
-    if (owns_base) cudaFree(d_res16);
-    if (owns_base) cudaFree(d_res8);
-    if (owns_base) cudaFree(d_row_scale);
-    if (owns_base) cudaFree(d_tile_scale);
+    free_words();
     cudaFree(d_q_bf16);
     cudaFree(d_q_fp8);
     cudaFree(d_q_scale);
     cudaFree(d_q_resid);
-    if (owns_base) cudaFree(d_tfnorm);
     cudaFree(d_serr);
     cudaFree(d_serr_acc);
     cudaFreeHost(h_serr_acc);
     cudaFree(d_fbq);
-    cudaFree(d_fbn);
-    cudaFreeHost(h_fbn);
     cudaFree(d_thr);
     cudaFree(d_cand_idx);
     cudaFree(d_cand_sim);
@@ -611,16 +635,14 @@ int CudaIndex::enqueue_prep_queries(const float* d_raw, uint64_t n, int mode, in
         if ((st = ivf_plan_words(*this, &p.zero[0], &p.zero_words[0]))) return st;
     } else if (path == 6) {
         if ((st = grow_device(d_floor, cap_floor, n, "tc workspace"))) return st;
-        if ((st = ensure_fbn())) return st;
-        p.zero[0] = reinterpret_cast<uint32_t*>(d_floor);
+            p.zero[0] = reinterpret_cast<uint32_t*>(d_floor);
         p.zero_words[0] = 2 * n;
         p.zero[1] = d_fbn;
         p.zero_words[1] = 1;
     } else if (path == 7) {
         if ((st = grow_device(d_q_resid, cap_q_resid, n, "query buffer"))) return st;
         if ((st = grow_device(d_cnt2, cap_cnt2, n, "pass-2 buffer"))) return st;
-        if ((st = ensure_fbn())) return st;
-        p.tf_slack = d_q_resid;
+            p.tf_slack = d_q_resid;
         p.tf_row_max = d_tfnorm + rows;
         p.tf_c_norm = tf32_c_norm();
         p.tf_collected = d_cnt2;
@@ -682,7 +704,6 @@ int CudaIndex::enqueue_tc(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o_idx, 
     if ((st = grow_device(d_thr, cap_thr, n, "tc workspace"))) return st;
     if ((st = grow_device(d_ws, cap_ws, per_query * n, "tc workspace"))) return st;
     if ((st = grow_device(d_ids, cap_ids, n, "pass-2 buffer"))) return st;
-    if ((st = ensure_fbn())) return st;
     if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_sim, cap_cand_sim, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_cnt, cap_cand_cnt, n, "tc workspace"))) return st;
@@ -851,15 +872,6 @@ int CudaIndex::encode_query_tmap(bool fp8, void* buf, uint32_t n, CUtensorMap* m
     return NNDEX_OK;
 }
 
-int CudaIndex::ensure_fbn() {
-    if (d_fbn) return NNDEX_OK;
-    cudaError_t e;
-    if ((e = cudaMalloc(&d_fbn, kFbnBytes)) != cudaSuccess ||
-        (e = cudaMallocHost(&h_fbn, kFbnBytes)) != cudaSuccess)
-        return cuda_error(e, "fallback buffer");
-    return NNDEX_OK;
-}
-
 // After pass 1: queries whose certificate held are final. The others run pass 2 (collect every row
 // whose upper bound reaches their exact k-th score, rerank exactly) — all on the device, sized for
 // the worst case (every query uncertified), the kernels reading the count that the compaction left.
@@ -869,7 +881,6 @@ int CudaIndex::enqueue_tc_pass2(bool fp8, uint32_t n, uint32_t kcap, uint64_t* o
     const uint32_t cap2 = kSecondPassCap;
     const uint64_t row_bytes = fp8 ? kf8 : kb16 * 2;
     const uint64_t n_alloc = (n + 127) / 128 * 128;
-    if ((st = ensure_fbn())) return st;
     if ((st = grow_device(d_ids, cap_ids, n, "pass-2 buffer"))) return st;
     if ((st = grow_device(d_q2_lp, cap_q2_lp, n_alloc * row_bytes, "pass-2 buffer"))) return st;
     if ((st = grow_device(d_q2_resid, cap_q2_resid, n, "pass-2 buffer"))) return st;
@@ -1037,17 +1048,24 @@ int CudaIndex::retry_tc_pass2(bool fp8, uint32_t m, uint32_t kcap, uint64_t* o_i
                                 d_rslots, o_idx, o_sim, o_cnt, d_ok2, s);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (overflow)");
     stats.kernel_launches += 6;
-    if ((st = grow_host(h_ids, cap_hids, m, "pinned buffer"))) return st;
-    if ((st = grow_host(h_ok2, cap_hok2, m, "pinned buffer"))) return st;
-    cudaMemcpyAsync(h_ids, d_fbq, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(h_ok2, d_ok2, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    // few enough (the usual case): in the page of the host's words
+    uint32_t* ids = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(h_flags) + kWordBytes);
+    uint32_t* ok = ids + kFewIds;
+    if (m > kFewIds) {
+        if ((st = grow_host(h_ids, cap_hids, m, "pinned buffer"))) return st;
+        if ((st = grow_host(h_ok2, cap_hok2, m, "pinned buffer"))) return st;
+        ids = h_ids;
+        ok = h_ok2;
+    }
+    cudaMemcpyAsync(ids, d_fbq, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(ok, d_ok2, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     if (w_err == d_err) cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(e, "search");
     if ((st = check_device_words())) return st;
     failed->clear();
     for (uint32_t i = 0; i < m; ++i)
-        if (!h_ok2[i]) failed->push_back(h_ids[i]);
+        if (!ok[i]) failed->push_back(ids[i]);
     return NNDEX_OK;
 }
 
@@ -1095,7 +1113,6 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     const uint64_t fb_per_query = static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap;
     if ((st = grow_device(d_ws, cap_ws, std::max(per_query, fb_per_query) * n, "scan workspace"))) return st;
     if ((st = grow_device(d_fbq, cap_fbq, n, "fallback buffer"))) return st;
-    if ((st = ensure_fbn())) return st;
     if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_sim, cap_cand_sim, static_cast<uint64_t>(n) * kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_cnt, cap_cand_cnt, n, "tc workspace"))) return st;
@@ -1848,10 +1865,11 @@ int index_begin(uint64_t rows, uint64_t dims, uint32_t flags, const nndex_cuda_o
     ix->normalized = (flags & NNDEX_FLAG_NORMALIZED) != 0;
     ix->approx = (flags & NNDEX_FLAG_APPROX) != 0;
     ix->opts = o;
-    cudaDeviceProp prop;
-    cudaGetDeviceProperties(&prop, device);
-    ix->sm_count = prop.multiProcessorCount;
-    ix->smem_optin = prop.sharedMemPerBlockOptin;
+    int value = 0;
+    if ((e = cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device)) == cudaSuccess) ix->sm_count = value;
+    if (e == cudaSuccess &&
+        (e = cudaDeviceGetAttribute(&value, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)) == cudaSuccess)
+        ix->smem_optin = static_cast<size_t>(value);
     auto fail = [&](int code) {
         delete ix;
         return code;
@@ -1860,39 +1878,58 @@ int index_begin(uint64_t rows, uint64_t dims, uint32_t flags, const nndex_cuda_o
         return fail(cuda_error(e, "cudaStreamCreate"));
     cudaEventCreate(&ix->ev0);
     cudaEventCreate(&ix->ev1);
-    if ((e = cudaMalloc(&ix->d_err, 2 * sizeof(unsigned long long))) != cudaSuccess) return fail(cuda_error(e, "alloc"));
-    ix->d_status = reinterpret_cast<uint32_t*>(ix->d_err + 1);
-    if ((e = cudaMallocHost(&ix->h_flags, 2 * sizeof(uint64_t))) != cudaSuccess) return fail(cuda_error(e, "alloc"));
-    const size_t base_bytes = ix->rows_alloc * ix->ds * sizeof(float);
-    if ((e = cudaMalloc(&ix->d_base, base_bytes)) != cudaSuccess) return fail(cuda_error(e, "base allocation"));
-    cudaMemsetAsync(ix->d_base + rows * ix->ds, 0, (ix->rows_alloc - rows) * ix->ds * sizeof(float), ix->stream);
-    cudaMemsetAsync(ix->d_err, 0, 2 * sizeof(unsigned long long), ix->stream);
-    ix->use_device_words();
-    // Row norms of the TF32 scans' bounds (8 bytes per row, written by K1; the last entry their maxima).
-    // Without them (no memory) FP32 batches take the FP32 scan.
-    if (cudaMalloc(&ix->d_tfnorm, (rows + 1) * sizeof(float2)) == cudaSuccess) {
-        cudaMemsetAsync(ix->d_tfnorm + rows, 0, sizeof(float2), ix->stream);
-    } else {
+    if ((e = ix->alloc_words()) != cudaSuccess) return fail(cuda_error(e, "alloc"));
+    // Everything on the device that lasts as long as the index, in one allocation: the driver takes 0.3
+    // to 1 ms for each, and as much to free it. Low-precision scoring copies: K1 writes them in the same
+    // pass as the rows.
+    const bool bf16 = (flags & NNDEX_FLAG_BF16) != 0, fp8 = (flags & NNDEX_FLAG_FP8) != 0;
+    if (bf16) ix->kb16 = (dims + 63) / 64 * 64;
+    if (fp8) ix->kf8 = (dims + 127) / 128 * 128;
+    auto carve = [&](Carver c, bool tf_norms) {
+        c.take(ix->d_base, ix->rows_alloc * ix->ds);
+        if (bf16) {
+            c.take(ix->d_base_bf16, ix->rows_alloc * ix->kb16);
+            c.take(ix->d_res16, rows);
+        }
+        if (fp8) {
+            c.take(ix->d_base_fp8, ix->rows_alloc * ix->kf8);
+            c.take(ix->d_row_scale, ix->rows_alloc);
+            c.take(ix->d_tile_scale, ix->rows_alloc / 256);
+            c.take(ix->d_res8, rows);
+        }
+        uint8_t* words = nullptr;
+        c.take(words, CudaIndex::kWordBytes);
+        ix->set_device_words(words);
+        // Row norms of the TF32 scans' bounds (8 bytes per row, written by K1; the last entry their maxima).
         ix->d_tfnorm = nullptr;
+        if (tf_norms) c.take(ix->d_tfnorm, rows + 1);
+        return c.used;
+    };
+    bool tf_norms = true;
+    e = cudaMalloc(&ix->d_mem, carve(Carver{}, true));
+    if (e != cudaSuccess) {  // without the norms (no memory) FP32 batches take the FP32 scan
         cudaGetLastError();
+        tf_norms = false;
+        e = cudaMalloc(&ix->d_mem, carve(Carver{}, false));
     }
-    // Low-precision scoring copies (K1 writes them in the same pass) and their residual norms.
-    if (flags & NNDEX_FLAG_BF16) {
-        ix->kb16 = (dims + 63) / 64 * 64;
-        if ((e = cudaMalloc(&ix->d_base_bf16, ix->rows_alloc * ix->kb16 * 2)) != cudaSuccess ||
-            (e = cudaMalloc(&ix->d_res16, rows * sizeof(float))) != cudaSuccess)
-            return fail(cuda_error(e, "BF16 copy allocation"));
-        cudaMemsetAsync(ix->d_base_bf16, 0, ix->rows_alloc * ix->kb16 * 2, ix->stream);
+    if (e != cudaSuccess) {
+        ix->d_mem = nullptr;
+        return fail(cuda_error(e, bf16 || fp8 ? "base and low-precision copies allocation" : "base allocation"));
     }
-    if (flags & NNDEX_FLAG_FP8) {
-        ix->kf8 = (dims + 127) / 128 * 128;
-        if ((e = cudaMalloc(&ix->d_base_fp8, ix->rows_alloc * ix->kf8)) != cudaSuccess ||
-            (e = cudaMalloc(&ix->d_row_scale, ix->rows_alloc * sizeof(float))) != cudaSuccess ||
-            (e = cudaMalloc(&ix->d_res8, rows * sizeof(float))) != cudaSuccess)
-            return fail(cuda_error(e, "FP8 copy allocation"));
-        cudaMemsetAsync(ix->d_base_fp8, 0, ix->rows_alloc * ix->kf8, ix->stream);
-        cudaMemsetAsync(ix->d_row_scale, 0, ix->rows_alloc * sizeof(float), ix->stream);
+    carve(Carver{static_cast<uint8_t*>(ix->d_mem)}, tf_norms);
+    // What K1 does not write: the rows that fill the last tile, and the words.
+    const uint64_t pad = ix->rows_alloc - rows;
+    cudaMemsetAsync(ix->d_err, 0, CudaIndex::kWordBytes, ix->stream);
+    if (tf_norms) cudaMemsetAsync(ix->d_tfnorm + rows, 0, sizeof(float2), ix->stream);
+    if (pad) {
+        cudaMemsetAsync(ix->d_base + rows * ix->ds, 0, pad * ix->ds * sizeof(float), ix->stream);
+        if (bf16) cudaMemsetAsync(ix->d_base_bf16 + rows * ix->kb16, 0, pad * ix->kb16 * 2, ix->stream);
+        if (fp8) {
+            cudaMemsetAsync(ix->d_base_fp8 + rows * ix->kf8, 0, pad * ix->kf8, ix->stream);
+            cudaMemsetAsync(ix->d_row_scale + rows, 0, pad * sizeof(float), ix->stream);
+        }
     }
+    ix->use_device_words();
     *out = ix;
     return NNDEX_OK;
 }
@@ -1937,15 +1974,12 @@ int index_finish(CudaIndex* ix) {
     if (ix->h_flags[0] != 0) return fail(err_code(static_cast<int>(~ix->h_flags[0] & 0xFF)));
     if (ix->d_res16 || ix->d_res8) {
         // ε of the certificate: the largest residual norm ‖x − x̂‖ over the rows.
-        unsigned int* d_max = nullptr;
-        if ((e = cudaMalloc(&d_max, 2 * sizeof(unsigned int))) != cudaSuccess) return fail(cuda_error(e, "alloc"));
-        cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned int), ix->stream);
+        unsigned int* d_max = ix->d_max;  // zero since index_begin
         if (ix->d_res16) launch_max_reduce(ix->d_res16, ix->rows, d_max, ix->stream);
         if (ix->d_res8) launch_max_reduce(ix->d_res8, ix->rows, d_max + 1, ix->stream);
         unsigned int hm[2] = {0, 0};
         cudaMemcpyAsync(hm, d_max, sizeof(hm), cudaMemcpyDeviceToHost, ix->stream);
         e = cudaStreamSynchronize(ix->stream);
-        cudaFree(d_max);
         if (e != cudaSuccess) return fail(cuda_error(e, "residual reduction"));
         std::memcpy(&ix->eps_bf16, &hm[0], 4);
         std::memcpy(&ix->eps_fp8, &hm[1], 4);
@@ -1973,8 +2007,6 @@ int index_finish(CudaIndex* ix) {
         return fail(set_error(NNDEX_ERR_CUDA, "cuda execution error: cuTensorMapEncodeTiled failed (FP8)"));
     if (ix->d_row_scale) {
         // FP8 scan: the scale extremes of each 256-row tile (its epilogue's per-tile cut)
-        if ((e = cudaMalloc(&ix->d_tile_scale, ix->rows_alloc / 256 * sizeof(float2))) != cudaSuccess)
-            return fail(cuda_error(e, "FP8 tile scales"));
         launch_tile_scale(ix->d_row_scale, ix->rows, ix->rows_alloc / 256, ix->d_tile_scale, ix->stream);
     }
     if (ix->approx) {
@@ -1995,7 +2027,7 @@ int create_index(const float* matrix, bool on_device, uint64_t n_values, uint64_
     int st = index_begin(rows, dims, flags, opts, &ix);
     if (st) return st;
     cudaError_t e = cudaSuccess;
-    // K1: upload in chunks (≈256 MB of raw rows each), validate + normalise + pad on the device.
+    // K1: upload in chunks (≈32 MB of raw rows each: a pageable copy is as fast as with 256, and there is less to map and free), validate + normalise + pad on the device.
     if (on_device) {
         // The caller may still be writing the matrix on any stream: wait for the device first.
         if ((e = cudaDeviceSynchronize()) != cudaSuccess) {
@@ -2004,18 +2036,17 @@ int create_index(const float* matrix, bool on_device, uint64_t n_values, uint64_
         }
         index_prep_rows(ix, matrix, 0, rows);
     } else {
-        uint64_t chunk_rows = std::max<uint64_t>(1, (256ull << 20) / (dims * sizeof(float)));
+        uint64_t chunk_rows = std::max<uint64_t>(1, (32ull << 20) / (dims * sizeof(float)));
         chunk_rows = std::min(chunk_rows, rows);
+        const int nbuf = chunk_rows < rows ? 2 : 1;
         float* d_raw[2] = {nullptr, nullptr};
         cudaEvent_t done[2];
-        for (int b = 0; b < 2; ++b) {
-            if ((e = cudaMalloc(&d_raw[b], chunk_rows * dims * sizeof(float))) != cudaSuccess) {
-                cudaFree(d_raw[0]);
-                delete ix;
-                return cuda_error(e, "upload staging");
-            }
-            cudaEventCreateWithFlags(&done[b], cudaEventDisableTiming);
+        if ((e = cudaMalloc(&d_raw[0], nbuf * chunk_rows * dims * sizeof(float))) != cudaSuccess) {
+            delete ix;
+            return cuda_error(e, "upload staging");
         }
+        d_raw[1] = d_raw[0] + (nbuf - 1) * chunk_rows * dims;
+        for (int b = 0; b < 2; ++b) cudaEventCreateWithFlags(&done[b], cudaEventDisableTiming);
         int b = 0;
         for (uint64_t r0 = 0; r0 < rows; r0 += chunk_rows, b ^= 1) {
             const uint64_t n = std::min(chunk_rows, rows - r0);
@@ -2027,10 +2058,8 @@ int create_index(const float* matrix, bool on_device, uint64_t n_values, uint64_
             cudaEventRecord(done[b], ix->stream);
         }
         cudaStreamSynchronize(ix->stream);
-        for (int i = 0; i < 2; ++i) {
-            cudaFree(d_raw[i]);
-            cudaEventDestroy(done[i]);
-        }
+        cudaFree(d_raw[0]);
+        for (int i = 0; i < 2; ++i) cudaEventDestroy(done[i]);
         if (e != cudaSuccess) {
             delete ix;
             return cuda_error(e, "upload");
@@ -2094,13 +2123,12 @@ int make_view(const CudaIndex& src, CudaIndex** out) {
     cudaError_t e;
     if ((e = cudaStreamCreateWithFlags(&v->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreate(&v->ev0)) != cudaSuccess || (e = cudaEventCreate(&v->ev1)) != cudaSuccess ||
-        (e = cudaMalloc(&v->d_err, 2 * sizeof(unsigned long long))) != cudaSuccess ||
-        (e = cudaMallocHost(&v->h_flags, 2 * sizeof(uint64_t))) != cudaSuccess) {
+        (e = cudaMalloc(&v->d_mem, CudaIndex::kWordBytes)) != cudaSuccess || (e = v->alloc_words()) != cudaSuccess) {
         delete v;
         return cuda_error(e, "index view");
     }
-    v->d_status = reinterpret_cast<uint32_t*>(v->d_err + 1);
-    cudaMemsetAsync(v->d_err, 0, 2 * sizeof(unsigned long long), v->stream);
+    v->set_device_words(static_cast<uint8_t*>(v->d_mem));
+    cudaMemsetAsync(v->d_err, 0, CudaIndex::kWordBytes, v->stream);
     v->use_device_words();
     cudaStreamSynchronize(v->stream);
     *out = v;

@@ -184,10 +184,27 @@ struct CudaIndex {
     float* h_sim = nullptr;
     uint32_t* h_cnt = nullptr;
     size_t res_bytes = 0;        // bytes of the current batch's results
-    // Status words, adjacent in one 16-byte allocation (d_status = the word after d_err), zero when
-    // clean: of construction and of device-buffer searches, read back with one copy into h_flags.
+    // The device's words and the host's, the first kWordBytes laid out alike. Status words (d_status = the word after
+    // d_err), zero when clean: of construction and of device-buffer searches, read back with one copy
+    // into h_flags. Then the counts of a two-pass batch (d_fbn, h_fbn), and construction's maxima (device)
+    // or an IVF search's counts (host).
+    static constexpr size_t kWordBytes = 256, kFbnAt = 64, kMaxAt = 128, kProbedAt = 192;
+    // The host's go on with two lists of an overflowed batch's queries, kFewIds each.
+    static constexpr size_t kHostWordBytes = 4096;
+    static constexpr uint32_t kFewIds = (kHostWordBytes - kWordBytes) / 8;
+    void* d_mem = nullptr;  // the allocation with the device's words, and an owner's rows and copies
     unsigned long long* d_err = nullptr;
     uint32_t* d_status = nullptr;
+    unsigned int* d_max = nullptr;  // the largest residual norms of the BF16 and FP8 copies
+    void set_device_words(uint8_t* at) {
+        d_err = reinterpret_cast<unsigned long long*>(at);
+        d_status = reinterpret_cast<uint32_t*>(d_err + 1);
+        d_fbn = reinterpret_cast<uint32_t*>(at + kFbnAt);
+        d_max = reinterpret_cast<unsigned int*>(at + kMaxAt);
+    }
+    void* words_page = nullptr;  // the registered page with the host's words, if they are in one
+    cudaError_t alloc_words();
+    void free_words();
     // The current call's: d_err / d_status, or for a host-buffer search h_flags itself (the kernels
     // only ever write them on an error, and a host-buffer search waits before it reads them).
     unsigned long long* w_err = nullptr;
@@ -262,7 +279,6 @@ struct CudaIndex {
     uint32_t* h_fbn = nullptr;  // pinned copy
     uint32_t* d_tcfail = nullptr;  // TC pass 2: positions (in d_ids) of the queries whose collection overflowed
     size_t cap_tcfail = 0;
-    int ensure_fbn();
     uint64_t h_fbn_rows() const { return *reinterpret_cast<const unsigned long long*>(h_fbn + 4); }
     cudaStream_t fbn_stream = nullptr;
     bool fbn_pending = false;

@@ -11,6 +11,19 @@
 
 namespace nndex {
 
+// Lays out arrays in one allocation, 1,024-byte aligned: run over a null base first for the size (used),
+// then over the memory.
+struct Carver {
+    uint8_t* base = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T*& p, size_t n) {
+        used = (used + 1023) / 1024 * 1024;
+        p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (n ? n : 1) * sizeof(T);
+    }
+};
+
 // Number of kernels launched by this library (process-wide). Called after each launch; with
 // NNDEX_SYNC_CHECK=1 in the environment it also waits for the device and prints the launch site of
 // the first CUDA error to stderr (a debugging aid: every launch then runs alone).

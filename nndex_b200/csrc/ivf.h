@@ -25,6 +25,7 @@ struct IvfIndex {
     uint64_t nlist = 0;          // clusters (1 = single-list index, never probed)
     uint64_t iters = 0;          // k-means iterations
     uint64_t nlist_pad = 0;      // nlist rounded up to 256 (assignment GEMM tiles, dims-major stride)
+    void* d_mem = nullptr;         // the allocation that the arrays below lie in
     float* d_centroids = nullptr;  // nlist × ds FP32, final centroids (zero padded)
     float* d_cent_t = nullptr;     // ds × nlist_pad FP32, the same centroids dims-major (probe)
     CUtensorMap tmap_cent{};       // the centroids, box {32 floats, 256 rows} (probe scores)
@@ -42,6 +43,7 @@ struct IvfIndex {
     __nv_bfloat16* d_reordered16 = nullptr;  // rows_alloc × kb16
     float* d_res16 = nullptr;                // rows (reordered order)
     float eps16 = 0.0f;
+    unsigned int* d_eps = nullptr;  // its device word, written with the layout
     CUtensorMap tmap_reordered16{};
     nndex_cuda_ivf_stats stats{};
 
@@ -74,7 +76,7 @@ struct IvfScratch {
     __nv_bfloat16* d_g16 = nullptr;     size_t cap_g16 = 0;        // gathered query blocks × 128 × kb16
     uint32_t* d_lane_qid = nullptr;     size_t cap_lane_qid = 0;   // gathered blocks × 128
     uint32_t* d_lane_slot = nullptr;    size_t cap_lane_slot = 0;
-    unsigned long long* h_probed = nullptr;  // pinned [8]: FP32 scan: rows probed (Σ over queries), streamed, union
+    unsigned long long* h_probed = nullptr;  // [8] of the index's host words: FP32 scan: rows probed (Σ over queries), streamed, union
 
     ~IvfScratch();
 };

@@ -1174,14 +1174,7 @@ __global__ void centroid_tf32_max_kernel(const float* __restrict__ cent, uint32_
 // ------------------------------------------------------------------------------------------
 
 IvfIndex::~IvfIndex() {
-    cudaFree(d_reordered16);
-    cudaFree(d_res16);
-    cudaFree(d_centroids);
-    cudaFree(d_cent_t);
-    cudaFree(d_cent_max);
-    cudaFree(d_reordered);
-    cudaFree(d_row_map);
-    cudaFree(d_offsets);
+    cudaFree(d_mem);
 }
 
 IvfScratch::~IvfScratch() {
@@ -1200,7 +1193,6 @@ IvfScratch::~IvfScratch() {
     cudaFree(d_list_slot);
     cudaFree(d_q_slot_off);
     cudaFree(d_ws);
-    cudaFreeHost(h_probed);
 }
 
 static uint64_t isqrt_u64(uint64_t n) {
@@ -1235,21 +1227,50 @@ uint64_t ivf_choose_nprobe(uint64_t nlist, uint64_t k, uint64_t rows) {
     return nprobe;
 }
 
+// Everything the index keeps, in one allocation (the driver takes 0.3 to 1 ms for each, and as much to
+// free it), with the words a build needs after its layout has begun.
+struct BuildKeep {
+    uint32_t* chosen = nullptr;    // nlist: the seeding's rows
+    uint32_t* amb_hist = nullptr;  // per iteration: rows of the full exact pass, rows decided among candidates
+    KppState* kst = nullptr;
+};
+
+static cudaError_t ivf_alloc(const CudaIndex& ix, IvfIndex& v, BuildKeep* keep) {
+    v.nlist_pad = (v.nlist + 255) / 256 * 256;
+    v.kb16 = (ix.dims + 63) / 64 * 64;
+    auto carve = [&](Carver c) {
+        c.take(v.d_reordered, ix.rows_alloc * ix.ds);
+        c.take(v.d_reordered16, ix.rows_alloc * v.kb16);
+        c.take(v.d_res16, ix.rows);
+        c.take(v.d_row_map, ix.rows);
+        c.take(v.d_centroids, v.nlist * ix.ds);
+        c.take(v.d_cent_t, ix.ds * v.nlist_pad);
+        c.take(v.d_cent_max, 1);
+        c.take(v.d_eps, 1);
+        c.take(v.d_offsets, v.nlist + 1);
+        if (keep) {
+            c.take(keep->chosen, v.nlist);
+            c.take(keep->amb_hist, 2 * v.iters);
+            c.take(keep->kst, 1);
+        }
+        return c.used;
+    };
+    const cudaError_t e = cudaMalloc(&v.d_mem, carve(Carver{}));
+    if (e != cudaSuccess) {
+        v.d_mem = nullptr;
+        return e;
+    }
+    carve(Carver{static_cast<uint8_t*>(v.d_mem)});
+    return cudaSuccess;
+}
+
 namespace {
 
 // Device scratch of one build, freed on every exit path.
+// Scratch of a build that does not fit the memory of its own result.
 struct BuildScratch {
-    std::vector<void*> ptrs;
-    ~BuildScratch() {
-        for (void* p : ptrs) cudaFree(p);
-    }
-    template <class T>
-    cudaError_t alloc(T*& p, size_t n) {
-        p = nullptr;
-        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), std::max<size_t>(n, 1) * sizeof(T));
-        if (e == cudaSuccess) ptrs.push_back(p);
-        return e;
-    }
+    void* p = nullptr;
+    ~BuildScratch() { cudaFree(p); }
 };
 
 struct Timer {
@@ -1269,30 +1290,24 @@ struct Timer {
 // Cluster-contiguous copies of the rows for the list scans, in the order of v.d_row_map: the FP32
 // rows and their BF16 copy with per-row residual bounds, whose maximum is raised into *d_eps.
 // Enqueued on ix.stream.
-static cudaError_t ivf_enqueue_layout(CudaIndex& ix, IvfIndex& v, unsigned int* d_eps) {
-    const uint64_t rows = ix.rows, ds = ix.ds;
+static cudaError_t ivf_enqueue_layout(CudaIndex& ix, IvfIndex& v) {
+    const uint64_t rows = ix.rows, ds = ix.ds, kb16 = v.kb16;
     const cudaStream_t s = ix.stream;
-    const uint64_t kb16 = (ix.dims + 63) / 64 * 64;
     cudaError_t e;
-    if ((e = cudaMalloc(&v.d_cent_max, sizeof(float2))) != cudaSuccess) return e;
+    cudaMemsetAsync(v.d_eps, 0, sizeof(unsigned int), s);
     cudaMemsetAsync(v.d_cent_max, 0, sizeof(float2), s);
     centroid_tf32_max_kernel<<<static_cast<unsigned>((v.nlist * 32 + 255) / 256), 256, 0, s>>>(
         v.d_centroids, static_cast<uint32_t>(ds), static_cast<uint32_t>(v.nlist), v.d_cent_max);
     count_launch();
-    if ((e = cudaMalloc(&v.d_reordered, ix.rows_alloc * ds * sizeof(float))) != cudaSuccess) return e;
     cudaMemsetAsync(v.d_reordered + rows * ds, 0, (ix.rows_alloc - rows) * ds * sizeof(float), s);
     const uint32_t gb = static_cast<uint32_t>(std::min<uint64_t>((rows * 32 + 255) / 256, ix.sm_count * 16ull));
     gather_rows_kernel<<<gb, 256, 0, s>>>(ix.d_base, static_cast<uint32_t>(ds), v.d_row_map, rows, v.d_reordered);
     count_launch();
-    v.kb16 = kb16;
-    if ((e = cudaMalloc(&v.d_reordered16, ix.rows_alloc * kb16 * sizeof(__nv_bfloat16))) != cudaSuccess ||
-        (e = cudaMalloc(&v.d_res16, rows * sizeof(float))) != cudaSuccess)
-        return e;
     cudaMemsetAsync(v.d_reordered16 + rows * kb16, 0, (ix.rows_alloc - rows) * kb16 * sizeof(__nv_bfloat16), s);
     bf16_rows_kernel<<<gb, 256, 0, s>>>(v.d_reordered, static_cast<uint32_t>(ds), rows, v.d_reordered16,
                                         static_cast<uint32_t>(kb16), v.d_res16);
     count_launch();
-    if ((e = launch_max_reduce(v.d_res16, rows, d_eps, s)) != cudaSuccess) return e;
+    if ((e = launch_max_reduce(v.d_res16, rows, v.d_eps, s)) != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
@@ -1327,51 +1342,79 @@ int ivf_build(CudaIndex& ix) {
     v.nlist = nlist;
     v.iters = iters;
     ix.ivf_scratch.nprobe = ix.opts.nprobe;
-    v.nlist_pad = (nlist + 255) / 256 * 256;
     const uint64_t kb = (ix.dims + 63) / 64 * 64;  // FP16 / BF16 row length (64-element K slabs)
-    BuildScratch tmp;
     cudaError_t e = cudaSuccess;
-    auto oom = [&](const char* what) { return cuda_error(e, what); };
-
-    // ---- persistent outputs ----
-    if ((e = cudaMalloc(&v.d_centroids, nlist * ds * sizeof(float))) != cudaSuccess) return oom("IVF centroids");
-    if ((e = cudaMalloc(&v.d_cent_t, ds * v.nlist_pad * sizeof(float))) != cudaSuccess) return oom("IVF centroids");
-    if ((e = cudaMalloc(&v.d_row_map, rows * sizeof(uint32_t))) != cudaSuccess) return oom("IVF row map");
-    if ((e = cudaMalloc(&v.d_offsets, (nlist + 1) * sizeof(uint32_t))) != cudaSuccess) return oom("IVF offsets");
+    BuildKeep keep;
+    if ((e = ivf_alloc(ix, v, &keep)) != cudaSuccess) return cuda_error(e, "IVF rows and centroids");
+    uint32_t* const chosen = keep.chosen;
+    KppState* const kst = keep.kst;
     cudaMemsetAsync(v.d_cent_t, 0, ds * v.nlist_pad * sizeof(float), s);
 
     // ---- scratch ----
-    // FP16 rows of the assignment GEMM; the seeding before it has its INT8 rows (ds ≤ kb bytes each) there.
-    __half* b16 = nullptr;
-    if ((e = tmp.alloc(b16, ix.rows_alloc * kb)) != cudaSuccess) return oom("IVF FP16 rows");
+    // The list-ordered rows are written last, so that until then their memory is the build's scratch: the
+    // BF16 rows' for the FP16 rows of the assignment GEMM (the seeding before it has its INT8 rows, ds ≤ kb
+    // bytes each, there), the FP32 rows' for the rest.
+    __half* b16 = reinterpret_cast<__half*>(v.d_reordered16);
     if (ix.rows_alloc > rows)
         cudaMemsetAsync(b16 + rows * kb, 0, (ix.rows_alloc - rows) * kb * sizeof(__half), s);
-    float *norm_up, *res_up, *min_d, *mean_f32;
-    float2* res_scale;
-    uint32_t *chosen, *assign, *amb, *amb_cnt, *hist, *list_size, *perm;
-    unsigned int* cmax;
-    unsigned long long* best;
-    double *partial, *sums;
-    KppState* kst;
-    __half* c16;
-    uint2* cand;
-    uint32_t *cand_cnt, *cand_list;
-    float* smax;
     // Rows of a sort block: a warp scatters them 32 at a time, one after another, so few, until the blocks'
     // histograms (nlist counts each) would outweigh the rows. 200,000 rows, 447 lists: 2,048 → 512 rows
     // took the scatter from 29 to 11 µs.
     const uint64_t sort_rows = nlist <= 1024 ? 512 : 2048;
     const uint32_t nblk_sort = static_cast<uint32_t>((rows + sort_rows - 1) / sort_rows);
-    if ((e = tmp.alloc(norm_up, rows)) || (e = tmp.alloc(res_up, rows)) || (e = tmp.alloc(min_d, rows)) ||
-        (e = tmp.alloc(res_scale, rows)) || (e = tmp.alloc(list_size, nlist)) ||
-        (e = tmp.alloc(mean_f32, ds)) || (e = tmp.alloc(chosen, nlist)) || (e = tmp.alloc(assign, rows)) ||
-        (e = tmp.alloc(amb, rows)) || (e = tmp.alloc(amb_cnt, 1)) ||
-        (e = tmp.alloc(hist, nlist * nblk_sort)) || (e = tmp.alloc(cmax, 2)) || (e = tmp.alloc(best, 1)) ||
-        (e = tmp.alloc(sums, nlist * ds)) || (e = tmp.alloc(kst, 1)) || (e = tmp.alloc(c16, v.nlist_pad * kb)) ||
-        (e = tmp.alloc(cand, rows)) || (e = tmp.alloc(cand_cnt, 1)) || (e = tmp.alloc(smax, rows)) ||
-        (e = tmp.alloc(cand_list, rows * kCandCap)))
-        return oom("IVF build scratch");
-    perm = v.d_row_map;
+    float *norm_up, *res_up, *min_d, *mean_f32, *smax;
+    float2* res_scale;
+    uint32_t *assign, *amb, *amb_cnt, *hist, *list_size, *cand_cnt, *cand_list;
+    unsigned int* cmax;
+    unsigned long long* best;
+    double *partial, *sums;
+    __half* c16;
+    uint2* cand;
+    // One resident wave of seeding blocks: every block streams its row range once, none waits for a second wave.
+    const size_t kpp_smem = ds * sizeof(float) + ds;
+    // Lanes a row that have all of it in flight with four chunks of 16 values each, from 513 values on eight
+    // with eight.
+    auto kpp = ds <= 256 ? kpp_step_kernel<4, 4> : ds <= 512 ? kpp_step_kernel<8, 4> : kpp_step_kernel<8, 8>;
+    cudaFuncSetAttribute(kpp, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kpp_smem));
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kpp, kKppThreads, kpp_smem);
+    const uint32_t kpp_target = static_cast<uint32_t>(ix.sm_count) * static_cast<uint32_t>(std::max(per_sm, 1));
+    const uint64_t rpb = ((rows + kpp_target - 1) / kpp_target + 31) / 32 * 32;
+    const uint32_t kpp_blocks = static_cast<uint32_t>((rows + rpb - 1) / rpb);
+    auto carve = [&](Carver c) {
+        c.take(norm_up, rows);
+        c.take(res_up, rows);
+        c.take(min_d, rows);
+        c.take(res_scale, rows);
+        c.take(smax, rows);
+        c.take(assign, rows);
+        c.take(amb, rows);
+        c.take(cand, rows);
+        c.take(cand_list, rows * kCandCap);
+        c.take(hist, nlist * nblk_sort);
+        c.take(list_size, nlist);
+        c.take(sums, nlist * ds);
+        c.take(c16, v.nlist_pad * kb);
+        c.take(mean_f32, ds);
+        c.take(partial, kpp_blocks);
+        c.take(best, 1);
+        c.take(cmax, 2);
+        c.take(amb_cnt, 1);
+        c.take(cand_cnt, 1);
+        return c.used;
+    };
+    BuildScratch tmp;
+    const size_t need = carve(Carver{});
+    uint8_t* scratch = reinterpret_cast<uint8_t*>(v.d_reordered);
+    if (need > ix.rows_alloc * ds * sizeof(float)) {
+        if ((e = cudaMalloc(&tmp.p, need)) != cudaSuccess) {
+            tmp.p = nullptr;
+            return cuda_error(e, "IVF build scratch");
+        }
+        scratch = static_cast<uint8_t*>(tmp.p);
+    }
+    carve(Carver{scratch});
+    uint32_t* const perm = v.d_row_map;
     cudaMemsetAsync(c16, 0, v.nlist_pad * kb * sizeof(__half), s);
 
     Timer t_all, t_seed, t_km, t_lay;
@@ -1400,18 +1443,6 @@ int ivf_build(CudaIndex& ix) {
     {
         kpp_init_kernel<<<1, 1, 0, s>>>(best, ix.opts.has_seed ? ix.opts.seed : rows * 2654435761ull + dp, kst, chosen);
         count_launch();
-        const size_t smem = ds * sizeof(float) + ds;
-        // Four lanes a row while they have all of it in flight (8 chunks of 16 values each), else eight.
-        auto kern = ds <= 256 ? kpp_step_kernel<4, 4> : ds <= 512 ? kpp_step_kernel<8, 4> : kpp_step_kernel<8, 8>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        // One resident wave: every block streams its row range once, none waits for a second wave.
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kKppThreads, smem);
-        const uint32_t blocks_target = static_cast<uint32_t>(ix.sm_count) * static_cast<uint32_t>(std::max(per_sm, 1));
-        uint64_t rpb = (rows + blocks_target - 1) / blocks_target;
-        rpb = (rpb + 31) / 32 * 32;
-        const uint32_t nb = static_cast<uint32_t>((rows + rpb - 1) / rpb);
-        if ((e = tmp.alloc(partial, nb)) != cudaSuccess) return oom("IVF seeding scratch");
         // FLT_MAX everywhere: the first step scores every row exactly.
         fill_f32_kernel<<<static_cast<unsigned>(std::min<uint64_t>((rows + 255) / 256, 65535)), 256, 0, s>>>(
             min_d, rows, FLT_MAX);
@@ -1420,14 +1451,14 @@ int ivf_build(CudaIndex& ix) {
         overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         overlap.val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(nb);
+        cfg.gridDim = dim3(kpp_blocks);
         cfg.blockDim = dim3(kKppThreads);
-        cfg.dynamicSmemBytes = smem;
+        cfg.dynamicSmemBytes = kpp_smem;
         cfg.stream = s;
         cfg.attrs = &overlap;
         cfg.numAttrs = 1;
         for (uint64_t c = 1; c < nlist; ++c) {
-            if ((e = cudaLaunchKernelEx(&cfg, kern, static_cast<const float*>(ix.d_base), static_cast<const signed char*>(b8),
+            if ((e = cudaLaunchKernelEx(&cfg, kpp, static_cast<const float*>(ix.d_base), static_cast<const signed char*>(b8),
                                         static_cast<uint32_t>(ds), static_cast<uint32_t>(dp), rows, rpb,
                                         static_cast<const float*>(norm_up), static_cast<const float2*>(res_scale), min_d,
                                         partial, kst, chosen, static_cast<uint32_t>(c))) != cudaSuccess)
@@ -1484,8 +1515,6 @@ int ivf_build(CudaIndex& ix) {
     cudaFuncSetAttribute(centroid_normalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(ds * sizeof(double)));
     std::vector<uint32_t> h_amb(2 * iters, 0);
-    uint32_t* d_amb_hist = nullptr;  // per iteration: rows of the full exact pass, rows decided among candidates
-    if ((e = tmp.alloc(d_amb_hist, 2 * iters)) != cudaSuccess) return oom("IVF build scratch");
     for (uint64_t it = 0; it < iters; ++it) {
         cudaMemsetAsync(cmax, 0, 2 * sizeof(unsigned int), s);
         cudaMemsetAsync(amb_cnt, 0, sizeof(uint32_t), s);
@@ -1501,8 +1530,8 @@ int ivf_build(CudaIndex& ix) {
         kmeans_assign_cand_kernel<<<ix.sm_count * 8, 256, 0, s>>>(ix.d_base, static_cast<uint32_t>(ds),
                                                                   static_cast<uint32_t>(dp), v.d_centroids, cand_list,
                                                                   cand, cand_cnt, assign);
-        cudaMemcpyAsync(d_amb_hist + 2 * it, amb_cnt, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
-        cudaMemcpyAsync(d_amb_hist + 2 * it + 1, cand_cnt, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+        cudaMemcpyAsync(keep.amb_hist + 2 * it, amb_cnt, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+        cudaMemcpyAsync(keep.amb_hist + 2 * it + 1, cand_cnt, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
         // Lists of this assignment (stable by row).
         cluster_hist_kernel<<<nblk_sort, 256, nlist * sizeof(uint32_t), s>>>(assign, rows, static_cast<uint32_t>(nlist),
                                                                              nblk_sort, static_cast<uint32_t>(sort_rows),
@@ -1527,8 +1556,7 @@ int ivf_build(CudaIndex& ix) {
 
     // List layout: the reordered FP32 rows and their BF16 copy.
     cudaEventRecord(t_lay.a, s);
-    cudaMemsetAsync(cmax, 0, sizeof(unsigned int), s);
-    if ((e = ivf_enqueue_layout(ix, v, cmax)) != cudaSuccess) return oom("IVF reordered rows");
+    if ((e = ivf_enqueue_layout(ix, v)) != cudaSuccess) return cuda_error(e, "IVF reordered rows");
     cudaEventRecord(t_lay.b, s);
     cudaEventRecord(t_all.b, s);
 
@@ -1536,12 +1564,12 @@ int ivf_build(CudaIndex& ix) {
     KppState h_st{};
     cudaMemcpyAsync(h_off.data(), v.d_offsets, (nlist + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(h_chosen.data(), chosen, nlist * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(h_amb.data(), d_amb_hist, 2 * iters * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(h_amb.data(), keep.amb_hist, 2 * iters * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(&h_st, kst, sizeof(h_st), cudaMemcpyDeviceToHost, s);
     uint32_t h_status = 0;
     unsigned int h_eps = 0;
     cudaMemcpyAsync(&h_status, ix.d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&h_eps, cmax, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&h_eps, v.d_eps, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(e, "IVF build");
     if (h_status == kStatusTimeout)
         return set_error(NNDEX_ERR_TIMEOUT, "cuda execution error: a bounded device wait timed out (IVF build)");
@@ -1611,21 +1639,11 @@ int ivf_restore(CudaIndex& ix, uint64_t nlist, const float* centroids, const uin
     auto ivf = std::make_shared<IvfIndex>();
     IvfIndex& v = *ivf;
     v.nlist = nlist;
-    v.nlist_pad = (nlist + 255) / 256 * 256;
     cudaError_t e;
     Timer t_all;
     cudaEventRecord(t_all.a, s);
-    if ((e = cudaMalloc(&v.d_centroids, nlist * ds * sizeof(float))) != cudaSuccess ||
-        (e = cudaMalloc(&v.d_cent_t, ds * v.nlist_pad * sizeof(float))) != cudaSuccess ||
-        (e = cudaMalloc(&v.d_row_map, rows * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMalloc(&v.d_offsets, (nlist + 1) * sizeof(uint32_t))) != cudaSuccess)
-        return cuda_error(e, "IVF layout");
+    if ((e = ivf_alloc(ix, v, nullptr)) != cudaSuccess) return cuda_error(e, "IVF layout");
     std::vector<uint32_t> off32(offsets, offsets + nlist + 1);
-    unsigned int* d_eps = nullptr;
-    if ((e = cudaMalloc(&d_eps, sizeof(unsigned int))) != cudaSuccess) return cuda_error(e, "IVF layout");
-    BuildScratch tmp;
-    tmp.ptrs.push_back(d_eps);
-    cudaMemsetAsync(d_eps, 0, sizeof(unsigned int), s);
     cudaMemsetAsync(v.d_centroids, 0, nlist * ds * sizeof(float), s);
     cudaMemsetAsync(v.d_cent_t, 0, ds * v.nlist_pad * sizeof(float), s);
     if ((e = cudaMemcpy2DAsync(v.d_centroids, ds * sizeof(float), centroids, dp * sizeof(float), dp * sizeof(float),
@@ -1640,10 +1658,10 @@ int ivf_restore(CudaIndex& ix, uint64_t nlist, const float* centroids, const uin
         v.d_centroids, static_cast<uint32_t>(ds), static_cast<uint32_t>(nlist), nullptr, static_cast<uint32_t>(kb),
         v.d_cent_t, v.nlist_pad, nullptr);
     count_launch();
-    if ((e = ivf_enqueue_layout(ix, v, d_eps)) != cudaSuccess) return cuda_error(e, "IVF reordered rows");
+    if ((e = ivf_enqueue_layout(ix, v)) != cudaSuccess) return cuda_error(e, "IVF reordered rows");
     cudaEventRecord(t_all.b, s);
     unsigned int h_eps = 0;
-    cudaMemcpyAsync(&h_eps, d_eps, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&h_eps, v.d_eps, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
     // the host arrays above are read by the copies until the stream drains
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(e, "IVF layout");
     v.h_offsets.assign(offsets, offsets + nlist + 1);

@@ -1195,9 +1195,6 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
             if ((st = plan_buffer(w, nlist))) return st;
             if ((st = grow(w.d_q_slot_off, w.cap_q_slot_off, nq + 1, "IVF plan buffer"))) return st;
             if ((st = grow(w.d_ws, w.cap_ws, pairs * chunks * k, "IVF slot workspace"))) return st;
-            if (!w.h_probed) bump_alloc_epoch();
-            if (!w.h_probed && cudaMallocHost(&w.h_probed, 8 * sizeof(unsigned long long)) != cudaSuccess)
-                return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
             zero_plan(w, nlist, s);
             const ProbeLaunch pl{&ix, queries, nq, dq, static_cast<uint32_t>(ix.dp), nlist, np, v.d_cent_t, v.nlist_pad,
                                  v.d_offsets, w.d_pscore, w.d_probes, w.d_list_cnt, w.d_q_slot_off, w.d_counters};
@@ -1259,9 +1256,6 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
     a.counters = w.d_counters;
     a.ws = w.d_ws;
     a.status = ix.w_status;
-    if (!w.h_probed) bump_alloc_epoch();
-    if (!w.h_probed && cudaMallocHost(&w.h_probed, 8 * sizeof(unsigned long long)) != cudaSuccess)
-        return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
     zero_plan(w, nlist, s);
     for (uint32_t q0 = 0; q0 < nq; q0 += sub) {
         const uint32_t n = std::min(sub, nq - q0);
@@ -1376,10 +1370,6 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     if ((st = grow(ix.d_tcfail, ix.cap_tcfail, nq, "pass-2 buffer"))) return st;
     if ((st = grow(ix.d_rslots, ix.cap_rslots, static_cast<size_t>(nq) * rerank_chunks(cap2) * k, "pass-2 buffer")))
         return st;
-    if ((st = ix.ensure_fbn())) return st;
-    if (!w.h_probed) bump_alloc_epoch();
-    if (!w.h_probed && cudaMallocHost(&w.h_probed, 8 * sizeof(unsigned long long)) != cudaSuccess)
-        return set_error(NNDEX_ERR_OUT_OF_MEMORY, "cuda execution error: pinned allocation failed");
 
     // ---- probe + plan (groups of 128 queries) + gathered query blocks ----
     // counters [8] and [9]: the work-item counters of the two tensor-core passes
