@@ -580,7 +580,12 @@ CudaIndex::TcPlan CudaIndex::plan_tc(uint64_t kcap, bool fp8) const {
     TcPlan out;
     if (kcap == 0) {
         out.stages = tc_stages_for(nchunks, 0, fp8, false, smem_optin);
-        if (!out.stages) {
+        // The query slabs stay in shared memory only beside a ring that is deep enough: a base slab a
+        // stage comes from L2 at best, and with two stages its latency shows on every slab. 1M × 512 in
+        // BF16, 512 queries: 829 us with two 32 KB stages beside the queries, 605 with four 48 KB stages
+        // that carry the query slabs too; × 448 (three stages) 586 -> 555. FP8 slabs pass through twice
+        // as fast, so the extra bytes weigh more: × 1,024 1,022 -> 876, × 768 (three stages) 696 -> 704.
+        if (out.stages < (fp8 ? 3u : 4u)) {
             out.stream_a = true;
             out.stages = tc_stages_for(nchunks, 0, fp8, true, smem_optin);
         }
