@@ -943,15 +943,18 @@ __global__ void __launch_bounds__(1024, 1)
 //   * each thread keeps the largest of its words, or of each of four shares of them (kR, k′ > 128); the
 //     k′-th largest of these maxima is a cut that at least k′ words reach, and hardly more do (the
 //     words are dealt round-robin);
-//   * the words that reach the cut are listed and sorted, and the first k′ re-scored. A list that
+//   * the words that reach the cut are listed and put in order, and the first k′ re-scored. A list that
 //     would not fit (mass ties) is truncated: any k rows give a valid T.
-// Bound by its sorts and the gather of the k′ rows. On 10M × 256 with 4,096 queries at k = 10: 107 us,
-// where the merge and rerank of the heaps took 217; 2M × 512 in FP8, 1,000 queries, k = 100: 191 us
-// (four shares; one maximum per thread of 1,024-thread blocks took 284), before 165.
+// Bound by the gather of the k′ rows and, for a batch that leaves SMs idle, by the chain of its steps. The
+// cut is found bit by bit with a block-wide count, the places by ranks: 64 queries at k′ = 32 took 12.3 us
+// with three bitonic sorts and take 6.7; 10M × 256 with 4,096 queries at k = 10 133 -> 94 (the merge and
+// rerank of the heaps before took 217); 2M × 512 in FP8, 1,000 queries, k = 100: 190 -> 173 (four shares;
+// one maximum per thread of 1,024-thread blocks was slower); 1,024 queries over 32 lists 41 -> 30.
 // ------------------------------------------------------------------------------------------
 namespace {
 constexpr int kThrThreads = 256;
 constexpr uint32_t kThrList = 2048;  // words listed per query
+constexpr uint32_t kThrRanked = 512;  // up to so many are put in order by their ranks
 constexpr uint32_t kThrExact = 1024;  // where the exact keys (≤ 512) start, past the k′ ≤ 512 groups
 
 // Order of a group's word: 0 for a group without rows (or with NaN scores only).
@@ -960,11 +963,36 @@ NNDEX_DEVICE_INLINE uint32_t group_order(uint32_t w) {
 }
 }  // namespace
 
+// The nth-largest of a block's kR values a thread (0 if the nth is 0): its bits from the highest, each by
+// one count over the block. counts: 32 words of shared memory, zeroed. 1 ≤ nth ≤ threads · kR.
+template <int kR>
+NNDEX_DEVICE_INLINE uint32_t block_nth_largest(const uint32_t (&v)[kR], uint32_t nth, uint32_t* counts) {
+    uint32_t p = 0;
+#pragma unroll 1
+    for (int bit = 31; bit >= 0; --bit) {
+        const uint32_t t = p | (1u << bit);
+        uint32_t c = 0;
+#pragma unroll
+        for (int r = 0; r < kR; ++r) c += v[r] >= t ? 1u : 0u;
+        if constexpr (kR == 1) {
+            c = static_cast<uint32_t>(__syncthreads_count(static_cast<int>(c)));
+        } else {
+            c = __reduce_add_sync(0xFFFFFFFFu, c);
+            if ((threadIdx.x & 31u) == 0) atomicAdd(&counts[bit], c);
+            __syncthreads();
+            c = counts[bit];
+        }
+        if (c >= nth) p = t;
+    }
+    return p;
+}
+
 template <int kR, bool kItems>
 __global__ void __launch_bounds__(kThrThreads) threshold_kernel(const TcThresholdArgs a) {
     constexpr int NT = kThrThreads;
     __shared__ uint64_t keys[kThrList];
-    __shared__ uint32_t count;
+    __shared__ uint32_t count, counts[32];
+    __shared__ uint64_t kth_s;
     extern __shared__ __align__(16) float q_s[];  // the query
     const uint32_t q = blockIdx.x, tid = threadIdx.x;
     const uint32_t wpt = kN / a.group;            // words per span of tiles
@@ -987,15 +1015,15 @@ __global__ void __launch_bounds__(kThrThreads) threshold_kernel(const TcThreshol
             best[r] = max(max(best[r], max(group_order(w[r].x), group_order(w[r].y))),
                           max(group_order(w[r].z), group_order(w[r].w)));
     }
-#pragma unroll
-    for (int r = 0; r < kR; ++r) keys[tid + r * NT] = best[r];
-    if (tid == 0) count = 0;
+    if (tid < 32) counts[tid] = 0;
+    if (tid == 0) {
+        count = 0;
+        kth_s = 0;
+    }
     __syncthreads();
-    block_bitonic_sort_desc(keys, NT * kR);
     const uint32_t nth = a.kp < static_cast<uint32_t>(NT * kR) ? a.kp : static_cast<uint32_t>(NT * kR);
-    uint32_t cut = static_cast<uint32_t>(keys[nth - 1]);
+    uint32_t cut = block_nth_largest<kR>(best, nth, counts);
     if (cut == 0) cut = 1;  // fewer groups than that: all of them
-    __syncthreads();
     for (uint32_t i0 = 0; i0 < n4; i0 += NT) {
         const uint32_t i = i0 + tid;
         uint4 w = make_uint4(kNoGroup, kNoGroup, kNoGroup, kNoGroup);
@@ -1012,21 +1040,39 @@ __global__ void __launch_bounds__(kThrThreads) threshold_kernel(const TcThreshol
     }
     __syncthreads();
     uint32_t m = count < kThrList ? count : kThrList;
-    uint32_t p2 = 1;
-    while (p2 < m) p2 <<= 1;
-    for (uint32_t i = m + tid; i < p2; i += NT) keys[i] = 0ull;
-    __syncthreads();
-    block_bitonic_sort_desc(keys, p2);
+    if (m <= kThrRanked) {  // few: each key's rank is its place
+        uint64_t mine[kThrRanked / NT];
+        uint32_t rank[kThrRanked / NT];
+#pragma unroll
+        for (uint32_t u = 0; u < kThrRanked / NT; ++u) {
+            mine[u] = tid + u * NT < m ? keys[tid + u * NT] : 0ull;
+            rank[u] = 0;
+        }
+        for (uint32_t j = 0; j < m; ++j) {
+            const uint64_t other = keys[j];
+#pragma unroll
+            for (uint32_t u = 0; u < kThrRanked / NT; ++u) rank[u] += other > mine[u] ? 1u : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t u = 0; u < kThrRanked / NT; ++u)
+            if (tid + u * NT < m) keys[rank[u]] = mine[u];
+        __syncthreads();
+    } else {
+        uint32_t p2 = 1;
+        while (p2 < m) p2 <<= 1;
+        for (uint32_t i = m + tid; i < p2; i += NT) keys[i] = 0ull;
+        __syncthreads();
+        block_bitonic_sort_desc(keys, p2);
+    }
     if (m > a.kp) m = a.kp;
-    uint32_t p2k = 1;
-    while (p2k < a.kp) p2k <<= 1;
     // the bound of a listed row's exact score: its approximate score (up to 32·span − 1 units of the
     // last place low, under span·2⁻¹⁸ of its magnitude) plus the largest slack
     const float low = static_cast<float>(a.span) * 7.62939453125e-06f;
     const float rq = a.q_resid[q], qs = a.q_scale ? a.q_scale[q] : 1.0f;
     const float slack = a.whole_slack ? rq : fmaf(a.eps_rows, 1.0f + rq, rq + a.eps_acc);
     const uint32_t ch = tid & 7u, nbox = a.ds / 32;
-    for (uint32_t j0 = 0; j0 < p2k; j0 += NT / 8) {
+    for (uint32_t j0 = 0; j0 < a.kp; j0 += NT / 8) {
         const uint32_t j = j0 + (tid >> 3);
         bool live = j < m;
         uint64_t row = 0;
@@ -1044,18 +1090,22 @@ __global__ void __launch_bounds__(kThrThreads) threshold_kernel(const TcThreshol
             bound = s + fabsf(s) * low + slack;
         }
         const float acc = dot_scan_order<8>(a.base + (live ? row : 0) * a.ds, q_s, nbox, ch, live);
-        if (ch == 0 && j < p2k) {
+        if (ch == 0 && j < a.kp) {
             keys[kThrExact + j] = live ? make_key(acc, static_cast<uint32_t>(row)) : 0ull;
-            if (j < a.kp) {
-                a.cand_idx[static_cast<size_t>(q) * a.kp + j] = live ? row : 0;
-                a.cand_sim[static_cast<size_t>(q) * a.kp + j] = live ? bound : 0.0f;
-            }
+            a.cand_idx[static_cast<size_t>(q) * a.kp + j] = live ? row : 0;
+            a.cand_sim[static_cast<size_t>(q) * a.kp + j] = live ? bound : 0.0f;
         }
     }
     __syncthreads();
-    block_bitonic_sort_desc(keys + kThrExact, p2k);
+    for (uint32_t i = tid; i < m; i += NT) {  // the k-th: k − 1 are larger (their rows differ, so no two are equal)
+        const uint64_t mine = keys[kThrExact + i];
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < m; ++j) rank += keys[kThrExact + j] > mine ? 1u : 0u;
+        if (mine && rank == a.k - 1) kth_s = mine;
+    }
+    __syncthreads();
     if (tid == 0) {
-        const uint64_t kth = keys[kThrExact + a.k - 1];
+        const uint64_t kth = kth_s;
         a.kth[q] = kth ? key_score(kth) : -INFINITY;
         a.cand_cnt[q] = m;
         a.cert[q] = 0;
