@@ -1113,7 +1113,7 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     const uint64_t per_query = static_cast<uint64_t>(ctas) * plan.kp_cta;
     // the FP32 scan that re-runs uncertified queries shares the candidate workspace
     ScanPlan fb_plan;
-    if (!plan_scan_fp32(n, static_cast<uint32_t>(ds), kcap, rows, sm_count, smem_optin, fb_plan))
+    if (!plan_fallback(6, n, kcap, fb_plan))
         return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: no FP32 scan plan for k=%u", kcap);
     const uint64_t fb_per_query = static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap;
     if ((st = grow_device(d_ws, cap_ws, std::max(per_query, fb_per_query) * n, "scan workspace"))) return st;
@@ -1177,18 +1177,51 @@ int CudaIndex::enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o
     r.certify = true;
     r.floor_keys = d_floor;  // rows the CTAs' lists left out score below it
     r.fb_ids = d_fbq;
-    r.fb_count = d_fbn;
+    r.fb_count = host_fallback ? h_fbn : d_fbn;
     if ((e = launch_rerank(r, s)) != cudaSuccess) return cuda_error(e, "rerank launch");
     // Uncertified queries re-run on the FP32 scan, on the device: the rerank listed them.
-    if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
+    if (!host_fallback) {
+        if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
+        fbn_stream = s;
+        fbn_pending = true;
+        stats.kernel_launches += 2;
+    }
     last_tc_n = n;
-    fbn_stream = s;
-    fbn_pending = true;
-    stats.kernel_launches += 5;
+    stats.kernel_launches += 3;
     stats.path = 6;
     stats.rerank_width = kp;
     stats.rows_scanned += rows * n;
     return NNDEX_OK;
+}
+
+// The FP32 scan that re-runs a TF32 batch's listed queries (path 6 or 7).
+bool CudaIndex::plan_fallback(int path, uint32_t n, uint32_t kcap, ScanPlan& plan) const {
+    if (!plan_scan_fp32(n, static_cast<uint32_t>(ds), kcap, rows, sm_count, smem_optin, plan)) return false;
+    if (path == 7) {  // usually few queries: up to a CTA per SM for each group of 16, within 256 MB of keys
+        const uint64_t per = std::min<uint64_t>(static_cast<uint64_t>(sm_count), (32ull << 20) / (static_cast<uint64_t>(n) * kcap));
+        plan.ctas_per_group = static_cast<uint32_t>(std::max<uint64_t>(plan.ctas_per_group, per));
+    }
+    return true;
+}
+
+// A host-buffer batch's listed queries, their number read where the batch was waited for: the two
+// launches, 8 us of a batch of 64 queries over 50k rows when none is listed, wait for one that is.
+int CudaIndex::finish_tf32(int path, uint32_t n, uint32_t kcap) {
+    stats.fp32_fallback_queries += h_fbn[0];
+    stats.certified = h_fbn[0] == 0 ? 1u : 0u;
+    if (h_fbn[0] == 0) return NNDEX_OK;
+    ScanPlan plan;
+    if (!plan_fallback(path, n, kcap, plan))
+        return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: no FP32 scan plan for k=%u", kcap);
+    cudaError_t e = cudaMemcpyAsync(d_fbn, h_fbn, sizeof(uint32_t), cudaMemcpyHostToDevice, stream);
+    if (e != cudaSuccess) return cuda_error(e, "fallback count");
+    int st;
+    if ((st = enqueue_fp32_fallback(plan, n, kcap, d_idx, d_sim, d_cnt, stream))) return st;
+    stats.kernel_launches += 2;
+    if (!mapped_io) cudaMemcpyAsync(h_res, d_res, res_bytes, cudaMemcpyDeviceToHost, stream);
+    cudaEventRecord(ev1, stream);
+    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_error(e, "search");
+    return check_device_words();
 }
 
 // The scan reads the listed queries' rows, the merge writes each result into the query's own output
@@ -1256,11 +1289,8 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
     const Tf32BatchPlan plan = plan_tf32_batch(n, kcap);
     ScanPlan fb_plan;
     // (a tuned plan is shared by the shapes of a power of two, some of which the rule may not take)
-    if (!plan.kp || !plan_scan_fp32(n, static_cast<uint32_t>(ds), kcap, rows, sm_count, smem_optin, fb_plan))
+    if (!plan.kp || !plan_fallback(7, n, kcap, fb_plan))
         return enqueue_exact_fp32(d_qn, n, kcap, kcap, o_idx, o_sim, o_cnt, s);
-    // The fallback usually has few queries: up to a CTA per SM for each group of 16, within 256 MB of keys.
-    const uint64_t fb_per = std::min<uint64_t>(static_cast<uint64_t>(sm_count), (32ull << 20) / (static_cast<uint64_t>(n) * kcap));
-    fb_plan.ctas_per_group = static_cast<uint32_t>(std::max<uint64_t>(fb_plan.ctas_per_group, fb_per));
     if ((st = grow_tf32_batch(plan, n, kcap, static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap))) {
         // without memory for the collections: the FP32 scan, whose workspace is far smaller
         if (st != NNDEX_ERR_OUT_OF_MEMORY) return st;
@@ -1337,13 +1367,16 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
     if (e != cudaSuccess) return cuda_error(e, "TF32 scan launch (pass 2)");
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, kSecondPassCap, kcap,
                                 d_kth, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, nullptr, nullptr, nullptr, nullptr,
-                                nullptr, d_fbq, d_fbn);
+                                nullptr, d_fbq, host_fallback ? h_fbn : d_fbn);
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
-    if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
+    if (!host_fallback) {
+        if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
+        fbn_stream = s;
+        fbn_pending = true;
+        stats.kernel_launches += 2;
+    }
     last_tc_n = n;
-    fbn_stream = s;
-    fbn_pending = true;
-    stats.kernel_launches += 7;
+    stats.kernel_launches += 5;
     stats.path = 7;
     stats.rerank_width = plan.kp;
     stats.pass1_tile_stride = plan.stride;
@@ -1421,6 +1454,7 @@ int CudaIndex::tune_host(uint64_t n, uint64_t kcap, int mode, TunePlan* plan) {
 int CudaIndex::enqueue_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
     int st;
     h_flags[0] = h_flags[1] = 0;  // (a replay's are reset by run_host_batch)
+    h_fbn[0] = 0;
     if (!mapped_io) cudaMemcpyAsync(d_qraw, h_q, n * dims * sizeof(float), cudaMemcpyHostToDevice, stream);
     if ((st = enqueue_prep_queries(mapped_io ? h_q : d_qraw, n, mode, path, stream))) return st;
     if (path == 4) {
@@ -1460,7 +1494,7 @@ int CudaIndex::enqueue_host_batch(uint64_t n, uint64_t kcap, int mode, int path)
 // the capture); otherwise directly. No path needs a host decision in the middle of its batch: the
 // FP32 scan (1), the tensor-core scans (2, 3, 5: pass 2 and its compaction run on the device; the
 // rare FP32 re-run of an overflowed collection follows the batch), the IVF list scan (4) and the
-// TF32 scans (6 and 7, their fallback on the device).
+// TF32 scans (6 and 7, the re-run of their listed queries likewise).
 int CudaIndex::run_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
     const bool graphable = use_graphs && !scan_timing && !error_report && !sync_check_enabled() &&
                            path >= 1 && path <= 7 &&
@@ -1479,6 +1513,7 @@ int CudaIndex::run_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
             break;
         }
         h_flags[0] = h_flags[1] = 0;
+        h_fbn[0] = 0;
         const cudaError_t e = cudaGraphLaunch(graphs[i].exec, stream);
         if (e != cudaSuccess) return cuda_error(e, "graph launch");
         // the capture's statistics: counters added to this call's, the rest as captured
@@ -1492,10 +1527,6 @@ int CudaIndex::run_host_batch(uint64_t n, uint64_t kcap, int mode, int path) {
         stats.ivf_rows_union = acc.ivf_rows_union;
         count_launch(static_cast<uint32_t>(graphs[i].launches));
         stats.graph = 2;
-        if (path == 6 || path == 7) {  // the replayed fallback's count is read back with the statistics
-            fbn_stream = stream;
-            fbn_pending = true;
-        }
         return NNDEX_OK;
     }
     if (!(same(graph_seen) && graph_seen.epoch == epoch)) {
@@ -1549,6 +1580,7 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
     stats = nndex_cuda_search_stats{};
     order_after_previous(stream);
     use_host_words();
+    host_fallback = !error_report;  // a report records what the device-side re-run has written
     const uint64_t kcap = std::min<uint64_t>(k, rows);
     if (kcap > kMaxFusedK)
         return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: k=%llu above the fused top-k limit %u",
@@ -1607,6 +1639,9 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
                 if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_error(e, "search");
             }
         }
+        if (host_fallback && (stats.path == 6 || stats.path == 7) &&
+            (st = finish_tf32(path, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap))))
+            return st;
         if (path == 4) {
             stats.rows_scanned += ivf_scratch.h_probed[0];
             stats.ivf_rows_streamed += ivf_scratch.h_probed[1];
@@ -1663,6 +1698,7 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
     if ((st = ensure_query_capacity(std::min<uint64_t>(nq, kMaxBatchChunk)))) return st;
     if (error_report && (st = serr_begin(nq, kcap, s))) return st;
     use_device_words();
+    host_fallback = false;
     cudaMemsetAsync(d_err, 0, 2 * sizeof(unsigned long long), s);
     bool synced = false, done = false;  // done: the last piece waited and its status words were clean
     for (uint64_t q0 = 0; q0 < nq; q0 += kMaxBatchChunk) {

@@ -282,6 +282,11 @@ struct CudaIndex {
     uint64_t h_fbn_rows() const { return *reinterpret_cast<const unsigned long long*>(h_fbn + 4); }
     cudaStream_t fbn_stream = nullptr;
     bool fbn_pending = false;
+    // A TF32 batch of a host-buffer search: its listed queries are counted in h_fbn, and re-run after the
+    // batch where there are any (finish_tf32).
+    bool host_fallback = false;
+    bool plan_fallback(int path, uint32_t n, uint32_t kcap, ScanPlan& plan) const;
+    int finish_tf32(int path, uint32_t n, uint32_t kcap);
     int fetch_fallback_stats();
 
     // scan-kernel timing (roofline reports)
