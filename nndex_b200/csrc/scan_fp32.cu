@@ -357,10 +357,11 @@ NNDEX_DEVICE_INLINE void merge_final(const uint64_t* keys, uint64_t n, uint32_t 
 
 }  // namespace
 
-// k ≤ kMergeBestK: one block per query (block_merge_best). Bound by latency: two rounds of loads, one
-// warp's selection, the ranks. One query's 148 lists of 10: 6.5 us, where the split kernel below spent
-// 12.5; 148 lists of 100: 13.6 (20); 16 queries with 148 lists of 64, 256 kept: 19 (29). Blocks of
-// 1,024 threads were no faster on the long lists.
+// k ≤ kMergeBestK: one block per query (block_merge_best). Bound by latency: two rounds of loads, the
+// counts that find the cut, the ranks. One query's 148 lists of 10: 5.7 us (7.3 with one warp's radix
+// selection of the cut), where the split kernel below spent 12.5; 148 lists of 100: 10.6 (13.7; 20); 16
+// queries with 148 lists of 64, 256 kept: 12.8 (20; 29). Blocks of 1,024 threads were no faster on the
+// long lists.
 template <int NT>
 __global__ void __launch_bounds__(NT) merge_best_kernel(const uint64_t* __restrict__ ws_keys, uint64_t per_query,
                                                         uint32_t k, uint32_t out_stride, uint64_t* __restrict__ idx_out,

@@ -219,16 +219,15 @@ NNDEX_DEVICE_INLINE void block_bitonic_sort_desc(uint64_t* a, uint32_t n) {
 
 // ---- the k best of a query's candidate keys, by one block ------------------------------------
 //
-// Each thread keeps the largest of the keys it reads (dealt round-robin); the k-th largest of these
-// maxima (one warp's radix select) is a cut that at least k keys reach and hardly more do, so one
-// more read lists about k keys, and their ranks among themselves place them. Exact whatever the
-// keys: only a list that does not hold every key above the cut sends the block to `overflow`.
+// Each thread keeps the largest of the keys it reads (dealt round-robin); the k-th largest score of these
+// maxima, found bit by bit with a block-wide count, is a cut that at least k keys reach and hardly more
+// do, so one more read lists about k keys, and their ranks among themselves place them. Exact whatever
+// the keys: only a list that does not hold every key that reaches the cut (mass ties) sends the block to
+// `overflow`.
 template <int NT>
 struct MergeScratch {
     static constexpr uint32_t kList = 1024;
     uint64_t list[kList];
-    uint32_t hist[256];
-    unsigned long long cut;
     uint32_t count;
 };
 
@@ -238,7 +237,6 @@ struct MergeScratch {
 template <int NT, class Get, class Put, class Overflow>
 NNDEX_DEVICE_INLINE uint32_t block_merge_best(Get&& get, uint32_t n, uint32_t k, MergeScratch<NT>& s, Put&& put,
                                               Overflow&& overflow) {
-    static_assert(NT <= static_cast<int>(MergeScratch<NT>::kList), "the maxima share the list");
     constexpr int U = 8;  // loads in flight; the keys stay in registers where one round reads them all
     const uint32_t tid = threadIdx.x;
     uint64_t best = 0, x[U];
@@ -248,21 +246,15 @@ NNDEX_DEVICE_INLINE uint32_t block_merge_best(Get&& get, uint32_t n, uint32_t k,
 #pragma unroll
         for (int u = 0; u < U; ++u) best = x[u] > best ? x[u] : best;
     }
-    // small k: the maxima of 2, 4, … threads together, still four times as many as k
-    uint32_t o = 1;
-    for (; o < 32 && NT / (2 * o) >= 4 * k && NT / (2 * o) >= 32; o <<= 1) {
-        const uint64_t other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other > best ? other : best;
-    }
-    if ((tid & (o - 1)) == 0) s.list[tid / o] = best;
     if (tid == 0) s.count = 0;
-    __syncthreads();
-    if (tid < 32) {
-        const uint64_t kth = warp_radix_kth(s.list, NT / o, k, s.hist);
-        if (tid == 0) s.cut = kth ? kth : 1ull;  // fewer keys than that: all of them
+    const uint32_t top = static_cast<uint32_t>(best >> 32);  // the score, in order
+    uint32_t score = 0;
+#pragma unroll 1
+    for (int bit = 31; bit >= 0; --bit) {
+        const uint32_t t = score | (1u << bit);
+        if (static_cast<uint32_t>(__syncthreads_count(top >= t)) >= k) score = t;
     }
-    __syncthreads();
-    const uint64_t cut = s.cut;
+    const uint64_t cut = score ? static_cast<uint64_t>(score) << 32 : 1ull;  // fewer keys than that: all of them
     for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
         if (n > U * NT) {
 #pragma unroll
@@ -282,7 +274,7 @@ NNDEX_DEVICE_INLINE uint32_t block_merge_best(Get&& get, uint32_t n, uint32_t k,
         return overflow();
     }
     const uint32_t kk = c < k ? c : k;
-    if (c <= 192) {
+    if (c <= 512) {
         for (uint32_t t = tid; t < c; t += NT) {
             const uint64_t mine = s.list[t];
             uint32_t rank = 0;
@@ -291,7 +283,7 @@ NNDEX_DEVICE_INLINE uint32_t block_merge_best(Get&& get, uint32_t n, uint32_t k,
         }
         return kk;
     }
-    uint32_t p2 = 256;
+    uint32_t p2 = 1024;
     while (p2 < c) p2 <<= 1;
     for (uint32_t t = c + tid; t < p2; t += NT) s.list[t] = 0ull;
     block_bitonic_sort_desc(s.list, p2);
