@@ -1,7 +1,8 @@
 // ivf_search.cu — K8/K9: IVF probe and the ragged list scan with exact FP32 rerank.
 //
 // Replaces candidate_clusters(_batch) (src/approx.rs:159-300) and search_approx /
-// search_batch_approx (src/cpu.rs:425-502). A batch runs as six launches and no host round trip:
+// search_batch_approx (src/cpu.rs:425-502). A batch runs without a host round trip (a small one, whose
+// (query, list, chunk) pairs are few, scans them pair by pair right after the probe, then merges):
 //   1. probe (two launches): per query, the nprobe best clusters by dot_small (FP64 in index order, f32
 //      result — the reference's value; score desc, lower index on ties): TF32 scores of every centroid
 //      from the tensor cores with a rigorous bound, and exact scores only of the clusters it leaves open.

@@ -16,10 +16,11 @@
 //   32 sampled rows, and threshold_kernel re-scores the rows of each query's k′ largest groups.
 //   Pass 2 (kMode 1), for the other queries only: collect every row with u_r ≥ T (no row with
 //   u_r < T can reach the top-k, since k rows already score ≥ T), and re-score them exactly.
-//   Only a query whose pass-2 set overflows its buffer is re-run on the FP32 scan.
+//   A query whose pass-2 set overflows its buffer gets a higher T from the rows it holds and another pass
+//   2; only one that overflows again is re-run on the FP32 scan.
 //
 // K3 layout. One CTA = 128 queries (one TMEM lane each; the query block is the MMA's A operand,
-// resident in shared memory) × one range of base rows. Warp 0 issues TMA loads of 256-row base
+// resident in shared memory or streamed with the base slabs) × one range of base rows. Warp 0 issues TMA loads of 256-row base
 // tiles, one 128-byte K slab per ring stage (128 B swizzle); warp 1 issues tcgen05.mma (M = 128,
 // N = 256, 4 instructions per slab) into one of two 256-column FP32 accumulators in TMEM; warps 2-5
 // read the finished accumulator with tcgen05.ld (each thread: one query's 256 scores, in 32-column

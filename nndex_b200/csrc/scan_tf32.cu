@@ -21,7 +21,8 @@
 // and the exact rerank (K4: the FP32 scan's own summation order) returns the top-k with the
 // certificate "exact k-th > k′-th bound": every other row's FP32 score is ≤ its u ≤ that bound. So a
 // certified query's rows and scores are bit for bit those of the FP32 scan; an uncertified one is
-// re-run on the FP32 scan by the host.
+// listed by the rerank and re-run on the FP32 scan (on the device behind the batch, or after it by a call
+// that waits for its batch).
 //
 // Layout: one CTA per (row range, block of 16 queries); ring stages of 128 base rows × one 128-byte
 // slab (32 FP32 values) plus the 16 queries' slab, both loaded by TMA with the 128-byte swizzle that
