@@ -8,13 +8,14 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <sys/mman.h>
+
 #include <algorithm>
 #include <chrono>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -232,21 +233,27 @@ void CudaIndex::drop_graphs() {
     graphs.clear();
 }
 
-// The host's words (kHostWordBytes, pinned). A page of the heap, registered, takes a third of the time that
-// a pinned allocation does (0.3 ms; the driver maps 2 MB for the first one of a process: 0.9 to 2.7).
+// The host's words (kHostWordBytes, pinned). A page of our own, registered, takes a third of the time that
+// a pinned allocation does (0.3 ms; the driver maps 2 MB for the first one of a process: 0.9 to 2.7). It is
+// kept out of forked children, as the driver's own pinned memory is: copy-on-write would leave the parent
+// another page than the one that the GPU writes.
 cudaError_t CudaIndex::alloc_words() {
-    words_page = std::aligned_alloc(kHostWordBytes, kHostWordBytes);
-    void* seen = nullptr;
-    if (words_page && cudaHostRegister(words_page, kHostWordBytes, cudaHostRegisterMapped) == cudaSuccess) {
-        if (cudaHostGetDevicePointer(&seen, words_page, 0) != cudaSuccess || seen != words_page)
-            cudaHostUnregister(words_page);  // the kernels are given the host's address
-        else
-            h_flags = static_cast<uint64_t*>(words_page);
+    void* page = mmap(nullptr, kHostWordBytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (page != MAP_FAILED) {
+        void* seen = nullptr;  // the kernels are given the host's address
+        if (madvise(page, kHostWordBytes, MADV_DONTFORK) == 0 &&
+            cudaHostRegister(page, kHostWordBytes, cudaHostRegisterMapped) == cudaSuccess) {
+            if (cudaHostGetDevicePointer(&seen, page, 0) == cudaSuccess && seen == page)
+                words_page = page;
+            else
+                cudaHostUnregister(page);
+        }
+        if (!words_page) munmap(page, kHostWordBytes);
     }
-    if (!h_flags) {
+    if (words_page) {
+        h_flags = static_cast<uint64_t*>(words_page);
+    } else {
         cudaGetLastError();
-        std::free(words_page);
-        words_page = nullptr;
         const cudaError_t e = cudaMallocHost(&h_flags, kHostWordBytes);
         if (e != cudaSuccess) return e;
     }
@@ -259,7 +266,7 @@ cudaError_t CudaIndex::alloc_words() {
 void CudaIndex::free_words() {
     if (words_page) {
         cudaHostUnregister(words_page);
-        std::free(words_page);
+        munmap(words_page, kHostWordBytes);
     } else {
         cudaFreeHost(h_flags);
     }
