@@ -385,6 +385,13 @@ NNDEX_API int nndex_cuda_autotune_import(nndex_cuda_index* index, const char* te
 /* Parses exported text without an index or a GPU: NNDEX_OK and the entry count, or
  * NNDEX_ERR_INVALID_ARGUMENT and the first bad line in the error message. */
 NNDEX_API int nndex_cuda_autotune_validate(const char* text, uint64_t* entries);
+/* The path (nndex_cuda_search_stats.path) that an exact index of this shape and these flags takes for a
+ * batch with the text's plans in its cache, without an index or a GPU (148 SMs). row_norms 0: an
+ * index that had no memory for the TF32 scans' row norms. A plan that cannot run on the index or
+ * does not hold the batch's k is left to the rules. */
+NNDEX_API int nndex_cuda_autotune_path(const char* text, uint64_t rows, uint64_t dims, uint32_t flags,
+                                       uint32_t precision, int row_norms, uint64_t query_rows, uint64_t k,
+                                       uint32_t* path);
 
 /* Lists probed per query by later approx searches (0 = choose_nprobe, src/approx.rs:318-336);
  * no counterpart in the reference, whose nprobe is always the policy's. */

@@ -192,6 +192,7 @@ SIGNATURES = {
     "nndex_cuda_autotune_export": (_i32, [_vp, C.c_char_p, _u64, C.POINTER(_u64)]),
     "nndex_cuda_autotune_import": (_i32, [_vp, C.c_char_p]),
     "nndex_cuda_autotune_validate": (_i32, [C.c_char_p, C.POINTER(_u64)]),
+    "nndex_cuda_autotune_path": (_i32, [C.c_char_p, _u64, _u64, _u32, _u32, _i32, _u64, _u64, C.POINTER(_u32)]),
     "nndex_cuda_last_score_errors": (_i32, [_vp, _u64, _u64, _vp]),
     "nndex_cuda_search_batch_device_noalloc": (_i32, [_vp, _vp, _u64, _u64, _u64, _vp, _vp, _vp, _vp]),
     "nndex_cuda_ivf_layout": (_i32, [_vp, C.POINTER(_u64), _vp, _vp, _vp, _vp]),

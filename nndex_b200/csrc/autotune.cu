@@ -152,11 +152,7 @@ CudaIndex::TunePlan CudaIndex::rule_plan(uint64_t nq, uint64_t kcap) const {
 
 std::vector<CudaIndex::TunePlan> CudaIndex::tune_candidates(uint64_t nq, uint64_t kcap) const {
     std::vector<TunePlan> c;
-    auto tc_ok = [&](bool fp8) {
-        if (fp8 ? !d_base_fp8 : !d_base_bf16) return false;
-        const TcPlan p1 = plan_tc(kcap, fp8);
-        return p1.kp >= kcap && p1.kp > 0 && plan_tc(0, fp8).stages > 0;
-    };
+    auto tc_ok = [&](bool fp8) { return tc_fits(kcap, fp8); };
     auto add_tc = [&](int path) {
         // pass 2 with one or two query blocks per CTA, where a batch has two blocks and they fit.
         // (CTA pairs, qb 3, are not timed: on 10M × 256 at 4,096 queries they tied one block in
@@ -218,13 +214,36 @@ std::vector<CudaIndex::TunePlan> CudaIndex::tune_candidates(uint64_t nq, uint64_
     return c;
 }
 
+// Whether this index can run the plan on this batch. A cached plan is shared by every batch of its bucket,
+// whose largest k (or smallest batch) it may not hold, and an imported one may name a copy of the rows, or
+// their TF32 norms, that this index does not have.
+bool CudaIndex::plan_fits(const TunePlan& plan, uint64_t nq, uint64_t kcap) const {
+    ScanPlan rerun;
+    switch (plan.path) {
+        case 2: return tc_fits(kcap, false);
+        case 3: return tc_fits(kcap, true);
+        case 4: return uses_ivf();
+        case 5: return uses_ivf() && ivf->d_reordered16;
+        case 6:
+            return plan_tf32(nq, kcap).kp &&
+                   plan_fallback(6, static_cast<uint32_t>(nq), static_cast<uint32_t>(kcap), rerun);
+        case 7: return plan_tf32_batch(nq, kcap).kp != 0;
+        default: return true;
+    }
+}
+
+// The cached plan of the batch's bucket, where it fits the batch (null: the rules choose).
+const CudaIndex::TuneEntry* CudaIndex::cached_plan(uint64_t nq, uint64_t kcap) const {
+    if (!autotune) return nullptr;
+    const auto it = tune_cache.find(tune_key(nq, kcap));
+    return it != tune_cache.end() && plan_fits(it->second.plan, nq, kcap) ? &it->second : nullptr;
+}
+
 CudaIndex::TunePlan CudaIndex::plan_for(uint64_t nq, uint64_t kcap, bool* measure) const {
     *measure = false;
-    if (autotune) {
-        auto it = tune_cache.find(tune_key(nq, kcap));
-        if (it != tune_cache.end()) return it->second.plan;
-        if (autotune == 1 && tune_candidates(nq, kcap).size() > 1) *measure = true;
-    }
+    if (const TuneEntry* ent = cached_plan(nq, kcap)) return ent->plan;
+    // (a bucket whose plan does not fit this batch keeps it for the others)
+    if (autotune == 1 && !tune_cache.count(tune_key(nq, kcap)) && tune_candidates(nq, kcap).size() > 1) *measure = true;
     return rule_plan(nq, kcap);
 }
 
@@ -292,6 +311,35 @@ int nndex_cuda_autotune_validate(const char* text, uint64_t* entries) {
     const int st = parse_cache(text, nullptr, [&](uint64_t, const CudaIndex::TuneEntry&) { ++n; });
     if (entries) *entries = n;
     return st;
+}
+
+int nndex_cuda_autotune_path(const char* text, uint64_t rows, uint64_t dims, uint32_t flags, uint32_t precision,
+                             int row_norms, uint64_t query_rows, uint64_t k, uint32_t* path) {
+    clear_error();
+    if (!path || rows == 0 || dims == 0 || query_rows == 0 || query_rows > kMaxBatchChunk || k == 0)
+        return set_error(NNDEX_ERR_INVALID_ARGUMENT, "cuda execution error: plan needs rows, dims, queries and k");
+    CudaIndex ix;  // no memory: the plan choice only looks at which copies there are
+    const int st = parse_cache(text, nullptr, [&](uint64_t key, const CudaIndex::TuneEntry& e) { ix.tune_cache[key] = e; });
+    if (st) return st;
+    ix.rows = rows;
+    ix.rows_alloc = (rows + 255) / 256 * 256;
+    ix.dims = dims;
+    ix.dp = (dims + 7) / 8 * 8;
+    ix.ds = (dims + 31) / 32 * 32;
+    ix.flags = flags;
+    ix.precision = precision;
+    if (flags & NNDEX_FLAG_BF16) {
+        ix.kb16 = (dims + 63) / 64 * 64;
+        ix.d_base_bf16 = reinterpret_cast<__nv_bfloat16*>(16);
+    }
+    if (flags & NNDEX_FLAG_FP8) {
+        ix.kf8 = (dims + 127) / 128 * 128;
+        ix.d_base_fp8 = reinterpret_cast<uint8_t*>(16);
+    }
+    if (row_norms) ix.d_tfnorm = reinterpret_cast<float2*>(16);
+    bool measure = false;
+    *path = static_cast<uint32_t>(ix.plan_for(query_rows, std::min(k, rows), &measure).path);
+    return NNDEX_OK;
 }
 
 }  // extern "C"

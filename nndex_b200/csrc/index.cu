@@ -443,26 +443,29 @@ int CudaIndex::check_device_words() {
 
 // ---- path choice (rules by batch size, k and the index's copies) ----------------------------
 
+// The tensor-core scan of the BF16 or FP8 copy holds k results (and there is such a copy).
+bool CudaIndex::tc_fits(uint64_t kcap, bool fp8) const {
+    if (fp8 ? !d_base_fp8 : !d_base_bf16) return false;
+    const TcPlan p1 = plan_tc(kcap, fp8);
+    return p1.stages > 0 && p1.kp >= kcap && p1.kp > 0 && plan_tc(0, fp8).stages > 0;
+}
+
 int CudaIndex::choose_path(uint64_t nq, uint64_t kcap) const {
-    const bool has16 = d_base_bf16 != nullptr, has8 = d_base_fp8 != nullptr;
-    auto tc_ok = [&](bool fp8) {
-        const TcPlan p1 = plan_tc(kcap, fp8);
-        return p1.kp >= kcap && p1.kp > 0 && plan_tc(0, fp8).stages > 0;
-    };
+    auto tc_ok = [&](bool fp8) { return tc_fits(kcap, fp8); };
     // Small batches (plan_tf32's range): the TF32 candidate scan, which reads the same FP32 base and
     // returns the same bits as the FP32 scan at the HBM rate, where the FP32 scan is bound by its
     // FMA issue.
     const int fp32_path = plan_tf32(nq, kcap).kp ? 6 : plan_tf32_batch(nq, kcap).kp ? 7 : 1;
     switch (precision) {
         case NNDEX_PRECISION_FP32: return fp32_path;
-        case NNDEX_PRECISION_BF16: return (has16 && tc_ok(false)) ? 2 : 1;
-        case NNDEX_PRECISION_FP8: return (has8 && tc_ok(true)) ? 3 : 1;
+        case NNDEX_PRECISION_BF16: return tc_ok(false) ? 2 : 1;
+        case NNDEX_PRECISION_FP8: return tc_ok(true) ? 3 : 1;
         default:
             // FP32 streaming is HBM-bound at small batches; the tensor cores win from a few dozen
             // queries per batch (the scan becomes compute-bound in FP32).
             if (nq >= 64) {
-                if (has16 && tc_ok(false)) return 2;
-                if (has8 && tc_ok(true)) return 3;
+                if (tc_ok(false)) return 2;
+                if (tc_ok(true)) return 3;
             }
             return fp32_path;
     }
@@ -1615,12 +1618,9 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
         TunePlan plan = plan_for(n, kcap, &measure);
         if (measure) {
             if ((st = tune_host(n, kcap, mode, &plan))) return st;
-        } else if (autotune) {
-            auto it = tune_cache.find(tune_key(n, kcap));
-            if (it != tune_cache.end()) {
-                stats.tuned = 2;
-                stats.tune_candidates = it->second.candidates;
-            }
+        } else if (const TuneEntry* ent = cached_plan(n, kcap)) {
+            stats.tuned = 2;
+            stats.tune_candidates = ent->candidates;
         }
         const int path = plan.path;
         serr_off = q0;
@@ -1758,12 +1758,9 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
             stats.tune_candidates = ent.candidates;
             plan = ent.plan;
             synced = true;
-        } else if (autotune) {
-            auto it = tune_cache.find(tune_key(n, kcap));
-            if (it != tune_cache.end()) {
-                stats.tuned = 2;
-                stats.tune_candidates = it->second.candidates;
-            }
+        } else if (const TuneEntry* ent = cached_plan(n, kcap)) {
+            stats.tuned = 2;
+            stats.tune_candidates = ent->candidates;
         }
         forced_stride = plan.stride;
         forced_qb = plan.qb;

@@ -356,6 +356,9 @@ struct CudaIndex {
     // The plan for a batch: cached, or by the rules; *measure when the tuner should time the
     // candidates on this batch first.
     TunePlan plan_for(uint64_t nq, uint64_t kcap, bool* measure) const;
+    const TuneEntry* cached_plan(uint64_t nq, uint64_t kcap) const;
+    bool plan_fits(const TunePlan& plan, uint64_t nq, uint64_t kcap) const;
+    bool tc_fits(uint64_t kcap, bool fp8) const;
     // The first host-buffer batch of a shape: every candidate plan timed on it (the queries in h_q).
     int tune_host(uint64_t n, uint64_t kcap, int mode, TunePlan* plan);
     struct TcPlan {
