@@ -476,6 +476,8 @@ NNDEX_API int nndex_cuda_check_bounded_wait(nndex_cuda_index* index, uint64_t bu
  * fail as if the GPU were out of memory (no cudaMalloc is attempted), and the calls that needed them
  * return NNDEX_ERR_OUT_OF_MEMORY. 0 cancels. For tests of callers' out-of-memory handling. */
 NNDEX_API void nndex_cuda_inject_alloc_failures(uint32_t count);
+/* The same, after `allocations` further ones that go ahead. */
+NNDEX_API void nndex_cuda_inject_alloc_failures_after(uint32_t allocations, uint32_t count);
 
 /* ---- launch planning (host only: no GPU, no index) ------------------------------------------ */
 

@@ -56,7 +56,11 @@ int nndex_cuda_check_bounded_wait(nndex_cuda_index* index, uint64_t budget_cycle
     return ix->check_device_words();
 }
 
-void nndex_cuda_inject_alloc_failures(uint32_t count) { inject_alloc_failures(count); }
+void nndex_cuda_inject_alloc_failures(uint32_t count) { inject_alloc_failures(0, count); }
+
+void nndex_cuda_inject_alloc_failures_after(uint32_t allocations, uint32_t count) {
+    inject_alloc_failures(allocations, count);
+}
 
 int nndex_cuda_plan_tc_ranges(uint64_t rows, uint64_t groups, uint32_t sm_count, uint64_t* nranges,
                               uint64_t* range_rows) {

@@ -30,17 +30,29 @@ namespace nndex {
 
 static std::atomic<uint64_t> g_launches{0};
 static std::atomic<uint64_t> g_alloc_epoch{0};
-static std::atomic<uint32_t> g_fail_allocs{0};  // host-side fault injection: allocations to fail
+static std::atomic<uint32_t> g_fail_skip{0}, g_fail_allocs{0};  // host-side fault injection: allocations to fail
 bool take_injected_alloc_failure() {
-    uint32_t n = g_fail_allocs.load(std::memory_order_relaxed);
+    uint32_t n = g_fail_skip.load(std::memory_order_relaxed);
+    while (n > 0 && !g_fail_skip.compare_exchange_weak(n, n - 1, std::memory_order_relaxed)) {
+    }
+    if (n > 0) return false;
+    n = g_fail_allocs.load(std::memory_order_relaxed);
     while (n > 0 && !g_fail_allocs.compare_exchange_weak(n, n - 1, std::memory_order_relaxed)) {
     }
     return n > 0;
 }
-void inject_alloc_failures(uint32_t n) { g_fail_allocs.store(n, std::memory_order_relaxed); }
+void inject_alloc_failures(uint32_t skip, uint32_t n) {
+    g_fail_skip.store(n ? skip : 0, std::memory_order_relaxed);
+    g_fail_allocs.store(n, std::memory_order_relaxed);
+}
 static thread_local cudaStream_t t_scratch_stream = nullptr;
 void set_scratch_stream(cudaStream_t s) { t_scratch_stream = s; }
 cudaStream_t scratch_stream() { return t_scratch_stream; }
+static void release_raw(void** p) {
+    if (*p && t_scratch_stream) cudaFreeAsync(*p, t_scratch_stream);
+    else if (*p) cudaFree(*p);
+    *p = nullptr;
+}
 cudaError_t regrow_raw(void** p, size_t bytes) {
     if (bytes == 0) bytes = 1;
     cudaStream_t s = t_scratch_stream;
@@ -650,14 +662,12 @@ int CudaIndex::enqueue_prep_queries(const float* d_raw, uint64_t n, int mode, in
         if ((st = ivf_plan_words(*this, &p.zero[0], &p.zero_words[0]))) return st;
     } else if (path == 6) {
         if ((st = grow_device(d_floor, cap_floor, n, "tc workspace"))) return st;
-            p.zero[0] = reinterpret_cast<uint32_t*>(d_floor);
+        p.zero[0] = reinterpret_cast<uint32_t*>(d_floor);
         p.zero_words[0] = 2 * n;
         p.zero[1] = d_fbn;
         p.zero_words[1] = 1;
     } else if (path == 7) {
-        if ((st = grow_device(d_q_resid, cap_q_resid, n, "query buffer"))) return st;
-        if ((st = grow_device(d_cnt2, cap_cnt2, n, "pass-2 buffer"))) return st;
-            p.tf_slack = d_q_resid;
+        p.tf_slack = d_q_resid;  // (settle_path has grown it, and d_cnt2)
         p.tf_row_max = d_tfnorm + rows;
         p.tf_c_norm = tf32_c_norm();
         p.tf_collected = d_cnt2;
@@ -1274,7 +1284,8 @@ int CudaIndex::enqueue_fp32_fallback(const ScanPlan& plan, uint32_t n, uint32_t 
 int CudaIndex::grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t kcap, uint64_t fb_keys) {
     int st;
     const uint64_t words = plan.nranges * plan.gm_tiles * (256 / plan.group);
-    if ((st = grow_device(d_ws, cap_ws, std::max((words + 1) / 2, fb_keys) * n, "scan workspace"))) return st;
+    if ((st = grow_device(d_q_resid, cap_q_resid, n, "query buffer"))) return st;
+    if ((st = grow_device(d_cnt2, cap_cnt2, n, "pass-2 buffer"))) return st;
     if ((st = grow_device(d_ids, cap_ids, n, "pass-2 buffer"))) return st;
     if ((st = grow_device(d_cand_idx, cap_cand_idx, static_cast<uint64_t>(n) * plan.kp, "tc workspace"))) return st;
     if ((st = grow_device(d_cand_sim, cap_cand_sim, static_cast<uint64_t>(n) * plan.kp, "tc workspace"))) return st;
@@ -1286,7 +1297,50 @@ int CudaIndex::grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t k
     if ((st = grow_device(d_rslots, cap_rslots, static_cast<uint64_t>(n) * rerank_chunks(kSecondPassCap) * kcap,
                           "pass-2 buffer")))
         return st;
-    return grow_device(d_fbq, cap_fbq, n, "fallback buffer");
+    if ((st = grow_device(d_fbq, cap_fbq, n, "fallback buffer"))) return st;
+    // last: the FP32 scan has its keys there too, and keeps what it has where one of the others fails
+    return grow_device(d_ws, cap_ws, std::max((words + 1) / 2, fb_keys) * n, "scan workspace");
+}
+
+// The path a batch planned on the two-pass TF32 scan takes, decided before anything of it is enqueued. Without
+// memory for the collections: the FP32 scan, whose workspace is far smaller. What the attempt had grown
+// is given back, and the next batches do not try again (each try would free, allocate and drop
+// every captured graph).
+int CudaIndex::settle_path(int* path, uint32_t n, uint32_t kcap) {
+    if (*path != 7) return NNDEX_OK;
+    if (tf32_rest) {
+        --tf32_rest;
+        *path = 1;
+        return NNDEX_OK;
+    }
+    const Tf32BatchPlan plan = plan_tf32_batch(n, kcap);
+    ScanPlan fb_plan;
+    if (!plan.kp || !plan_fallback(7, n, kcap, fb_plan)) {
+        *path = 1;
+        return NNDEX_OK;
+    }
+    struct Grown {
+        void** p;
+        size_t* cap;
+        size_t before;
+    };
+    auto at = [](auto& p, size_t& cap) { return Grown{reinterpret_cast<void**>(&p), &cap, cap}; };
+    const Grown grown[] = {at(d_q_resid, cap_q_resid),   at(d_cnt2, cap_cnt2),         at(d_ids, cap_ids),
+                           at(d_cand_idx, cap_cand_idx), at(d_cand_sim, cap_cand_sim), at(d_cand_cnt, cap_cand_cnt),
+                           at(d_cert, cap_cert),         at(d_kth, cap_kth),           at(d_rows2, cap_rows2),
+                           at(d_ok2, cap_ok2),           at(d_rslots, cap_rslots),     at(d_fbq, cap_fbq)};
+    const int st = grow_tf32_batch(plan, n, kcap, static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap);
+    if (st != NNDEX_ERR_OUT_OF_MEMORY) return st;
+    cudaGetLastError();
+    clear_error();
+    for (const Grown& g : grown) {
+        if (*g.cap == g.before) continue;
+        release_raw(g.p);
+        *g.cap = 0;
+    }
+    tf32_rest = kTf32Rest;
+    *path = 1;
+    return NNDEX_OK;
 }
 
 // Two-pass TF32 scan (FP32 indexes, 17 queries and more): K3's sampled pass 1 and collecting pass 2 on
@@ -1298,16 +1352,8 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
     int st;
     const Tf32BatchPlan plan = plan_tf32_batch(n, kcap);
     ScanPlan fb_plan;
-    // (a tuned plan is shared by the shapes of a power of two, some of which the rule may not take)
     if (!plan.kp || !plan_fallback(7, n, kcap, fb_plan))
-        return enqueue_exact_fp32(d_qn, n, kcap, kcap, o_idx, o_sim, o_cnt, s);
-    if ((st = grow_tf32_batch(plan, n, kcap, static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap))) {
-        // without memory for the collections: the FP32 scan, whose workspace is far smaller
-        if (st != NNDEX_ERR_OUT_OF_MEMORY) return st;
-        cudaGetLastError();
-        clear_error();
-        return enqueue_exact_fp32(d_qn, n, kcap, kcap, o_idx, o_sim, o_cnt, s);
-    }
+        return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: no two-pass TF32 plan for k=%u", kcap);
     CUtensorMap tmap_q;  // the queries straight from the prepared buffer: rows past n read as zeros
     if (!encode_tmap_2d(&tmap_q, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d_qn, ds, n, ds * sizeof(float), 32, 128,
                         CU_TENSOR_MAP_SWIZZLE_128B))
@@ -1422,7 +1468,9 @@ int CudaIndex::tune_host(uint64_t n, uint64_t kcap, int mode, TunePlan* plan) {
             forced_stride = cands[c].stride;
             forced_qb = cands[c].qb;
             const auto t0 = std::chrono::steady_clock::now();
-            cst = enqueue_host_batch(n, kcap, mode, cands[c].path);
+            int path = cands[c].path;
+            cst = settle_path(&path, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap));
+            if (cst == NNDEX_OK) cst = enqueue_host_batch(n, kcap, mode, path);
             const cudaError_t e = cudaStreamSynchronize(stream);
             if (cst == NNDEX_OK && e != cudaSuccess) cst = cuda_error(e, "search");
             if (cst == NNDEX_OK) cst = check_device_words();
@@ -1622,7 +1670,8 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
             stats.tuned = 2;
             stats.tune_candidates = ent->candidates;
         }
-        const int path = plan.path;
+        int path = plan.path;
+        if ((st = settle_path(&path, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap)))) return st;
         serr_off = q0;
         forced_stride = plan.stride;
         forced_qb = plan.qb;
@@ -1669,6 +1718,7 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
 int CudaIndex::run_device_chunk(const float* dq, uint64_t n, uint64_t kcap, int path, uint64_t* oi, float* os,
                                 uint32_t* oc, cudaStream_t s, bool* synced) {
     int st;
+    if ((st = settle_path(&path, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap)))) return st;
     if ((st = enqueue_prep_queries(dq, n, normalized ? 2 : 0, path, s))) return st;
     const uint32_t n32 = static_cast<uint32_t>(n), k32 = static_cast<uint32_t>(kcap);
     if (path == 4) return ivf_search(*this, d_qn, n32, k32, oi, os, oc, s);

@@ -29,12 +29,17 @@ constexpr size_t kMappedIoBytes = 64 << 10;
 // 11,410 / 962.
 constexpr uint64_t kTf32BatchMinWork = 250000000ull;
 
+// After a batch that the two-pass TF32 scan could not serve, this many go to the FP32 scan before it is tried
+// again: a batch that tries in vain costs at most about twice the FP32 scan, so 3 % over 32.
+constexpr uint32_t kTf32Rest = 31;
+
 // Incremented whenever a scratch or staging buffer of any index is (re)allocated: a captured
 // CUDA graph is valid only while the epoch it was captured in lasts.
 uint64_t alloc_epoch();
 void bump_alloc_epoch();
-// Host-side fault injection (tests): the next n scratch allocations fail as out of memory.
-void inject_alloc_failures(uint32_t n);
+// Host-side fault injection (tests): after `skip` scratch allocations that go ahead, the next n fail as out
+// of memory.
+void inject_alloc_failures(uint32_t skip, uint32_t n);
 bool take_injected_alloc_failure();
 // Scratch growth. By default a buffer that must grow is freed with cudaFree (which waits for the
 // whole device) and reallocated with cudaMalloc. A serving slot instead grows its buffers in
@@ -396,6 +401,8 @@ struct CudaIndex {
                        cudaStream_t s, std::vector<uint32_t>* failed);
     int enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
     int enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
+    int settle_path(int* path, uint32_t n, uint32_t kcap);
+    uint32_t tf32_rest = 0;  // batches of the two-pass TF32 scan's shapes still to go to the FP32 scan
     int grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t kcap, uint64_t fb_keys);
     // The FP32 scan of the d_fbn[0] queries listed in d_fbq, into their own output rows (enqueued
     // for up to n of them; its launches return at once when there are none).
