@@ -479,6 +479,11 @@ NNDEX_API void nndex_cuda_inject_alloc_failures(uint32_t count);
 /* The same, after `allocations` further ones that go ahead. */
 NNDEX_API void nndex_cuda_inject_alloc_failures_after(uint32_t allocations, uint32_t count);
 
+/* The next `count` re-runs of queries that a tensor-core scan could not finish (pass-2 overflows, uncertified
+ * queries of a host-buffer batch) are followed by a bounded device wait that runs out, and their calls
+ * return NNDEX_ERR_TIMEOUT. 0 cancels. For tests of the status checks behind the re-runs. */
+NNDEX_API void nndex_cuda_inject_rerun_timeouts(uint32_t count);
+
 /* ---- launch planning (host only: no GPU, no index) ------------------------------------------ */
 
 /* The row ranges the tensor-core scan splits `rows` rows into for `groups` CTAs per range (its

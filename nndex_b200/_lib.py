@@ -202,6 +202,7 @@ SIGNATURES = {
     "nndex_cuda_check_bounded_wait": (_i32, [_vp, _u64]),
     "nndex_cuda_inject_alloc_failures": (None, [_u32]),
     "nndex_cuda_inject_alloc_failures_after": (None, [_u32, _u32]),
+    "nndex_cuda_inject_rerun_timeouts": (None, [_u32]),
     "nndex_cuda_plan_tc_ranges": (_i32, [_u64, _u64, _u32, C.POINTER(_u64), C.POINTER(_u64)]),
     "nndex_cuda_plan_fp32_scan": (_i32, [_u32, _u32, _u32, _u64, _u32, _u64, C.POINTER(_u32), C.POINTER(_u32),
                                          C.POINTER(_u32)]),

@@ -30,6 +30,13 @@ __global__ void bounded_wait_probe_kernel(long long budget, uint32_t* status) {
 
 }  // namespace
 
+namespace nndex {
+void launch_unanswered_wait(long long budget_cycles, uint32_t* status, cudaStream_t s) {
+    bounded_wait_probe_kernel<<<1, 32, 0, s>>>(budget_cycles, status);
+    count_launch();
+}
+}  // namespace nndex
+
 extern "C" {
 
 int nndex_cuda_check_bounded_wait(nndex_cuda_index* index, uint64_t budget_cycles) {
@@ -43,8 +50,7 @@ int nndex_cuda_check_bounded_wait(nndex_cuda_index* index, uint64_t budget_cycle
     cudaSetDevice(ix->device);
     ix->order_after_previous(ix->stream);
     cudaMemsetAsync(ix->d_status, 0, sizeof(uint32_t), ix->stream);
-    bounded_wait_probe_kernel<<<1, 32, 0, ix->stream>>>(static_cast<long long>(budget_cycles), ix->d_status);
-    count_launch();
+    launch_unanswered_wait(static_cast<long long>(budget_cycles), ix->d_status, ix->stream);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "wait check launch");
     ix->h_flags[0] = 0;  // no validation error involved
@@ -61,6 +67,8 @@ void nndex_cuda_inject_alloc_failures(uint32_t count) { inject_alloc_failures(0,
 void nndex_cuda_inject_alloc_failures_after(uint32_t allocations, uint32_t count) {
     inject_alloc_failures(allocations, count);
 }
+
+void nndex_cuda_inject_rerun_timeouts(uint32_t count) { inject_rerun_timeouts(count); }
 
 int nndex_cuda_plan_tc_ranges(uint64_t rows, uint64_t groups, uint32_t sm_count, uint64_t* nranges,
                               uint64_t* range_rows) {

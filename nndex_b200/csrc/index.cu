@@ -45,6 +45,14 @@ void inject_alloc_failures(uint32_t skip, uint32_t n) {
     g_fail_skip.store(n ? skip : 0, std::memory_order_relaxed);
     g_fail_allocs.store(n, std::memory_order_relaxed);
 }
+static std::atomic<uint32_t> g_rerun_timeouts{0};
+bool take_injected_rerun_timeout() {
+    uint32_t n = g_rerun_timeouts.load(std::memory_order_relaxed);
+    while (n > 0 && !g_rerun_timeouts.compare_exchange_weak(n, n - 1, std::memory_order_relaxed)) {
+    }
+    return n > 0;
+}
+void inject_rerun_timeouts(uint32_t n) { g_rerun_timeouts.store(n, std::memory_order_relaxed); }
 static thread_local cudaStream_t t_scratch_stream = nullptr;
 void set_scratch_stream(cudaStream_t s) { t_scratch_stream = s; }
 cudaStream_t scratch_stream() { return t_scratch_stream; }
@@ -1116,9 +1124,16 @@ int CudaIndex::rerun_exact_fp32(const std::vector<uint32_t>& qs, uint32_t kcap, 
                         cudaMemcpyDeviceToDevice, s);
         if (o_cnt) cudaMemcpyAsync(o_cnt + q, d_fb_cnt + i, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
     }
+    return wait_rerun(s);
+}
+
+// Waits for a re-run that followed its batch, and reads the status words again: a device wait that ran out
+// in it has left part of the queries' results unwritten.
+int CudaIndex::wait_rerun(cudaStream_t s) {
+    if (take_injected_rerun_timeout()) launch_unanswered_wait(kInjectedWaitCycles, w_status, s);
+    if (w_err == d_err) cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
     const cudaError_t e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_error(e, "search");
-    return NNDEX_OK;
+    return e != cudaSuccess ? cuda_error(e, "search") : check_device_words();
 }
 
 // K12 (small batches, FP32 precision): the TF32 candidate scan, the merge of each query's per-CTA
@@ -1240,8 +1255,7 @@ int CudaIndex::finish_tf32(int path, uint32_t n, uint32_t kcap) {
     stats.kernel_launches += 2;
     if (!mapped_io) cudaMemcpyAsync(h_res, d_res, res_bytes, cudaMemcpyDeviceToHost, stream);
     cudaEventRecord(ev1, stream);
-    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_error(e, "search");
-    return check_device_words();
+    return wait_rerun(stream);
 }
 
 // The scan reads the listed queries' rows, the merge writes each result into the query's own output

@@ -41,6 +41,11 @@ void bump_alloc_epoch();
 // of memory.
 void inject_alloc_failures(uint32_t skip, uint32_t n);
 bool take_injected_alloc_failure();
+// The next n re-runs of listed queries are followed by a device wait that runs out (tests).
+void inject_rerun_timeouts(uint32_t n);
+bool take_injected_rerun_timeout();
+constexpr long long kInjectedWaitCycles = 2000000;  // about 1 ms
+void launch_unanswered_wait(long long budget_cycles, uint32_t* status, cudaStream_t s);
 // Scratch growth. By default a buffer that must grow is freed with cudaFree (which waits for the
 // whole device) and reallocated with cudaMalloc. A serving slot instead grows its buffers in
 // stream order on its own stream (cudaFreeAsync / cudaMallocAsync), so a slot meeting a larger
@@ -409,6 +414,7 @@ struct CudaIndex {
     int enqueue_fp32_fallback(const ScanPlan& plan, uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim,
                               uint32_t* o_cnt, cudaStream_t s);
     // The FP32 scan for the listed queries (rows of d_qn), written into their output slots.
+    int wait_rerun(cudaStream_t s);
     int rerun_exact_fp32(const std::vector<uint32_t>& qs, uint32_t kcap, uint64_t* o_idx, float* o_sim,
                          uint32_t* o_cnt, cudaStream_t s);
     int stream_status();

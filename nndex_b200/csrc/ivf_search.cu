@@ -1582,8 +1582,7 @@ int ivf_finish_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
                         cudaMemcpyDeviceToDevice, s);
         if (o_cnt) cudaMemcpyAsync(o_cnt + q, ix.d_fb_cnt + i, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
     }
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(e, "IVF search");
-    return NNDEX_OK;
+    return ix.wait_rerun(s);
 }
 
 }  // namespace nndex
