@@ -1116,13 +1116,14 @@ int CudaIndex::rerun_exact_fp32(const std::vector<uint32_t>& qs, uint32_t kcap, 
     const uint32_t path = stats.path;
     if ((st = enqueue_exact_fp32(d_qsub, mf, kcap, kcap, d_fb_idx, d_fb_sim, d_fb_cnt, s))) return st;
     stats.path = path;
+    // (a small host batch's outputs are in pinned host memory)
     for (uint32_t i = 0; i < mf; ++i) {
         const uint64_t q = qs[i];
         cudaMemcpyAsync(o_idx + q * kcap, d_fb_idx + static_cast<uint64_t>(i) * kcap, kcap * sizeof(uint64_t),
-                        cudaMemcpyDeviceToDevice, s);
+                        cudaMemcpyDefault, s);
         cudaMemcpyAsync(o_sim + q * kcap, d_fb_sim + static_cast<uint64_t>(i) * kcap, kcap * sizeof(float),
-                        cudaMemcpyDeviceToDevice, s);
-        if (o_cnt) cudaMemcpyAsync(o_cnt + q, d_fb_cnt + i, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+                        cudaMemcpyDefault, s);
+        if (o_cnt) cudaMemcpyAsync(o_cnt + q, d_fb_cnt + i, sizeof(uint32_t), cudaMemcpyDefault, s);
     }
     return wait_rerun(s);
 }

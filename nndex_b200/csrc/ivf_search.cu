@@ -1574,13 +1574,14 @@ int ivf_finish_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     const nndex_cuda_search_stats keep = ix.stats;
     if ((st = ivf_search(ix, ix.d_qsub, mf, k, ix.d_fb_idx, ix.d_fb_sim, ix.d_fb_cnt, s))) return st;
     ix.stats = keep;
+    // (a small host batch's outputs are in pinned host memory)
     for (uint32_t i = 0; i < mf; ++i) {
         const uint64_t q = failed[i];
         cudaMemcpyAsync(o_idx + q * k, ix.d_fb_idx + static_cast<uint64_t>(i) * k, k * sizeof(uint64_t),
-                        cudaMemcpyDeviceToDevice, s);
+                        cudaMemcpyDefault, s);
         cudaMemcpyAsync(o_sim + q * k, ix.d_fb_sim + static_cast<uint64_t>(i) * k, k * sizeof(float),
-                        cudaMemcpyDeviceToDevice, s);
-        if (o_cnt) cudaMemcpyAsync(o_cnt + q, ix.d_fb_cnt + i, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+                        cudaMemcpyDefault, s);
+        if (o_cnt) cudaMemcpyAsync(o_cnt + q, ix.d_fb_cnt + i, sizeof(uint32_t), cudaMemcpyDefault, s);
     }
     return ix.wait_rerun(s);
 }
