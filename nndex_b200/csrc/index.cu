@@ -1494,6 +1494,8 @@ int CudaIndex::tune_host(uint64_t n, uint64_t kcap, int mode, TunePlan* plan) {
             if (cst == NNDEX_OK && cands[c].path == 5)
                 cst = ivf_finish_tc(*this, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap), d_idx, d_sim, d_cnt,
                                     stream);
+            if (cst == NNDEX_OK && host_fallback && (stats.path == 6 || stats.path == 7))
+                cst = finish_tf32(path, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap));  // part of its time
             ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         }
         forced_stride = 0;
