@@ -1652,7 +1652,7 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
                            float* sim_out, uint64_t* counts_out) {
     std::lock_guard<std::mutex> lock(mu);
     cudaSetDevice(device);
-    stats = nndex_cuda_search_stats{};
+    begin_call();
     order_after_previous(stream);
     use_host_words();
     host_fallback = !error_report;  // a report records what the device-side re-run has written
@@ -1764,7 +1764,7 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
                              float* d_sim_out, uint32_t* d_cnt_out, cudaStream_t s, int synchronize) {
     std::lock_guard<std::mutex> lock(mu);
     cudaSetDevice(device);
-    stats = nndex_cuda_search_stats{};
+    begin_call();
     if (!s) s = cudaStreamLegacy;
     order_after_previous(s);
     const uint64_t kcap = std::min<uint64_t>(k, rows);
@@ -1905,10 +1905,16 @@ int CudaIndex::serr_fetch_stats() {
     return NNDEX_OK;
 }
 
+// A new call's statistics: what was still to be read into the last one's is dropped with them (its stream may
+// be gone by now).
+void CudaIndex::begin_call() {
+    stats = nndex_cuda_search_stats{};
+    ms_pending = fbn_pending = serr_pending = false;
+}
+
 // The index's scratch buffers are shared by every call: work enqueued on one stream must not
 // overlap work of an earlier call on another stream.
 void CudaIndex::order_after_previous(cudaStream_t s) {
-    ms_pending = false;
     if (done_ev && done_stream && done_stream != s) cudaStreamWaitEvent(s, done_ev, 0);
 }
 void CudaIndex::mark_done(cudaStream_t s) {

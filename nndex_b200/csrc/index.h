@@ -427,6 +427,7 @@ struct CudaIndex {
     }
     void order_after_previous(cudaStream_t s);
     void mark_done(cudaStream_t s);
+    void begin_call();
 };
 
 // Tensor map of a row-major matrix (inner × outer elements), 2-D boxes.

@@ -65,7 +65,7 @@ int search_device_noalloc(CudaIndex* ix, const float* d_queries, uint64_t nq, ui
     std::lock_guard<std::mutex> lock(ix->mu);
     cudaError_t e = cudaSetDevice(ix->device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
-    ix->stats = nndex_cuda_search_stats{};
+    ix->begin_call();
     if (ix->uses_ivf())
         return set_error(NNDEX_ERR_UNSUPPORTED,
                          "cuda execution error: the no-allocation entry point serves exact indexes only");
