@@ -1020,7 +1020,6 @@ int CudaIndex::finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_si
         else if (m * 2 <= n) tc_sample_stride = 1;
         if (tc_sample_stride != before) drop_graphs();  // a captured batch keeps its stride
     }
-    stats.fp32_fallback_queries = 0;
     tc_patched = false;
     int st;
     stats.pass2_rows += h_fbn_rows();
@@ -1028,7 +1027,7 @@ int CudaIndex::finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_si
     std::vector<uint32_t> failed;
     if ((st = retry_tc_pass2(stats.path == 3, failed_n, kcap, o_idx, o_sim, o_cnt, s, &failed))) return st;
     tc_patched = true;
-    stats.fp32_fallback_queries = static_cast<uint32_t>(failed.size());
+    stats.fp32_fallback_queries += static_cast<uint32_t>(failed.size());
     if (failed.empty()) return NNDEX_OK;
     // ---- the FP32 scan for queries whose collected set overflowed again ----
     return rerun_exact_fp32(failed, kcap, o_idx, o_sim, o_cnt, s);
@@ -1244,7 +1243,7 @@ bool CudaIndex::plan_fallback(int path, uint32_t n, uint32_t kcap, ScanPlan& pla
 // launches, 8 us of a batch of 64 queries over 50k rows when none is listed, wait for one that is.
 int CudaIndex::finish_tf32(int path, uint32_t n, uint32_t kcap) {
     stats.fp32_fallback_queries += h_fbn[0];
-    stats.certified = h_fbn[0] == 0 ? 1u : 0u;
+    stats.certified = stats.fp32_fallback_queries == 0 ? 1u : 0u;
     if (h_fbn[0] == 0) return NNDEX_OK;
     ScanPlan plan;
     if (!plan_fallback(path, n, kcap, plan))
@@ -1459,12 +1458,12 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
 // The device-side fallback's count into the statistics (waits for its stream once).
 int CudaIndex::fetch_fallback_stats() {
     if (!fbn_pending) return NNDEX_OK;
-    cudaMemcpyAsync(h_fbn, d_fbn, sizeof(uint32_t), cudaMemcpyDeviceToHost, fbn_stream);
+    cudaMemcpyAsync(h_fbn, fbn_pieces ? d_fbn_sum : d_fbn, sizeof(uint32_t), cudaMemcpyDeviceToHost, fbn_stream);
     const cudaError_t e = cudaStreamSynchronize(fbn_stream);
     if (e != cudaSuccess) return cuda_error(e, "fallback count");
     fbn_pending = false;
-    stats.fp32_fallback_queries = h_fbn[0];
-    stats.certified = h_fbn[0] == 0 ? 1u : 0u;
+    stats.fp32_fallback_queries += h_fbn[0];
+    stats.certified = stats.fp32_fallback_queries == 0 ? 1u : 0u;
     return NNDEX_OK;
 }
 
@@ -1774,6 +1773,9 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
     use_device_words();
     host_fallback = false;
     cudaMemsetAsync(d_err, 0, 2 * sizeof(unsigned long long), s);
+    // the pieces of a larger call share the word of the listed queries' number: it is added up after each
+    fbn_pieces = nq > kMaxBatchChunk;
+    if (fbn_pieces) cudaMemsetAsync(d_fbn_sum, 0, sizeof(uint32_t), s);
     bool synced = false, done = false;  // done: the last piece waited and its status words were clean
     for (uint64_t q0 = 0; q0 < nq; q0 += kMaxBatchChunk) {
         const uint64_t n = std::min<uint64_t>(kMaxBatchChunk, nq - q0);
@@ -1836,6 +1838,7 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
         forced_stride = 0;
         forced_qb = 0;
         if (st) return st;
+        if (fbn_pieces && (stats.path == 6 || stats.path == 7)) launch_add_word(d_fbn_sum, d_fbn, s);
         synced |= done;
         if (error_report) {
             done = false;

@@ -210,6 +210,7 @@ struct CudaIndex {
         d_err = reinterpret_cast<unsigned long long*>(at);
         d_status = reinterpret_cast<uint32_t*>(d_err + 1);
         d_fbn = reinterpret_cast<uint32_t*>(at + kFbnAt);
+        d_fbn_sum = d_fbn + kFbnBytes / sizeof(uint32_t);
         d_max = reinterpret_cast<unsigned int*>(at + kMaxAt);
     }
     void* words_page = nullptr;  // the registered page with the host's words, if they are in one
@@ -286,6 +287,8 @@ struct CudaIndex {
     // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, spare, rows pass 2 collected (64 bits)}
     static constexpr size_t kFbnBytes = 6 * sizeof(uint32_t);
     uint32_t* d_fbn = nullptr;
+    uint32_t* d_fbn_sum = nullptr;  // the word behind them: the first one summed over a device-buffer call's pieces
+    bool fbn_pieces = false;        // the pending count is that sum
     uint32_t* h_fbn = nullptr;  // pinned copy
     uint32_t* d_tcfail = nullptr;  // TC pass 2: positions (in d_ids) of the queries whose collection overflowed
     size_t cap_tcfail = 0;

@@ -315,6 +315,7 @@ struct BatchReport {
     const unsigned long long* flags = nullptr;     // 2: the error word, the status word
     unsigned long long* host_flags = nullptr;
 };
+void launch_add_word(uint32_t* sum, const uint32_t* word, cudaStream_t s);  // *sum += *word
 void launch_compact_zero_flags(const uint32_t* flags, uint32_t n, uint32_t* ids, uint32_t* count, cudaStream_t s,
                                const uint32_t* live = nullptr, const BatchReport& report = BatchReport{});
 

@@ -1544,7 +1544,7 @@ int ivf_finish_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     ix.stats.ivf_rows_union = w.h_probed[5];
     ix.stats.certified = m == 0 ? 1u : 0u;
     ix.stats.second_pass_queries = m;
-    ix.stats.fp32_fallback_queries = failed_n;
+    ix.stats.fp32_fallback_queries += failed_n;
     ix.tc_patched = failed_n != 0;
     int st;
     ix.stats.pass2_rows += ix.h_fbn_rows();

@@ -1587,6 +1587,13 @@ __global__ void __launch_bounds__(1024) compact_zero_flags_kernel(const uint32_t
     if (rep.host_flags && threadIdx.x < 2) rep.host_flags[threadIdx.x] = rep.flags[threadIdx.x];
 }
 
+__global__ void add_word_kernel(uint32_t* __restrict__ sum, const uint32_t* __restrict__ word) { *sum += *word; }
+
+void launch_add_word(uint32_t* sum, const uint32_t* word, cudaStream_t s) {
+    add_word_kernel<<<1, 1, 0, s>>>(sum, word);
+    count_launch();
+}
+
 void launch_compact_zero_flags(const uint32_t* flags, uint32_t n, uint32_t* ids, uint32_t* count, cudaStream_t s,
                                const uint32_t* live, const BatchReport& report) {
     compact_zero_flags_kernel<<<1, 1024, 0, s>>>(flags, n, ids, count, live, report);

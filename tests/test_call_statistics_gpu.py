@@ -30,3 +30,25 @@ def test_device_time_outlives_a_wait_check():
     index.search(q, k=K)
     assert _lib.lib().nndex_cuda_check_bounded_wait(index.handle, 100_000) == _lib.NNDEX_ERR_TIMEOUT
     assert index.last_search_stats()["device_ms"] > 0
+
+
+def test_listed_queries_are_summed_over_the_pieces_of_a_large_call():
+    # a call runs in pieces of 16,384 queries
+    rng = np.random.default_rng(2)
+    m = rng.standard_normal((20_000, 32), dtype=np.float32)
+    m[3_000:3_000 + COPIES] = m[3_000]
+    q = rng.standard_normal((16_384 + 400, 32), dtype=np.float32)
+    q[:50] = m[3_000] + np.float32(1e-3) * rng.standard_normal((50, 32), dtype=np.float32)
+    q[-10:] = q[:10]
+    index = NNdex(m, autotune=False)
+    counts = {}
+    for name, part in (("first", q[:16_384]), ("rest", q[16_384:]), ("all", q)):
+        on_device(index, part, synchronize=0)
+        st = index.last_search_stats()
+        assert st["path"] == 7
+        counts[name] = st["fp32_fallback_queries"]
+    assert counts["first"] >= 50 and counts["rest"] >= 10
+    assert counts["all"] == counts["first"] + counts["rest"], counts
+    index.search(q, k=K)
+    st = index.last_search_stats()
+    assert (st["fp32_fallback_queries"], st["certified"]) == (counts["all"], 0), st
