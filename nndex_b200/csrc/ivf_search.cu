@@ -266,7 +266,11 @@ __global__ void __launch_bounds__(256)
 //    Bound by latency (its barriers, then the rows between the bounds from L2). 1,024 queries against 1,414
 //    centroids of 384 dims: scores 17 us + pick 36, where the FP64 scores of every pair and the warp
 //    selection took 94 + 25; one query against 512 of 128: 4.5 + 8.2, before 15 + 7.4. (Exact scores
-//    as one thread's chain of FP64 adds per list: pick 54 and 10 us.)
+//    as one thread's chain of FP64 adds per list: pick 54 and 10 us.) Where more lists lie between the bounds
+//    than shared memory holds (equal centroids, from rows of few distinct values), their exact scores go
+//    back to memory and a radix selection takes the best: 8,192 lists of 3 distinct centroids, 1 query
+//    150 us, 1,024 queries 1.02 ms; ranks among all lists, quadratic, took 8.4 and 36 ms, the FP64 scores
+//    of every pair 0.22 and 0.78.
 constexpr uint32_t kProbePick = 512;
 constexpr uint32_t kProbeBand = 256;  // lists between the certain ones scored from shared memory
 
@@ -279,6 +283,7 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 8 : 1)
                           uint32_t* __restrict__ list_cnt, uint32_t* __restrict__ q_slot_off,
                           unsigned long long* __restrict__ counters, int no_plan) {
     __shared__ MergeScratch<NT> s;
+    __shared__ BlockSelectScratch sel;
     __shared__ uint64_t band_key[kProbeBand];
     __shared__ uint32_t picked[kProbePick], band[kProbeBand];
     __shared__ double norm_part[2][NT / 32];
@@ -327,16 +332,18 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 8 : 1)
         sh_err = static_cast<double>(nq) * static_cast<double>(c.x) * static_cast<double>(dp) * 4.5e-16;  // 2·2⁻⁵³·2
     }
     __syncthreads();
-    bool all_exact = !(sh_e2 <= FLT_MAX);  // no bound: every list by its exact score
+    const bool all_exact = !(sh_e2 <= FLT_MAX);  // no bound: every list by its exact score
     if (np < nlist && !all_exact) {
+        auto get = [&](uint32_t i) { return make_key(sq[i], i); };
         block_merge_best<NT>(
-            [&](uint32_t i) { return make_key(sq[i], i); }, nlist, np, s,
+            get, nlist, np, s,
             [&](uint32_t j, uint64_t key) {
                 if (j == np - 1) sh_l = key_score(key);
             },
-            [&]() {
-                all_exact = true;  // (mass ties)
-                return 0u;
+            [&]() {  // mass ties
+                const uint64_t kth = block_radix_kth_of(get, nlist, np, sel, 32);
+                if (tid == 0) sh_l = key_score(kth);
+                return np;
             });
         __syncthreads();
     }
@@ -367,19 +374,30 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 8 : 1)
         }
     } else {
         // too many to hold: their exact scores replace the approximate ones, the others' are set apart
-        for (uint32_t i0 = 0; i0 < nlist; i0 += NT / 8) {
-            const uint32_t i = i0 + tid / 8;
+        for (uint32_t i0 = tid & ~31u; i0 < nlist; i0 += NT) {  // 32 lists a warp, four of them at a time
+            const uint32_t lane = tid & 31u, i = i0 + lane;
             const bool maybe = i < nlist && (all_exact || (sq[i] <= hi && sq[i] >= lo));
-            const float x = dot_f64_row8(q_d, centroids + static_cast<uint64_t>(maybe ? i : 0) * ds, dp, sh_err, tid & 7u, maybe);
-            if (i < nlist && (tid & 7u) == 0) sq[i] = maybe ? fold_zero(x) : -FLT_MAX;
+            if (i < nlist && !maybe) sq[i] = -FLT_MAX;
+            uint32_t left = __ballot_sync(0xFFFFFFFFu, maybe);
+            while (left) {
+                uint32_t mine = left;  // the lane's list: the (lane / 8)-th that is left
+                for (uint32_t g = lane >> 3; g > 0; --g) mine &= mine - 1;
+                const bool on = mine != 0;
+                const uint32_t c = on ? i0 + __ffs(mine) - 1 : i0;
+                const float x = dot_f64_row8(q_d, centroids + static_cast<uint64_t>(c) * ds, dp, sh_err, lane & 7u, on);
+                if (on && (lane & 7u) == 0) sq[c] = fold_zero(x);
+                for (uint32_t g = 0; g < 4; ++g) left &= left - 1;
+            }
         }
         __syncthreads();
-        for (uint32_t i = tid; i < nlist; i += NT) {
-            if (sq[i] == -FLT_MAX) continue;
-            const uint64_t key = make_key(sq[i], i);
-            uint32_t rank = 0;
-            for (uint32_t j = 0; j < nlist; ++j) rank += (sq[j] != -FLT_MAX && make_key(sq[j], j) > key) ? 1u : 0u;
-            if (rank < r) picked[nin + rank] = i;
+        // their best r: the keys (score, list) are distinct, so exactly r reach the r-th
+        auto get = [&](uint32_t i) { return sq[i] == -FLT_MAX ? 0ull : make_key(sq[i], i); };
+        const uint64_t kth = block_radix_kth_of(get, nlist, r, sel);
+        for (uint32_t i0 = 0; i0 < nlist; i0 += NT) {
+            const uint32_t i = i0 + tid;
+            const bool take = i < nlist && get(i) >= kth;
+            const uint32_t a = warp_append(&n_in, take);
+            if (take && a < kProbePick) picked[a] = i;
         }
     }
     __syncthreads();
@@ -1098,15 +1116,18 @@ cudaError_t launch_probe(uint32_t pqb, const ProbeLaunch& a, bool no_plan, cudaS
         t.p.status = ix.w_status;
         if ((e = launch_scan_tc(t, kTcTf32, 3, s)) != cudaSuccess) return e;
         const size_t smem = a.ds * sizeof(double);
-        // a few lists: small blocks, of which many fit an SM
-        auto pick = a.np <= 64 ? ivf_probe_pick_kernel<128> : ivf_probe_pick_kernel<512>;
+        // A few lists: small blocks, of which many fit an SM; but a large block where the lists to look through
+        // are thousands and the queries too few to fill the SMs with small ones (8,192 lists: 1 query 82 us
+        // with 128 threads, 72 with 512; 256 queries 357 and 357; 1,024 queries 677 and 723).
+        const bool small = a.np <= 64 && (a.nlist <= 2048 || a.nq > 2 * static_cast<uint32_t>(ix.sm_count));
+        auto pick = small ? ivf_probe_pick_kernel<128> : ivf_probe_pick_kernel<512>;
         if (smem > 24 * 1024 &&
             (e = cudaFuncSetAttribute(pick, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))) != cudaSuccess)
             return e;
-        pick<<<a.nq, a.np <= 64 ? 128 : 512, smem, s>>>(a.scores, a.ct_stride, a.nlist, a.np, a.queries, a.ds, a.dp,
-                                                        ix.ivf->d_centroids, ix.ivf->d_cent_max, ix.tf32_c_norm(),
-                                                        a.offsets, a.probes, a.list_cnt, a.q_slot_off, a.counters,
-                                                        no_plan ? 1 : 0);
+        pick<<<a.nq, small ? 128 : 512, smem, s>>>(a.scores, a.ct_stride, a.nlist, a.np, a.queries, a.ds, a.dp,
+                                                   ix.ivf->d_centroids, ix.ivf->d_cent_max, ix.tf32_c_norm(),
+                                                   a.offsets, a.probes, a.list_cnt, a.q_slot_off, a.counters,
+                                                   no_plan ? 1 : 0);
         count_launch();
     } else {
         if ((a.nlist + kProbeCentroids - 1) / kProbeCentroids > 65535u) return cudaErrorInvalidValue;

@@ -151,17 +151,18 @@ struct BlockSelectScratch {
     unsigned long long kth;
 };
 
-// Exact k-th largest among keys[0..n) (global or shared), 1 <= k <= n. All threads of the block
-// call it; warp 0 resolves bins. Keys equal to 0 take part like any other key.
-NNDEX_DEVICE_INLINE uint64_t block_radix_kth(const uint64_t* keys, uint64_t n, uint32_t k, BlockSelectScratch& s) {
+// Exact k-th largest among the keys get(0 … n), 1 <= k <= n, or with low its bits from `low` (a multiple of 8)
+// up. All threads of the block call it; warp 0 resolves bins. Keys equal to 0 take part like any other key.
+template <class Get>
+NNDEX_DEVICE_INLINE uint64_t block_radix_kth_of(Get&& get, uint64_t n, uint32_t k, BlockSelectScratch& s, int low = 0) {
     uint64_t prefix = 0, mask = 0;
     uint32_t krem = k;
 #pragma unroll 1
-    for (int shift = 56; shift >= 0; shift -= 8) {
+    for (int shift = 56; shift >= low; shift -= 8) {
         for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s.hist[i] = 0;
         __syncthreads();
         for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint64_t key = keys[i];
+            const uint64_t key = get(i);
             if ((key & mask) == prefix) atomicAdd(&s.hist[(key >> shift) & 0xFFu], 1u);
         }
         __syncthreads();
@@ -185,7 +186,7 @@ NNDEX_DEVICE_INLINE uint64_t block_radix_kth(const uint64_t* keys, uint64_t n, u
             __syncthreads();
             uint64_t m = ~0ull;
             for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
-                const uint64_t key = keys[i];
+                const uint64_t key = get(i);
                 if ((key & mask) == prefix && key < m) m = key;
             }
             m = warp_min_u64(m);
@@ -195,6 +196,11 @@ NNDEX_DEVICE_INLINE uint64_t block_radix_kth(const uint64_t* keys, uint64_t n, u
         }
     }
     return prefix;
+}
+
+// The same of keys[0..n) in global or shared memory.
+NNDEX_DEVICE_INLINE uint64_t block_radix_kth(const uint64_t* keys, uint64_t n, uint32_t k, BlockSelectScratch& s) {
+    return block_radix_kth_of([&](uint64_t i) { return keys[i]; }, n, k, s);
 }
 
 // Bitonic sort of n (power of two, <= blockDim.x * 32) keys in shared memory, descending.
