@@ -789,12 +789,13 @@ __global__ void __launch_bounds__((kPairW + 1) * 32)
 // 4. Merge: per query, the k best keys of its slots, sorted; unused result slots (0, 0.0f).
 // ------------------------------------------------------------------------------------------
 // k ≤ kMergeBestK (block_merge_best).
-__global__ void __launch_bounds__(256)
+template <int NT>
+__global__ void __launch_bounds__(NT)
     ivf_merge_best_kernel(const uint64_t* __restrict__ ws, const uint32_t* __restrict__ q_slot_off, uint32_t slots,
                           uint32_t k, uint64_t* __restrict__ idx_out, float* __restrict__ sim_out, uint32_t* __restrict__ count_out,
                           const unsigned long long* __restrict__ counters,
                           unsigned long long* __restrict__ host_probed) {
-    __shared__ MergeScratch<256> s;
+    __shared__ MergeScratch<NT> s;
     const uint32_t q = blockIdx.x;
     // the plan's row totals for the statistics, into pinned memory
     if (host_probed && q == 0 && threadIdx.x < 3) host_probed[threadIdx.x] = counters[3 + threadIdx.x];
@@ -804,7 +805,7 @@ __global__ void __launch_bounds__(256)
     const uint32_t n = (q_slot_off ? q_slot_off[q + 1] - q_slot_off[q] : slots) * k;
     uint64_t* oi = idx_out + static_cast<uint64_t>(q) * k;
     float* os = sim_out + static_cast<uint64_t>(q) * k;
-    const uint32_t kk = block_merge_best<256>(
+    const uint32_t kk = block_merge_best<NT>(
         [&](uint32_t i) { return keys[i]; }, n, k, s,
         [&](uint32_t j, uint64_t key) {
             oi[j] = key_row(key);
@@ -1022,11 +1023,23 @@ cudaError_t launch_scan(const CUtensorMap& tmap, const IvfScanArgs& a, uint32_t 
     return cudaGetLastError();
 }
 
+void launch_ivf_merge_best(const IvfScratch& w, const uint32_t* q_slot_off, uint32_t slots, uint32_t nq, uint32_t k,
+                           uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, const unsigned long long* counters,
+                           unsigned long long* host_probed, cudaStream_t s) {
+    // The cut is the k-th largest of the threads' maxima, which about NT · ln(NT / (NT − k)) keys reach: with
+    // 256 threads twice k at 200, six times at 256 (more than the list holds).
+    if (k <= 128)
+        ivf_merge_best_kernel<256><<<nq, 256, 0, s>>>(w.d_ws, q_slot_off, slots, k, o_idx, o_sim, o_cnt, counters,
+                                                      host_probed);
+    else
+        ivf_merge_best_kernel<512><<<nq, 512, 0, s>>>(w.d_ws, q_slot_off, slots, k, o_idx, o_sim, o_cnt, counters,
+                                                      host_probed);
+}
+
 void launch_ivf_merge(const IvfScratch& w, uint32_t nq, uint32_t k, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
                       const unsigned long long* counters, unsigned long long* host_probed, cudaStream_t s) {
     if (k <= kMergeBestK) {
-        ivf_merge_best_kernel<<<nq, 256, 0, s>>>(w.d_ws, w.d_q_slot_off, 0, k, o_idx, o_sim, o_cnt, counters,
-                                                 host_probed);
+        launch_ivf_merge_best(w, w.d_q_slot_off, 0, nq, k, o_idx, o_sim, o_cnt, counters, host_probed, s);
     } else {
         uint32_t p2 = 1;
         while (p2 < k) p2 <<= 1;
@@ -1249,8 +1262,7 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
             ivf_scan_pair_kernel<<<dim3(chunks, np, nq), (kPairW + 1) * 32, psmem, s>>>(v.tmap_reordered, a, w.d_probes, np,
                                                                                        static_cast<uint32_t>(chunk));
             ix.scan_event_end(s, ev_a);
-            ivf_merge_best_kernel<<<nq, 256, 0, s>>>(w.d_ws, nullptr, np * chunks, k, o_idx, o_sim, o_cnt, w.d_counters,
-                                                     w.h_probed);
+            launch_ivf_merge_best(w, nullptr, np * chunks, nq, k, o_idx, o_sim, o_cnt, w.d_counters, w.h_probed, s);
             count_launch(2);
             if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "IVF scan launch");
             ix.stats.kernel_launches += 4;
