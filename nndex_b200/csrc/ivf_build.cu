@@ -33,6 +33,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <functional>
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -1314,8 +1315,11 @@ static cudaError_t ivf_enqueue_layout(CudaIndex& ix, IvfIndex& v) {
 // Once the layout has completed (v.h_offsets set): the longest list, the BF16 residual bound and
 // the tensor maps of the reordered copies.
 static int ivf_complete_layout(CudaIndex& ix, IvfIndex& v, unsigned int eps_bits) {
-    v.max_list = 0;
-    for (uint64_t c = 0; c < v.nlist; ++c) v.max_list = std::max<uint64_t>(v.max_list, v.h_offsets[c + 1] - v.h_offsets[c]);
+    v.longest_rows.assign(v.nlist + 1, 0);
+    for (uint64_t c = 0; c < v.nlist; ++c) v.longest_rows[c + 1] = v.h_offsets[c + 1] - v.h_offsets[c];
+    std::sort(v.longest_rows.begin() + 1, v.longest_rows.end(), std::greater<uint64_t>());
+    v.max_list = v.nlist ? v.longest_rows[1] : 0;
+    for (uint64_t c = 0; c < v.nlist; ++c) v.longest_rows[c + 1] += v.longest_rows[c];
     if (!encode_tmap_2d(&v.tmap_reordered, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, v.d_reordered, ix.ds, ix.rows_alloc,
                         ix.ds * sizeof(float), 32, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tmap_2d(&v.tmap_reordered16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, v.d_reordered16, v.kb16,

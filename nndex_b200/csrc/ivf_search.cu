@@ -1008,6 +1008,28 @@ size_t ivf_scan_smem(uint32_t qb, uint32_t dq, uint32_t cap) {
 // queries 151 / 205, 16 (512 pairs) 246 / 274, 32 431 / 377; 8 lists, 64 queries 355 / 327.
 constexpr uint64_t kPairLimit = 512;
 
+// Rows of a CTA that give every SM about two, for lists of average length.
+uint64_t pair_share(const CudaIndex& ix, uint64_t pairs) {
+    return pairs * (ix.rows / ix.ivf->nlist + 1) / (2 * static_cast<uint64_t>(ix.sm_count));
+}
+
+// Uneven lists: whether the pairs do without a plan at whatever lists the queries probe. A plan reads a list once
+// for 16 queries, the pairs once for each, so what they may read beyond average lists (the longest ones,
+// by every query) has to cost less than the plan, 40 to 50 us: 350 MB, about 33 us from L2. And a long
+// list is cut into at most 32 chunks, which must not outlast the rest: 2 MB each beyond an even share.
+// 400k × 128 in 512 lists, 16 probed, k = 10, plan / pairs: a quarter of the rows in one list, queries beside
+// it: 8 (400 MB) 110 / 116 us, 16 110 / 157, 32 154 / 237; half of them: 1 query (3.2 MB) 107 / 122, 32 201
+// / 367; list sizes by a power law: 4 queries (320 MB) 106 / 86, 16 107 / 140.
+constexpr uint64_t kPairExtraBytes = 350000000ull, kPairChunkBytes = 2ull << 20;
+
+bool pairs_even(const CudaIndex& ix, uint64_t nq, uint64_t np) {
+    const IvfIndex& v = *ix.ivf;
+    const uint64_t row = ix.ds * sizeof(float), longest = (v.max_list + 31) / 32;
+    const uint64_t most = v.longest_rows[np], average = np * ix.rows / v.nlist;
+    return (most - std::min(most, average)) * nq * row <= kPairExtraBytes &&
+           (longest <= pair_share(ix, nq * np) || longest * row <= kPairChunkBytes);
+}
+
 size_t ivf_pair_smem(uint32_t dq, uint32_t cap) {
     return 1024 + static_cast<size_t>(kStages) * kPairW * 16 * 128 + static_cast<size_t>(dq) * 4 +
            static_cast<size_t>(cap) * 8 + kPairW * 256 * 4 + 8 + 8 + kStages * 16 + 16;
@@ -1225,9 +1247,8 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
     // Small batches whose lists serve at most one query on average: (query, list, chunk) CTAs, no plan.
     // Chunks of as many 256 rows as give every SM about two (of the longest list at most 32).
     const uint64_t pairs = static_cast<uint64_t>(nq) * np;
-    if (pairs <= nlist && pairs <= kPairLimit && k <= kMergeBestK) {
-        const uint64_t rows_est = pairs * (ix.rows / nlist + 1);
-        uint64_t chunk = std::max<uint64_t>(rows_est / (2 * static_cast<uint64_t>(ix.sm_count)), (v.max_list + 31) / 32);
+    if (pairs <= nlist && pairs <= kPairLimit && k <= kMergeBestK && pairs_even(ix, nq, np)) {
+        uint64_t chunk = std::max<uint64_t>(pair_share(ix, pairs), (v.max_list + 31) / 32);
         chunk = std::max<uint64_t>(256, (chunk + 255) / 256 * 256);
         const uint32_t chunks = static_cast<uint32_t>(std::max<uint64_t>(1, (v.max_list + chunk - 1) / chunk));
         const uint32_t pcap = ((k + 2 * kPairW * 16) + 31) / 32 * 32;
