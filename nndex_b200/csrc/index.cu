@@ -681,7 +681,7 @@ int CudaIndex::enqueue_prep_queries(const float* d_raw, uint64_t n, int mode, in
         p.tf_collected = d_cnt2;
         p.tf_over = kSecondPassCap + 1;
         p.zero[1] = d_fbn;
-        p.zero_words[1] = 1;
+        p.zero_words[1] = 4;
     }
     if (path == 2 || path == 3 || path == 5) {
         const uint64_t nq_alloc = (n + 127) / 128 * 128;
@@ -1242,15 +1242,18 @@ bool CudaIndex::plan_fallback(int path, uint32_t n, uint32_t kcap, ScanPlan& pla
 // A host-buffer batch's listed queries, their number read where the batch was waited for: the two
 // launches, 8 us of a batch of 64 queries over 50k rows when none is listed, wait for one that is.
 int CudaIndex::finish_tf32(int path, uint32_t n, uint32_t kcap) {
-    stats.fp32_fallback_queries += h_fbn[0];
+    const uint32_t listed = path == 7 ? h_fbn[3] & 0xFFFFu : h_fbn[0];
+    stats.fp32_fallback_queries += listed;
     stats.certified = stats.fp32_fallback_queries == 0 ? 1u : 0u;
-    if (h_fbn[0] == 0) return NNDEX_OK;
+    if (listed == 0) return NNDEX_OK;
     ScanPlan plan;
     if (!plan_fallback(path, n, kcap, plan))
         return set_error(NNDEX_ERR_UNSUPPORTED, "cuda execution error: no FP32 scan plan for k=%u", kcap);
-    cudaError_t e = cudaMemcpyAsync(d_fbn, h_fbn, sizeof(uint32_t), cudaMemcpyHostToDevice, stream);
-    if (e != cudaSuccess) return cuda_error(e, "fallback count");
     int st;
+    if (path == 6) {  // counted in host memory
+        const cudaError_t e = cudaMemcpyAsync(d_fbn, h_fbn, sizeof(uint32_t), cudaMemcpyHostToDevice, stream);
+        if (e != cudaSuccess) return cuda_error(e, "fallback count");
+    }
     if ((st = enqueue_fp32_fallback(plan, n, kcap, d_idx, d_sim, d_cnt, stream))) return st;
     stats.kernel_launches += 2;
     if (!mapped_io) cudaMemcpyAsync(h_res, d_res, res_bytes, cudaMemcpyDeviceToHost, stream);
@@ -1319,9 +1322,15 @@ int CudaIndex::grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t k
 // The path a batch planned on the two-pass TF32 scan takes, decided before anything of it is enqueued. Without
 // memory for the collections: the FP32 scan, whose workspace is far smaller. What the attempt had grown
 // is given back, and the next batches do not try again (each try would free, allocate and drop
-// every captured graph).
+// every captured graph). Where most of a batch's collections overflowed (many rows within the bound of the k-th
+// score: copies of a few rows, tight clusters), the FP32 scan had nearly all of the work to do again, and
+// the next batches go to it likewise: 200k × 128, 8 distinct rows, 64 queries 306 us on the FP32 scan, 508
+// through both; 256 queries 746 and 1,557.
 int CudaIndex::settle_path(int* path, uint32_t n, uint32_t kcap) {
     if (*path != 7) return NNDEX_OK;
+    // what the last such batch to finish said of itself (a device-buffer batch may still be running)
+    const uint32_t last = __atomic_exchange_n(h_fbn + 3, 0u, __ATOMIC_RELAXED);
+    if (2 * (last & 0xFFFFu) > last >> 16) tf32_rest = kTf32Rest;
     if (tf32_rest) {
         --tf32_rest;
         *path = 1;
@@ -1437,7 +1446,7 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
     if (e != cudaSuccess) return cuda_error(e, "TF32 scan launch (pass 2)");
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, kSecondPassCap, kcap,
                                 d_kth, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, nullptr, nullptr, nullptr, nullptr,
-                                nullptr, d_fbq, host_fallback ? h_fbn : d_fbn);
+                                nullptr, OverflowList{d_fbq, d_fbn, d_fbn + 3, h_fbn + 3});
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
     if (!host_fallback) {
         if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;

@@ -284,7 +284,8 @@ struct CudaIndex {
     // scan, spare}), read back with the statistics.
     uint32_t* d_fbq = nullptr;  // the re-run queries' indices
     size_t cap_fbq = 0;
-    // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, spare, rows pass 2 collected (64 bits)}
+    // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, a ticket (host: what the last two-pass TF32 batch
+    // to finish listed, OverflowList), rows pass 2 collected (64 bits)}
     static constexpr size_t kFbnBytes = 6 * sizeof(uint32_t);
     uint32_t* d_fbn = nullptr;
     uint32_t* d_fbn_sum = nullptr;  // the word behind them: the first one summed over a device-buffer call's pieces

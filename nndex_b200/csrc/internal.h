@@ -353,7 +353,13 @@ cudaError_t launch_gather_queries(const uint32_t* ids, uint32_t m, const void* q
 // list-ordered copy by collected position. slot_keys: m × rerank_chunks(cap2) × k keys of scratch.
 // With fail (m positions in ids whose collections overflowed): the k-th exact score of the rows they
 // did collect is a higher T, written to kth (by query), and the queries to fail_ids; no results.
-// With over_ids: queries whose collection overflowed are appended there, counted in over_count.
+// With over.ids: queries whose collection overflowed are appended there.
+struct OverflowList {
+    uint32_t* ids = nullptr;
+    uint32_t* count = nullptr;   // their number, zeroed before
+    uint32_t* ticket = nullptr;  // a word zeroed before
+    uint32_t* host = nullptr;    // pinned: m << 16 | their number, once every query is done (m < 32,768)
+};
 uint32_t rerank_chunks(uint32_t cap2);
 cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float* queries, const uint32_t* ids,
                                     uint32_t m, const uint32_t* rows2, const uint32_t* cnt2, uint32_t cap2, uint32_t k,
@@ -361,7 +367,7 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
                                     uint32_t* cnt_out, uint32_t* ok_out, cudaStream_t stream, bool by_query = false,
                                     const uint32_t* live = nullptr, const uint32_t* row_map = nullptr,
                                     const uint32_t* fail = nullptr, float* kth = nullptr, uint32_t* fail_ids = nullptr,
-                                    uint32_t* over_ids = nullptr, uint32_t* over_count = nullptr);
+                                    const OverflowList& over = OverflowList{});
 cudaError_t launch_max_reduce(const float* v, uint64_t n, unsigned int* out, cudaStream_t stream);
 // FP8: {min, max} row scale of each 256-row tile (tiles = rows_alloc / 256).
 void launch_tile_scale(const float* row_scale, uint64_t rows, uint64_t tiles, float2* out, cudaStream_t s);

@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(256)
                         const uint64_t* __restrict__ slot_keys, uint32_t chunks, uint64_t* __restrict__ idx_out,
                         float* __restrict__ sim_out, uint32_t* __restrict__ cnt_out, uint32_t* __restrict__ ok_out,
                         const uint32_t* __restrict__ fail, float* __restrict__ kth, uint32_t* __restrict__ fail_ids,
-                        uint32_t* __restrict__ over_ids, uint32_t* __restrict__ over_count, uint32_t seg) {
+                        const OverflowList over, uint32_t seg) {
     extern __shared__ uint64_t keys[];  // chunks·k keys, at least p2(k)
     __shared__ BlockSelectScratch sel;
     const uint32_t i = blockIdx.x;
@@ -1244,13 +1244,17 @@ __global__ void __launch_bounds__(256)
     const uint32_t q = ids[at0];
     uint32_t total = cnt2[by_query ? q : at0];
     if (fail && total > cap2) total = cap2;
-    if (total > cap2) {  // the collected set overflowed: finish_tc raises the query's T, or re-runs it
-        if (threadIdx.x == 0) {
-            ok_out[i] = 0;
-            if (over_ids) over_ids[atomicAdd(over_count, 1u)] = q;
+    const bool overflowed = total > cap2;  // finish_tc raises the query's T, or re-runs it; or it is listed
+    if (threadIdx.x == 0) {
+        if (overflowed) ok_out[i] = 0;
+        if (over.ids) {
+            if (overflowed) over.ids[atomicAdd(over.count, 1u)] = q;
+            // the last of the queries tells the host how many there were and how many are listed
+            const uint32_t mine = 0x10000u | (overflowed ? 1u : 0u), before = atomicAdd(over.ticket, mine);
+            if (before >> 16 == gridDim.x - 1) *over.host = before + mine;
         }
-        return;
     }
+    if (overflowed) return;
     const uint32_t segs = (total + seg - 1) / seg, items = segs < chunks ? segs : chunks;
     const uint64_t* src = slot_keys + static_cast<size_t>(i) * chunks * k;
     if (threadIdx.x == 0) sel.count = 0;
@@ -1498,14 +1502,14 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
                                     const float* thr, uint64_t* slot_keys, uint64_t* idx_out, float* sim_out,
                                     uint32_t* cnt_out, uint32_t* ok_out, cudaStream_t stream, bool by_query,
                                     const uint32_t* live, const uint32_t* row_map, const uint32_t* fail, float* kth,
-                                    uint32_t* fail_ids, uint32_t* over_ids, uint32_t* over_count) {
+                                    uint32_t* fail_ids, const OverflowList& over) {
     if (m == 0) return cudaSuccess;
     const uint32_t chunks = rerank_chunks(cap2);
     // A small batch's collections are dealt over all of a query's items, 32 rows (one round of a block) at
     // a time: 37 queries of about 300 rows took 19.2 us in one item each and 4.7 so, 64 queries 9.3 -> 6.2.
     // A large batch fills the chip with whole items, which load the query and select their best once.
     const uint32_t seg = m <= 64 ? 32u : m <= 256 ? 128u : kRerankChunk;
-    if (k == 0 || k > kRerankChunk || chunks > 65535u) return cudaErrorInvalidValue;
+    if (k == 0 || k > kRerankChunk || chunks > 65535u || (over.ids && m > 0x7FFFu)) return cudaErrorInvalidValue;
     const size_t qsmem = static_cast<size_t>(ds) * sizeof(float);
     if (qsmem > 48 * 1024) {
         const cudaError_t ea = cudaFuncSetAttribute(rerank_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1521,7 +1525,7 @@ cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float*
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     kern<<<m, 256, smem, stream>>>(ids, cnt2, cap2, k, by_query ? 1 : 0, live, slot_keys, chunks, idx_out, sim_out,
-                                   cnt_out, ok_out, fail, kth, fail_ids, over_ids, over_count, seg);
+                                   cnt_out, ok_out, fail, kth, fail_ids, over, seg);
     count_launch(2);
     return cudaGetLastError();
 }
