@@ -202,6 +202,12 @@ struct CudaIndex {
     // The host's go on with two lists of an overflowed batch's queries, kFewIds each.
     static constexpr size_t kHostWordBytes = 4096;
     static constexpr uint32_t kFewIds = (kHostWordBytes - kWordBytes) / 8;
+    // Behind them: the queries and the results of batches up to kMappedIoBytes each.
+    static constexpr size_t kHostBytes = kHostWordBytes + 2 * kMappedIoBytes;
+    bool in_words(const void* p) const {
+        const uint8_t *at = static_cast<const uint8_t*>(p), *words = reinterpret_cast<const uint8_t*>(h_flags);
+        return words && at >= words && at < words + kHostBytes;
+    }
     void* d_mem = nullptr;  // the allocation with the device's words, and an owner's rows and copies
     unsigned long long* d_err = nullptr;
     uint32_t* d_status = nullptr;
@@ -213,7 +219,7 @@ struct CudaIndex {
         d_fbn_sum = d_fbn + kFbnBytes / sizeof(uint32_t);
         d_max = reinterpret_cast<unsigned int*>(at + kMaxAt);
     }
-    void* words_page = nullptr;  // the registered page with the host's words, if they are in one
+    void* words_page = nullptr;  // the registered memory with the host's words, if they are in such
     cudaError_t alloc_words();
     void free_words();
     // The current call's: d_err / d_status, or for a host-buffer search h_flags itself (the kernels
