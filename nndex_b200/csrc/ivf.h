@@ -36,6 +36,7 @@ struct IvfIndex {
     std::vector<uint64_t> h_offsets;
     std::vector<uint64_t> h_init_rows;  // rows chosen by k-means++ (diagnostics / parity)
     std::vector<uint64_t> longest_rows;  // nlist + 1: rows of the n longest lists
+    uint64_t own_list_rows = 0;          // rows of the list that a row lies in, on average over the rows
     uint64_t max_list = 0;
     CUtensorMap tmap_reordered{};
     // BF16 copy of the reordered rows for the tensor-core list scan: kb16 = dims rounded up to 64,

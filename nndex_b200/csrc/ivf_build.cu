@@ -673,10 +673,9 @@ __global__ void centroid_prep_kernel(const float* __restrict__ cent, uint32_t ds
 
 // ------------------------------------------------------------------------------------------
 // K5: assignment on the tensor cores. Persistent CTAs walk 128-row tiles; for each, every
-// 256-centroid tile is one M=128 × N=256 BF16 GEMM (K in 64-element slabs, A and B slabs staged
+// 256-centroid tile is one M=128 × N=256 FP16 GEMM (K in 64-element slabs, A and B slabs staged
 // together by TMA, 4-deep ring) into one of two TMEM accumulators; the epilogue keeps per row the
-// best approximate score (and its centroid) and the second best. Certified rows are assigned;
-// the others are queued for the exact pass.
+// best approximate score (pass A), or lists the centroids within the bound of it (pass B).
 // ------------------------------------------------------------------------------------------
 namespace {
 constexpr int kAsM = 128;
@@ -1267,8 +1266,7 @@ static cudaError_t ivf_alloc(const CudaIndex& ix, IvfIndex& v, BuildKeep* keep) 
 
 namespace {
 
-// Device scratch of one build, freed on every exit path.
-// Scratch of a build that does not fit the memory of its own result.
+// Scratch of a build that does not fit the memory of its own result, freed on every exit path.
 struct BuildScratch {
     void* p = nullptr;
     ~BuildScratch() { cudaFree(p); }
@@ -1319,6 +1317,9 @@ static int ivf_complete_layout(CudaIndex& ix, IvfIndex& v, unsigned int eps_bits
     for (uint64_t c = 0; c < v.nlist; ++c) v.longest_rows[c + 1] = v.h_offsets[c + 1] - v.h_offsets[c];
     std::sort(v.longest_rows.begin() + 1, v.longest_rows.end(), std::greater<uint64_t>());
     v.max_list = v.nlist ? v.longest_rows[1] : 0;
+    double squares = 0.0;
+    for (uint64_t c = 1; c <= v.nlist; ++c) squares += static_cast<double>(v.longest_rows[c]) * static_cast<double>(v.longest_rows[c]);
+    v.own_list_rows = static_cast<uint64_t>(squares / static_cast<double>(ix.rows));
     for (uint64_t c = 0; c < v.nlist; ++c) v.longest_rows[c + 1] += v.longest_rows[c];
     if (!encode_tmap_2d(&v.tmap_reordered, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, v.d_reordered, ix.ds, ix.rows_alloc,
                         ix.ds * sizeof(float), 32, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||

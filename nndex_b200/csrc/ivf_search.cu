@@ -1013,20 +1013,23 @@ uint64_t pair_share(const CudaIndex& ix, uint64_t pairs) {
     return pairs * (ix.rows / ix.ivf->nlist + 1) / (2 * static_cast<uint64_t>(ix.sm_count));
 }
 
-// Uneven lists: whether the pairs do without a plan at whatever lists the queries probe. A plan reads a list once
-// for 16 queries, the pairs once for each, so what they may read beyond average lists (the longest ones,
-// by every query) has to cost less than the plan, 40 to 50 us: 350 MB, about 33 us from L2. And a long
-// list is cut into at most 32 chunks, which must not outlast the rest: 2 MB each beyond an even share.
-// 400k × 128 in 512 lists, 16 probed, k = 10, plan / pairs: a quarter of the rows in one list, queries beside
-// it: 8 (400 MB) 110 / 116 us, 16 110 / 157, 32 154 / 237; half of them: 1 query (3.2 MB) 107 / 122, 32 201
-// / 367; list sizes by a power law: 4 queries (320 MB) 106 / 86, 16 107 / 140.
-constexpr uint64_t kPairExtraBytes = 350000000ull, kPairChunkBytes = 2ull << 20;
+// Uneven lists: whether the pairs do without a plan. A plan reads a list once for 16 queries, the pairs once for
+// each, so what they read beyond average lists has to cost no more than the plan, 40 to 60 us: 700 MB, about
+// 65 us from L2. Queries like the rows probe lists like the rows' own (own_list_rows), at most the longest
+// ones. And a long list is cut into at most 32 chunks, which must not outlast the rest: 2 MB each beyond an
+// even share. Plan / pairs, k = 10, queries beside the longest list: 400k × 128, 16 of 512 lists, a quarter
+// of the rows in one: 8 queries (400 MB) 110 / 116 us, 16 (800 MB) 110 / 157, 32 154 / 237; half of them, 1
+// query (3.2 MB a chunk) 107 / 122, 32 201 / 367; sizes by a power law: 4 queries (320 MB) 106 / 86, 16
+// (1.3 GB) 107 / 140. Lists of a Zipf mixture, queries of its own, k = 1: 1.56M × 366, 8 of 1,249 lists, 6
+// queries (120 MB) 184 / 123; 729k × 238, 32 of 853, 8 queries (270 MB) 159 / 120; 1.9M × 253, 32 of 1,370,
+// 16 queries (850 MB) 236 / 232.
+constexpr uint64_t kPairExtraBytes = 700000000ull, kPairChunkBytes = 2ull << 20;
 
 bool pairs_even(const CudaIndex& ix, uint64_t nq, uint64_t np) {
     const IvfIndex& v = *ix.ivf;
     const uint64_t row = ix.ds * sizeof(float), longest = (v.max_list + 31) / 32;
-    const uint64_t most = v.longest_rows[np], average = np * ix.rows / v.nlist;
-    return (most - std::min(most, average)) * nq * row <= kPairExtraBytes &&
+    const uint64_t likely = std::min(np * v.own_list_rows, v.longest_rows[np]), average = np * ix.rows / v.nlist;
+    return (likely - std::min(likely, average)) * nq * row <= kPairExtraBytes &&
            (longest <= pair_share(ix, nq * np) || longest * row <= kPairChunkBytes);
 }
 
@@ -1049,7 +1052,8 @@ void launch_ivf_merge_best(const IvfScratch& w, const uint32_t* q_slot_off, uint
                            uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, const unsigned long long* counters,
                            unsigned long long* host_probed, cudaStream_t s) {
     // The cut is the k-th largest of the threads' maxima, which about NT · ln(NT / (NT − k)) keys reach: with
-    // 256 threads twice k at 200, six times at 256 (more than the list holds).
+    // 256 threads twice k at 200, six times at 256 (more than the list holds). One query over 32 lists of
+    // 1M × 384, a call with 256 / 512 threads: k = 100 77 / 78 us, 130 82 / 76, 200 94 / 81, 256 194 / 84.
     if (k <= 128)
         ivf_merge_best_kernel<256><<<nq, 256, 0, s>>>(w.d_ws, q_slot_off, slots, k, o_idx, o_sim, o_cnt, counters,
                                                       host_probed);
@@ -1486,7 +1490,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
         a.p.gm_group = 8;
         a.p.gm_span = span;
         ix.scan_event_begin(s, ev_a);
-        e = launch_scan_tc(a, false, 2, s);
+        e = launch_scan_tc(a, kTcBf16, 2, s);
         ix.scan_event_end(s, ev_a);
         if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch");
         TcThresholdArgs t;
@@ -1522,7 +1526,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
         a.p.thr_global = ix.d_thr;
         a.p.ws_keys = w.d_ws;
         ix.scan_event_begin(s, ev_a);
-        e = launch_scan_tc(a, false, 0, s);
+        e = launch_scan_tc(a, kTcBf16, 0, s);
         ix.scan_event_end(s, ev_a);
         if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch");
         launch_ivf_merge(w, nq, kp, ix.d_cand_idx, ix.d_cand_sim, ix.d_cand_cnt, nullptr, nullptr, s);
@@ -1564,7 +1568,7 @@ int ivf_search_tc(CudaIndex& ix, uint32_t nq, uint32_t k, uint64_t* o_idx, float
     a.p.live_q = d_m;  // item mode: the whole pass returns at once when every query certified
     a.p.it_next = w.d_counters + 9;
     ix.scan_event_begin(s, ev_a);
-    e = launch_scan_tc(a, false, 1, s);
+    e = launch_scan_tc(a, kTcBf16, 1, s);
     ix.scan_event_end(s, ev_a);
     if (e != cudaSuccess) return cuda_error(e, "IVF tensor-core scan launch (pass 2)");
     e = launch_rerank_collected(v.d_reordered, static_cast<uint32_t>(ix.ds), ix.d_qn, ix.d_ids, nq, ix.d_rows2,
