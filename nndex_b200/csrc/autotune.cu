@@ -218,15 +218,12 @@ std::vector<CudaIndex::TunePlan> CudaIndex::tune_candidates(uint64_t nq, uint64_
 // whose largest k (or smallest batch) it may not hold, and an imported one may name a copy of the rows, or
 // their TF32 norms, that this index does not have.
 bool CudaIndex::plan_fits(const TunePlan& plan, uint64_t nq, uint64_t kcap) const {
-    ScanPlan rerun;
     switch (plan.path) {
         case 2: return tc_fits(kcap, false);
         case 3: return tc_fits(kcap, true);
         case 4: return uses_ivf();
         case 5: return uses_ivf() && ivf->d_reordered16;
-        case 6:
-            return plan_tf32(nq, kcap).kp &&
-                   plan_fallback(6, static_cast<uint32_t>(nq), static_cast<uint32_t>(kcap), rerun);
+        case 6: return plan_tf32(nq, kcap).kp != 0;
         case 7: return plan_tf32_batch(nq, kcap).kp != 0;
         default: return true;
     }
@@ -236,12 +233,21 @@ bool CudaIndex::plan_fits(const TunePlan& plan, uint64_t nq, uint64_t kcap) cons
 const CudaIndex::TuneEntry* CudaIndex::cached_plan(uint64_t nq, uint64_t kcap) const {
     if (!autotune) return nullptr;
     const auto it = tune_cache.find(tune_key(nq, kcap));
-    return it != tune_cache.end() && plan_fits(it->second.plan, nq, kcap) ? &it->second : nullptr;
+    if (it == tune_cache.end()) return nullptr;
+    // (the answer for the shape that asked last is kept: planning takes up to 10 us of the host's time)
+    const TuneEntry& e = it->second;
+    if (e.fit_nq != nq || e.fit_k != kcap || e.fit_width != rerank_width) {
+        e.fits = plan_fits(e.plan, nq, kcap);
+        e.fit_nq = nq;
+        e.fit_k = kcap;
+        e.fit_width = rerank_width;
+    }
+    return e.fits ? &e : nullptr;
 }
 
-CudaIndex::TunePlan CudaIndex::plan_for(uint64_t nq, uint64_t kcap, bool* measure) const {
+CudaIndex::TunePlan CudaIndex::plan_for(uint64_t nq, uint64_t kcap, bool* measure, const TuneEntry** cached) const {
     *measure = false;
-    if (const TuneEntry* ent = cached_plan(nq, kcap)) return ent->plan;
+    if ((*cached = cached_plan(nq, kcap))) return (*cached)->plan;
     // (a bucket whose plan does not fit this batch keeps it for the others)
     if (autotune == 1 && !tune_cache.count(tune_key(nq, kcap)) && tune_candidates(nq, kcap).size() > 1) *measure = true;
     return rule_plan(nq, kcap);
@@ -338,7 +344,8 @@ int nndex_cuda_autotune_path(const char* text, uint64_t rows, uint64_t dims, uin
     }
     if (row_norms) ix.d_tfnorm = reinterpret_cast<float2*>(16);
     bool measure = false;
-    *path = static_cast<uint32_t>(ix.plan_for(query_rows, std::min(k, rows), &measure).path);
+    const CudaIndex::TuneEntry* cached = nullptr;
+    *path = static_cast<uint32_t>(ix.plan_for(query_rows, std::min(k, rows), &measure, &cached).path);
     return NNDEX_OK;
 }
 

@@ -1256,7 +1256,8 @@ bool CudaIndex::plan_fallback(int path, uint32_t n, uint32_t kcap, ScanPlan& pla
 // A host-buffer batch's listed queries, their number read where the batch was waited for: the two
 // launches, 8 us of a batch of 64 queries over 50k rows when none is listed, wait for one that is.
 int CudaIndex::finish_tf32(int path, uint32_t n, uint32_t kcap) {
-    const uint32_t listed = path == 7 ? h_fbn[3] & 0xFFFFu : h_fbn[0];
+    const uint32_t listed = h_fbn[0] & 0xFFFFu;
+    if (path == 7 && 2 * listed > n) tf32_rest = kTf32Rest;  // (settle_path)
     stats.fp32_fallback_queries += listed;
     stats.certified = stats.fp32_fallback_queries == 0 ? 1u : 0u;
     if (listed == 0) return NNDEX_OK;
@@ -1342,7 +1343,7 @@ int CudaIndex::grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t k
 // through both; 256 queries 746 and 1,557.
 int CudaIndex::settle_path(int* path, uint32_t n, uint32_t kcap) {
     if (*path != 7) return NNDEX_OK;
-    // what the last such batch to finish said of itself (a device-buffer batch may still be running)
+    // what the last device-buffer batch to finish said of itself (one may still be running)
     const uint32_t last = __atomic_exchange_n(h_fbn + 3, 0u, __ATOMIC_RELAXED);
     if (2 * (last & 0xFFFFu) > last >> 16) tf32_rest = kTf32Rest;
     if (tf32_rest) {
@@ -1350,6 +1351,8 @@ int CudaIndex::settle_path(int* path, uint32_t n, uint32_t kcap) {
         *path = 1;
         return NNDEX_OK;
     }
+    if (settled_n == n && settled_k == kcap && settled_epoch == alloc_epoch()) return NNDEX_OK;
+    settled_n = 0;
     const Tf32BatchPlan plan = plan_tf32_batch(n, kcap);
     ScanPlan fb_plan;
     if (!plan.kp || !plan_fallback(7, n, kcap, fb_plan)) {
@@ -1367,6 +1370,11 @@ int CudaIndex::settle_path(int* path, uint32_t n, uint32_t kcap) {
                            at(d_cert, cap_cert),         at(d_kth, cap_kth),           at(d_rows2, cap_rows2),
                            at(d_ok2, cap_ok2),           at(d_rslots, cap_rslots),     at(d_fbq, cap_fbq)};
     const int st = grow_tf32_batch(plan, n, kcap, static_cast<uint64_t>(fb_plan.ctas_per_group) * kcap);
+    if (st == NNDEX_OK) {
+        settled_n = n;
+        settled_k = kcap;
+        settled_epoch = alloc_epoch();
+    }
     if (st != NNDEX_ERR_OUT_OF_MEMORY) return st;
     cudaGetLastError();
     clear_error();
@@ -1460,7 +1468,7 @@ int CudaIndex::enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, fl
     if (e != cudaSuccess) return cuda_error(e, "TF32 scan launch (pass 2)");
     e = launch_rerank_collected(d_base, static_cast<uint32_t>(ds), d_qn, d_ids, n, d_rows2, d_cnt2, kSecondPassCap, kcap,
                                 d_kth, d_rslots, o_idx, o_sim, o_cnt, d_ok2, s, false, nullptr, nullptr, nullptr, nullptr,
-                                nullptr, OverflowList{d_fbq, d_fbn, d_fbn + 3, h_fbn + 3});
+                                nullptr, OverflowList{d_fbq, d_fbn, d_fbn + 3, host_fallback ? h_fbn : h_fbn + 3});
     if (e != cudaSuccess) return cuda_error(e, "rerank launch (pass 2)");
     if (!host_fallback) {
         if ((st = enqueue_fp32_fallback(fb_plan, n, kcap, o_idx, o_sim, o_cnt, s))) return st;
@@ -1702,12 +1710,13 @@ int CudaIndex::search_host(const float* queries, uint64_t nq, uint64_t k, int mo
         }
         std::memcpy(h_q, queries + q0 * dims, n * dims * sizeof(float));
         bool measure = false;
-        TunePlan plan = plan_for(n, kcap, &measure);
+        const TuneEntry* cached = nullptr;
+        TunePlan plan = plan_for(n, kcap, &measure, &cached);
         if (measure) {
             if ((st = tune_host(n, kcap, mode, &plan))) return st;
-        } else if (const TuneEntry* ent = cached_plan(n, kcap)) {
+        } else if (cached) {
             stats.tuned = 2;
-            stats.tune_candidates = ent->candidates;
+            stats.tune_candidates = cached->candidates;
         }
         int path = plan.path;
         if ((st = settle_path(&path, static_cast<uint32_t>(n), static_cast<uint32_t>(kcap)))) return st;
@@ -1807,7 +1816,8 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
         uint32_t* oc = d_cnt_out ? d_cnt_out + q0 : nullptr;
         const float* dq = d_queries + q0 * dims;
         bool measure = false;
-        TunePlan plan = plan_for(n, kcap, &measure);
+        const TuneEntry* cached = nullptr;
+        TunePlan plan = plan_for(n, kcap, &measure, &cached);
         if (measure) {
             // the first batch of this shape: time every candidate plan on it, keep the fastest
             std::vector<TunePlan> cands = tune_candidates(n, kcap);
@@ -1850,9 +1860,9 @@ int CudaIndex::search_device(const float* d_queries, uint64_t nq, uint64_t k, ui
             stats.tune_candidates = ent.candidates;
             plan = ent.plan;
             synced = true;
-        } else if (const TuneEntry* ent = cached_plan(n, kcap)) {
+        } else if (cached) {
             stats.tuned = 2;
-            stats.tune_candidates = ent->candidates;
+            stats.tune_candidates = cached->candidates;
         }
         forced_stride = plan.stride;
         forced_qb = plan.qb;

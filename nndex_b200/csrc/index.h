@@ -21,12 +21,13 @@ constexpr uint32_t kSecondPassCap = 8192;
 // Host-buffer batches up to this size, queries and results each, run without copies.
 constexpr size_t kMappedIoBytes = 64 << 10;
 
-// FP32 batches take the two-pass TF32 scan from this much work (rows × stored dims × queries). Its nine
-// launches cost about 45 us whatever the batch, the FP32 scan's FMAs about 20 us per 1e8 beyond its own
-// 50. Batches in a row through device buffers, FP32 scan against two-pass scan: 50k × 128 with 17
-// queries (1.1e8) 61 / 70 us, 32 (2.0e8) 66 / 71, 64 (4.1e8) 94 / 72, 256 (1.6e9) 216 / 78;
-// 5k × 768, 32 queries (1.2e8) 67 / 80; 300k × 100, 37 queries 232 / 111; 1M × 768, 256 queries
-// 11,410 / 962.
+// FP32 batches take the two-pass TF32 scan from this much work (rows × stored dims × queries). Its launches
+// (six on host buffers, eight on device buffers) take 50 to 70 us whatever the batch, the FP32 scan's FMAs
+// about 10 us per 1e8 beyond its own 40. Device-buffer batches in a row, FP32 scan / two-pass scan, k = 10:
+// 50k × 128 with 32 queries (2.0e8) 52 / 57 us, 40 (2.6e8) 62 / 56 (k = 100: 72 / 72), 64 (4.1e8) 72 / 56,
+// 256 (1.6e9) 189 / 66; 5k × 768 with 64 (2.5e8) 54 / 71, 128 (4.9e8) 76 / 70; 20k × 64, 128 queries (1.6e8)
+// 56 / 56; 300k × 100, 37 queries 203 / 82; 1M × 768, 256 queries 11,285 / 857. On host buffers, where two of
+// the launches wait for a listed query, it already wins below the line (50k × 128, 32 queries 80 / 70).
 constexpr uint64_t kTf32BatchMinWork = 250000000ull;
 
 // After a batch that the two-pass TF32 scan could not serve, this many go to the FP32 scan before it is tried
@@ -290,8 +291,8 @@ struct CudaIndex {
     // scan, spare}), read back with the statistics.
     uint32_t* d_fbq = nullptr;  // the re-run queries' indices
     size_t cap_fbq = 0;
-    // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, a ticket (host: what the last two-pass TF32 batch
-    // to finish listed, OverflowList), rows pass 2 collected (64 bits)}
+    // {TF32 re-runs, TC pass-2 queries, TC pass-2 overflows, a ticket (host: what the last device-buffer batch of
+    // the two-pass TF32 scan listed, OverflowList), rows pass 2 collected (64 bits)}
     static constexpr size_t kFbnBytes = 6 * sizeof(uint32_t);
     uint32_t* d_fbn = nullptr;
     uint32_t* d_fbn_sum = nullptr;  // the word behind them: the first one summed over a device-buffer call's pieces
@@ -367,15 +368,18 @@ struct CudaIndex {
         TunePlan plan;
         double ms = 0.0;      // its wall time per batch when measured
         uint32_t candidates = 0;
+        mutable uint64_t fit_nq = 0, fit_k = 0;  // the shape (and rerank width) that `fits` was last asked for
+        mutable uint32_t fit_width = 0;
+        mutable bool fits = false;
     };
     int autotune = 1;  // 0 = rules only, 1 = measure once per shape, 2 = cached plans, else rules
     std::map<uint64_t, TuneEntry> tune_cache;
     uint64_t tune_key(uint64_t nq, uint64_t kcap) const;
     std::vector<TunePlan> tune_candidates(uint64_t nq, uint64_t kcap) const;
     TunePlan rule_plan(uint64_t nq, uint64_t kcap) const;
-    // The plan for a batch: cached, or by the rules; *measure when the tuner should time the
+    // The plan for a batch: cached (*cached), or by the rules; *measure when the tuner should time the
     // candidates on this batch first.
-    TunePlan plan_for(uint64_t nq, uint64_t kcap, bool* measure) const;
+    TunePlan plan_for(uint64_t nq, uint64_t kcap, bool* measure, const TuneEntry** cached) const;
     const TuneEntry* cached_plan(uint64_t nq, uint64_t kcap) const;
     bool plan_fits(const TunePlan& plan, uint64_t nq, uint64_t kcap) const;
     bool tc_fits(uint64_t kcap, bool fp8) const;
@@ -417,6 +421,9 @@ struct CudaIndex {
     int enqueue_tf32(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
     int enqueue_tf32_batch(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
     int settle_path(int* path, uint32_t n, uint32_t kcap);
+    // the shape that settle_path last had the buffers for; they are still there while nothing was reallocated
+    uint32_t settled_n = 0, settled_k = 0;
+    uint64_t settled_epoch = 0;
     uint32_t tf32_rest = 0;  // batches of the two-pass TF32 scan's shapes still to go to the FP32 scan
     int grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t kcap, uint64_t fb_keys);
     // The FP32 scan of the d_fbn[0] queries listed in d_fbq, into their own output rows (enqueued

@@ -358,7 +358,7 @@ struct OverflowList {
     uint32_t* ids = nullptr;
     uint32_t* count = nullptr;   // their number, zeroed before
     uint32_t* ticket = nullptr;  // a word zeroed before
-    uint32_t* host = nullptr;    // pinned: m << 16 | their number, once every query is done (m < 32,768)
+    uint32_t* host = nullptr;    // pinned: m << 16 | their number, once every query is done, unless it is 0 (m < 32,768)
 };
 uint32_t rerank_chunks(uint32_t cap2);
 cudaError_t launch_rerank_collected(const float* vecs, uint32_t ds, const float* queries, const uint32_t* ids,

@@ -1225,7 +1225,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // Per uncertified query i: the best k over its items' slots, sorted, into the query's outputs (a
-// collection that overflowed its buffer marks the query for the FP32 scan instead).
+// collection that overflowed its buffer marks the query instead, or lists it in `over`).
 // Latency for a small batch: with the selection and the sort, 37 queries at k = 33 took 13.4 us from 16
 // items' keys, 10.5 with ranks; 4,096 queries at k = 10 44 -> 19.
 constexpr uint32_t kMergeRanked = 512;  // up to so many keys are put in order by their ranks
@@ -1244,14 +1244,14 @@ __global__ void __launch_bounds__(256)
     const uint32_t q = ids[at0];
     uint32_t total = cnt2[by_query ? q : at0];
     if (fail && total > cap2) total = cap2;
-    const bool overflowed = total > cap2;  // finish_tc raises the query's T, or re-runs it; or it is listed
+    const bool overflowed = total > cap2;  // the host raises the query's T or re-runs it; or it is listed
     if (threadIdx.x == 0) {
         if (overflowed) ok_out[i] = 0;
         if (over.ids) {
             if (overflowed) over.ids[atomicAdd(over.count, 1u)] = q;
-            // the last of the queries tells the host how many there were and how many are listed
-            const uint32_t mine = 0x10000u | (overflowed ? 1u : 0u), before = atomicAdd(over.ticket, mine);
-            if (before >> 16 == gridDim.x - 1) *over.host = before + mine;
+            // the last of the queries tells the host how many there were and how many are listed, if any is
+            const uint32_t mine = 0x10000u | (overflowed ? 1u : 0u), all = atomicAdd(over.ticket, mine) + mine;
+            if (all >> 16 == gridDim.x && (all & 0xFFFFu)) *over.host = all;
         }
     }
     if (overflowed) return;
