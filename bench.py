@@ -652,9 +652,9 @@ def run_mixed(args, dev, L, world):
     os_ = torch.empty((nq, k), dtype=torch.float32, device=dev)
     stats = _lib.SearchStats()
     out = {}
-    # The FP32 arm is the plain FP32 scan (the index's own choice for FP32 batches of this size is the
-    # TF32 scan with FP32 rerank): a plan in the tuner's cache, with --mixed-stride / --mixed-qb also the
-    # given stride and blocks for both low precisions.
+    # The FP32 arm is the plain FP32 scan, by a plan in the tuner's cache (with --mixed-stride / --mixed-qb also
+    # the given stride and blocks for both low precisions). What the index itself chooses for FP32 batches of
+    # this size, the two-pass TF32 scan with FP32 rerank, is an arm of its own.
     n = C.c_uint64(0)
     L.nndex_cuda_autotune_export(h, None, 0, C.byref(n))
     buf = C.create_string_buffer(n.value)
@@ -668,8 +668,11 @@ def run_mixed(args, dev, L, world):
         raise RuntimeError(_lib.last_error())
     sample = min(args.mixed_oracle_queries, nq)
     ref_i, ref_s = fp64_topk(base, q[:sample], k)
-    for name, prec in (("fp32", NNDEX_PRECISION_FP32), ("bf16", NNDEX_PRECISION_BF16), ("fp8", NNDEX_PRECISION_FP8)):
+    for name, prec in (("fp32", NNDEX_PRECISION_FP32), ("fp32_chosen", NNDEX_PRECISION_FP32),
+                       ("bf16", NNDEX_PRECISION_BF16), ("fp8", NNDEX_PRECISION_FP8)):
         L.nndex_cuda_set_precision(h, prec, 0)
+        # "fp32_chosen": FP32 by the index's own choice, without the plan that holds it to the FP32 scan
+        L.nndex_cuda_set_autotune(h, 0 if name == "fp32_chosen" else 1)
         steps = max(1, min(args.mixed_steps, 2 if name == "fp32" else args.mixed_steps))
         for _ in range(2):  # warm-up (the second also runs with the autotuned k′)
             if L.nndex_cuda_search_batch_device(h, q.data_ptr(), nq, dims, k, oi.data_ptr(), os_.data_ptr(), None,
@@ -690,7 +693,7 @@ def run_mixed(args, dev, L, world):
                                                 sptr, 1) != 0:
                 raise RuntimeError(_lib.last_error())
             L.nndex_cuda_last_search_stats(h, C.byref(stats))
-            if stats.path in (2, 3):
+            if stats.path in (2, 3, 7):
                 second += stats.second_pass_queries
                 fallbacks += stats.fp32_fallback_queries
                 p2rows += stats.pass2_rows
@@ -715,6 +718,7 @@ def run_mixed(args, dev, L, world):
             h, q.data_ptr(), nq, dims, k, oi.data_ptr(), os_.data_ptr(), None, sptr, 1))
         scan_total = scan_ms.value  # all scan-kernel launches of the timed batches
         out[name] = {
+            "path": int(stats.path),
             "queries_per_s": total_q / (max_ms / 1e3),
             "ms_per_batch": max_ms / steps,
             "scan_ms_per_batch": scan_total / steps,
@@ -735,15 +739,17 @@ def run_mixed(args, dev, L, world):
     del base
     torch.cuda.empty_cache()
     fp32 = out["fp32"]["queries_per_s"]
+    chosen = out["fp32_chosen"]["queries_per_s"]
     for name in ("bf16", "fp8"):
         out[name]["speedup_vs_fp32"] = out[name]["queries_per_s"] / fp32
+        out[name]["speedup_vs_fp32_chosen"] = out[name]["queries_per_s"] / chosen
     bf16_peak = measured_bf16_peak()
     bf16_sus = measured_bf16_peak(sustained=True)
     alg = {name: out[name]["algorithmic_tflops"] for name in ("bf16", "fp8")}
     return {
         "workload": f"exact top-{k}, base {rows}x{dims} ({args.mixed_centers}-centre Gaussian mixture, "
                     f"sigma={args.mixed_sigma}, unit rows), batch {nq}; BF16/FP8 tensor-core scan + FP32 rerank "
-                    f"vs the FP32 scan; recall on {sample} queries vs a float64 brute force",
+                    f"vs the FP32 scan and vs the index's own FP32 path; recall on {sample} queries vs a float64 brute force",
         "results": out,
         "roofline": {"bound": "tensor", "kernel": "scan_tc_kernel",
                      "flops": "algorithmic 2*N*D*batch per batch, over the whole batch time (both passes, "

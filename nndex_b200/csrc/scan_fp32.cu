@@ -171,7 +171,7 @@ __global__ void __launch_bounds__((W + 1) * 32, 1)
                           uint32_t dq, uint64_t rows, uint32_t k, uint32_t cap,
                           const uint32_t* __restrict__ row_map, uint64_t* __restrict__ ws_keys,
                           uint32_t* __restrict__ status, const uint32_t* __restrict__ live,
-                     const uint32_t* __restrict__ ids) {
+                          const uint32_t* __restrict__ ids) {
     if (live) {  // a fallback launch: only the queries to re-run
         if (*live < nq) nq = *live;
         if (blockIdx.y * QB >= nq) return;
