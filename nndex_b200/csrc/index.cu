@@ -1039,12 +1039,33 @@ int CudaIndex::finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_si
     stats.pass2_rows += h_fbn_rows();
     if (failed_n == 0) return NNDEX_OK;
     std::vector<uint32_t> failed;
-    if ((st = retry_tc_pass2(stats.path == 3, failed_n, kcap, o_idx, o_sim, o_cnt, s, &failed))) return st;
+    if (tc_retry_rest) {
+        --tc_retry_rest;
+        if ((st = overflowed_queries(m, failed_n, s, &failed))) return st;
+    } else {
+        if ((st = retry_tc_pass2(stats.path == 3, failed_n, kcap, o_idx, o_sim, o_cnt, s, &failed))) return st;
+        // in vain for most: more rows tie with the k-th score than a collection holds, as they will next time
+        if (2 * failed.size() > failed_n) tc_retry_rest = kTcRetryRest;
+    }
     tc_patched = true;
     stats.fp32_fallback_queries += static_cast<uint32_t>(failed.size());
     if (failed.empty()) return NNDEX_OK;
     // ---- the FP32 scan for queries whose collected set overflowed again ----
     return rerun_exact_fp32(failed, kcap, o_idx, o_sim, o_cnt, s);
+}
+
+// The queries whose collection overflowed, without another pass.
+int CudaIndex::overflowed_queries(uint32_t m, uint32_t failed_n, cudaStream_t s, std::vector<uint32_t>* failed) {
+    int st;
+    if ((st = grow_host(h_ids, cap_hids, m, "pinned buffer"))) return st;
+    if ((st = grow_host(h_ok2, cap_hok2, failed_n, "pinned buffer"))) return st;
+    cudaMemcpyAsync(h_ids, d_ids, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(h_ok2, d_tcfail, failed_n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_error(e, "search");
+    failed->resize(failed_n);
+    for (uint32_t i = 0; i < failed_n; ++i) (*failed)[i] = h_ids[h_ok2[i]];
+    return NNDEX_OK;
 }
 
 // A collection overflows when T is far below the query's true k-th score (a sampled pass 1, or FP8's
