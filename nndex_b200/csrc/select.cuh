@@ -227,9 +227,9 @@ NNDEX_DEVICE_INLINE void block_bitonic_sort_desc(uint64_t* a, uint32_t n) {
 //
 // Each thread keeps the largest of the keys it reads (dealt round-robin); the k-th largest score of these
 // maxima, found bit by bit with a block-wide count, is a cut that at least k keys reach and hardly more
-// do, so one more read lists about k keys, and their ranks among themselves place them. Exact whatever
-// the keys: only a list that does not hold every key that reaches the cut (mass ties) sends the block to
-// `overflow`.
+// do, so one more read lists about k keys, and their ranks among themselves place them. Scores tied with
+// the cut by the thousand take the row's part of the key into it. Exact whatever the keys: only a list that
+// does not hold every key that reaches the cut even so sends the block to `overflow`.
 template <int NT>
 struct MergeScratch {
     static constexpr uint32_t kList = 1024;
@@ -260,21 +260,38 @@ NNDEX_DEVICE_INLINE uint32_t block_merge_best(Get&& get, uint32_t n, uint32_t k,
         const uint32_t t = score | (1u << bit);
         if (static_cast<uint32_t>(__syncthreads_count(top >= t)) >= k) score = t;
     }
-    const uint64_t cut = score ? static_cast<uint64_t>(score) << 32 : 1ull;  // fewer keys than that: all of them
-    for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
-        if (n > U * NT) {
+    uint64_t cut = score ? static_cast<uint64_t>(score) << 32 : 1ull;  // fewer keys than that: all of them
+    auto list = [&]() {
+        for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
+            if (n > U * NT) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? get(i0 + u * NT + tid) : 0ull;
-        }
+                for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? get(i0 + u * NT + tid) : 0ull;
+            }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const bool take = x[u] >= cut;
-            const uint32_t at = warp_append(&s.count, take);
-            if (take && at < MergeScratch<NT>::kList) s.list[at] = x[u];
+            for (int u = 0; u < U; ++u) {
+                const bool take = x[u] >= cut;
+                const uint32_t at = warp_append(&s.count, take);
+                if (take && at < MergeScratch<NT>::kList) s.list[at] = x[u];
+            }
         }
+        __syncthreads();
+        return s.count;
+    };
+    uint32_t c = list();
+    if (c > MergeScratch<NT>::kList && score) {
+        // more keys tie with the cut's score than the list holds: the rest of the key decides, like the score
+        const uint32_t low = static_cast<uint32_t>(best);
+        uint32_t rest = 0;
+#pragma unroll 1
+        for (int bit = 31; bit >= 0; --bit) {
+            const uint32_t t = rest | (1u << bit);
+            if (static_cast<uint32_t>(__syncthreads_count(top > score || (top == score && low >= t))) >= k) rest = t;
+        }
+        cut |= rest;
+        if (tid == 0) s.count = 0;
+        __syncthreads();
+        c = list();
     }
-    __syncthreads();
-    const uint32_t c = s.count;
     if (c > MergeScratch<NT>::kList) {
         __syncthreads();
         return overflow();
