@@ -236,11 +236,12 @@ const CudaIndex::TuneEntry* CudaIndex::cached_plan(uint64_t nq, uint64_t kcap) c
     if (it == tune_cache.end()) return nullptr;
     // (the answer for the shape that asked last is kept: planning takes up to 10 us of the host's time)
     const TuneEntry& e = it->second;
-    if (e.fit_nq != nq || e.fit_k != kcap || e.fit_width != rerank_width) {
+    if (e.fit_nq != nq || e.fit_k != kcap || e.fit_width != rerank_width || e.fit_host != host_fallback) {
         e.fits = plan_fits(e.plan, nq, kcap);
         e.fit_nq = nq;
         e.fit_k = kcap;
         e.fit_width = rerank_width;
+        e.fit_host = host_fallback;
     }
     return e.fits ? &e : nullptr;
 }

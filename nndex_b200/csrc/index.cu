@@ -546,7 +546,6 @@ CudaIndex::Tf32BatchPlan CudaIndex::plan_tf32_batch(uint64_t nq, uint64_t kcap) 
         return v && v[0] == '0';
     }();
     if (off || !d_tfnorm || nq < 17 || kcap == 0 || kcap > kMaxGroupCandidates / 2) return p;
-    if (rows * ds * nq < kTf32BatchMinWork) return p;
     const uint64_t kp = std::min<uint64_t>(rows, std::max<uint64_t>(32, 2 * kcap));
     // Pass 1 on every stride-th tile: few enough that the groups of 8 rows are at least 16 per
     // candidate, and that pass 2 collects about stride × k ≤ 2,048 rows per query.
@@ -556,6 +555,7 @@ CudaIndex::Tf32BatchPlan CudaIndex::plan_tf32_batch(uint64_t nq, uint64_t kcap) 
                           (stride > 8 && tiles < 16384)))
         stride /= 2;
     if (tiles * 32 < 4 * kp) return p;
+    if (rows * nq * (ds + 64) < tf32_batch_costs(rows, ds, nq, kcap, stride, host_fallback)) return p;
     const uint32_t nchunks = static_cast<uint32_t>(ds / 32);
     bool stream_a = false;
     const uint32_t stages = tc_tf32_stages_for(nchunks, smem_optin, &stream_a);
@@ -1372,7 +1372,8 @@ int CudaIndex::settle_path(int* path, uint32_t n, uint32_t kcap) {
         *path = 1;
         return NNDEX_OK;
     }
-    if (settled_n == n && settled_k == kcap && settled_epoch == alloc_epoch()) return NNDEX_OK;
+    if (settled_n == n && settled_k == kcap && settled_host == host_fallback && settled_epoch == alloc_epoch())
+        return NNDEX_OK;
     settled_n = 0;
     const Tf32BatchPlan plan = plan_tf32_batch(n, kcap);
     ScanPlan fb_plan;
@@ -1394,6 +1395,7 @@ int CudaIndex::settle_path(int* path, uint32_t n, uint32_t kcap) {
     if (st == NNDEX_OK) {
         settled_n = n;
         settled_k = kcap;
+        settled_host = host_fallback;
         settled_epoch = alloc_epoch();
     }
     if (st != NNDEX_ERR_OUT_OF_MEMORY) return st;

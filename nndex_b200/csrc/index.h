@@ -21,14 +21,20 @@ constexpr uint32_t kSecondPassCap = 8192;
 // Host-buffer batches up to this size, queries and results each, run without copies.
 constexpr size_t kMappedIoBytes = 64 << 10;
 
-// FP32 batches take the two-pass TF32 scan from this much work (rows × stored dims × queries). Its launches
-// (six on host buffers, eight on device buffers) take 50 to 70 us whatever the batch, the FP32 scan's FMAs
-// about 10 us per 1e8 beyond its own 40. Device-buffer batches in a row, FP32 scan / two-pass scan, k = 10:
-// 50k × 128 with 32 queries (2.0e8) 52 / 57 us, 40 (2.6e8) 62 / 56 (k = 100: 72 / 72), 64 (4.1e8) 72 / 56,
-// 256 (1.6e9) 189 / 66; 5k × 768 with 64 (2.5e8) 54 / 71, 128 (4.9e8) 76 / 70; 20k × 64, 128 queries (1.6e8)
-// 56 / 56; 300k × 100, 37 queries 203 / 82; 1M × 768, 256 queries 11,285 / 857. On host buffers, where two of
-// the launches wait for a listed query, it already wins below the line (50k × 128, 32 queries 80 / 70).
-constexpr uint64_t kTf32BatchMinWork = 250000000ull;
+// FP32 batches take the two-pass TF32 scan where the FP32 scan's work, rows × queries × (stored dims + 64), is at
+// least what the other's parts cost in the same measure (about 8 us per 1e8): its launches, beyond the FP32
+// scan's; the rows that a query's threshold and rerank gather, k × dims; a query's blocks; and, of a base beyond
+// L2, the rows that pass 1 reads besides. A host-buffer batch has two launches fewer (its listed queries wait
+// until there is one) and waits in any case. Fitted to 1,600 batches of 1,000 to 1M rows × 32 to 1,536 dims, 17
+// to 9,000 queries, k of 1 to 256 on normal rows: by this line 10 of them (host: 10) take more than 5 % longer
+// than on the FP32 scan, 45 (26) could have been 5 % faster on the other side; by 2.5e8 multiply-adds alone 158
+// took longer, up to 2.4 times as long. FP32 / two-pass scan, device buffers: 50k × 128, k = 10, 32 queries
+// 52 / 57 us, 40 62 / 56, 256 189 / 66; 1,200 × 128, 1,628 queries 85 / 144; 20k × 512, 25 queries, k = 10 72 / 76,
+// k = 256 83 / 132; 100k × 512, 32 queries, k = 10 154 / 116, k = 256 187 / 244; 1M × 768, 256 queries 11,285 / 857.
+inline uint64_t tf32_batch_costs(uint64_t rows, uint64_t ds, uint64_t nq, uint64_t k, uint64_t stride, bool host) {
+    const uint64_t again = rows * ds * sizeof(float) > (126ull << 20) ? rows * ds / stride * 8 : 0;
+    return (host ? 80000000ull : 290000000ull) + k * ds * 10000 + nq * (host ? 300000 : 600000) + again;
+}
 
 // After a batch that the two-pass TF32 scan could not serve, this many go to the FP32 scan before it is tried
 // again: a batch that tries in vain costs at most about twice the FP32 scan, so 3 % over 32.
@@ -373,9 +379,9 @@ struct CudaIndex {
         TunePlan plan;
         double ms = 0.0;      // its wall time per batch when measured
         uint32_t candidates = 0;
-        mutable uint64_t fit_nq = 0, fit_k = 0;  // the shape (and rerank width) that `fits` was last asked for
+        mutable uint64_t fit_nq = 0, fit_k = 0;  // the batch (and rerank width) that `fits` was last asked for
         mutable uint32_t fit_width = 0;
-        mutable bool fits = false;
+        mutable bool fit_host = false, fits = false;
     };
     int autotune = 1;  // 0 = rules only, 1 = measure once per shape, 2 = cached plans, else rules
     std::map<uint64_t, TuneEntry> tune_cache;
@@ -431,6 +437,7 @@ struct CudaIndex {
     // the shape that settle_path last had the buffers for; they are still there while nothing was reallocated
     uint32_t settled_n = 0, settled_k = 0;
     uint64_t settled_epoch = 0;
+    bool settled_host = false;
     uint32_t tf32_rest = 0;  // batches of the two-pass TF32 scan's shapes still to go to the FP32 scan
     int grow_tf32_batch(const Tf32BatchPlan& plan, uint32_t n, uint32_t kcap, uint64_t fb_keys);
     // The FP32 scan of the d_fbn[0] queries listed in d_fbq, into their own output rows (enqueued

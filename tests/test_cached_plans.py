@@ -57,6 +57,15 @@ def test_low_precision_plans_need_their_copy_and_room_for_k():
     assert held[0] and not held[-1] and sorted(held, reverse=True) == held
 
 
+@pytest.mark.parametrize("rows,dims,nq,k,path", [
+    (1_200, 128, 1_628, 10, 1), (1_200, 512, 652, 10, 1), (2_500, 32, 5_001, 10, 1),   # few rows for many queries
+    (20_000, 512, 25, 256, 1), (100_000, 512, 32, 256, 1), (10_000, 512, 79, 100, 1),  # few queries, much to gather
+    (100_000, 512, 32, 10, 7), (100_000, 128, 63, 256, 7), (40_000, 128, 157, 100, 7), (5_000, 512, 626, 10, 7),
+])
+def test_two_pass_plan_weighs_its_own_costs(rows, dims, nq, k, path):
+    assert path_of(7, rows, dims, nq, k) == path
+
+
 @pytest.mark.gpu
 def test_batches_outside_a_cached_plan_are_answered():
     rng = np.random.default_rng(0)
