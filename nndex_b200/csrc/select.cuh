@@ -7,6 +7,8 @@
 // exactly k of them, and the result set equals the canonical top-k (similarity desc, index asc).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace nndex {
@@ -227,9 +229,11 @@ NNDEX_DEVICE_INLINE void block_bitonic_sort_desc(uint64_t* a, uint32_t n) {
 //
 // Each thread keeps the largest of the keys it reads (dealt round-robin); the k-th largest score of these
 // maxima, found bit by bit with a block-wide count, is a cut that at least k keys reach and hardly more
-// do, so one more read lists about k keys, and their ranks among themselves place them. Scores tied with
-// the cut by the thousand take the row's part of the key into it. Exact whatever the keys: only a list that
-// does not hold every key that reaches the cut even so sends the block to `overflow`.
+// do, so one more read lists about k keys, and their ranks among themselves place them. Where more keys reach
+// the cut than the list holds, either scores tie with it by the thousand, and the row's part of the key is taken
+// into the cut, or lists filled only at their start had fallen to hardly more than k threads, and the keys are
+// dealt again, each round turned by 37 threads. Exact whatever the keys: only keys that do not fit even so send
+// the block to `overflow`.
 template <int NT>
 struct MergeScratch {
     static constexpr uint32_t kList = 1024;
@@ -243,54 +247,69 @@ struct MergeScratch {
 template <int NT, class Get, class Put, class Overflow>
 NNDEX_DEVICE_INLINE uint32_t block_merge_best(Get&& get, uint32_t n, uint32_t k, MergeScratch<NT>& s, Put&& put,
                                               Overflow&& overflow) {
+    static_assert((NT & (NT - 1)) == 0, "rounds are turned within a power of two");
     constexpr int U = 8;  // loads in flight; the keys stay in registers where one round reads them all
     const uint32_t tid = threadIdx.x;
-    uint64_t best = 0, x[U];
-    for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? get(i0 + u * NT + tid) : 0ull;
-#pragma unroll
-        for (int u = 0; u < U; ++u) best = x[u] > best ? x[u] : best;
-    }
-    if (tid == 0) s.count = 0;
-    const uint32_t top = static_cast<uint32_t>(best >> 32);  // the score, in order
-    uint32_t score = 0;
-#pragma unroll 1
-    for (int bit = 31; bit >= 0; --bit) {
-        const uint32_t t = score | (1u << bit);
-        if (static_cast<uint32_t>(__syncthreads_count(top >= t)) >= k) score = t;
-    }
-    uint64_t cut = score ? static_cast<uint64_t>(score) << 32 : 1ull;  // fewer keys than that: all of them
-    auto list = [&]() {
+    // lists the keys that reach the cut; their number
+    auto attempt = [&](auto turn) {
+        uint64_t best = 0, x[U];
+        auto load = [&](uint32_t i0, int u) {
+            const uint32_t base = i0 + u * NT;
+            const uint32_t i = base + (decltype(turn)::value ? (tid + decltype(turn)::value * (base / NT)) & (NT - 1) : tid);
+            return i < n ? get(i) : 0ull;
+        };
         for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
-            if (n > U * NT) {
 #pragma unroll
-                for (int u = 0; u < U; ++u) x[u] = i0 + u * NT + tid < n ? get(i0 + u * NT + tid) : 0ull;
-            }
+            for (int u = 0; u < U; ++u) x[u] = load(i0, u);
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool take = x[u] >= cut;
-                const uint32_t at = warp_append(&s.count, take);
-                if (take && at < MergeScratch<NT>::kList) s.list[at] = x[u];
-            }
+            for (int u = 0; u < U; ++u) best = x[u] > best ? x[u] : best;
         }
-        __syncthreads();
-        return s.count;
-    };
-    uint32_t c = list();
-    if (c > MergeScratch<NT>::kList && score) {
-        // more keys tie with the cut's score than the list holds: the rest of the key decides, like the score
-        const uint32_t low = static_cast<uint32_t>(best);
-        uint32_t rest = 0;
+        if (tid == 0) s.count = 0;
+        const uint32_t top = static_cast<uint32_t>(best >> 32);  // the score, in order
+        uint32_t score = 0;
 #pragma unroll 1
         for (int bit = 31; bit >= 0; --bit) {
-            const uint32_t t = rest | (1u << bit);
-            if (static_cast<uint32_t>(__syncthreads_count(top > score || (top == score && low >= t))) >= k) rest = t;
+            const uint32_t t = score | (1u << bit);
+            if (static_cast<uint32_t>(__syncthreads_count(top >= t)) >= k) score = t;
         }
-        cut |= rest;
-        if (tid == 0) s.count = 0;
-        __syncthreads();
-        c = list();
+        uint64_t cut = score ? static_cast<uint64_t>(score) << 32 : 1ull;  // fewer keys than that: all of them
+        auto list = [&]() {
+            for (uint32_t i0 = 0; i0 < n; i0 += U * NT) {
+                if (n > U * NT) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) x[u] = load(i0, u);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const bool take = x[u] >= cut;
+                    const uint32_t at = warp_append(&s.count, take);
+                    if (take && at < MergeScratch<NT>::kList) s.list[at] = x[u];
+                }
+            }
+            __syncthreads();
+            return s.count;
+        };
+        uint32_t c = list();
+        if (c > MergeScratch<NT>::kList && __syncthreads_count(score && top == score) >= 8) {
+            // (with the score of many threads' best) thousands of keys tie: the rest of the key decides, like the score
+            const uint32_t low = static_cast<uint32_t>(best);
+            uint32_t rest = 0;
+#pragma unroll 1
+            for (int bit = 31; bit >= 0; --bit) {
+                const uint32_t t = rest | (1u << bit);
+                if (static_cast<uint32_t>(__syncthreads_count(top > score || (top == score && low >= t))) >= k) rest = t;
+            }
+            cut |= rest;
+            if (tid == 0) s.count = 0;
+            __syncthreads();
+            c = list();
+        }
+        return c;
+    };
+    uint32_t c = attempt(std::integral_constant<uint32_t, 0>{});
+    if (c > MergeScratch<NT>::kList) {
+        __syncthreads();  // before the count starts anew
+        c = attempt(std::integral_constant<uint32_t, 37>{});
     }
     if (c > MergeScratch<NT>::kList) {
         __syncthreads();
