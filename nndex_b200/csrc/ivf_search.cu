@@ -140,7 +140,9 @@ NNDEX_DEVICE_INLINE uint64_t warp_radix_kth(const float* scores, uint32_t n, uin
 // memory, as doubles, and a centroid row, n values (a multiple of 8), by 8 consecutive lanes (j of 8, all
 // of the warp calling); every lane returns it. The lanes add in another order: both sums are within
 // n·2⁻⁵³·Σ|xy| ≤ err / 2 of the exact value, so where every value within err rounds to one f32, that is the
-// reference's. Where it does not (about once in 10⁷) they add in index order.
+// reference's. Where it does not (about once in 10⁷) they add in index order, unless every product is zero (a
+// zero centroid, or one without a dimension in common with the query), which any order adds up to zero: a
+// query that had 1,000 empty lists of 1,500 in question took 228 us in index order.
 NNDEX_DEVICE_INLINE float dot_f64_row8(const double* q_s, const float* __restrict__ row, uint32_t n, double err,
                                        uint32_t j, bool live) {
     double s = 0.0;
@@ -157,9 +159,21 @@ NNDEX_DEVICE_INLINE float dot_f64_row8(const double* q_s, const float* __restric
     s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
     s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
     s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
-    if (live && __double2float_rn(s - err) != __double2float_rn(s + err)) {
-        s = 0.0;
-        for (uint32_t d = 0; d < n; ++d) s = fma(q_s[d], static_cast<double>(row[d]), s);
+    const bool doubt = live && __double2float_rn(s - err) != __double2float_rn(s + err);
+    if (__any_sync(0xFFFFFFFFu, doubt)) {
+        bool product = false;
+        if (doubt)
+            for (uint32_t d = 4 * j; d < n; d += 32) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(row + d));
+                product |= (v.x != 0.0f && q_s[d] != 0.0) || (v.y != 0.0f && q_s[d + 1] != 0.0) ||
+                           (v.z != 0.0f && q_s[d + 2] != 0.0) || (v.w != 0.0f && q_s[d + 3] != 0.0);
+            }
+        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, product);
+        if (doubt) {
+            s = 0.0;
+            if (lanes >> (threadIdx.x & 24u) & 0xFFu)
+                for (uint32_t d = 0; d < n; ++d) s = fma(q_s[d], static_cast<double>(row[d]), s);
+        }
     }
     return __double2float_rn(s);
 }
@@ -268,9 +282,9 @@ __global__ void __launch_bounds__(256)
 //    selection took 94 + 25; one query against 512 of 128: 4.5 + 8.2, before 15 + 7.4. (Exact scores
 //    as one thread's chain of FP64 adds per list: pick 54 and 10 us.) Where more lists lie between the bounds
 //    than shared memory holds (equal centroids, from rows of few distinct values), their exact scores go
-//    back to memory and a radix selection takes the best: 8,192 lists of 3 distinct centroids, 1 query
-//    150 us, 1,024 queries 1.02 ms; ranks among all lists, quadratic, took 8.4 and 36 ms, the FP64 scores
-//    of every pair 0.22 and 0.78.
+//    back to memory and a second merge takes the best: 8,192 lists of 3 distinct centroids, 1 query 140 us,
+//    1,024 queries 0.96 ms; ranks among all lists, quadratic, took 8.4 and 36 ms, the FP64 scores of every
+//    pair 0.22 and 0.78.
 constexpr uint32_t kProbePick = 512;
 constexpr uint32_t kProbeBand = 256;  // lists between the certain ones scored from shared memory
 
@@ -390,15 +404,20 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 8 : 1)
             }
         }
         __syncthreads();
-        // their best r: the keys (score, list) are distinct, so exactly r reach the r-th
+        // their best r
         auto get = [&](uint32_t i) { return sq[i] == -FLT_MAX ? 0ull : make_key(sq[i], i); };
-        const uint64_t kth = block_radix_kth_of(get, nlist, r, sel);
-        for (uint32_t i0 = 0; i0 < nlist; i0 += NT) {
-            const uint32_t i = i0 + tid;
-            const bool take = i < nlist && get(i) >= kth;
-            const uint32_t a = warp_append(&n_in, take);
-            if (take && a < kProbePick) picked[a] = i;
-        }
+        block_merge_best<NT>(
+            get, nlist, r, s, [&](uint32_t j, uint64_t key) { picked[nin + j] = key_row(key); },
+            [&]() {  // the keys (score, list) are distinct, so exactly r reach the r-th
+                const uint64_t kth = block_radix_kth_of(get, nlist, r, sel);
+                for (uint32_t i0 = 0; i0 < nlist; i0 += NT) {
+                    const uint32_t i = i0 + tid;
+                    const bool take = i < nlist && get(i) >= kth;
+                    const uint32_t a = warp_append(&n_in, take);
+                    if (take && a < kProbePick) picked[a] = i;
+                }
+                return r;
+            });
     }
     __syncthreads();
     const uint32_t n = np < nlist ? np : nlist;
