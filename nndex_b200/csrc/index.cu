@@ -1039,19 +1039,32 @@ int CudaIndex::finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_si
     stats.pass2_rows += h_fbn_rows();
     if (failed_n == 0) return NNDEX_OK;
     std::vector<uint32_t> failed;
-    if (tc_retry_rest) {
+    if (tc_retry_rest && failed_n <= tc_retry_rest_m) {
         --tc_retry_rest;
         if ((st = overflowed_queries(m, failed_n, s, &failed))) return st;
     } else {
         if ((st = retry_tc_pass2(stats.path == 3, failed_n, kcap, o_idx, o_sim, o_cnt, s, &failed))) return st;
-        // in vain for most: more rows tie with the k-th score than a collection holds, as they will next time
-        if (2 * failed.size() > failed_n) tc_retry_rest = kTcRetryRest;
+        if (!retry_paid(failed_n, static_cast<uint32_t>(failed.size()))) {
+            tc_retry_rest = kTcRetryRest;
+            tc_retry_rest_m = failed_n;
+        }
     }
     tc_patched = true;
     stats.fp32_fallback_queries += static_cast<uint32_t>(failed.size());
     if (failed.empty()) return NNDEX_OK;
     // ---- the FP32 scan for queries whose collected set overflowed again ----
     return rerun_exact_fp32(failed, kcap, o_idx, o_sim, o_cnt, s);
+}
+
+// Whether the second pass 2 of m queries, which left `failed` of them overflowed, cost less than the FP32 scan of
+// the others (us): a re-run query takes about 16 of copies, its share of a scan per 16 queries that the scan
+// no longer runs for; the pass about 20, then the exact scores of 8,192 rows a query. 64k × 1,024 in FP8,
+// k = 100, with / without: 16 queries, 9 left, 853 / 704; 128, 82 left, 2,517 / 2,664; 512, 295 left, 7,324 /
+// 9,221; 32k × 1,024, 2, none left, 584 / 441; 256k × 1,024 2, none left, 441 / 489; 128k × 256 16, 5 of them
+// overflowed, none left, 312 / 354.
+bool CudaIndex::retry_paid(uint32_t m, uint32_t failed) const {
+    const double d = static_cast<double>(ds), scans = (m + 15) / 16 - (failed + 15) / 16;
+    return 16.0 * (m - failed) + scans * static_cast<double>(rows) * d * 5.3e-7 > 20.0 + 0.1 * d + m * d * 3.3e-3;
 }
 
 // The queries whose collection overflowed, without another pass.

@@ -40,9 +40,9 @@ inline uint64_t tf32_batch_costs(uint64_t rows, uint64_t ds, uint64_t nq, uint64
 // again: a batch that tries in vain costs at most about twice the FP32 scan, so 3 % over 32.
 constexpr uint32_t kTf32Rest = 31;
 
-// Likewise the second pass 2 of overflowed collections (paths 2 and 3), where it left most of them overflowed: it
-// costs 50 to 350 us of a batch then (458k × 11 in BF16, 32 tight clusters, 123 queries: 2,023 us without it,
-// 2,353 with it; 9 queries over 316k × 175 in FP8 457 and 516).
+// Likewise the second pass 2 of overflowed collections (paths 2 and 3), where it cost more than the FP32 scan of
+// what it served (CudaIndex::retry_paid). In vain for all of them: 458k × 11 in BF16, 32 tight clusters, 123 queries 2,023
+// us without it, 2,353 with it; 9 queries over 316k × 175 in FP8 457 and 516.
 constexpr uint32_t kTcRetryRest = 31;
 
 // Incremented whenever a scratch or staging buffer of any index is (re)allocated: a captured
@@ -427,7 +427,10 @@ struct CudaIndex {
     int finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt, cudaStream_t s);
     // Pass 2 once more for the m queries whose collection overflowed (positions in d_ids: d_tcfail),
     // against the T of the rows they did collect; the ones that overflow again are left in *failed.
-    uint32_t tc_retry_rest = 0;  // batches whose overflowed queries still go to the FP32 scan without it
+    // batches whose overflowed queries still go to the FP32 scan without it, where they are at most so many (more
+    // of them share the pass, and may be worth it)
+    uint32_t tc_retry_rest = 0, tc_retry_rest_m = 0;
+    bool retry_paid(uint32_t m, uint32_t failed) const;
     int overflowed_queries(uint32_t m, uint32_t failed_n, cudaStream_t s, std::vector<uint32_t>* failed);
     int retry_tc_pass2(bool fp8, uint32_t m, uint32_t kcap, uint64_t* o_idx, float* o_sim, uint32_t* o_cnt,
                        cudaStream_t s, std::vector<uint32_t>* failed);
