@@ -1052,6 +1052,15 @@ bool pairs_even(const CudaIndex& ix, uint64_t nq, uint64_t np) {
            (longest <= pair_share(ix, nq * np) || longest * row <= kPairChunkBytes);
 }
 
+// The pairs leave a query's merge, one block, a slot of k keys for each chunk of the longest list, whatever the
+// list: many probes, a large k and one long list make it hundreds of thousands of keys, most of them empty, at
+// about 0.8 ns each, where a plan has slots for the chunks that there are. Pairs against plan, 879 batches of 1 to
+// 32 queries, k of 10 to 256, by keys a query: 40,000 to 80,000 0.9 of the time (median), 80,000 to 100,000 0.99,
+// up to 130,000 1.03, up to 400,000 1.15, beyond 2.5. 569k × 150, 128 of 144 lists, k = 256, one query (688,128
+// keys) 361 / 198 us; 1.27M × 50, 64 of 152, k = 100 (204,800) 285 / 166; 326k × 95, 4 queries, 128 of 2,366
+// lists, k = 100 (217,600) 435 / 192.
+constexpr uint64_t kPairMergeKeys = 100000;
+
 size_t ivf_pair_smem(uint32_t dq, uint32_t cap) {
     return 1024 + static_cast<size_t>(kStages) * kPairW * 16 * 128 + static_cast<size_t>(dq) * 4 +
            static_cast<size_t>(cap) * 8 + kPairW * 256 * 4 + 8 + 8 + kStages * 16 + 16;
@@ -1270,10 +1279,11 @@ int ivf_search(CudaIndex& ix, const float* queries, uint32_t nq, uint32_t k, uin
     // Small batches whose lists serve at most one query on average: (query, list, chunk) CTAs, no plan.
     // Chunks of as many 256 rows as give every SM about two (of the longest list at most 32).
     const uint64_t pairs = static_cast<uint64_t>(nq) * np;
-    if (pairs <= nlist && pairs <= kPairLimit && k <= kMergeBestK && pairs_even(ix, nq, np)) {
-        uint64_t chunk = std::max<uint64_t>(pair_share(ix, pairs), (v.max_list + 31) / 32);
-        chunk = std::max<uint64_t>(256, (chunk + 255) / 256 * 256);
-        const uint32_t chunks = static_cast<uint32_t>(std::max<uint64_t>(1, (v.max_list + chunk - 1) / chunk));
+    uint64_t chunk = std::max<uint64_t>(pair_share(ix, pairs), (v.max_list + 31) / 32);
+    chunk = std::max<uint64_t>(256, (chunk + 255) / 256 * 256);
+    const uint32_t chunks = static_cast<uint32_t>(std::max<uint64_t>(1, (v.max_list + chunk - 1) / chunk));
+    if (pairs <= nlist && pairs <= kPairLimit && k <= kMergeBestK && pairs_even(ix, nq, np) &&
+        static_cast<uint64_t>(np) * chunks * k <= kPairMergeKeys) {
         const uint32_t pcap = ((k + 2 * kPairW * 16) + 31) / 32 * 32;
         const size_t psmem = ivf_pair_smem(dq, pcap);
         uint32_t stages = 0;
