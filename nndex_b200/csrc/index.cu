@@ -1061,10 +1061,12 @@ int CudaIndex::finish_tc(uint32_t n, uint32_t kcap, uint64_t* o_idx, float* o_si
 // no longer runs for; the pass about 20, then the exact scores of 8,192 rows a query. 64k × 1,024 in FP8,
 // k = 100, with / without: 16 queries, 9 left, 853 / 704; 128, 82 left, 2,517 / 2,664; 512, 295 left, 7,324 /
 // 9,221; 32k × 1,024, 2, none left, 584 / 441; 256k × 1,024 2, none left, 441 / 489; 128k × 256 16, 5 of them
-// overflowed, none left, 312 / 354.
+// overflowed, none left, 312 / 354. And it reads the copy: 1.3M × 8 in FP8, 8 queries, one of them overflowed, none
+// left, 458 / 351; 3.5M × 34, 141, 135 left, 7,343 / 6,603; 2M × 8, 26, 24 left, 1,555 / 1,258.
 bool CudaIndex::retry_paid(uint32_t m, uint32_t failed) const {
-    const double d = static_cast<double>(ds), scans = (m + 15) / 16 - (failed + 15) / 16;
-    return 16.0 * (m - failed) + scans * static_cast<double>(rows) * d * 5.3e-7 > 20.0 + 0.1 * d + m * d * 3.3e-3;
+    const double d = static_cast<double>(ds), scans = (m + 15) / 16 - (failed + 15) / 16, n = static_cast<double>(rows);
+    const double copy = n * static_cast<double>(stats.path == 3 ? kf8 : 2 * kb16) * ((m + 127) / 128);
+    return 16.0 * (m - failed) + scans * n * d * 5.3e-7 > 20.0 + 0.1 * d + m * d * 3.3e-3 + copy * 1.5e-7;
 }
 
 // The queries whose collection overflowed, without another pass.
